@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "../../include/clv.h"
+#include "normal64.cuh"
 
 namespace clv {
 
@@ -160,13 +161,9 @@ __device__ __forceinline__ uint2 noise_words(uint64_t seed, uint32_t chain, uint
 }
 
 __device__ __forceinline__ double2 box_muller64(uint32_t x, uint32_t y) {
-    const double two_m32 = 2.3283064365386963e-10;
-    const double u1 = ((double)x + 0.5) * two_m32;
-    const double u2 = (double)y * two_m32;
-    const double r = sqrt(-2.0 * log(u1));
-    double s, c;
-    sincospi(2.0 * u2, &s, &c);
-    return make_double2(r * c, r * s);
+    double2 z;
+    normal64(x, y, z.x, z.y);
+    return z;
 }
 
 // FP32 arithmetic on the same words as box_muller64 with the hardware logarithm,

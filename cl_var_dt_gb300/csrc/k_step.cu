@@ -173,16 +173,11 @@ update_kernel(const ChainDev *__restrict__ chains, const ChainState *__restrict_
         const uint32_t lin = (uint32_t)((long long)tau * ch.V + s);
         const bool lone = lone_component(a0, ch.ncomp);
         const uint4 o = philox_block(ch.seed, (uint32_t)task.chain, nstep, (int)blockIdx.y, lone ? lin >> 1 : lin);
-        for (int a = a0; a < a1; ++a) {
-            const bool hi = lone ? (lin & 1) != 0 : (a & 1) != 0;
-            const uint32_t wx = hi ? o.z : o.x, wy = hi ? o.w : o.y;
-            if (sizeof(R) == 8) {
-                const double2 g = box_muller64(wx, wy);
-                zu[a - a0].x = (R)g.x; zu[a - a0].y = (R)g.y;
-            } else {
-                const float2 g = box_muller32(wx, wy);
-                zu[a - a0].x = (R)g.x; zu[a - a0].y = (R)g.y;
-            }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (a0 + u >= a1) break;
+            const bool hi = lone ? (lin & 1) != 0 : u != 0;
+            zu[u] = unit_normal<R, C2>(hi ? o.z : o.x, hi ? o.w : o.y);
         }
     };
     if (early) draw(pre);
@@ -192,14 +187,17 @@ update_kernel(const ChainDev *__restrict__ chains, const ChainState *__restrict_
     if (nstep != pre) draw(nstep);
     const double dtd = __ldcg(&stc->dt);
     const R dt = (R)dtd, sd = (R)sqrt(dtd);
-    for (int a = a0; a < a1; ++a) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int a = a0 + u;
+        if (a >= a1) break;
         C2 z;
         if (NOISE == CLV_NOISE_EXTERNAL) {
             const long long r = ch.noise_off + (((long long)a * ch.V + s) * ch.nt + tau) * 2;
             z.x = (R)noise[r];
             z.y = (R)noise[r + 1];
         } else {
-            z = zu[a - a0];
+            z = zu[u];
         }
         z.x = mul_rn<R>(sd, z.x);
         z.y = mul_rn<R>(sd, z.y);
