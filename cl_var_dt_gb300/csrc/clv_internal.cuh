@@ -30,6 +30,18 @@ template <class C2> __device__ __forceinline__ C2 cmul(C2 a, C2 b) {
 template <class C2, class R> __device__ __forceinline__ C2 cscale(R s, C2 a) { C2 r; r.x = s * a.x; r.y = s * a.y; return r; }
 template <class C2> __device__ __forceinline__ C2 cconj(C2 a) { C2 r; r.x = a.x; r.y = -a.y; return r; }
 
+// Arithmetic with the rounding written out (the compiler contracts nothing across these).
+template <class R> __device__ __forceinline__ R mul_rn(R a, R b);
+template <> __device__ __forceinline__ double mul_rn<double>(double a, double b) { return __dmul_rn(a, b); }
+template <> __device__ __forceinline__ float mul_rn<float>(float a, float b) { return __fmul_rn(a, b); }
+template <class R> __device__ __forceinline__ R add_rn(R a, R b);
+template <> __device__ __forceinline__ double add_rn<double>(double a, double b) { return __dadd_rn(a, b); }
+template <> __device__ __forceinline__ float add_rn<float>(float a, float b) { return __fadd_rn(a, b); }
+
+template <class R> __device__ __forceinline__ R fma_rn(R a, R b, R c);
+template <> __device__ __forceinline__ double fma_rn<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
+template <> __device__ __forceinline__ float fma_rn<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
 // One axis of one chain, as seen by the kinetic line filter.
 struct AxisDev {
     int n;                 // line length (lattice extent along the axis)

@@ -20,7 +20,9 @@ __device__ __forceinline__ C2 times_si(C2 z) {
     return r;
 }
 
-// Complex add/sub of the butterflies.  FP32 uses the packed two-lane FP32
+// Arithmetic of the butterflies.  FP64 writes every rounding out, so that all plans that
+// run the same butterflies give the same bits wherever they are inlined, with the fused
+// multiply-adds placed by hand (FP64 operations are the bound).  FP32 uses the packed two-lane FP32
 // instructions of sm_100+ (add/sub .rn.f32x2: two IEEE single additions, the
 // same results as the scalar pair), so one instruction moves a complex sum.
 template <class C2> __device__ __forceinline__ C2 vadd(C2 a, C2 b) { return cadd(a, b); }
@@ -46,6 +48,43 @@ template <> __device__ __forceinline__ float2 vsub<float2>(float2 a, float2 b) {
     return f2_unpack(r);
 }
 
+template <> __device__ __forceinline__ double2 vadd<double2>(double2 a, double2 b) {
+    return make_double2(__dadd_rn(a.x, b.x), __dadd_rn(a.y, b.y));
+}
+template <> __device__ __forceinline__ double2 vsub<double2>(double2 a, double2 b) {
+    return make_double2(__dadd_rn(a.x, -b.x), __dadd_rn(a.y, -b.y));
+}
+// s z for a real s; z w (twiddle)
+__device__ __forceinline__ float2 vscale(float s, float2 z) { return make_float2(s * z.x, s * z.y); }
+__device__ __forceinline__ double2 vscale(double s, double2 z) { return make_double2(__dmul_rn(s, z.x), __dmul_rn(s, z.y)); }
+__device__ __forceinline__ float2 vmul(float2 z, float2 w) { return cmul(z, w); }
+__device__ __forceinline__ double2 vmul(double2 z, double2 w) {
+    return make_double2(__fma_rn(z.x, w.x, -__dmul_rn(z.y, w.y)), __fma_rn(z.x, w.y, __dmul_rn(z.y, w.x)));
+}
+// p = e + s z and m = e - s z for a real constant s
+__device__ __forceinline__ void vaxpy2(float2 e, float s, float2 z, float2 &p, float2 &m) {
+    const float2 w = vscale(s, z);
+    p = vadd(e, w);
+    m = vsub(e, w);
+}
+__device__ __forceinline__ void vaxpy2(double2 e, double s, double2 z, double2 &p, double2 &m) {
+    p = make_double2(__fma_rn(s, z.x, e.x), __fma_rn(s, z.y, e.y));
+    m = make_double2(__fma_rn(-s, z.x, e.x), __fma_rn(-s, z.y, e.y));
+}
+
+// p = f a + g b and m = f a - g b for real f, g: at FP64 two products and four fused
+// multiply-adds instead of four products and four sums
+__device__ __forceinline__ void vpair(float f, float2 a, float g, float2 b, float2 &p, float2 &m) {
+    const float2 x = vscale(f, a), y = vscale(g, b);
+    p = vadd(x, y);
+    m = vsub(x, y);
+}
+__device__ __forceinline__ void vpair(double f, double2 a, double g, double2 b, double2 &p, double2 &m) {
+    vaxpy2(vscale(f, a), g, b, p, m);
+}
+
+// Radix<C2, R>::run<S> is the butterfly, run_scaled<S>(a, f) the butterfly of f[r] a[r]
+// (the first inverse pass after the filter).
 template <class C2, int R>
 struct Radix;
 
@@ -64,12 +103,22 @@ template <class C2>
 struct Radix<C2, 4> {
     template <int S>
     static __device__ __forceinline__ void run(C2 *a) {
-        const C2 s02 = vadd(a[0], a[2]), d02 = vsub(a[0], a[2]);
-        const C2 s13 = vadd(a[1], a[3]), d13 = times_si<S>(vsub(a[1], a[3]));
+        finish<S>(a, vadd(a[0], a[2]), vsub(a[0], a[2]), vadd(a[1], a[3]), vsub(a[1], a[3]));
+    }
+    template <int S>
+    static __device__ __forceinline__ void finish(C2 *a, C2 s02, C2 d02, C2 s13, C2 d13) {
+        d13 = times_si<S>(d13);
         a[0] = vadd(s02, s13);
         a[2] = vsub(s02, s13);
         a[1] = vadd(d02, d13);
         a[3] = vsub(d02, d13);
+    }
+    template <int S, class RR>
+    static __device__ __forceinline__ void run_scaled(C2 *a, RR f0, RR f1, RR f2, RR f3) {
+        C2 s02, d02, s13, d13;
+        vpair(f0, a[0], f2, a[2], s02, d02);
+        vpair(f1, a[1], f3, a[3], s13, d13);
+        finish<S>(a, s02, d02, s13, d13);
     }
     static __device__ __forceinline__ void run(C2 *a, int S) {
         if (S < 0) run<-1>(a); else run<1>(a);
@@ -80,26 +129,38 @@ template <class C2>
 struct Radix<C2, 8> {
     template <int S>
     static __device__ __forceinline__ void run(C2 *a) {
-        using R = decltype(a[0].x);
-        const R h = (R)0.70710678118654752440;
         C2 e[4] = {a[0], a[2], a[4], a[6]};
         C2 o[4] = {a[1], a[3], a[5], a[7]};
         Radix<C2, 4>::template run<S>(e);
         Radix<C2, 4>::template run<S>(o);
-        // twiddles exp(S 2 pi i q/8), q = 1, 2, 3
-        C2 w1, w3;
+        finish<S>(a, e, o);
+    }
+    template <int S, class RR>
+    static __device__ __forceinline__ void run_scaled(C2 *a, const RR *f) {
+        C2 e[4] = {a[0], a[2], a[4], a[6]};
+        C2 o[4] = {a[1], a[3], a[5], a[7]};
+        Radix<C2, 4>::template run_scaled<S>(e, f[0], f[2], f[4], f[6]);
+        Radix<C2, 4>::template run_scaled<S>(o, f[1], f[3], f[5], f[7]);
+        finish<S>(a, e, o);
+    }
+    template <int S>
+    static __device__ __forceinline__ void finish(C2 *a, const C2 *e, const C2 *o) {
+        using R = decltype(a[0].x);
+        const R h = (R)0.70710678118654752440;
+        // twiddles exp(S 2 pi i q/8), q = 1, 2, 3: h t1, S i, h t3
+        C2 t1, t3;
         if (S < 0) {
-            w1.x = h * (o[1].x + o[1].y); w1.y = h * (o[1].y - o[1].x);
-            w3.x = h * (o[3].y - o[3].x); w3.y = -h * (o[3].x + o[3].y);
+            t1.x = add_rn<R>(o[1].x, o[1].y); t1.y = add_rn<R>(o[1].y, -o[1].x);
+            t3.x = add_rn<R>(o[3].y, -o[3].x); t3.y = -add_rn<R>(o[3].x, o[3].y);
         } else {
-            w1.x = h * (o[1].x - o[1].y); w1.y = h * (o[1].y + o[1].x);
-            w3.x = -h * (o[3].x + o[3].y); w3.y = h * (o[3].x - o[3].y);
+            t1.x = add_rn<R>(o[1].x, -o[1].y); t1.y = add_rn<R>(o[1].y, o[1].x);
+            t3.x = -add_rn<R>(o[3].x, o[3].y); t3.y = add_rn<R>(o[3].x, -o[3].y);
         }
         const C2 w2 = times_si<S>(o[2]);
         a[0] = vadd(e[0], o[0]); a[4] = vsub(e[0], o[0]);
-        a[1] = vadd(e[1], w1);   a[5] = vsub(e[1], w1);
+        vaxpy2(e[1], h, t1, a[1], a[5]);
         a[2] = vadd(e[2], w2);   a[6] = vsub(e[2], w2);
-        a[3] = vadd(e[3], w3);   a[7] = vsub(e[3], w3);
+        vaxpy2(e[3], h, t3, a[3], a[7]);
     }
     static __device__ __forceinline__ void run(C2 *a, int S) {
         if (S < 0) run<-1>(a); else run<1>(a);
@@ -109,10 +170,10 @@ struct Radix<C2, 8> {
 // z * w for a constant w = (wr, wi)
 template <class C2, class R>
 __device__ __forceinline__ C2 cmulc(C2 z, R wr, R wi) {
-    C2 r;
-    r.x = z.x * wr - z.y * wi;
-    r.y = z.x * wi + z.y * wr;
-    return r;
+    C2 w;
+    w.x = wr;
+    w.y = wi;
+    return vmul(z, w);
 }
 
 // 16 = 4 x 4: x[4 n1 + n2] -> radix 4 over n1 (index k1), twiddle W16^(n2 k1),
@@ -163,11 +224,15 @@ struct Radix<C2, 3> {
         using R = decltype(a[0].x);
         const R half = (R)0.5, s3 = (R)0.86602540378443864676;
         const C2 t1 = vadd(a[1], a[2]), t2 = vsub(a[1], a[2]);
-        C2 m; m.x = a[0].x - half * t1.x; m.y = a[0].y - half * t1.y;
-        const C2 r = times_si<S>(cscale(s3, t2));
+        C2 m; m.x = fma_rn<R>(-half, t1.x, a[0].x); m.y = fma_rn<R>(-half, t1.y, a[0].y);
         a[0] = vadd(a[0], t1);
-        a[1] = vadd(m, r);
-        a[2] = vsub(m, r);
+        if constexpr (sizeof(R) == 8) {
+            vaxpy2(m, s3, times_si<S>(t2), a[1], a[2]);
+        } else {
+            const C2 r = times_si<S>(vscale(s3, t2));
+            a[1] = vadd(m, r);
+            a[2] = vsub(m, r);
+        }
     }
     static __device__ __forceinline__ void run(C2 *a, int S) {
         if (S < 0) run<-1>(a); else run<1>(a);
@@ -211,10 +276,11 @@ struct Radix<C2, 5> {
         const R s1 = (R)0.95105651629515357212, s2 = (R)0.58778525229247312917;
         const C2 t1 = vadd(a[1], a[4]), t2 = vadd(a[2], a[3]);
         const C2 t3 = vsub(a[1], a[4]), t4 = vsub(a[2], a[3]);
-        C2 b1; b1.x = a[0].x + c1 * t1.x + c2 * t2.x; b1.y = a[0].y + c1 * t1.y + c2 * t2.y;
-        C2 b2; b2.x = a[0].x + c2 * t1.x + c1 * t2.x; b2.y = a[0].y + c2 * t1.y + c1 * t2.y;
-        C2 q1; q1.x = s1 * t3.x + s2 * t4.x; q1.y = s1 * t3.y + s2 * t4.y;
-        C2 q2; q2.x = s2 * t3.x - s1 * t4.x; q2.y = s2 * t3.y - s1 * t4.y;
+        C2 b1, b2, q1, q2;
+        b1.x = fma_rn<R>(c2, t2.x, fma_rn<R>(c1, t1.x, a[0].x)); b1.y = fma_rn<R>(c2, t2.y, fma_rn<R>(c1, t1.y, a[0].y));
+        b2.x = fma_rn<R>(c1, t2.x, fma_rn<R>(c2, t1.x, a[0].x)); b2.y = fma_rn<R>(c1, t2.y, fma_rn<R>(c2, t1.y, a[0].y));
+        q1.x = fma_rn<R>(s1, t3.x, mul_rn<R>(s2, t4.x)); q1.y = fma_rn<R>(s1, t3.y, mul_rn<R>(s2, t4.y));
+        q2.x = fma_rn<R>(s2, t3.x, -mul_rn<R>(s1, t4.x)); q2.y = fma_rn<R>(s2, t3.y, -mul_rn<R>(s1, t4.y));
         q1 = times_si<S>(q1);
         q2 = times_si<S>(q2);
         a[0] = vadd(a[0], vadd(t1, t2));
@@ -290,5 +356,18 @@ struct Radix<C2, 64> {
         }
     }
 };
+
+template <class C2, int R, int S, class RR>
+__device__ __forceinline__ void radix_scaled(C2 *a, const RR *f) {
+    if constexpr (R == 4) {
+        Radix<C2, 4>::template run_scaled<S>(a, f[0], f[1], f[2], f[3]);
+    } else if constexpr (R == 8) {
+        Radix<C2, 8>::template run_scaled<S>(a, f);
+    } else {
+#pragma unroll
+        for (int q = 0; q < R; ++q) a[q] = vscale(f[q], a[q]);
+        Radix<C2, R>::template run<S>(a);
+    }
+}
 
 }  // namespace clv

@@ -92,7 +92,7 @@ __device__ __forceinline__ void warp_pass(const C2 *s, C2 *d, int inner, int n, 
             if (r > 0 && k > 0) {
                 C2 t = tw[k * r * tstep];
                 if (S > 0) t.y = -t.y;  // table holds exp(-2 pi i k/n)
-                x = cmul(x, t);
+                x = vmul(x, t);
             }
             v[r] = x;
         }
@@ -102,7 +102,7 @@ __device__ __forceinline__ void warp_pass(const C2 *s, C2 *d, int inner, int n, 
         for (int q = 0; q < R; ++q) {
             const int idx = o + q * Ns;
             C2 val = v[q];
-            if (f) val = cscale(f[idx] * cst, val);
+            if (f) val = vscale(f[idx] * cst, val);
             d[idx * inner] = val;
         }
     }
@@ -155,7 +155,7 @@ __device__ __forceinline__ void warp_pass_1d(const C2 *s, C2 *d, int n, int Ns, 
             if (r > 0 && k > 0) {
                 C2 t = tw[k * r * tstep];
                 if (S > 0) t.y = -t.y;
-                x = cmul(x, t);
+                x = vmul(x, t);
             }
             v[r] = x;
         }
@@ -182,13 +182,14 @@ __device__ __forceinline__ void warp_mid_1d(const C2 *s, C2 *d, int n, const C2 
         for (int r = 0; r < R; ++r) {
             const int idx = j + r * nR;
             C2 x = s[PS ? padi(idx) : idx];
-            if (r > 0 && j > 0) x = cmul(x, tw[j * r]);
+            if (r > 0 && j > 0) x = vmul(x, tw[j * r]);
             v[r] = x;
         }
         Radix<C2, R>::run(v, -1);
+        RR g[R];
 #pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = cscale(f[j + q * nR] * cst, v[q]);
-        Radix<C2, R>::run(v, +1);
+        for (int q = 0; q < R; ++q) g[q] = f[j + q * nR] * cst;
+        radix_scaled<C2, R, 1>(v, g);
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int idx = j * R + q;
@@ -290,7 +291,7 @@ __device__ __forceinline__ void ct_pass(const C2 *s, C2 *d, const C2 *tw, int la
                     t = tw[k * r * tstep];
                     if (S > 0) t.y = -t.y;
                 }
-                x = cmul(x, t);
+                x = vmul(x, t);
             }
             v[r] = x;
         }
@@ -315,13 +316,14 @@ __device__ __forceinline__ void ct_mid(const C2 *s, C2 *d, const C2 *tw, const R
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             C2 x = sl[PS ? padi(r * nR) : r * nR];
-            if (nR > 1 && r > 0) x = cmul(x, PT ? tw[(r - 1) * nR + j] : tw[j * r]);
+            if (nR > 1 && r > 0) x = vmul(x, PT ? tw[(r - 1) * nR + j] : tw[j * r]);
             v[r] = x;
         }
         Radix<C2, R>::template run<-1>(v);
+        RR g[R];
 #pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = cscale(f[j + q * nR] * cst, v[q]);
-        Radix<C2, R>::template run<1>(v);
+        for (int q = 0; q < R; ++q) g[q] = f[j + q * nR] * cst;
+        radix_scaled<C2, R, 1>(v, g);
         C2 *dl = d + (PD ? padi(j * R) : j * R);
 #pragma unroll
         for (int q = 0; q < R; ++q) dl[q] = v[q];
@@ -428,7 +430,7 @@ __device__ __forceinline__ void g4_pass(const C2 *s, C2 *d, const C2 *tw, int t)
             if (NS > 1 && r > 0) {
                 C2 w = tw[k * r * tstep];
                 if (S > 0) w.y = -w.y;
-                x = cmul(x, w);
+                x = vmul(x, w);
             }
             v[r] = x;
         }
@@ -452,13 +454,14 @@ __device__ __forceinline__ void g4_mid(const C2 *s, C2 *d, const C2 *tw, const R
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             C2 x = sl[PS ? padi(r * nR) : r * nR];
-            if (nR > 1 && r > 0) x = cmul(x, tw[j * r]);
+            if (nR > 1 && r > 0) x = vmul(x, tw[j * r]);
             v[r] = x;
         }
         Radix<C2, 4>::template run<-1>(v);
+        RR g[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = cscale(f[j + q * nR] * cst, v[q]);
-        Radix<C2, 4>::template run<1>(v);
+        for (int q = 0; q < 4; ++q) g[q] = f[j + q * nR] * cst;
+        radix_scaled<C2, 4, 1>(v, g);
         C2 *dl = d + padi(j * 4);
 #pragma unroll
         for (int q = 0; q < 4; ++q) dl[q] = v[q];
@@ -796,6 +799,14 @@ fused_step_kernel(const LaunchFused A) {
     R mxr = 0, smr = 0;
     int bad = 0;
     const DriftConsts<R> dk(ch);
+    // FP64: the pair (psibar(tau), psi(tau-1)) carried from the previous imaginary time (44
+    // of the site's 740 FP64 operations; FP32 recomputes it: the registers cost occupancy)
+    constexpr bool kCarry = FAST && MODEL == CLV_MODEL_SPIN1 && sizeof(R) == 8;
+    Spin1Link<C2> link[kCarry ? SPT : 1];
+    if constexpr (kCarry) {
+#pragma unroll
+        for (int k = 0; k < SPT; ++k) link[k] = spin1_link<R>(dk, Qc[k], Pp[k]);
+    }
     const uint64_t seed = ch.seed;
     const int ref_rule = !FAST && A.dt_rule == CLV_DT_REF_MEANMAX;
     int ia = 0, ic = 0;  // ring positions of psi(tau) and psibar(tau+1)
@@ -917,9 +928,11 @@ fused_step_kernel(const LaunchFused A) {
             if (MODEL == CLV_MODEL_REF4)
                 drift_ref4_vals<R>(dk, Pp[k], vpc[k], vpp[k], Qc[k], vcp[k], Kp[k], kp, K, Kc,
                                    FAST ? 3 : (do_psi ? 1 : 0) | (do_bar ? 2 : 0), cmask);
-            else
-                // (recomputing the bilinears of (psibar(tau), psi(tau-1)) measured faster
-                // here than carrying them: the registers cost occupancy)
+            else if constexpr (kCarry) {
+                spin1_drift_psi<R>(link[k], Pp[k], vpc[k], Kp[k], K);
+                link[k] = spin1_link<R>(dk, vcp[k], vpc[k]);
+                spin1_drift_bar<R>(link[k], vcp[k], Qc[k], kp, Kc);
+            } else
                 drift_spin1_vals<R>(dk, Pp[k], vpc[k], Qc[k], vcp[k], Kp[k], kp, K, Kc,
                                     FAST ? 3 : (do_psi ? 1 : 0) | (do_bar ? 2 : 0));
             if (!FAST && A.mode == FUSED_MAXONLY && A.drift_out) {

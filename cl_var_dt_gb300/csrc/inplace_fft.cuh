@@ -66,7 +66,7 @@ struct InPlace {
             Radix<C2, R>::template run<-1>(v);
             if constexpr (S > 1) {
 #pragma unroll
-                for (int q = 1; q < R; ++q) v[q] = cmul(v[q], tw[q * k * (N / L)]);
+                for (int q = 1; q < R; ++q) v[q] = vmul(v[q], tw[q * k * (N / L)]);
             }
 #pragma unroll
             for (int q = 0; q < R; ++q) t[l * LS + (a0 + q * S) * ES] = v[q];
@@ -94,7 +94,7 @@ struct InPlace {
                 if (S > 1 && q > 0) {
                     C2 w = tw[q * k * (N / L)];
                     w.y = -w.y;
-                    x = cmul(x, w);
+                    x = vmul(x, w);
                 }
                 v[q] = x;
             }
@@ -113,9 +113,9 @@ struct InPlace {
     }
 
     // The last forward pass (span R_last, no twiddles), the filter f at each output's
-    // frequency times cst, and the first inverse pass, in registers.
+    // frequency, and the first inverse pass, in registers.
     template <class C2, class RR>
-    static __device__ __forceinline__ void mid(C2 *t, int LS, int ES, const RR *f, RR cst) {
+    static __device__ __forceinline__ void mid(C2 *t, int LS, int ES, const RR *f) {
         constexpr int nR = N / RL, NB = NL * nR, PER = (NB + T - 1) / T;
 #pragma unroll(U)
         for (int p = 0; p < PER; ++p) {
@@ -127,9 +127,16 @@ struct InPlace {
             for (int m = 0; m < RL; ++m) v[m] = t[l * LS + (j * RL + m) * ES];
             Radix<C2, RL>::template run<-1>(v);
             const int fj = mid_freq(j);
+            if constexpr (sizeof(RR) == 8) {
+                RR g[RL];
 #pragma unroll
-            for (int q = 0; q < RL; ++q) v[q] = cscale(f[fj + q * nR] * cst, v[q]);
-            Radix<C2, RL>::template run<1>(v);
+                for (int q = 0; q < RL; ++q) g[q] = f[fj + q * nR];
+                radix_scaled<C2, RL, 1>(v, g);
+            } else {  // (value by value: the FP32 planes run at their register caps)
+#pragma unroll
+                for (int q = 0; q < RL; ++q) v[q] = vscale(f[fj + q * nR], v[q]);
+                Radix<C2, RL>::template run<1>(v);
+            }
 #pragma unroll
             for (int m = 0; m < RL; ++m) t[l * LS + (j * RL + m) * ES] = v[m];
         }
@@ -164,7 +171,7 @@ struct InPlace {
             const int l = b % NL, k = b / NL;
             Radix<C2, R0>::template run<-1>(v[u]);
 #pragma unroll
-            for (int q = 1; q < R0; ++q) v[u][q] = cmul(v[u][q], tw[q * k]);
+            for (int q = 1; q < R0; ++q) v[u][q] = vmul(v[u][q], tw[q * k]);
 #pragma unroll
             for (int q = 0; q < R0; ++q) t[l * LS + (k + q * S) * ES] = v[u][q];
         }
@@ -191,9 +198,9 @@ struct InPlace {
     // Filter all NL lines of the tile along their axis, in place, from forward pass P0
     // on (P0 = 1: the caller ran pass 0); ends with a block barrier.
     template <class C2, class RR, int P0>
-    static __device__ __forceinline__ void filter(C2 *t, int LS, int ES, const C2 *tw, const RR *f, RR cst) {
+    static __device__ __forceinline__ void filter(C2 *t, int LS, int ES, const C2 *tw, const RR *f) {
         fwd<C2, P0>(t, LS, ES, tw);
-        mid<C2, RR>(t, LS, ES, f, cst);
+        mid<C2, RR>(t, LS, ES, f);
         __syncthreads();
         inv<C2, NF - 2>(t, LS, ES, tw);
     }

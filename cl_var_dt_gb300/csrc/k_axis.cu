@@ -61,7 +61,7 @@ __device__ __forceinline__ void cta_pass(const C2 *s, C2 *d, int SS, int SD, int
             if (NS > 1 && r > 0) {
                 C2 t = tw[k * r * tstep];
                 if (S > 0) t.y = -t.y;
-                x = cmul(x, t);
+                x = vmul(x, t);
             }
             v[r] = x;
         }
@@ -76,10 +76,10 @@ __device__ __forceinline__ void cta_pass(const C2 *s, C2 *d, int SS, int SD, int
     __syncthreads();
 }
 
-// Last forward pass, real filter f[k] * cst, first inverse pass, in registers.
+// Last forward pass, real filter f[k], first inverse pass, in registers.
 template <class C2, class RR, int N, int R>
 __device__ __forceinline__ void cta_mid(const C2 *s, C2 *d, int SS, int SD, int nl, const C2 *tw,
-                                        const RR *f, RR cst) {
+                                        const RR *f) {
     constexpr int nR = N / R;
     for (int b = threadIdx.x; b < nl * nR; b += blockDim.x) {
         const int l = b / nR, j = b - l * nR;
@@ -89,13 +89,14 @@ __device__ __forceinline__ void cta_mid(const C2 *s, C2 *d, int SS, int SD, int 
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             C2 x = ls[padi(j + r * nR)];
-            if (nR > 1 && r > 0) x = cmul(x, tw[j * r]);
+            if (nR > 1 && r > 0) x = vmul(x, tw[j * r]);
             v[r] = x;
         }
         Radix<C2, R>::template run<-1>(v);
+        RR g[R];
 #pragma unroll
-        for (int q = 0; q < R; ++q) v[q] = cscale(f[j + q * nR] * cst, v[q]);
-        Radix<C2, R>::template run<1>(v);
+        for (int q = 0; q < R; ++q) g[q] = f[j + q * nR];
+        radix_scaled<C2, R, 1>(v, g);
 #pragma unroll
         for (int q = 0; q < R; ++q) ld[padi(j * R + q)] = v[q];
     }
@@ -129,14 +130,14 @@ __device__ __forceinline__ void cta_inv2(C2 *A, C2 *B, int PP, int nl, const C2 
 // B as dense lines; one block barrier per pass.
 template <class C2, class RR, int N>
 __device__ __forceinline__ void cta_lines_filter(C2 *A, C2 *B, int PP, int nl, const C2 *tw,
-                                                 const RR *f, RR cst) {
+                                                 const RR *f) {
     constexpr int NF = ax_nfac(N);
     constexpr int RL = ax_fac(N, NF - 1);
     static_assert(NF >= 2, "compile-time plans need two radix factors");
     cta_fwd2<C2, N, 0, 1, true>(A, B, PP, nl, tw);
     // the middle pass has index NF - 1: it reads A when NF - 1 is even
     constexpr bool MID_A = ((NF - 1) % 2) == 0;
-    cta_mid<C2, RR, N, RL>(MID_A ? A : B, MID_A ? B : A, PP, PP, nl, tw, f, cst);
+    cta_mid<C2, RR, N, RL>(MID_A ? A : B, MID_A ? B : A, PP, PP, nl, tw, f);
     cta_inv2<C2, N, NF - 2, RL, !MID_A>(A, B, PP, nl, tw);
 }
 
@@ -170,6 +171,9 @@ __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
     C2 *dst = reinterpret_cast<C2 *>(field ? A.dst1 : A.dst0) + soff;
     const long long base = inner == 1 ? (long long)task.l0 * n
                                       : (long long)(task.l0 / inner) * n * inner + (task.l0 % inner);
+    // the component constant goes into the CTA's filter table (a tile that runs on across
+    // slices takes none)
+    const R cst = A.with_const ? (R)ch.comp_const[task.slice / ch.nt] : (R)1;
     if constexpr (N > 0) {
         if (inner > 1 && nl == W) {
             // in place: element a of tile line w at tile[w * PL + a], in global memory at
@@ -186,13 +190,12 @@ __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
                 const R *f = A.filter ? efilt_of<R>(ax) : filt_of<R>(ax);
                 for (int i = threadIdx.x; i < n; i += blockDim.x) {
                     twS[i] = tw[i];
-                    fS[i] = f[i];
+                    fS[i] = f[i] * cst;
                 }
             }
             __syncthreads();
-            const R cst = A.with_const ? (R)ch.comp_const[task.slice / ch.nt] : (R)1;
             IP::template fwd<C2, 1>(tile, PL, 1, twS);
-            IP::template mid<C2, R>(tile, PL, 1, fS, cst);
+            IP::template mid<C2, R>(tile, PL, 1, fS);
             __syncthreads();
             IP::template inv<C2, IP::NF - 2, 1>(tile, PL, 1, twS);
             IP::template dit<C2, 0, true>(tile, PL, 1, twS, dst + base, 1, inner, A.accumulate != 0);
@@ -228,23 +231,21 @@ __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
         const R *f = A.filter ? efilt_of<R>(ax) : filt_of<R>(ax);
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
             twS[i] = tw[i];
-            fS[i] = f[i];
+            fS[i] = f[i] * cst;
         }
     }
     __syncthreads();
-    const int c = task.slice / ch.nt;
-    const R cst = A.with_const ? (R)ch.comp_const[c] : (R)1;
     const int px = padded_line(n);
     const C2 *res = tile;  // dense result lines at pitch PL
     if constexpr (N > 0) {
-        cta_lines_filter<C2, R, N>(tile, scr, PL, nl, twS, fS, cst);
+        cta_lines_filter<C2, R, N>(tile, scr, PL, nl, twS, fS);
         res = scr;
     } else {
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
         C2 *scrX = scr + 2 * px * warp, *scrY = scrX + px;
         for (int w = warp; w < nl; w += nwarps) {
             C2 *line = tile + w * PL;
-            warp_line_filter_1d<C2, R>(line, scrX, scrY, ax, twS, fS, cst, lane);
+            warp_line_filter_1d<C2, R>(line, scrX, scrY, ax, twS, fS, (R)1, lane);
             for (int i = lane; i < n; i += 32) line[i] = scrX[i];
             __syncwarp();
         }
@@ -300,7 +301,7 @@ __global__ void __launch_bounds__(64, 6) axis_line_kernel(const LaunchAxis A) {
     const float cst = A.with_const ? (float)ch.comp_const[task.slice / ch.nt] : 1.0f;
     Radix<C2, N>::template run<-1>(v);
 #pragma unroll
-    for (int k = 0; k < N; ++k) v[k] = cscale(f[k] * cst, v[k]);
+    for (int k = 0; k < N; ++k) v[k] = vscale(f[k] * cst, v[k]);
     Radix<C2, N>::template run<1>(v);
     const bool acc = A.accumulate != 0;
 #pragma unroll

@@ -38,7 +38,7 @@ __device__ __forceinline__ void stockham_pass(const C2 *__restrict__ src, C2 *__
             if (r > 0 && k > 0) {
                 C2 t = tw[k * r * step];
                 t.y = S < 0 ? t.y : -t.y;  // table holds exp(-2 pi i k/n)
-                x = cmul(x, t);
+                x = vmul(x, t);
             }
             v[r] = x;
         }

@@ -86,7 +86,7 @@ __device__ __forceinline__ void plane_lines_in_registers(const LaunchAxis &A) {
         Radix<C2, N>::template run<-1>(v);
         const R *f = ph ? fc : fr;
 #pragma unroll
-        for (int k = 0; k < N; ++k) v[k] = cscale(f[k], v[k]);
+        for (int k = 0; k < N; ++k) v[k] = vscale(f[k], v[k]);
         Radix<C2, N>::template run<1>(v);
         const int s0 = ph ? l * PL : l, sa = ph ? 1 : PL;  // element a of the line in the tile
 #pragma unroll
@@ -127,17 +127,16 @@ __device__ __forceinline__ void plane_in_place(const LaunchAxis &A) {
     }
     {
         const R *f0 = filt_of<R>(axr), *f1 = filt_of<R>(axc);
+        const R cst = A.with_const ? (R)ch.comp_const[task.slice / ch.nt] : (R)1;
         for (int i = threadIdx.x; i < N; i += T) {
             twS[i] = tw[i];
             fr[i] = f0[i];
-            fc[i] = f1[i];
+            fc[i] = f1[i] * cst;
         }
     }
     __syncthreads();
-    const int c = task.slice / ch.nt;
-    const R cst = A.with_const ? (R)ch.comp_const[c] : (R)1;
-    IP::template filter<C2, R, 1>(tile, 1, PL, twS, fr, (R)1);  // along the columns (the slower axis)
-    IP::template filter<C2, R, 0>(tile, PL, 1, twS, fc, cst);  // along the rows (contiguous axis)
+    IP::template filter<C2, R, 1>(tile, 1, PL, twS, fr);  // along the columns (the slower axis)
+    IP::template filter<C2, R, 0>(tile, PL, 1, twS, fc);  // along the rows (contiguous axis)
 #pragma unroll
     for (int i = 0; i < EPT; ++i) {
         const int e = threadIdx.x + i * T;

@@ -66,10 +66,11 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
         const int t = tau < 0 ? tau + T : (tau >= T ? tau - T : tau);
         return ((long long)c * T + t) * V + s;
     };
+    const DriftConsts<R> dk(ch);
     const int tau0 = task.tau0, tau1 = task.tau1;
     // carried: psi(tau-1), kin(tau-1), psibar(tau), psi(tau)
     C2 Pp[NC], Kp[NC], Qc[NC], Pc[NC];
-    Spin1Bilinears<C2> Bm;  // spin-1: bilinears of (psibar(tau), psi(tau-1)), carried
+    Spin1Link<C2> Bm;  // spin-1: the pair (psibar(tau), psi(tau-1)), carried
     // prefetched for the next tau: psi(tau+1), psibar(tau+1), kin(tau), kinbar(tau+1)
     C2 nP[NC], nQ[NC], nK[NC], nKc[NC];
     auto load_next = [&](int tau) {
@@ -89,13 +90,12 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
             Qc[c] = gpsic[at(c, tau0)];
             Pc[c] = gpsi[at(c, tau0)];
         }
-        if constexpr (MODEL == CLV_MODEL_SPIN1) Bm = spin1_bilinears<C2, R>(Qc, Pp);
+        if constexpr (MODEL == CLV_MODEL_SPIN1) Bm = spin1_link<R>(dk, Qc, Pp);
         load_next(tau0);
     }
 
     R mxr = 0, smr = 0;
     int bad = 0;
-    const DriftConsts<R> dk(ch);
     const uint64_t seed = ch.seed;
     const int ref_rule = A.dt_rule == CLV_DT_REF_MEANMAX;
     if (act) {
@@ -109,9 +109,9 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
                 drift_ref4_vals<R>(dk, Pp, Pc, vpp, Qc, vcp, Kp, kp, K, Kc);
             else
             {
-                const Spin1Bilinears<C2> Bp = spin1_bilinears<C2, R>(vcp, Pc);
-                drift_spin1_vals_b<R>(dk, Bm, Bp, Pp, Pc, Qc, vcp, Kp, kp, K, Kc);
-                Bm = Bp;
+                spin1_drift_psi<R>(Bm, Pp, Pc, Kp, K);
+                Bm = spin1_link<R>(dk, vcp, Pc);
+                spin1_drift_bar<R>(Bm, vcp, Qc, kp, Kc);
             }
             if (A.mode == FUSED_MAXONLY && A.drift_out) {
                 // the stored-drift update reads the drift instead of a second drift pass
