@@ -13,6 +13,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <string>
 #include <vector>
 
@@ -53,6 +54,39 @@ bool factorize(int n, int *fac, int &nf) {
     return n == 1;
 }
 
+// In-place plan of the tile filter: as few radices of 2 .. 16 as the length allows, the most
+// even such split, larger ones first.
+bool tile_factors(int n, int *fac, int &nf) {
+    static const int radices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+    if (n <= 1) return false;
+    for (int want = 1; want <= kMaxTileFactors; ++want) {
+        int best[kMaxTileFactors], cur[kMaxTileFactors], sum = 1 << 30;
+        auto search = [&](auto &&self, int rest, int depth, int most) -> void {
+            if (depth == want) {
+                int s = 0;
+                for (int i = 0; i < want; ++i) s += cur[i];
+                if (rest == 1 && s < sum) {
+                    sum = s;
+                    std::copy(cur, cur + want, best);
+                }
+                return;
+            }
+            for (int r : radices)
+                if (r <= most && rest % r == 0) {
+                    cur[depth] = r;
+                    self(self, rest / r, depth + 1, r);
+                }
+        };
+        search(search, n, 0, 16);
+        if (sum < (1 << 30)) {
+            nf = want;
+            std::copy(best, best + want, fac);
+            return true;
+        }
+    }
+    return false;
+}
+
 }  // namespace
 
 namespace clv {
@@ -88,7 +122,7 @@ struct clv_engine {
     FusedTask *fused_tasks = nullptr;
     double2 *fused_partials = nullptr;
     int slot_stride = 0, comp_stride = 0;
-    int fused_tab_n = 0, fused_tab_bytes = 0, fused_spt = 1, fused_ln = 0;
+    int fused_tab_n = 0, fused_tab_bytes = 0, fused_ln = 0;
     size_t fused_smem = 0;
     int fused_ctas_per_sm = 0;
     int num_sms = 0;
@@ -103,12 +137,19 @@ struct clv_engine {
         int axis, n, pitch, with_const;
         int W;          // lines per tile
         int plane = 0;  // 1: square planes over axes (axis, axis + 1) by the plane filter
+        int tile = 0;   // 1: tile filter (k_tile.cuh), tasks in ttasks; n = 0 when lengths differ
+        int threads = 128;
+        int whole = 0;  // tile filter over whole slices
+        std::vector<TileFilterTask> ttasks;
+        TileFilterTask *td = nullptr;
         int strided = 1;  // every chain's lines of this axis are neighbours in memory (stride > 1)
         size_t smem;
         std::vector<AxisTask> tasks;
         AxisTask *d = nullptr;
     };
     bool tiled = false;
+    std::vector<TileFilterPlan> tile_plans_h;
+    TileFilterPlan *tile_plans = nullptr;
     std::vector<AxisGroup> axis_groups;
     bool energy_axis = false;             // kinetic energy of the observables by axis filters
     std::vector<AxisGroup> energy_groups;
@@ -202,7 +243,7 @@ int build_tables(clv_engine *e) {
     long long off = 0, noff = 0;
     int obs_off = 0;
     // host staging for every table, uploaded at once
-    struct Pending { void **dst; std::vector<unsigned char> bytes; };
+    struct Pending { void **dst; std::vector<unsigned char> bytes; size_t off; };
     std::vector<Pending> pend;
     auto table = [&](auto **dst, auto &&vec) {
         Pending p;
@@ -272,6 +313,28 @@ int build_tables(clv_engine *e) {
             table(&ax.filt32, f32);
             table(&ax.efilt64, e64);
             table(&ax.efilt32, e32);
+            // the tile filter's plan, and the filters in the order its forward passes leave
+            // the frequencies: position sum_p q_p (L_p / R_p) holds sum_p q_p (R_0 ... R_{p-1})
+            if (!tile_factors(n, ax.tfac, ax.tnf)) ax.tnf = 0;
+            if (ax.tnf) {
+                std::vector<double> tf64(n), te64(n);
+                for (int i = 0; i < n; ++i) {
+                    int rest = i, L = n, w = 1, k = 0;
+                    for (int p = 0; p < ax.tnf; ++p) {
+                        L /= ax.tfac[p];
+                        k += rest / L * w;
+                        rest %= L;
+                        w *= ax.tfac[p];
+                    }
+                    tf64[i] = f64[k];
+                    te64[i] = e64[k];
+                }
+                std::vector<float> tf32(tf64.begin(), tf64.end()), te32(te64.begin(), te64.end());
+                table(&ax.tfilt64, tf64);
+                table(&ax.tfilt32, tf32);
+                table(&ax.tefilt64, te64);
+                table(&ax.tefilt32, te32);
+            }
             // per-pass twiddles of the fused kernel's compile-time line plans, from the
             // same rounded values
             if (n == 64 || n == 128 || n == 256 || n == 512) {
@@ -324,14 +387,23 @@ int build_tables(clv_engine *e) {
     e->total_elems = off;
     e->noise_total = noff;
     e->acc_F_total = obs_off;
-    // upload tables; device pointers are patched into the host chain copies
+    // upload the tables in one allocation and one copy, equal ones (chains of one length and
+    // imaginary-time step) once; device pointers are patched into the host chain copies
+    std::map<std::vector<unsigned char>, size_t> at;
+    std::vector<unsigned char> pool;
     for (auto &p : pend) {
-        void *dptr = nullptr;
-        int rc = e->alloc(&dptr, p.bytes.size());
-        if (rc) return rc;
-        CK(cudaMemcpy(dptr, p.bytes.data(), p.bytes.size(), cudaMemcpyHostToDevice));
-        *p.dst = dptr;
+        const auto it = at.emplace(std::move(p.bytes), pool.size());
+        p.off = it.first->second;
+        if (it.second) {
+            const auto &b = it.first->first;
+            pool.insert(pool.end(), b.begin(), b.end());
+            pool.resize((pool.size() + 255) / 256 * 256);
+        }
     }
+    unsigned char *dptr = nullptr;
+    if (int rc = e->alloc(&dptr, pool.size())) return rc;
+    if (!pool.empty()) CK(cudaMemcpy(dptr, pool.data(), pool.size(), cudaMemcpyHostToDevice));
+    for (auto &p : pend) *p.dst = dptr + p.off;
     return CLV_OK;
 }
 
@@ -411,7 +483,6 @@ LaunchFused fused_launch(const clv_engine *e, int from, int mode, bool ext) {
     L.comp_stride = e->comp_stride;
     L.tab_n = e->fused_tab_n;
     L.tab_bytes = e->fused_tab_bytes;
-    L.spt = e->fused_spt;
     L.ln = e->fused_ln;
     L.split = e->fused_split ? 1 : 0;
     L.smem_bytes = e->fused_smem;
@@ -442,33 +513,63 @@ LaunchTiled tiled_launch(const clv_engine *e, int from, int mode, bool ext) {
     return L;
 }
 
+// The launches of a group list.  Kinetic filter (two fields, src1 not null): the groups of
+// axis 0 read the fields, the others continue in kin/kinbar.  Kinetic energy (src1 null):
+// every axis reads src0, the first writes kin and the others add to it.
+template <class R>
+int run_groups(clv_engine *e, const std::vector<clv_engine::AxisGroup> &groups, const void *src0, const void *src1,
+               EventTrail *trail = nullptr) {
+    const bool energy = src1 == nullptr;
+    for (const auto &g : groups) {
+        const void *s0 = (energy || g.axis == 0) ? src0 : e->kin, *s1 = g.axis == 0 ? src1 : e->kinc;
+        if (g.tile) {
+            LaunchTileFilter T{};
+            T.chains = e->chains_d;
+            T.plans = e->tile_plans;
+            T.tasks = g.td;
+            T.ntasks = (int)g.ttasks.size();
+            T.src0 = s0;
+            T.src1 = s1;
+            T.dst0 = e->kin;
+            T.dst1 = e->kinc;
+            T.nfields = energy ? 1 : 2;
+            T.filter = energy;
+            T.accumulate = energy && g.axis > 0;
+            T.threads = g.threads;
+            T.smem_bytes = g.smem;
+            CK(launch_tile_filter<R>(T, e->stream));
+        } else {
+            LaunchAxis A{};
+            A.chains = e->chains_d;
+            A.tasks = g.d;
+            A.ntasks = (int)g.tasks.size();
+            A.axis = g.axis;
+            A.n = g.n;
+            A.W = g.W;
+            A.pitch = g.pitch;
+            A.with_const = g.with_const;
+            A.src0 = s0;
+            A.src1 = s1;
+            A.dst0 = e->kin;
+            A.dst1 = e->kinc;
+            A.smem_bytes = g.smem;
+            A.nfields = energy ? 1 : 2;
+            A.filter = energy;
+            A.accumulate = energy && g.axis > 0;
+            A.strided = g.strided;
+            if (g.plane) CK(launch_plane_filter<R>(A, e->stream));
+            else CK(launch_axis_filter<R>(A, e->stream));
+        }
+        if (trail) CK(trail->mark(e->stream));
+    }
+    return CLV_OK;
+}
+
 // Tiled step: kinetic filter axis by axis into kin/kinbar, then the streaming
 // drift/noise/update kernel (speculative dt with redo, or reduce then apply).
 template <class R>
 int enqueue_tiled(clv_engine *e, bool external_noise, EventTrail *trail, int from) {
-    for (const auto &g : e->axis_groups) {
-        LaunchAxis A{};
-        A.chains = e->chains_d;
-        A.tasks = g.d;
-        A.ntasks = (int)g.tasks.size();
-        A.axis = g.axis;
-        A.n = g.n;
-        A.W = g.W;
-        A.pitch = g.pitch;
-        A.with_const = g.with_const;
-        A.src0 = g.axis == 0 ? e->fld[from][0] : e->kin;
-        A.src1 = g.axis == 0 ? e->fld[from][1] : e->kinc;
-        A.dst0 = e->kin;
-        A.dst1 = e->kinc;
-        A.smem_bytes = g.smem;
-        A.nfields = 2;
-        A.filter = 0;
-        A.accumulate = 0;
-        A.strided = g.strided;
-        if (g.plane) CK(launch_plane_filter<R>(A, e->stream));
-        else CK(launch_axis_filter<R>(A, e->stream));
-        if (trail) CK(trail->mark(e->stream));
-    }
+    if (int rc = run_groups<R>(e, e->axis_groups, e->fld[from][0], e->fld[from][1], trail)) return rc;
     if (e->speculate && e->dt_rule == CLV_DT_K_OVER_MAX) {
         CK(launch_tiled<R>(tiled_launch(e, from, FUSED_SPEC, external_noise), e->stream));
         if (trail) CK(trail->mark(e->stream));
@@ -597,7 +698,10 @@ int enqueue_step(clv_engine *e, bool external_noise, EventTrail *trail, int from
         if (trail) CK(trail->mark(e->stream));
         return CLV_OK;
     }
-    int rc = run_kinetic<R>(e, e->fld[from][0], e->fld[from][1], e->kin, e->kinc, 0, 2, trail);
+    // lines beyond the tiled path's: the tile filter, or the line filter where the tile path
+    // is switched off (CLV_TILED=0)
+    int rc = e->axis_groups.empty() ? run_kinetic<R>(e, e->fld[from][0], e->fld[from][1], e->kin, e->kinc, 0, 2, trail)
+                                    : run_groups<R>(e, e->axis_groups, e->fld[from][0], e->fld[from][1], trail);
     if (rc) return rc;
     LaunchSites L = e->sites();
     L.psi = e->fld[from][0];
@@ -617,9 +721,6 @@ int enqueue_step_any(clv_engine *e, bool ext, EventTrail *trail, int from) {
                                         : enqueue_step<float>(e, ext, trail, from);
 }
 
-// Choose the fused path when every chain's slice fits the shared-memory plan,
-// and split each chain's imaginary times into chunks that fill the GPU.
-// Fused tasks for chunks of L imaginary times; sets each chain's CTA range.
 // Fused step tasks: chunks of L imaginary times.  Under the reference's step rule
 // (two passes on the generic kernel), when the chunks are fewer than the SMs (the
 // reference's own 256 x 32 lattice: 32 chunks), each chunk becomes a psi CTA and a
@@ -671,22 +772,17 @@ void build_fused_tasks(clv_engine *e, int L) {
     }
 }
 
-// Tiled step tasks: 256 sites x chunks of L imaginary times.
+// Tiled step tasks: 256 consecutive (chunk, site) pairs, chunks of L imaginary times.
 void build_tiled_tasks(clv_engine *e, int L) {
     e->chunk = L;
     e->tile_tasks_h.clear();
     for (int c = 0; c < (int)e->chains_h.size(); ++c) {
         ChainDev &d = e->chains_h[c];
-        const int ntile = (d.V + 255) / 256;
         const int nchunk = std::max(1, (d.nt + L - 1) / L);
+        const int ntile = (int)(((long long)d.V * nchunk + 255) / 256);
         d.fused_block0 = (int)e->tile_tasks_h.size();
-        d.fused_nblocks = ntile * nchunk;
-        int part = 0;
-        for (int k = 0; k < nchunk; ++k) {
-            const int t0 = (int)((long long)d.nt * k / nchunk);
-            const int t1 = (int)((long long)d.nt * (k + 1) / nchunk);
-            for (int t = 0; t < ntile; ++t) e->tile_tasks_h.push_back({c, t * 256, t0, t1, part++});
-        }
+        d.fused_nblocks = ntile;
+        for (int t = 0; t < ntile; ++t) e->tile_tasks_h.push_back({c, t * 256, nchunk, t});
     }
 }
 
@@ -706,25 +802,16 @@ int plan_fused(clv_engine *e) {
     // even so that every component row stays 16-byte aligned for the bulk copies
     const int cs = padded_line(vmax);
     const int stride = fused_slot_stride(e->ncomp, vmax, (int)esz);
-    const int spt = vmax <= 256 ? 1 : (vmax <= 512 ? 2 : (vmax <= 1024 ? 4 : 0));
-    if (spt == 0) return CLV_OK;
-    // compile-time plan when every chain is a 1D line of one common length
+    // every chain a 1D line of one common length of 64, 128 or 256 sites: other shapes and
+    // mixed batches take the tiled path, whose filters work on whole tiles of lines (a warp
+    // per line and a thread per site of the batch's largest slice left 64 chains of 60-site
+    // lines to 30 x 30 planes at 2.43 ms per step; tiled: 0.13 ms)
     int ln = e->chains_h[0].nx;
     for (auto &d : e->chains_h)
         if (d.ny != 1 || d.nz != 1 || d.nx != ln) ln = 0;
-    if (ln != 64 && ln != 128 && ln != 256) ln = 0;
+    if (ln != 64 && ln != 128 && ln != 256) return CLV_OK;
     if (std::getenv("CLV_NO_STATIC_PLAN")) ln = 0;
-    // shared tables: twiddles and filters of the filtered axes of the largest chain
-    int tab_n = 0;
-    for (auto &d : e->chains_h) {
-        int n = 0;
-        for (int a = 0; a < 3; ++a) {
-            if (d.axis[a].n <= 1) continue;
-            if (e->kinetic == CLV_KIN_REF_LINEAR_PX && a > 0) break;
-            n += d.axis[a].n;
-        }
-        tab_n = std::max(tab_n, n);
-    }
+    const int tab_n = vmax;  // twiddles and filter of the lines
     const int tab_bytes = fused_tab_bytes(tab_n, (int)esz, ln);
     const int nslots = (e->model == CLV_MODEL_REF4 ? 3 : 2) + 2 + 5;
     const size_t smem = tab_bytes + (size_t)nslots * stride * esz;
@@ -733,21 +820,16 @@ int plan_fused(clv_engine *e) {
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device));
     e->num_sms = nsm;
     if (smem + 2048 > (size_t)dev_smem) return CLV_OK;  // room for the kernel's static shared memory
-    // the compile-time-line kernels derive the same geometry from ln alone
-    if (ln > 0 && (tab_n != ln || stride != fused_slot_stride(e->ncomp, ln, (int)esz)))
-        return fail(CLV_ERR_STATE, "fused slot geometry of the line kernels");
     e->slot_stride = stride;
     e->comp_stride = cs;
     e->fused_smem = smem;
     e->fused_tab_n = tab_n;
     e->fused_tab_bytes = tab_bytes;
-    e->fused_spt = spt;
     e->fused_ln = ln;
     e->use_tma = aligned && !(std::getenv("CLV_NO_TMA"));
     e->speculate = !(std::getenv("CLV_NO_SPECULATE"));
     LaunchFused probe{};
     probe.model = e->model;
-    probe.spt = spt;
     probe.ln = ln;
     probe.smem_bytes = smem;
     int per_sm = 0;
@@ -784,14 +866,122 @@ int plan_fused(clv_engine *e) {
     return CLV_OK;
 }
 
-// Tiled path for the chains the fused kernel cannot hold: every filtered axis
-// needs lines of at most 512 sites and shared memory for a tile of up to W
-// adjacent lines and its FFT scratch (axis_tile_lines, axis_smem_bytes).
-// Otherwise the engine keeps the separate line-filter / drift / update kernels.
+// The tile-filter group for tiles of `elems` shared elements along axis `a` (0 for whole
+// slices): tiles of one size class share a launch, whatever their shapes.
+clv_engine::AxisGroup &tile_group(const clv_engine *e, std::vector<clv_engine::AxisGroup> &groups, int a, int n,
+                                  bool whole, int elems, size_t smem) {
+    const bool wide = elems > (e->elem_bytes == 8 ? tile_wide<float>() : tile_wide<double>());
+    const int threads = wide ? 256 : 128;
+    for (auto &g : groups)
+        if (g.tile && g.axis == a && g.threads == threads) {
+            if (g.n != n) g.n = 0;
+            g.whole |= whole;
+            g.smem = std::max(g.smem, smem);
+            return g;
+        }
+    clv_engine::AxisGroup g{};
+    g.axis = a;
+    g.n = n;
+    g.tile = 1;
+    g.whole = whole;
+    g.threads = threads;
+    g.smem = smem;
+    groups.push_back(std::move(g));
+    return groups.back();
+}
+
+size_t tile_smem(const clv_engine *e, int elems, int nsum, int rows) {
+    return (size_t)(elems + nsum) * e->elem_bytes + (size_t)(nsum + rows) * (e->elem_bytes / 2) + 16;
+}
+
+int tile_plan(clv_engine *e, const TileFilterPlan &p) {
+    for (int i = 0; i < (int)e->tile_plans_h.size(); ++i)
+        if (!std::memcmp(&e->tile_plans_h[i], &p, sizeof p)) return i;
+    e->tile_plans_h.push_back(p);
+    return (int)e->tile_plans_h.size() - 1;
+}
+
+// Whole slices of chain c: tiles of consecutive imaginary times of one component, about
+// tile_target elements (one slice when it is larger).
+int add_tile_slices(clv_engine *e, int c, bool energy, std::vector<clv_engine::AxisGroup> &groups) {
+    const ChainDev &d = e->chains_h[c];
+    int last = 0;
+    for (int a = 1; a < 3; ++a)
+        if (d.axis[a].n > 1) last = a;
+    TileFilterPlan p;
+    std::memset(&p, 0, sizeof p);
+    const int cols = d.axis[last].n, rows1 = d.V / cols;
+    int nsum = 0;
+    for (int a = 0; a <= last; ++a) {
+        if (d.axis[a].n <= 1) continue;
+        if (!energy && e->kinetic == CLV_KIN_REF_LINEAR_PX && a > 0) break;
+        if (!d.axis[a].tnf) return fail(CLV_ERR_STATE, "tile filter plan");
+        p.axis[p.naxes] = a;
+        p.inner[p.naxes++] = d.axis[a].inner;
+        nsum += d.axis[a].n;
+    }
+    p.pitch = cols | 1;
+    p.with_const = !energy && e->kinetic == CLV_KIN_EXP;
+    const int target = e->elem_bytes == 8 ? tile_target<float>() : tile_target<double>();
+    const int ns = std::max(1, std::min(d.nt, target / d.V));
+    p.tile_elems = (ns * rows1 * p.pitch + 1) / 2 * 2;
+    const int id = tile_plan(e, p);
+    auto &g = tile_group(e, groups, 0, p.naxes == 1 ? d.axis[p.axis[0]].n : 0, p.naxes > 1, p.tile_elems,
+                         tile_smem(e, p.tile_elems, nsum, ns * rows1));
+    for (int k = 0; k < d.ncomp; ++k)
+        for (int t = 0; t < d.nt; t += ns)
+            g.ttasks.push_back({c, id, k * d.nt + t, 0, std::min(ns, d.nt - t) * rows1, cols});
+    return CLV_OK;
+}
+
+// Tiles of lines of axis a of chain c: a strided axis in tiles of adjacent lines (16-line
+// multiples keep the rows' 128-byte segments), the innermost one in tiles of whole lines.
+int add_tile_axis(clv_engine *e, int c, int a, bool energy, std::vector<clv_engine::AxisGroup> &groups) {
+    const ChainDev &d = e->chains_h[c];
+    const AxisDev &ax = d.axis[a];
+    if (!ax.tnf) return fail(CLV_ERR_STATE, "tile filter plan");
+    const int n = ax.n, lines = d.V / n;
+    const int target = e->elem_bytes == 8 ? tile_target<float>() : tile_target<double>();
+    TileFilterPlan p;
+    std::memset(&p, 0, sizeof p);
+    p.naxes = 1;
+    p.axis[0] = a;
+    p.with_const = !energy && e->kinetic == CLV_KIN_EXP && a == 0;
+    if (ax.inner > 1) {
+        int W = target / n;
+        W = W >= 16 ? W / 16 * 16 : (W >= 8 ? 8 : 4);
+        W = std::min(W, ax.inner);
+        p.inner[0] = 0;
+        p.pitch = W | 1;
+        p.gstride = ax.inner;
+        p.tile_elems = (n * p.pitch + 1) / 2 * 2;
+        const int id = tile_plan(e, p);
+        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, n));
+        for (int sl = 0; sl < d.ncomp * d.nt; ++sl)
+            for (int hi = 0; hi < lines / ax.inner; ++hi)
+                for (int l = 0; l < ax.inner; l += W)
+                    g.ttasks.push_back({c, id, sl, hi * n * ax.inner + l, n, std::min(W, ax.inner - l)});
+    } else {
+        const int W = std::max(1, std::min(lines, target / n));
+        p.inner[0] = 1;
+        p.pitch = n | 1;
+        p.tile_elems = (W * p.pitch + 1) / 2 * 2;
+        const int id = tile_plan(e, p);
+        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, W));
+        for (int sl = 0; sl < d.ncomp * d.nt; ++sl)
+            for (int l = 0; l < lines; l += W)
+                g.ttasks.push_back({c, id, sl, l * n, std::min(W, lines - l), n});
+    }
+    return CLV_OK;
+}
+
 // Axis-filter launch groups, one per (axis, line length): kinetic (energy =
 // false: the step's filter, every filtered axis, the component constant on the
-// first) or kinetic energy (energy = true: k_a^2/2 on every axis, summed).  False
-// when a line is longer than 512 sites or a tile does not fit shared memory.
+// first) or kinetic energy (energy = true: k_a^2/2 on every axis, summed).  Square planes
+// of 32 to 128 (kinetic) take the plane filter; other slices of up to tile_slice_max sites
+// the tile filter with every axis on chip; the axes of larger slices the axis filter where
+// it has their length, else the tile filter.  *ok false when a tile does not fit shared
+// memory.
 int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGroup> &groups, bool &ok) {
     ok = false;
     groups.clear();
@@ -817,6 +1007,11 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
                 }
             }
             if (occ < 1) pa = -1;
+        }
+        // other small slices: every filtered axis while the slice is on chip
+        if (pa < 0 && d.V <= (esz == 8 ? tile_slice_max<float>() : tile_slice_max<double>())) {
+            if (int rc = add_tile_slices(e, c, energy, groups)) return rc;
+            continue;
         }
         for (int a = 0; a < 3; ++a) {
             const AxisDev &ax = d.axis[a];
@@ -846,20 +1041,23 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
                 continue;
             }
             const int n = ax.n, lines = d.V / n;
-            if (n > 512) return CLV_OK;
             const bool ct = axis_compile_time_plan(n);
-            const int W = esz == 8 ? axis_tile_lines<float>(ct ? n : 0) : axis_tile_lines<double>(ct ? n : 0);
+            if (!ct) {
+                if (int rc = add_tile_axis(e, c, a, energy, groups)) return rc;
+                continue;
+            }
+            const int W = esz == 8 ? axis_tile_lines<float>(n) : axis_tile_lines<double>(n);
             int gi = -1;
             for (int g = 0; g < (int)groups.size(); ++g)
-                if (!groups[g].plane && groups[g].axis == a && groups[g].n == n) gi = g;
+                if (!groups[g].plane && !groups[g].tile && groups[g].axis == a && groups[g].n == n) gi = g;
             if (gi < 0) {
                 clv_engine::AxisGroup g;
                 g.axis = a;
                 g.n = n;
-                g.pitch = axis_pitch(n, ct);
+                g.pitch = axis_pitch(n);
                 g.W = W;
                 g.with_const = !energy && e->kinetic == CLV_KIN_EXP && a == 0;
-                g.smem = axis_smem_bytes(n, ct, W, esz);
+                g.smem = axis_smem_bytes(n, W, esz);
                 if (g.smem + 1024 > (size_t)dev_smem) return CLV_OK;
                 int occ = 0;
                 if (e->precision == CLV_PREC_F64) CK(setup_axis_filter<double>(n, g.smem, &occ));
@@ -887,6 +1085,13 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
             }
         }
     }
+    for (auto &g : groups)
+        if (g.tile) {
+            int occ = 0;
+            if (e->precision == CLV_PREC_F64) CK(setup_tile_filter<double>(g.smem, &occ));
+            else CK(setup_tile_filter<float>(g.smem, &occ));
+            if (occ < 1) return CLV_OK;
+        }
     std::stable_sort(groups.begin(), groups.end(),
                      [](const clv_engine::AxisGroup &x, const clv_engine::AxisGroup &y) { return x.axis < y.axis; });
     ok = true;
@@ -900,11 +1105,18 @@ int plan_tiled(clv_engine *e) {
     int nsm = 0;
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, e->device));
     std::vector<clv_engine::AxisGroup> groups;
-    for (auto &d : e->chains_h)
-        if (d.nt < 2) return CLV_OK;
-    bool ok = false;
+    bool ok = false, longer = false;
     if (int rc = build_axis_groups(e, false, groups, ok)) return rc;
     if (!ok) return CLV_OK;
+    for (auto &d : e->chains_h) {
+        if (d.nt < 2) longer = true;
+        for (int a = 0; a < 3; ++a)
+            longer |= d.axis[a].n > kTiledMaxLine && !(a > 0 && e->kinetic == CLV_KIN_REF_LINEAR_PX);
+    }
+    if (longer) {
+        e->axis_groups = std::move(groups);
+        return CLV_OK;
+    }
     int occ = 0;
     if (e->precision == CLV_PREC_F64) CK(setup_tiled<double>(e->model, &occ));
     else CK(setup_tiled<float>(e->model, &occ));
@@ -913,7 +1125,7 @@ int plan_tiled(clv_engine *e) {
     // chunks amortise the halo slice and the prologue; clv_autotune refines it);
     // fewer for problems too small to fill the GPU
     long long tile_taus = 0;
-    for (auto &d : e->chains_h) tile_taus += (long long)((d.V + 255) / 256) * d.nt;
+    for (auto &d : e->chains_h) tile_taus += ((long long)d.V * d.nt + 255) / 256;
     const long long Lw = tile_taus / ((long long)occ * nsm);
     int L = (int)(Lw >= 8 ? std::min<long long>(64, Lw) : std::max<long long>(1, Lw));
     if (const char *cl = std::getenv("CLV_CHUNK")) L = std::max(1, atoi(cl));
@@ -1077,10 +1289,12 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
         if (!e->line_tasks_h[a].empty() &&
             (rc = e->alloc(&e->line_tasks[a], e->line_tasks_h[a].size() * sizeof(LineTask))))
             return bail(rc);
-    for (auto &g : e->axis_groups)
-        if ((rc = e->alloc(&g.d, g.tasks.size() * sizeof(AxisTask)))) return bail(rc);
-    for (auto &g : e->energy_groups)
-        if ((rc = e->alloc(&g.d, g.tasks.size() * sizeof(AxisTask)))) return bail(rc);
+    for (auto *gs : {&e->axis_groups, &e->energy_groups})
+        for (auto &g : *gs)
+            if ((rc = g.tile ? e->alloc(&g.td, g.ttasks.size() * sizeof(TileFilterTask))
+                             : e->alloc(&g.d, g.tasks.size() * sizeof(AxisTask))))
+                return bail(rc);
+    if ((rc = e->alloc(&e->tile_plans, e->tile_plans_h.size() * sizeof(TileFilterPlan)))) return bail(rc);
     auto up = [&](void *d, const void *h, size_t b) {
         return cudaMemcpy(d, h, b, cudaMemcpyHostToDevice);
     };
@@ -1092,8 +1306,11 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
         return bail(fail(CLV_ERR_CUDA, cudaGetErrorString(ce)));
     for (auto *gs : {&e->axis_groups, &e->energy_groups})
         for (auto &g : *gs)
-            if ((ce = up(g.d, g.tasks.data(), g.tasks.size() * sizeof(AxisTask))) != cudaSuccess)
+            if ((ce = g.tile ? up(g.td, g.ttasks.data(), g.ttasks.size() * sizeof(TileFilterTask))
+                             : up(g.d, g.tasks.data(), g.tasks.size() * sizeof(AxisTask))) != cudaSuccess)
                 return bail(fail(CLV_ERR_CUDA, cudaGetErrorString(ce)));
+    if ((ce = up(e->tile_plans, e->tile_plans_h.data(), e->tile_plans_h.size() * sizeof(TileFilterPlan))) != cudaSuccess)
+        return bail(fail(CLV_ERR_CUDA, cudaGetErrorString(ce)));
     if ((ce = up(e->chains_d, e->chains_h.data(), nch * sizeof(ChainDev))) != cudaSuccess ||
         (ce = up(e->site_tasks, e->site_tasks_h.data(), e->site_tasks_h.size() * sizeof(SiteTask))) != cudaSuccess ||
         (ce = up(e->obs_tasks, e->obs_tasks_h.data(), e->obs_tasks_h.size() * sizeof(SiteTask))) != cudaSuccess ||
@@ -1448,27 +1665,10 @@ int clv_evaluate(clv_engine *e) {
             e->sample_count = 0;
         }
         if (e->energy_axis) {
-            // kinetic energy sum_a (k_a^2/2) psi: the first axis writes, the others add
-            for (const auto &g : e->energy_groups) {
-                LaunchAxis A{};
-                A.chains = e->chains_d;
-                A.tasks = g.d;
-                A.ntasks = (int)g.tasks.size();
-                A.axis = g.axis;
-                A.n = g.n;
-                A.W = g.W;
-                A.pitch = g.pitch;
-                A.with_const = 0;
-                A.src0 = e->psi();
-                A.dst0 = e->kin;
-                A.smem_bytes = g.smem;
-                A.nfields = 1;
-                A.filter = 1;
-                A.accumulate = g.axis > 0;
-                A.strided = g.strided;
-                if (e->precision == CLV_PREC_F64) CK(launch_axis_filter<double>(A, e->stream));
-                else CK(launch_axis_filter<float>(A, e->stream));
-            }
+            // kinetic energy sum_a (k_a^2/2) psi
+            const int rc = e->precision == CLV_PREC_F64 ? run_groups<double>(e, e->energy_groups, e->psi(), nullptr)
+                                                        : run_groups<float>(e, e->energy_groups, e->psi(), nullptr);
+            if (rc) return rc;
         } else {
             int rc = e->precision == CLV_PREC_F64
                          ? run_kinetic<double>(e, e->psi(), nullptr, e->kin, nullptr, 1, 1)
@@ -1561,7 +1761,6 @@ static int apply_plan(clv_engine *e, int L, int tma, int ln, int sd) {
         if (ln != e->fused_ln) {
             LaunchFused probe{};
             probe.model = e->model;
-            probe.spt = e->fused_spt;
             probe.ln = ln;
             probe.smem_bytes = e->fused_smem;
             int per_sm = 0;
@@ -1698,6 +1897,15 @@ int clv_autotune(clv_engine *e, int trial_steps, char *report, int capacity) {
     return CLV_OK;
 }
 
+// Name of a filter launch: planes and axes with their length, tile launches over whole slices
+// or over lines of several lengths without one.
+static std::string group_name(const clv_engine::AxisGroup &g) {
+    if (g.tile && (g.whole || !g.n))
+        return (g.whole ? "slices" : "lines" + std::to_string(g.axis)) + (g.threads > 128 ? "_wide" : "");
+    return (g.plane ? "plane" + std::to_string(g.axis) + std::to_string(g.axis + 1) : "axis" + std::to_string(g.axis)) +
+           "_n" + std::to_string(g.n);
+}
+
 int clv_get_plan(clv_engine *e, char *buf, int capacity) {
     if (!e || !buf || capacity < 1) return fail(CLV_ERR_ARG, "null argument");
     std::string p;
@@ -1708,14 +1916,13 @@ int clv_get_plan(clv_engine *e, char *buf, int capacity) {
         else p = "fused:fused_reduce,fused_apply";
     } else if (e->tiled) {
         p = "tiled:";
-        for (const auto &g : e->axis_groups)
-            p += (g.plane ? "plane" + std::to_string(g.axis) + std::to_string(g.axis + 1) : "axis" + std::to_string(g.axis)) +
-                 "_n" + std::to_string(g.n) + ",";
+        for (const auto &g : e->axis_groups) p += group_name(g) + ",";
         p += (e->speculate && e->dt_rule == CLV_DT_K_OVER_MAX) ? "tiled_step,tiled_redo"
              : e->store_drift ? "tiled_reduce,stored_drift_update" : "tiled_reduce,tiled_apply";
     } else {
         p = "unfused:";
-        for (int a = 0; a < 3; ++a) {
+        for (const auto &g : e->axis_groups) p += group_name(g) + ",";
+        for (int a = 0; a < 3 && e->axis_groups.empty(); ++a) {
             if (e->line_tasks_h[a].empty()) continue;
             if (e->kinetic == CLV_KIN_REF_LINEAR_PX && a > 0) break;
             p += "kinetic_axis" + std::to_string(a) + ",";

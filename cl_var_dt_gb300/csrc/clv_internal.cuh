@@ -12,6 +12,7 @@ namespace clv {
 
 constexpr int kMaxFactors = 16;
 constexpr int kMaxComp = 4;
+constexpr int kMaxTileFactors = 4;  // 2048 = 16 16 8
 
 // Precision traits: R is the arithmetic type of the bulk field work.
 template <class R> struct Cx;
@@ -58,6 +59,12 @@ struct AxisDev {
     // (layout tw_*_off, n = 64 ... 512); null for other lengths
     const double2 *ptw64;
     const float2 *ptw32;
+    // in-place plan of the tile filter (k_tile.cuh): radices 2 .. 16, and the two filters in
+    // its order of frequencies (position i after the forward passes)
+    int tnf;
+    int tfac[kMaxTileFactors];
+    const double *tfilt64, *tefilt64;
+    const float *tfilt32, *tefilt32;
 };
 
 // Per-chain constants (device copy, read-only during steps).

@@ -13,6 +13,9 @@ namespace clv {
 constexpr int kMaxBundleElems64 = 2048;
 constexpr int kMaxBundleElems32 = 4096;
 constexpr int kMaxLine = 2048;
+// Longest line of the tiled path; longer ones (to kMaxLine) take the line filter with the
+// separate drift and update kernels.
+constexpr int kTiledMaxLine = 1536;
 
 struct LaunchLineFilter {
     const ChainDev *chains;
@@ -64,7 +67,6 @@ struct LaunchFused {
     int comp_stride;    // elements between the components of one slot (padded V)
     int tab_n;          // twiddle/filter entries staged in shared memory
     int tab_bytes;      // bytes before the first slot (barriers + tables)
-    int spt;            // lattice sites per thread (1, 2 or 4)
     int ln;             // every chain a 1D line of ln sites (64, 128, 256), else 0
     int split;          // tasks step psi and psibar in separate CTAs (FusedTask::side)
     size_t smem_bytes;
@@ -231,12 +233,53 @@ struct LaunchAxis {
     int strided;     // every task's lines are neighbours in memory (axis stride > 1)
 };
 
-// Step over precomputed kinetic terms: a CTA streams imaginary times
-// [tau0, tau1) of 256 consecutive sites of one chain.
+// Tile filter (k_tile.cuh): a tile of one field -- whole slices, or a strided or
+// contiguous tile of lines of one axis -- filtered along every axis of its plan.
+struct TileFilterPlan {
+    int naxes;
+    int axis[3];        // in the order of processing
+    int inner[3];       // tile elements (padding aside) between two sites of the axis; 1: the
+                        // rows' own axis, 0: the task's columns (a strided tile)
+    int pitch;          // shared elements between rows (odd)
+    int gstride;        // global elements between rows, 0: rows follow one another
+    int with_const;     // multiply the component constant
+    int tile_elems;     // shared elements of a full tile
+};
+struct TileFilterTask {
+    int chain, plan;
+    int slice;          // c * nt + tau of the first element
+    int off;            // elements from the slice's start
+    int rows, cols;
+};
+struct LaunchTileFilter {
+    const ChainDev *chains;
+    const TileFilterPlan *plans;
+    const TileFilterTask *tasks;
+    int ntasks;
+    const void *src0, *src1;
+    void *dst0, *dst1;
+    int nfields;        // 2: psi and psibar (blockIdx.x % 2), 1: src0 -> dst0 only
+    int filter;         // 0: kinetic filter, 1: kinetic-energy filter (sum over the axes)
+    int accumulate;     // 1: dst += filtered
+    int threads;        // 128, 256 for tiles above kTileWide elements
+    size_t smem_bytes;
+};
+// Elements of a tile of lines, of a whole slice kept on chip (several CTAs per SM), and
+// where a CTA takes 256 threads instead of 128.
+template <class R> __host__ __device__ constexpr int tile_target() { return sizeof(R) == 4 ? 4096 : 2048; }
+template <class R> __host__ __device__ constexpr int tile_slice_max() { return sizeof(R) == 4 ? 12288 : 6144; }
+template <class R> __host__ __device__ constexpr int tile_wide() { return sizeof(R) == 4 ? 6144 : 3072; }
+template <class R> cudaError_t launch_tile_filter(const LaunchTileFilter &L, cudaStream_t s);
+template <class R> cudaError_t setup_tile_filter(size_t smem_bytes, int *ctas_per_sm);
+
+// Step over precomputed kinetic terms: the chain's imaginary times are split into nchunk
+// chunks, and its (chunk, site) pairs, flattened, are taken 256 at a time; every thread
+// streams its site through its chunk.  A slice of 60 sites so fills its warps with four
+// chunks and a bit.
 struct TileTask {
     int chain;
-    int site0;
-    int tau0, tau1;
+    int flat0;  // chunk * V + site of the CTA's first thread
+    int nchunk;
     int part;   // index of the CTA's step-rule partial within the chain
 };
 
@@ -283,9 +326,8 @@ template <class R> cudaError_t launch_plane_filter(const LaunchAxis &L, cudaStre
 template <class R> cudaError_t setup_plane_filter(int n, size_t smem_bytes, int *ctas_per_sm);
 template <class R> cudaError_t launch_tiled(const LaunchTiled &L, cudaStream_t s);
 template <class R> cudaError_t setup_tiled(int model, int *ctas_per_sm);
-// Axis filter geometry.  Compile-time plans exist for lines of 32, 64, 96, 128,
-// 256 and 512 sites.  Lines per tile (FP32; half at FP64): 64 for 32, 32 for 64,
-// 16 for 96 and 128, 8 for 256, 512 and runtime plans (n = 0 here), so that a
+// Axis filter geometry, lines of 32, 64, 96, 128, 256 and 512 sites.  Lines per tile
+// (FP32; half at FP64): 64 for 32, 32 for 64, 16 for 96 and 128, 8 for 256 and 512, so that a
 // radix-8 pass has about a butterfly for each of the 256 threads and a tile with
 // its scratch fits in a quarter of an SM's shared memory.
 __host__ __device__ constexpr bool axis_compile_time_plan(int n) {
@@ -299,19 +341,13 @@ __host__ __device__ constexpr int axis_tile_lines(int n) {
 __host__ __device__ constexpr size_t axis_tab_bytes(int n, size_t esz) { return ((size_t)n * (esz + esz / 2) + 15) / 16 * 16; }
 // tile elements (W lines at pitch PL), rounded to keep the scratch 16-byte aligned
 __host__ __device__ constexpr int axis_tile_elems(int n, int PL, int W) { return (W * PL + 1) / 2 * 2; }
-// line pitch of the tile: odd (no bank conflicts for the transposing accesses); for
-// the compile-time plans large enough to hold a padded line, since the tile is one
-// of the two buffers the passes alternate between
-__host__ __device__ constexpr int axis_pitch(int n, bool compile_time_plan) {
-    return compile_time_plan ? (padded_line(n) | 1) : (n | 1);
-}
-// shared bytes of one CTA: tables, tile, scratch (one more tile for the CTA-wide
-// compile-time plan, two padded lines per warp for the runtime plan)
-__host__ __device__ constexpr size_t axis_smem_bytes(int n, bool compile_time_plan, int W, size_t esz) {
-    return axis_tab_bytes(n, esz) +
-           (compile_time_plan ? 2 * (size_t)axis_tile_elems(n, axis_pitch(n, true), W)
-                              : (size_t)axis_tile_elems(n, axis_pitch(n, false), W) + 2 * 8 * padded_line(n)) *
-               esz;
+// line pitch of the tile: odd (no bank conflicts for the transposing accesses), large
+// enough to hold a padded line, since the tile is one of the two buffers the passes
+// alternate between
+__host__ __device__ constexpr int axis_pitch(int n) { return padded_line(n) | 1; }
+// shared bytes of one CTA: tables, tile, scratch tile
+__host__ __device__ constexpr size_t axis_smem_bytes(int n, int W, size_t esz) {
+    return axis_tab_bytes(n, esz) + 2 * (size_t)axis_tile_elems(n, axis_pitch(n), W) * esz;
 }
 
 size_t loop_smem_bytes(int model, int ln, int esz);

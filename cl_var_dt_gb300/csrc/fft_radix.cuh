@@ -1,4 +1,4 @@
-// fft_radix.cuh -- in-register DFT butterflies of radix 2, 3, 4, 5, 8, 12, 16 used by
+// fft_radix.cuh -- in-register DFT butterflies of radix 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16 used by
 // the shared-memory Stockham FFTs (line filter and fused step).
 //
 // Radix<C2, R>::run<S>(a) replaces a[0..R) by y_q = sum_r a_r exp(S 2 pi i r q / R)
@@ -291,6 +291,77 @@ struct Radix<C2, 5> {
     }
     static __device__ __forceinline__ void run(C2 *a, int S) {
         if (S < 0) run<-1>(a); else run<1>(a);
+    }
+};
+
+// Coprime factors N = N1 N2 without twiddles (Good-Thomas): x[(N2 n1 + N1 n2) mod N] ->
+// radix N1 over n1 (index k1) for each n2, radix N2 over n2 (index k2) ->
+// X[(E1 k1 + E2 k2) mod N] with E1 = 1 mod N1, 0 mod N2 and E2 = 0 mod N1, 1 mod N2.
+template <class C2, int N1, int N2>
+struct GoodThomas {
+    static constexpr int N = N1 * N2;
+    static constexpr int unit(int m, int other) {  // the multiple of `other` that is 1 mod m
+        int e = other;
+        while (e % m != 1) e += other;
+        return e;
+    }
+    static constexpr int E1 = unit(N1, N2), E2 = unit(N2, N1);
+    template <int S>
+    static __device__ __forceinline__ void run(C2 *a) {
+        C2 y[N2][N1];
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) {
+            C2 t[N1];
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1) t[n1] = a[(N2 * n1 + N1 * n2) % N];
+            Radix<C2, N1>::template run<S>(t);
+#pragma unroll
+            for (int k1 = 0; k1 < N1; ++k1) y[n2][k1] = t[k1];
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) {
+            C2 t[N2];
+#pragma unroll
+            for (int n2 = 0; n2 < N2; ++n2) t[n2] = y[n2][k1];
+            Radix<C2, N2>::template run<S>(t);
+#pragma unroll
+            for (int k2 = 0; k2 < N2; ++k2) a[(E1 * k1 + E2 * k2) % N] = t[k2];
+        }
+    }
+};
+template <class C2> struct Radix<C2, 6> : GoodThomas<C2, 2, 3> {};
+template <class C2> struct Radix<C2, 10> : GoodThomas<C2, 2, 5> {};
+template <class C2> struct Radix<C2, 15> : GoodThomas<C2, 3, 5> {};
+
+// 9 = 3 x 3: x[3 n1 + n2] -> radix 3 over n1 (index k1), twiddle W9^(n2 k1), radix 3 over
+// n2 (index k2) -> X[k1 + 3 k2].
+template <class C2>
+struct Radix<C2, 9> {
+    template <int S>
+    static __device__ __forceinline__ void run(C2 *a) {
+        using R = decltype(a[0].x);
+        // W9^m = (cos(2 pi m / 9), S sin(2 pi m / 9)), m = 1, 2, 4
+        const R c[3] = {(R)0.76604444311897803520, (R)0.17364817766693034885, (R)-0.93969262078590838405};
+        const R s[3] = {(R)(S * 0.64278760968653932632), (R)(S * 0.98480775301220805937), (R)(S * 0.34202014332566873304)};
+        C2 y[3][3];
+#pragma unroll
+        for (int n2 = 0; n2 < 3; ++n2) {
+            C2 t[3] = {a[n2], a[3 + n2], a[6 + n2]};
+            Radix<C2, 3>::template run<S>(t);
+#pragma unroll
+            for (int k1 = 0; k1 < 3; ++k1) y[n2][k1] = t[k1];
+        }
+        y[1][1] = cmulc(y[1][1], c[0], s[0]);
+        y[1][2] = cmulc(y[1][2], c[1], s[1]);
+        y[2][1] = cmulc(y[2][1], c[1], s[1]);
+        y[2][2] = cmulc(y[2][2], c[2], s[2]);
+#pragma unroll
+        for (int k1 = 0; k1 < 3; ++k1) {
+            C2 t[3] = {y[0][k1], y[1][k1], y[2][k1]};
+            Radix<C2, 3>::template run<S>(t);
+#pragma unroll
+            for (int k2 = 0; k2 < 3; ++k2) a[k1 + 3 * k2] = t[k2];
+        }
     }
 };
 

@@ -1,5 +1,5 @@
-// fused_impl.cuh -- the whole Langevin step of chains whose spatial slice fits in
-// shared memory, in one kernel that streams through imaginary time.
+// fused_impl.cuh -- the whole Langevin step of 1D chains of 64, 128 or 256 sites, their
+// slices in shared memory, in one kernel that streams through imaginary time.
 //
 // A CTA owns imaginary times [tau0, tau1) of one chain.  Field slices
 // (all components of one tau, contiguous in the [c][tau][x][y][z] layout) arrive
@@ -75,190 +75,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
     return false;
 }
 
-// ------------------------------------------------------- warp line filter
-// One Stockham pass of radix R over one line (length n, element stride `inner`)
-// executed by the 32 lanes of a warp.  When f != nullptr (last forward pass) the
-// output, in natural frequency order, is multiplied by f[k] * cst.
-template <class C2, class RR, int R>
-__device__ __forceinline__ void warp_pass(const C2 *s, C2 *d, int inner, int n, int Ns, int S,
-                                          const C2 *tw, const RR *f, RR cst, int lane) {
-    const int nR = n / R, tstep = n / (Ns * R);
-    for (int j = lane; j < nR; j += 32) {
-        const int k = j % Ns;
-        C2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            C2 x = s[(j + r * nR) * inner];
-            if (r > 0 && k > 0) {
-                C2 t = tw[k * r * tstep];
-                if (S > 0) t.y = -t.y;  // table holds exp(-2 pi i k/n)
-                x = vmul(x, t);
-            }
-            v[r] = x;
-        }
-        Radix<C2, R>::run(v, S);
-        const int o = (j / Ns) * Ns * R + k;
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-            const int idx = o + q * Ns;
-            C2 val = v[q];
-            if (f) val = vscale(f[idx] * cst, val);
-            d[idx * inner] = val;
-        }
-    }
-}
-
-// Filter one line in place: forward FFT, real filter, inverse FFT along the
-// line starting at buf + base.  Passes alternate buf -> tmp -> buf ...; their
-// number 2*nf is even, so the result lands back in buf.  Warp-synchronous.
-template <class C2, class RR>
-__device__ __forceinline__ void warp_line_filter(C2 *buf, C2 *tmp, int base, const AxisDev &ax,
-                                                 const C2 *tw, const RR *f, RR cst, int lane) {
-    C2 *src = buf + base, *dst = tmp + base;
-    for (int dir = 0; dir < 2; ++dir) {
-        const int S = dir == 0 ? -1 : +1;
-        int Ns = 1;
-        for (int p = 0; p < ax.nf; ++p) {
-            const int R = ax.fac[p];
-            const RR *fp = (dir == 0 && p == ax.nf - 1) ? f : nullptr;
-            switch (R) {
-                case 8: warp_pass<C2, RR, 8>(src, dst, ax.inner, ax.n, Ns, S, tw, fp, cst, lane); break;
-                case 4: warp_pass<C2, RR, 4>(src, dst, ax.inner, ax.n, Ns, S, tw, fp, cst, lane); break;
-                case 2: warp_pass<C2, RR, 2>(src, dst, ax.inner, ax.n, Ns, S, tw, fp, cst, lane); break;
-                case 3: warp_pass<C2, RR, 3>(src, dst, ax.inner, ax.n, Ns, S, tw, fp, cst, lane); break;
-                default: warp_pass<C2, RR, 5>(src, dst, ax.inner, ax.n, Ns, S, tw, fp, cst, lane); break;
-            }
-            __syncwarp();
-            C2 *t = src; src = dst; dst = t;
-            Ns *= R;
-        }
-    }
-}
-
-// ------------------------------------------------- contiguous-line fast path
-// Lines of a 1D chain are contiguous.  Intermediate layouts are padded with one
+// ---------------------------------------------------------- contiguous lines
+// Intermediate layouts are padded with one
 // spare element after every 16, which removes the shared-memory bank conflicts
 // of the strided Stockham stores.
 __device__ __forceinline__ int padi(int i) { return i + (i >> 4); }
-
-template <class C2, int R, bool PS, bool PD>
-__device__ __forceinline__ void warp_pass_1d(const C2 *s, C2 *d, int n, int Ns, int S, const C2 *tw,
-                                             int lane) {
-    const int nR = n / R, tstep = n / (Ns * R);
-    for (int j = lane; j < nR; j += 32) {
-        const int k = j % Ns;
-        C2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int idx = j + r * nR;
-            C2 x = s[PS ? padi(idx) : idx];
-            if (r > 0 && k > 0) {
-                C2 t = tw[k * r * tstep];
-                if (S > 0) t.y = -t.y;
-                x = vmul(x, t);
-            }
-            v[r] = x;
-        }
-        Radix<C2, R>::run(v, S);
-        const int o = (j / Ns) * Ns * R + k;
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-            const int idx = o + q * Ns;
-            d[PD ? padi(idx) : idx] = v[q];
-        }
-    }
-}
-
-// Last forward pass (radix R, Ns = n/R), real filter, first inverse pass
-// (radix R, Ns = 1) in registers: lane j holds frequencies j + q n/R after the
-// forward butterfly, which are exactly the inputs of its inverse butterfly.
-template <class C2, class RR, int R, bool PS, bool PD>
-__device__ __forceinline__ void warp_mid_1d(const C2 *s, C2 *d, int n, const C2 *tw, const RR *f,
-                                            RR cst, int lane) {
-    const int nR = n / R;
-    for (int j = lane; j < nR; j += 32) {
-        C2 v[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int idx = j + r * nR;
-            C2 x = s[PS ? padi(idx) : idx];
-            if (r > 0 && j > 0) x = vmul(x, tw[j * r]);
-            v[r] = x;
-        }
-        Radix<C2, R>::run(v, -1);
-        RR g[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) g[q] = f[j + q * nR] * cst;
-        radix_scaled<C2, R, 1>(v, g);
-#pragma unroll
-        for (int q = 0; q < R; ++q) {
-            const int idx = j * R + q;
-            d[PD ? padi(idx) : idx] = v[q];
-        }
-    }
-}
-
-template <class C2, bool PS, bool PD>
-__device__ __forceinline__ void pass_1d(int R, const C2 *s, C2 *d, int n, int Ns, int S,
-                                        const C2 *tw, int lane) {
-    switch (R) {
-        case 8: warp_pass_1d<C2, 8, PS, PD>(s, d, n, Ns, S, tw, lane); break;
-        case 4: warp_pass_1d<C2, 4, PS, PD>(s, d, n, Ns, S, tw, lane); break;
-        case 2: warp_pass_1d<C2, 2, PS, PD>(s, d, n, Ns, S, tw, lane); break;
-        case 3: warp_pass_1d<C2, 3, PS, PD>(s, d, n, Ns, S, tw, lane); break;
-        default: warp_pass_1d<C2, 5, PS, PD>(s, d, n, Ns, S, tw, lane); break;
-    }
-}
-template <class C2, class RR, bool PS, bool PD>
-__device__ __forceinline__ void mid_1d(int R, const C2 *s, C2 *d, int n, const C2 *tw, const RR *f,
-                                       RR cst, int lane) {
-    switch (R) {
-        case 8: warp_mid_1d<C2, RR, 8, PS, PD>(s, d, n, tw, f, cst, lane); break;
-        case 4: warp_mid_1d<C2, RR, 4, PS, PD>(s, d, n, tw, f, cst, lane); break;
-        case 2: warp_mid_1d<C2, RR, 2, PS, PD>(s, d, n, tw, f, cst, lane); break;
-        case 3: warp_mid_1d<C2, RR, 3, PS, PD>(s, d, n, tw, f, cst, lane); break;
-        default: warp_mid_1d<C2, RR, 5, PS, PD>(s, d, n, tw, f, cst, lane); break;
-    }
-}
-
-// Filter of one contiguous line: src (dense) -> ... -> out (dense).  The 2 nf - 1
-// passes alternate the padded buffers X and Y and end in X == out: out may
-// alias X and Y may alias src (src is read only by the first pass).
-template <class C2, class RR>
-__device__ __forceinline__ void warp_line_filter_1d(const C2 *src, C2 *X, C2 *Y, const AxisDev &ax,
-                                                    const C2 *tw, const RR *f, RR cst, int lane) {
-    const int n = ax.n, nf = ax.nf;
-    if (nf == 1) {
-        mid_1d<C2, RR, false, false>(ax.fac[0], src, X, n, tw, f, cst, lane);
-        __syncwarp();
-        return;
-    }
-    int Ns = 1;
-    const C2 *cur = src;
-    C2 *nxt = X, *oth = Y;
-    for (int p = 0; p < nf - 1; ++p) {
-        if (p == 0) pass_1d<C2, false, true>(ax.fac[p], cur, nxt, n, Ns, -1, tw, lane);
-        else pass_1d<C2, true, true>(ax.fac[p], cur, nxt, n, Ns, -1, tw, lane);
-        __syncwarp();
-        Ns *= ax.fac[p];
-        cur = nxt;
-        C2 *t = nxt; nxt = oth; oth = t;
-    }
-    const int Rl = ax.fac[nf - 1];
-    mid_1d<C2, RR, true, true>(Rl, cur, nxt, n, tw, f, cst, lane);
-    __syncwarp();
-    cur = nxt;
-    { C2 *t = nxt; nxt = oth; oth = t; }
-    Ns = Rl;
-    for (int p = nf - 2; p >= 0; --p) {
-        if (p == 0) pass_1d<C2, true, false>(ax.fac[p], cur, nxt, n, Ns, +1, tw, lane);
-        else pass_1d<C2, true, true>(ax.fac[p], cur, nxt, n, Ns, +1, tw, lane);
-        __syncwarp();
-        Ns *= ax.fac[p];
-        cur = nxt;
-        C2 *t = nxt; nxt = oth; oth = t;
-    }
-}
 
 // ------------------------------------ compile-time plans for power-of-two lines
 // Stockham pass with every size known at compile time (NS a power of two).
@@ -359,8 +180,10 @@ __device__ __forceinline__ void ct_inv(const C2 *&cur, C2 *&nxt, C2 *&oth, const
     }
 }
 
-// Same contract as warp_line_filter_1d for a compile-time length N = 2^k.  PT:
-// tw holds the per-pass tables (tw_*_off), else the length-N table.
+// Filter of one contiguous line of a compile-time length N = 2^k: src (dense) -> ... ->
+// out (dense).  The 2 NF - 1 passes alternate the padded buffers X and Y and end in X ==
+// out: out may alias X and Y may alias src (src is read only by the first pass).  PT: tw
+// holds the per-pass tables (tw_*_off), else the length-N table.
 template <class C2, class RR, int N, bool PT = false>
 __device__ __forceinline__ void warp_line_filter_ct(const C2 *src, C2 *X, C2 *Y, const C2 *tw,
                                                     const RR *f, RR cst, int lane) {
@@ -387,17 +210,14 @@ static_assert(tw_mid_off(256) == 56 && tw_inv_off(256, 1) == 248 && tw_inv_off(2
               tw_entries(256) == 500, "pass tables of 256");
 static_assert(tw_entries(128) == 56 + 64 + 14 + 112 && tw_entries(64) == 56 + 56, "pass-table sizes");
 
-// Contiguous-line filter: compile-time plan for the common power-of-two
-// lengths, runtime plan otherwise.
+// Contiguous-line filter of a length known at run time (the plan without per-pass tables).
 template <class C2, class RR>
-__device__ __forceinline__ void line_filter_1d(const C2 *src, C2 *X, C2 *Y, const AxisDev &ax,
-                                               const C2 *tw, const RR *f, RR cst, int lane) {
-    switch (ax.n) {
+__device__ __forceinline__ void line_filter_1d(const C2 *src, C2 *X, C2 *Y, int n, const C2 *tw, const RR *f, RR cst,
+                                               int lane) {
+    switch (n) {
         case 64: warp_line_filter_ct<C2, RR, 64>(src, X, Y, tw, f, cst, lane); break;
         case 128: warp_line_filter_ct<C2, RR, 128>(src, X, Y, tw, f, cst, lane); break;
-        case 256: warp_line_filter_ct<C2, RR, 256>(src, X, Y, tw, f, cst, lane); break;
-        case 512: warp_line_filter_ct<C2, RR, 512>(src, X, Y, tw, f, cst, lane); break;
-        default: warp_line_filter_1d<C2, RR>(src, X, Y, ax, tw, f, cst, lane); break;
+        default: warp_line_filter_ct<C2, RR, 256>(src, X, Y, tw, f, cst, lane); break;
     }
 }
 
@@ -521,71 +341,20 @@ __device__ __forceinline__ const R *filt_of(const AxisDev &ax);
 template <> __device__ __forceinline__ const double *filt_of<double>(const AxisDev &ax) { return ax.filt64; }
 template <> __device__ __forceinline__ const float *filt_of<float>(const AxisDev &ax) { return ax.filt32; }
 
-// Kinetic filter of NJ slices (slice j in buf_j, partner tmp_j; components at
-// stride cs): every warp takes whole lines, one block barrier per axis.  The
-// kinetic term ends in tmp_j for 1D chains (contiguous-line path) and in buf_j
-// otherwise.  twS/fS: shared tables.
-template <class R, int LN>
-__device__ void slices_filter(const ChainDev &ch, int ncomp, int cs, int kinetic, int NJ,
-                              typename Cx<R>::T *buf0, typename Cx<R>::T *tmp0,
-                              typename Cx<R>::T *buf1, typename Cx<R>::T *tmp1,
-                              const typename Cx<R>::T *twS, const R *fS) {
-    using C2 = typename Cx<R>::T;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    const int V = ch.V;
-    if (LN || (ch.ny == 1 && ch.nz == 1)) {
-        const AxisDev &ax = ch.axis[0];
-        const bool wc = kinetic == CLV_KIN_EXP;
-        for (int t = warp; t < NJ * ncomp; t += nwarps) {
-            const int job = t >= ncomp;
-            const int c = t - job * ncomp;
-            C2 *b = (job ? buf1 : buf0) + c * cs, *x = (job ? tmp1 : tmp0) + c * cs;
-            const R cst = wc ? (R)ch.comp_const[c] : (R)1;
-            if constexpr (LN > 0) warp_line_filter_ct<C2, R, LN>(b, x, b, twS, fS, cst, lane);
-            else line_filter_1d<C2, R>(b, x, b, ax, twS, fS, cst, lane);
-        }
-        __syncthreads();
-        return;
-    }
-    int toff = 0;
-    bool first_axis = true;
-    for (int a = 0; a < 3; ++a) {
-        const AxisDev &ax = ch.axis[a];
-        if (ax.n <= 1) continue;
-        if (kinetic == CLV_KIN_REF_LINEAR_PX && a > 0) break;
-        const int lpc = V / ax.n;
-        const int per_job = ncomp * lpc;
-        const bool wc = first_axis && kinetic == CLV_KIN_EXP;
-        for (int t = warp; t < NJ * per_job; t += nwarps) {
-            const int job = t >= per_job;
-            const int L = t - job * per_job;
-            const int c = L / lpc, l = L - c * lpc;
-            const int base = c * cs + (l / ax.inner) * ax.n * ax.inner + (l % ax.inner);
-            const R cst = wc ? (R)ch.comp_const[c] : (R)1;
-            warp_line_filter<C2, R>(job ? buf1 : buf0, job ? tmp1 : tmp0, base, ax,
-                                    twS + toff, fS + toff, cst, lane);
-        }
-        __syncthreads();
-        toff += ax.n;
-        first_axis = false;
-    }
-}
-
 // -------------------------------------------------------------- the kernel
-// SPT: lattice sites per thread (V <= 256 * SPT).  LN > 0: every chain of the
-// launch is a 1D line of LN sites (compile-time sizes and plan), LN = 0: any
-// slice shape.  FAST (LN > 0 only): the production variant -- K/max step rule,
+// One lattice site per thread.  LN: the chains' line length at compile time, 0: at run time
+// (the autotuner's alternative).  FAST (LN > 0 only): the production variant -- K/max step rule,
 // in-register Philox noise, bulk copies, no stored drift, both fields per CTA --
 // with those choices fixed at compile time, so the per-tau frame carries no
 // branches on them.
 // Per-site state carried in registers across imaginary times: psi(tau-1),
 // kin(tau-1), psibar(tau).
 
-template <class R, int MODEL, int SPT, int LN, bool FAST = false>
+template <class R, int MODEL, int LN, bool FAST = false>
 // FP64 1D lines off the production variant (the reference's step rule on few CTAs):
 // registers capped at two CTAs' worth, so that the programmatic update's CTAs (its
 // noise drawn while this pass runs) fit beside this kernel's on every SM.
-__global__ void __launch_bounds__(256, (sizeof(R) == 4 && SPT == 1) ? 3 : ((LN > 0 && !FAST) ? 2 : 1))
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : ((LN > 0 && !FAST) ? 2 : 1))
 fused_step_kernel(const LaunchFused A) {
     using C2 = typename Cx<R>::T;
     constexpr int NC = MODEL == CLV_MODEL_REF4 ? 4 : 3;
@@ -609,7 +378,6 @@ fused_step_kernel(const LaunchFused A) {
 
     const int V = LN ? LN : ch.V, T = ch.nt, cs = LN ? padded_line(LN) : A.comp_stride;
     const int TV = T * V;  // elements of one component of the chain
-    const bool kin_in_partner = LN || (ch.ny == 1 && ch.nz == 1);  // contiguous-line FFT path
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);  // NPS + NQS barriers
     C2 *twS = reinterpret_cast<C2 *>(smem + 64);
     R *fS = reinterpret_cast<R *>(smem + 64 + A.tab_n * sizeof(C2));
@@ -643,20 +411,13 @@ fused_step_kernel(const LaunchFused A) {
         for (int i = 0; i < NPS + NQS; ++i) mbar_init(&bars[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // shared copies of the twiddle and filter tables of the chain's filtered axes
+    // shared copies of the twiddle and filter tables
     {
-        int toff = 0;
-        for (int a = 0; a < 3; ++a) {
-            const AxisDev &ax = ch.axis[a];
-            if (ax.n <= 1) continue;
-            if (A.kinetic == CLV_KIN_REF_LINEAR_PX && a > 0) break;
-            const C2 *tw = tw_of<R>(ax);
-            const R *f = filt_of<R>(ax);
-            for (int i = threadIdx.x; i < ax.n; i += blockDim.x) {
-                twS[toff + i] = tw[i];
-                fS[toff + i] = f[i];
-            }
-            toff += ax.n;
+        const C2 *tw = tw_of<R>(ch.axis[0]);
+        const R *f = filt_of<R>(ch.axis[0]);
+        for (int i = threadIdx.x; i < V; i += blockDim.x) {
+            twS[i] = tw[i];
+            fS[i] = f[i];
         }
         if constexpr (LN > 0) {
             const C2 *pt = ptw_of<R>(ch.axis[0]);
@@ -703,7 +464,7 @@ fused_step_kernel(const LaunchFused A) {
 
     const int tau0 = task.tau0, tau1 = task.tau1;
     const int last_psi = MODEL == CLV_MODEL_REF4 ? tau1 : tau1 - 1;  // last psi time read
-    C2 Pp[SPT][NC], Kp[SPT][NC], Qc[SPT][NC];  // psi(tau-1), kin(tau-1), psibar(tau)
+    C2 Pp[NC], Kp[NC], Qc[NC];  // psi(tau-1), kin(tau-1), psibar(tau)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = FAST ? 8 : blockDim.x >> 5;
     // 1D chains: one warp per line (2 NC lines); the remaining warps draw the
     // Philox noise of the imaginary time into shared memory meanwhile: at FP32 every
@@ -712,14 +473,13 @@ fused_step_kernel(const LaunchFused A) {
     // first pair only (8 % faster than all three).
     constexpr int SMEM_PAIRS = (NC == 3 && sizeof(R) == 8) ? 1 : (NC + 1) / 2;
     const bool noise_smem =
-        kin_in_partner && writes && (FAST || A.noise == CLV_NOISE_PHILOX) && 2 * NC < nwarps;
-    const AxisDev &ax0 = ch.axis[0];
+        writes && (FAST || A.noise == CLV_NOISE_PHILOX) && 2 * NC < nwarps;
     const bool wc = A.kinetic == CLV_KIN_EXP;
     // kinetic filter of component c of a 1D slice: src (read only) -> X, scratch Y
     auto line1d = [&](const C2 *src, C2 *X, C2 *Y, int c) {
         const R cst = wc ? (R)ch.comp_const[c] : (R)1;
         if constexpr (LN > 0) warp_line_filter_ct<C2, R, LN, true>(src + c * cs, X + c * cs, Y + c * cs, twT, fS, cst, lane);
-        else line_filter_1d<C2, R>(src + c * cs, X + c * cs, Y + c * cs, ax0, twS, fS, cst, lane);
+        else line_filter_1d<C2, R>(src + c * cs, X + c * cs, Y + c * cs, V, twS, fS, cst, lane);
     };
     // FP64 lines of 256 sites when a CTA filters at most four lines per imaginary time
     // (the chunks split by field and component halves of the few-CTA problems, e.g. the
@@ -759,33 +519,18 @@ fused_step_kernel(const LaunchFused A) {
     wait_slot(0);
     wait_slot(NPS);
     __syncthreads();
+    const int s = threadIdx.x;
+    if (s < V)
 #pragma unroll
-    for (int k = 0; k < SPT; ++k) {
-        const int s = threadIdx.x + k * 256;
-        if (s < V)
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                Pp[k][c] = slot(0)[c * cs + s];
-                Qc[k][c] = slot(NPS)[c * cs + s];
-            }
-    }
-    if (kin_in_partner) {
-        filter_lines(do_psi ? cmask & ((1 << NC) - 1) : 0, slot(0), part0, ybuf0, nullptr, nullptr, nullptr);
-        __syncthreads();
-    } else {
-        __syncthreads();
-        if (do_psi) slices_filter<R, LN>(ch, NC, cs, A.kinetic, 1, slot(0), part0, nullptr, nullptr, twS, fS);
-    }
-    {
-        const C2 *kin0 = kin_in_partner ? part0 : slot(0);
-#pragma unroll
-        for (int k = 0; k < SPT; ++k) {
-            const int s = threadIdx.x + k * 256;
-            if (s < V)
-#pragma unroll
-                for (int c = 0; c < NC; ++c) Kp[k][c] = kin0[c * cs + s];
+        for (int c = 0; c < NC; ++c) {
+            Pp[c] = slot(0)[c * cs + s];
+            Qc[c] = slot(NPS)[c * cs + s];
         }
-    }
+    filter_lines(do_psi ? cmask & ((1 << NC) - 1) : 0, slot(0), part0, ybuf0, nullptr, nullptr, nullptr);
+    __syncthreads();
+    if (s < V)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) Kp[c] = part0[c * cs + s];
     __syncthreads();
     if (!abort_cta) {  // a CTA whose prologue copy timed out issues nothing more and leaves
         for (int i = 0; i < NPS; ++i)
@@ -795,18 +540,15 @@ fused_step_kernel(const LaunchFused A) {
     }
 
     // step-rule reduction in the working precision per thread (the max is exact;
-    // the REF mean sums at most SPT * (tau1 - tau0) values), FP64 across the CTA
+    // the REF mean sums at most tau1 - tau0 values), FP64 across the CTA
     R mxr = 0, smr = 0;
     int bad = 0;
     const DriftConsts<R> dk(ch);
     // FP64: the pair (psibar(tau), psi(tau-1)) carried from the previous imaginary time (44
     // of the site's 740 FP64 operations; FP32 recomputes it: the registers cost occupancy)
     constexpr bool kCarry = FAST && MODEL == CLV_MODEL_SPIN1 && sizeof(R) == 8;
-    Spin1Link<C2> link[kCarry ? SPT : 1];
-    if constexpr (kCarry) {
-#pragma unroll
-        for (int k = 0; k < SPT; ++k) link[k] = spin1_link<R>(dk, Qc[k], Pp[k]);
-    }
+    Spin1Link<C2> link;
+    if constexpr (kCarry) link = spin1_link<R>(dk, Qc, Pp);
     const uint64_t seed = ch.seed;
     const int ref_rule = !FAST && A.dt_rule == CLV_DT_REF_MEANMAX;
     int ia = 0, ic = 0;  // ring positions of psi(tau) and psibar(tau+1)
@@ -824,21 +566,8 @@ fused_step_kernel(const LaunchFused A) {
             if (tau - 1 + NPS <= last_psi) issue(fp, gpsi, tau - 1 + NPS);
             if (tau + NQS <= tau1) issue(fq, gpsic, tau + NQS);
         }
-        C2 vpc[SPT][NC], vcp[SPT][NC], vpp[SPT][NC];
-        auto read_fields = [&]() {
-#pragma unroll
-            for (int k = 0; k < SPT; ++k) {
-                const int s = threadIdx.x + k * 256;
-                if (s < V)
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        vpc[k][c] = slot(sp)[c * cs + s];
-                        vcp[k][c] = slot(sq)[c * cs + s];
-                        if (MODEL == CLV_MODEL_REF4) vpp[k][c] = slot(spp)[c * cs + s];
-                    }
-            }
-        };
-        if (kin_in_partner) {
+        C2 vpc[NC], vcp[NC], vpp[NC];
+        {
             // kin(tau) -> part0, kinbar(tau+1) -> part1; the field slots stay intact
             // (kin(tau) only feeds the next imaginary time: the chunk's last skips it)
             if (warp < 2 * NC || (kPairLines && !noise_smem)) {
@@ -897,43 +626,31 @@ fused_step_kernel(const LaunchFused A) {
                     }
                 }
             }
-            __syncthreads();
-            read_fields();
-        } else {
-            read_fields();
-            __syncthreads();
-            // in place: kin(tau) into the psi(tau) slot, kinbar(tau+1) into the psibar(tau+1) slot
-            // (the chunk's last imaginary time needs kinbar(tau+1) only)
-            const bool kin_psi = do_psi && tau + 1 < tau1;
-            if (kin_psi && do_bar)
-                slices_filter<R, LN>(ch, NC, cs, A.kinetic, 2, slot(sp), part0, slot(sq), part1, twS, fS);
-            else if (do_bar)
-                slices_filter<R, LN>(ch, NC, cs, A.kinetic, 1, slot(sq), part1, nullptr, nullptr, twS, fS);
-            else if (kin_psi)
-                slices_filter<R, LN>(ch, NC, cs, A.kinetic, 1, slot(sp), part0, nullptr, nullptr, twS, fS);
         }
-        const C2 *kinb = kin_in_partner ? part0 : slot(sp);   // kin(tau)
-        const C2 *kinq = kin_in_partner ? part1 : slot(sq);   // kinbar(tau+1)
+        __syncthreads();
+        if (s < V) {
 #pragma unroll
-        for (int k = 0; k < SPT; ++k) {
-            const int s = threadIdx.x + k * 256;
-            if (s >= V) continue;
+            for (int c = 0; c < NC; ++c) {
+                vpc[c] = slot(sp)[c * cs + s];
+                vcp[c] = slot(sq)[c * cs + s];
+                if (MODEL == CLV_MODEL_REF4) vpp[c] = slot(spp)[c * cs + s];
+            }
             C2 kp[NC], K[NC], Kc[NC];
             if (!FAST && side) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) K[c] = Kc[c] = mk<C2>(0.0, 0.0);
             }
 #pragma unroll
-            for (int c = 0; c < NC; ++c) kp[c] = kinq[c * cs + s];
+            for (int c = 0; c < NC; ++c) kp[c] = part1[c * cs + s];
             if (MODEL == CLV_MODEL_REF4)
-                drift_ref4_vals<R>(dk, Pp[k], vpc[k], vpp[k], Qc[k], vcp[k], Kp[k], kp, K, Kc,
+                drift_ref4_vals<R>(dk, Pp, vpc, vpp, Qc, vcp, Kp, kp, K, Kc,
                                    FAST ? 3 : (do_psi ? 1 : 0) | (do_bar ? 2 : 0), cmask);
             else if constexpr (kCarry) {
-                spin1_drift_psi<R>(link[k], Pp[k], vpc[k], Kp[k], K);
-                link[k] = spin1_link<R>(dk, vcp[k], vpc[k]);
-                spin1_drift_bar<R>(link[k], vcp[k], Qc[k], kp, Kc);
+                spin1_drift_psi<R>(link, Pp, vpc, Kp, K);
+                link = spin1_link<R>(dk, vcp, vpc);
+                spin1_drift_bar<R>(link, vcp, Qc, kp, Kc);
             } else
-                drift_spin1_vals<R>(dk, Pp[k], vpc[k], Qc[k], vcp[k], Kp[k], kp, K, Kc,
+                drift_spin1_vals<R>(dk, Pp, vpc, Qc, vcp, Kp, kp, K, Kc,
                                     FAST ? 3 : (do_psi ? 1 : 0) | (do_bar ? 2 : 0));
             if (!FAST && A.mode == FUSED_MAXONLY && A.drift_out) {
                 // the apply step reads the drift instead of recomputing filter and drift
@@ -1003,16 +720,16 @@ fused_step_kernel(const LaunchFused A) {
                         zz.y = mul_rn<R>(sd, z[u].y);
                         const int gi = cc * TV + tau * V + s;  // < 2^31 (plan_fused)
                         if (!own(cc)) continue;
-                        if (do_psi) opsi[gi] = langevin_update<R>(vpc[k][cc], K[cc], dt, zz, false);
-                        if (do_bar) opsic[gi] = langevin_update<R>(Qc[k][cc], Kc[cc], dt, zz, true);
+                        if (do_psi) opsi[gi] = langevin_update<R>(vpc[cc], K[cc], dt, zz, false);
+                        if (do_bar) opsic[gi] = langevin_update<R>(Qc[cc], Kc[cc], dt, zz, true);
                     }
                 }
             }
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                Pp[k][c] = vpc[k][c];
-                Kp[k][c] = kinb[c * cs + s];
-                Qc[k][c] = vcp[k][c];
+                Pp[c] = vpc[c];
+                Kp[c] = part0[c * cs + s];
+                Qc[c] = vcp[c];
             }
         }
         ia = (ia + 1) % NPS;
@@ -1071,25 +788,23 @@ fused_step_kernel(const LaunchFused A) {
 }
 
 // Kernel pointer of one instantiation (defined in k_fused_<precision>_<model>.cu).
-void *fused_kernel_f32_ref4(int spt, int ln, bool fast);
-void *fused_kernel_f32_spin1(int spt, int ln, bool fast);
-void *fused_kernel_f64_ref4(int spt, int ln, bool fast);
-void *fused_kernel_f64_spin1(int spt, int ln, bool fast);
+void *fused_kernel_f32_ref4(int ln, bool fast);
+void *fused_kernel_f32_spin1(int ln, bool fast);
+void *fused_kernel_f64_ref4(int ln, bool fast);
+void *fused_kernel_f64_spin1(int ln, bool fast);
 
 template <class R, int MODEL>
-void *fused_fn(int spt, int ln, bool fast) {
+void *fused_fn(int ln, bool fast) {
     switch (ln) {
-        case 64: return fast ? (void *)fused_step_kernel<R, MODEL, 1, 64, true>
-                             : (void *)fused_step_kernel<R, MODEL, 1, 64>;
-        case 128: return fast ? (void *)fused_step_kernel<R, MODEL, 1, 128, true>
-                              : (void *)fused_step_kernel<R, MODEL, 1, 128>;
-        case 256: return fast ? (void *)fused_step_kernel<R, MODEL, 1, 256, true>
-                              : (void *)fused_step_kernel<R, MODEL, 1, 256>;
+        case 64: return fast ? (void *)fused_step_kernel<R, MODEL, 64, true>
+                             : (void *)fused_step_kernel<R, MODEL, 64>;
+        case 128: return fast ? (void *)fused_step_kernel<R, MODEL, 128, true>
+                              : (void *)fused_step_kernel<R, MODEL, 128>;
+        case 256: return fast ? (void *)fused_step_kernel<R, MODEL, 256, true>
+                              : (void *)fused_step_kernel<R, MODEL, 256>;
         default: break;
     }
-    if (spt == 1) return (void *)fused_step_kernel<R, MODEL, 1, 0>;
-    if (spt == 2) return (void *)fused_step_kernel<R, MODEL, 2, 0>;
-    return (void *)fused_step_kernel<R, MODEL, 4, 0>;
+    return (void *)fused_step_kernel<R, MODEL, 0>;
 }
 
 }  // namespace clv

@@ -19,12 +19,11 @@
 //   tile never round-trips through separate load and store phases.
 // * Otherwise lines that are neighbours in memory are loaded with W-wide coalesced
 //   rows and transposed into shared memory (for the innermost axis the tile is one
-//   contiguous block).  For the common line lengths the whole CTA runs the Stockham
+//   contiguous block).  The whole CTA runs the Stockham
 //   passes of all the tile's lines together (compile-time mixed-radix plan; the last
 //   forward radix, the filter and the first inverse radix fused in registers; a
-//   scratch tile), the last inverse pass writing back into the tile; other lengths
-//   use a runtime plan with one warp per line.  The tile is stored with the same
-//   coalesced rows.
+//   scratch tile).  The tile is stored with the same coalesced rows.  (Other lengths, and
+//   slices small enough to be kept whole, take the tile filter, k_tile.cuh.)
 // Tile lines are kept at an odd pitch, so line-wise reads and transposing stores are
 // free of bank conflicts; every element is read once and written once per axis.
 #include "clv_internal.cuh"
@@ -146,21 +145,20 @@ struct AxisPlan {
     static __host__ __device__ constexpr int fac(int n, int p) { return ax_fac(n, p); }
 };
 
-// N > 0: compile-time line length (32, 64, 96, 128, 256, 512): CTA-wide passes
-// alternating between the tile and one scratch tile (both at a pitch that holds
-// a padded line), the result in the scratch tile.  N = 0: runtime plan, one warp
-// per line (per-warp scratch of two padded lines), the result back in the tile.
+// N: line length (32, 64, 96, 128, 256, 512): CTA-wide passes alternating between the tile
+// and one scratch tile (both at a pitch that holds a padded line), the result in the
+// scratch tile.
 template <class R, int N>
 __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
     using C2 = typename Cx<R>::T;
     constexpr int W = axis_tile_lines<R>(N);
-    constexpr int PER = N > 0 ? W * N / 256 : 1;  // elements per thread of a full tile
+    constexpr int PER = W * N / 256;  // elements per thread of a full tile
     extern __shared__ __align__(128) unsigned char smem[];
     const AxisTask task = A.tasks[A.nfields == 2 ? blockIdx.x >> 1 : blockIdx.x];
     const int field = A.nfields == 2 ? (int)(blockIdx.x & 1) : 0;
     const ChainDev &ch = A.chains[task.chain];
     const AxisDev &ax = ch.axis[A.axis];
-    const int n = N ? N : ax.n;
+    constexpr int n = N;
     const int PL = A.pitch, inner = ax.inner, nl = task.nl, total = nl * n;
     C2 *twS = reinterpret_cast<C2 *>(smem);
     R *fS = reinterpret_cast<R *>(smem + (size_t)n * sizeof(C2));
@@ -174,7 +172,7 @@ __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
     // the component constant goes into the CTA's filter table (a tile that runs on across
     // slices takes none)
     const R cst = A.with_const ? (R)ch.comp_const[task.slice / ch.nt] : (R)1;
-    if constexpr (N > 0) {
+    {
         if (inner > 1 && nl == W) {
             // in place: element a of tile line w at tile[w * PL + a], in global memory at
             // base + w + a * inner
@@ -202,7 +200,7 @@ __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
             return;
         }
     }
-    if (N > 0 && nl == W) {
+    if (nl == W) {
         // full tile: every load of the thread in flight before the first store
         C2 v[PER];
 #pragma unroll
@@ -235,22 +233,8 @@ __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
         }
     }
     __syncthreads();
-    const int px = padded_line(n);
-    const C2 *res = tile;  // dense result lines at pitch PL
-    if constexpr (N > 0) {
-        cta_lines_filter<C2, R, N>(tile, scr, PL, nl, twS, fS);
-        res = scr;
-    } else {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-        C2 *scrX = scr + 2 * px * warp, *scrY = scrX + px;
-        for (int w = warp; w < nl; w += nwarps) {
-            C2 *line = tile + w * PL;
-            warp_line_filter_1d<C2, R>(line, scrX, scrY, ax, twS, fS, (R)1, lane);
-            for (int i = lane; i < n; i += 32) line[i] = scrX[i];
-            __syncwarp();
-        }
-        __syncthreads();
-    }
+    cta_lines_filter<C2, R, N>(tile, scr, PL, nl, twS, fS);
+    const C2 *res = scr;  // dense result lines at pitch PL
     const bool acc = A.accumulate != 0;
     if (inner == 1) {
         for (int e = threadIdx.x; e < total; e += blockDim.x) {
@@ -320,14 +304,14 @@ static const void *axis_kernel_ptr(int n) {
         case 128: return (const void *)axis_filter_kernel<R, 128>;
         case 256: return (const void *)axis_filter_kernel<R, 256>;
         case 512: return (const void *)axis_filter_kernel<R, 512>;
-        default: return (const void *)axis_filter_kernel<R, 0>;
+        default: return nullptr;
     }
 }
 
 template <class R>
 cudaError_t setup_axis_filter(int n, size_t smem_bytes, int *ctas_per_sm) {
     const void *fn = axis_kernel_ptr<R>(n);
-    // the runtime-plan kernel serves every other line length: keep the largest request
+    if (!fn) return cudaErrorInvalidValue;
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, fn);
     if (e != cudaSuccess) return e;
@@ -345,6 +329,7 @@ cudaError_t launch_axis_filter(const LaunchAxis &L, cudaStream_t s) {
     if (sizeof(R) == 4 && L.n == 64 && L.strided)
         return cudaLaunchKernel((const void *)axis_line_kernel<64>, dim3(L.ntasks), dim3(32 * L.nfields), args, 0, s);
     const void *fn = axis_kernel_ptr<R>(L.n);
+    if (!fn) return cudaErrorInvalidValue;
     return cudaLaunchKernel(fn, dim3(L.nfields * L.ntasks), dim3(256), args, L.smem_bytes, s);
 }
 

@@ -6,10 +6,10 @@
 namespace clv {
 
 template <class R>
-static void *fused_kernel_of(int model, int spt, int ln, bool fast) {
+static void *fused_kernel_of(int model, int ln, bool fast) {
     if (sizeof(R) == 4)
-        return model == CLV_MODEL_REF4 ? fused_kernel_f32_ref4(spt, ln, fast) : fused_kernel_f32_spin1(spt, ln, fast);
-    return model == CLV_MODEL_REF4 ? fused_kernel_f64_ref4(spt, ln, fast) : fused_kernel_f64_spin1(spt, ln, fast);
+        return model == CLV_MODEL_REF4 ? fused_kernel_f32_ref4(ln, fast) : fused_kernel_f32_spin1(ln, fast);
+    return model == CLV_MODEL_REF4 ? fused_kernel_f64_ref4(ln, fast) : fused_kernel_f64_spin1(ln, fast);
 }
 
 // The production variant (fused_step_kernel's FAST) serves launches that use
@@ -22,7 +22,7 @@ static bool fused_fast(const LaunchFused &L) {
 template <class R>
 cudaError_t launch_fused(const LaunchFused &L, cudaStream_t s) {
     if (L.ntasks == 0) return cudaSuccess;
-    void *fn = fused_kernel_of<R>(L.model, L.spt, L.ln, fused_fast(L));
+    void *fn = fused_kernel_of<R>(L.model, L.ln, fused_fast(L));
     void *args[] = {const_cast<LaunchFused *>(&L)};
     return cudaLaunchKernel(fn, dim3(L.ntasks), dim3(256), args, L.smem_bytes, s);
 }
@@ -37,7 +37,7 @@ cudaError_t setup_fused(const LaunchFused &L, int *ctas_per_sm) {
     if (e != cudaSuccess) return e;
     void *fn = nullptr;
     for (int fast = 0; fast < (L.ln > 0 ? 2 : 1); ++fast) {
-        fn = fused_kernel_of<R>(L.model, L.spt, L.ln, fast != 0);
+        fn = fused_kernel_of<R>(L.model, L.ln, fast != 0);
         cudaFuncAttributes fa{};
         e = cudaFuncGetAttributes(&fa, fn);
         if (e == cudaSuccess)

@@ -1,0 +1,7 @@
+// tile_filter_kernel<double> (k_tile.cuh).
+#include "k_tile.cuh"
+
+namespace clv {
+template cudaError_t setup_tile_filter<double>(size_t, int *);
+template cudaError_t launch_tile_filter<double>(const LaunchTileFilter &, cudaStream_t);
+}  // namespace clv

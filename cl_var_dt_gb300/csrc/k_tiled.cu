@@ -2,8 +2,8 @@
 // fused kernel, after the kinetic terms have been filtered along every axis
 // (k_axis.cu writes kin = e^{-eps H_kin} psi and kinbar for all imaginary times).
 //
-// A CTA owns 256 consecutive spatial sites of one chain (one thread per site)
-// and streams through imaginary times [tau0, tau1).  psi(tau-1), psi(tau),
+// A thread owns one spatial site of one chain over a chunk of imaginary times
+// [tau0, tau1) and streams through it; a CTA takes 256 consecutive (chunk, site) pairs.  psi(tau-1), psi(tau),
 // kin(tau-1) and psibar(tau) are carried in registers from the previous tau;
 // each iteration loads psi(tau+1), psibar(tau+1), kin(tau) and kinbar(tau+1),
 // prefetched one tau ahead, so every array is read once per step (plus one halo
@@ -36,7 +36,7 @@ __device__ __forceinline__ void normal_pair(uint64_t seed, uint32_t chain, uint6
 }
 
 
-// One task: imaginary times [tau0, tau1) of 256 sites of one chain.
+// One task: 256 consecutive (chunk, site) pairs of one chain.
 template <class R, int MODEL>
 __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask task) {
     using C2 = typename Cx<R>::T;
@@ -46,8 +46,9 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
     if (A.mode == FUSED_APPLY && A.only_rejected && st->accepted) return;  // uniform per CTA
 
     const int V = ch.V, T = ch.nt;
-    const int s = task.site0 + threadIdx.x;
-    const bool act = s < V;
+    const int flat = task.flat0 + threadIdx.x;
+    const int chunk = flat / V, s = flat - chunk * V;
+    const bool act = chunk < task.nchunk;
     const C2 *gpsi = reinterpret_cast<const C2 *>(A.psi_in) + ch.off;
     const C2 *gpsic = reinterpret_cast<const C2 *>(A.psic_in) + ch.off;
     const C2 *gkin = reinterpret_cast<const C2 *>(A.kin) + ch.off;
@@ -67,7 +68,7 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
         return ((long long)c * T + t) * V + s;
     };
     const DriftConsts<R> dk(ch);
-    const int tau0 = task.tau0, tau1 = task.tau1;
+    const int tau0 = (int)((long long)T * chunk / task.nchunk), tau1 = (int)((long long)T * (chunk + 1) / task.nchunk);
     // carried: psi(tau-1), kin(tau-1), psibar(tau), psi(tau)
     C2 Pp[NC], Kp[NC], Qc[NC], Pc[NC];
     Spin1Link<C2> Bm;  // spin-1: the pair (psibar(tau), psi(tau-1)), carried

@@ -1,0 +1,100 @@
+"""The tile filter (csrc/k_tile.cuh) and the flattened step tasks: lines of every radix,
+whole small slices, strided and contiguous tiles with remainders, mixed batches; steps and
+observables against the FP64 oracle."""
+import numpy as np
+import pytest
+from conftest import rel_err
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def clv():
+    import cl_var_dt_gb300 as m
+    m.build()
+    return m
+
+
+def spin1(clv, **kw):
+    base = dict(nx=60, ny=1, nz=1, nt=6, eps=0.05, mu=0.8, c0=0.3, c1=-0.05, q=0.02, K=0.05, dt_max=1e-3, seed=12)
+    base.update(kw)
+    return clv.ChainParams(**base)
+
+
+def oracle_params(oracle, c):
+    return oracle.spin1_params(nx=c.nx, ny=c.ny, nz=c.nz, nt=c.nt, eps=c.eps, mu=c.mu, c0=c.c0, c1=c.c1, q=c.q,
+                               Kc=c.K, dt_max=c.dt_max)
+
+
+# every radix alone and in two and three passes; slices of one and several per tile; tiles
+# of lines with remainders (a last strided tile of one column: 81 = 5 x 16 + 1 at FP64)
+SHAPES = [dict(nx=n, nt=5) for n in (2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 25, 27, 30, 45, 48, 50, 60, 81, 90,
+                                     100, 135, 144, 150, 200, 225, 240, 250, 360, 375, 400, 480, 500)] + [
+    dict(nx=30, ny=30, nt=7), dict(nx=24, ny=20, nt=5), dict(nx=2, ny=2, nt=2), dict(nx=100, ny=81, nt=2),
+    dict(nx=100, ny=100, nt=2), dict(nx=8, ny=6, nz=4, nt=9), dict(nx=20, ny=18, nz=15, nt=3),
+    dict(nx=6, ny=1, nz=10, nt=4), dict(nx=48, ny=20, nz=15, nt=2), dict(nx=3, ny=160, nz=50, nt=2)]
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda d: "x".join(str(v) for v in d.values()))
+def test_spin1_step_and_observables(clv, oracle, shape, prec):
+    c = spin1(clv, **shape)
+    p = oracle_params(oracle, c)
+    tol = 1e-12 if prec == "f64" else 1e-5
+    with clv.Engine(c, model=clv.MODEL_SPIN1, precision=clv.PREC_F64 if prec == "f64" else clv.PREC_F32) as e:
+        assert e.plan()[0] == "tiled"
+        e.init_spin1()
+        psi, psic = oracle.spin1_init(p, c.seed, 0)
+        e.step(1)
+        psi, psic, dt, _, _ = oracle.step(p, psi, psic, seed=c.seed, chain=0, step_index=0)
+        gp, gc = e.get_fields(0)
+        assert rel_err(gp, psi) < tol and rel_err(gc, psic) < tol
+        assert abs(e.step_info()["dt"][0] - dt) <= tol * dt
+        e.evaluate()
+        want, got = oracle.spin1_observables(p, gp, gc), e.spin1_samples(0)[0]
+        assert np.max(np.abs(got - want)) < tol * max(1.0, float(np.max(np.abs(want))))
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("chunk", [None, "1", "4"])
+def test_mixed_batch(clv, oracle, monkeypatch, prec, chunk):
+    """Shapes of different kinds in one engine; chains whose (chunk, site) pairs end inside a CTA."""
+    if chunk:
+        monkeypatch.setenv("CLV_CHUNK", chunk)
+    shapes = [dict(nx=60, nt=25), dict(nx=128, nt=8), dict(nx=30, ny=30, nt=5), dict(nx=24, ny=20, nt=9),
+              dict(nx=500, nt=3), dict(nx=64, ny=64, nt=2), dict(nx=100, ny=128, nt=2), dict(nx=2, nt=2)]
+    chains = [spin1(clv, mu=0.4 + 0.1 * i, seed=3 + i, **s) for i, s in enumerate(shapes)]
+    tol = 1e-12 if prec == "f64" else 1e-5
+    with clv.Engine(chains, model=clv.MODEL_SPIN1, precision=clv.PREC_F64 if prec == "f64" else clv.PREC_F32) as e:
+        e.init_spin1()
+        e.step(1)
+        for i, c in enumerate(chains):
+            p = oracle_params(oracle, c)
+            psi, psic = oracle.spin1_init(p, c.seed, i)
+            psi, psic, _, _, _ = oracle.step(p, psi, psic, seed=c.seed, chain=i, step_index=0)
+            gp, gc = e.get_fields(i)
+            assert rel_err(gp, psi) < tol and rel_err(gc, psic) < tol, shapes[i]
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [dict(nx=48, ny=10, nz=9, nt=4), dict(nx=90, nt=6), dict(nx=48, ny=40, nz=6, nt=2)],
+                         ids=lambda d: "x".join(str(v) for v in d.values()))
+def test_ref4_tile_filter_equals_line_filter(clv, monkeypatch, shape, prec):
+    """The reference's kinetic term (x axis only) by the tile filter and by the separate
+    line-filter, drift and update kernels."""
+    c = clv.ChainParams(**shape, eps=0.02, a_x=1.0, G=0.1, Q=0.02, P=0.05, mu=-0.5, DT=0.002, seed=7)
+    rng = np.random.default_rng(5)
+    out = []
+    for env in (None, "0"):
+        if env:
+            monkeypatch.setenv("CLV_FUSED", env)
+            monkeypatch.setenv("CLV_TILED", env)
+        with clv.Engine(c, model=clv.MODEL_REF4, precision=clv.PREC_F64 if prec == "f64" else clv.PREC_F32) as e:
+            assert e.plan()[0] == ("unfused" if env else "tiled")
+            if not out:
+                f = (rng.standard_normal(e.shape(0)) + 1j * rng.standard_normal(e.shape(0))) * 0.3 + 0.5
+            e.set_fields(0, f, np.conj(f))
+            e.step(3)
+            out.append(e.get_fields(0))
+    tol = 1e-13 if prec == "f64" else 2e-6
+    assert rel_err(out[0][0], out[1][0]) < tol and rel_err(out[0][1], out[1][1]) < tol
