@@ -204,13 +204,44 @@ __device__ __forceinline__ C2 langevin_update(C2 p, C2 K, R dt, C2 z, bool conj)
     return o;
 }
 
-// Maximum that is NaN when either argument is (max.NaN.f32), so a reduction of
-// |drift|^2 carries a non-finite drift to the chain's finish by itself.
+// Maximum of values that are not negative or NaN, NaN when either argument is, so that a
+// reduction of |drift| carries a non-finite drift to the chain's finish by itself.  FP64
+// compares the bit patterns as integers (ordered alike, NaN above infinity): no operation
+// on the FP64 pipe.
 __device__ __forceinline__ float max_nan(float a, float b) {
     float r;
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
+__device__ __forceinline__ double max_nan(double a, double b) {
+    const unsigned long long x = (unsigned long long)__double_as_longlong(a), y = (unsigned long long)__double_as_longlong(b);
+    return __longlong_as_double((long long)(x > y ? x : y));
+}
+
+// |z| of a drift value for the reference's rule.  FP64: the library's hypot takes about 60
+// operations of the FP64 pipe, as many as a third of the drift; between 2^-511 and 2^497
+// the sum of squares neither overflows nor underflows, and its root takes five (a single-
+// precision reciprocal root of the mantissa, its bits moved by integer operations, and two
+// Newton steps on the root with the residual formed by a fused multiply-add): within 1.1
+// units in the last place.
+__device__ __forceinline__ float abs_drift(float2 z) { return hypotf(z.x, z.y); }
+__device__ __forceinline__ double abs_drift(double2 z) {
+    const unsigned hx = (unsigned)__double2hiint(z.x) & 0x7fffffffu, hy = (unsigned)__double2hiint(z.y) & 0x7fffffffu;
+    if ((hx > hy ? hx : hy) - 0x20000000u >= 0x3f000000u) return hypot(z.x, z.y);
+    const double s = __fma_rn(z.x, z.x, __dmul_rn(z.y, z.y));
+    // s = m 4^k, 1 <= m < 4
+    const int hs = __double2hiint(s), k = ((hs >> 20) - 1023) >> 1, hm = hs - (k << 21), lo = __double2loint(s);
+    const double m = __hiloint2double(hm, lo);
+    const float y = rsqrtf(__int_as_float(((hm - 0x38000000) << 3) | (int)((unsigned)lo >> 29)));
+    const int yb = __float_as_int(y), yh = (yb >> 3) + 0x38000000, yl = (int)((unsigned)yb << 29);
+    const double y0 = __hiloint2double(yh, yl), h = __hiloint2double(yh - 0x00100000, yl);  // y, y / 2
+    double g = __dmul_rn(m, y0);
+    g = __fma_rn(__fma_rn(-g, g, m), h, g);
+    g = __fma_rn(__fma_rn(-g, g, m), h, g);
+    return __hiloint2double(__double2hiint(g) + (k << 20), __double2loint(g));
+}
+__device__ __forceinline__ bool not_finite(float a) { return !isfinite(a); }
+__device__ __forceinline__ bool not_finite(double a) { return ((unsigned)__double2hiint(a) & 0x7ff00000u) == 0x7ff00000u; }
 
 // Block-wide (max, sum) with warp shuffles; result valid in thread 0.
 __device__ __forceinline__ void block_max_sum(double &mx, double &sm) {

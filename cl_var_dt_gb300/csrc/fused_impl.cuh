@@ -665,24 +665,15 @@ fused_step_kernel(const LaunchFused A) {
             if (A.mode != FUSED_APPLY) {
                 if (ref_rule) {
                     if (own(0)) {  // (a psibar CTA's K is zero)
-                        const R a0 = hypot(K[0].x, K[0].y);
-                        mxr = fmax(mxr, a0);
+                        const R a0 = abs_drift(K[0]);
+                        mxr = max_nan(mxr, a0);
                         smr += a0;
-                        bad |= !isfinite(a0);
+                        bad |= not_finite(a0);
                     }
                 } else {
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        if (!own(c)) continue;
-                        const R m1 = abs2<R>(K[c]);
-                        const R m2 = abs2<R>(Kc[c]);
-                        if constexpr (sizeof(R) == 4) {
-                            mxr = max_nan(mxr, max_nan(m1, m2));  // a NaN reaches the finish
-                        } else {
-                            mxr = fmax(mxr, fmax(m1, m2));
-                            smr += m1 + m2;  // unused by the rule; carries a NaN to the finish
-                        }
-                    }
+                    for (int c = 0; c < NC; ++c)
+                        if (own(c)) mxr = max_nan(mxr, max_nan(abs2<R>(K[c]), abs2<R>(Kc[c])));
                 }
             }
             if (writes) {

@@ -221,25 +221,17 @@ __global__ void __launch_bounds__(256, 1) loop_step_kernel(const LaunchLoop A) {
                 drift_spin1_vals<R>(dk, pm, pc, qc, cp, km, kp, K, Kc, do_psi ? 1 : 2);
             if (A.dt_rule == CLV_DT_REF_MEANMAX) {
                 if (own(0)) {  // (a psibar CTA's K is zero)
-                    const R a0 = hypot(K[0].x, K[0].y);
-                    mxr = fmax(mxr, a0);
+                    const R a0 = abs_drift(K[0]);
+                    mxr = max_nan(mxr, a0);
                     smr += a0;
-                    bad |= !isfinite(a0);
+                    bad |= not_finite(a0);
                 }
             } else {
                 // K/max rule: max |K|^2 over this CTA's field and components (the chain's
-                // maximum is the same whichever CTA finds it); FP64 carries a NaN in the sum
+                // maximum is the same whichever CTA finds it)
 #pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    if (!own(c)) continue;
-                    const R m = abs2<R>(do_psi ? K[c] : Kc[c]);
-                    if constexpr (sizeof(R) == 4) {
-                        mxr = max_nan(mxr, m);
-                    } else {
-                        mxr = fmax(mxr, m);
-                        smr += m;
-                    }
-                }
+                for (int c = 0; c < NC; ++c)
+                    if (own(c)) mxr = max_nan(mxr, abs2<R>(do_psi ? K[c] : Kc[c]));
             }
         }
         double mx = (double)mxr, sm = (double)smr;

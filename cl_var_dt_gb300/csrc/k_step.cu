@@ -80,10 +80,10 @@ drift_kernel(const ChainDev *__restrict__ chains, ChainState *__restrict__ state
         }
         if (RULE == CLV_DT_REF_MEANMAX) {
             // component 0 of the psi drift only (launch quirk of :363-366)
-            const double a0 = (double)hypot(K[0].x, K[0].y);
+            const double a0 = (double)abs_drift(K[0]);
             mx = a0;
             sm = a0;
-            bad = !isfinite(a0);
+            bad = not_finite(a0);
         } else {
 #pragma unroll
             for (int a = 0; a < NC; ++a) {

@@ -125,18 +125,13 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
             }
             if (A.mode != FUSED_APPLY) {
                 if (ref_rule) {
-                    const R a0 = hypot(K[0].x, K[0].y);
-                    mxr = fmax(mxr, a0);
+                    const R a0 = abs_drift(K[0]);
+                    mxr = max_nan(mxr, a0);
                     smr += a0;
-                    bad |= !isfinite(a0);
+                    bad |= not_finite(a0);
                 } else {
 #pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        const R m1 = abs2<R>(K[c]);
-                        const R m2 = abs2<R>(Kc[c]);
-                        mxr = fmax(mxr, fmax(m1, m2));
-                        smr += m1 + m2;  // unused by the rule; carries a NaN to the finish
-                    }
+                    for (int c = 0; c < NC; ++c) mxr = max_nan(mxr, max_nan(abs2<R>(K[c]), abs2<R>(Kc[c])));
                 }
             }
             if (writes) {
