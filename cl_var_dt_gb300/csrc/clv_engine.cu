@@ -786,6 +786,36 @@ void build_tiled_tasks(clv_engine *e, int L) {
     }
 }
 
+// Imaginary times per CTA of the step kernels: the chunk length whose CTAs, spread over the
+// SMs, finish soonest.  An SM's time is its share of the CTAs times a CTA's length plus the
+// halo that every chunk pays, and the share is a whole number: 192 CTAs on 152 SMs cost as
+// much as 304 (the FP64 reduce pass on 128 x 128 with chunks of 43: 1.11 ms; of 18: 0.78 ms;
+// the FP64 step of 32 chains of 256 x 128 with 320 CTAs: 1.32 ms, with 288: 1.03 ms).  width:
+// sites a CTA takes of a chunk, 0: all of them.
+int choose_chunk(const clv_engine *e, int nsm, int width, double halo) {
+    int tmax = 1;
+    double work = 0;
+    for (auto &d : e->chains_h) {
+        tmax = std::max(tmax, d.nt);
+        work += width ? (double)d.V * d.nt / width : (double)d.nt;
+    }
+    int best = 1;
+    double cost = 0;
+    for (int L = 1; L <= std::min(64, tmax); ++L) {
+        long long ctas = 0;
+        for (auto &d : e->chains_h) {
+            const long long nchunk = (d.nt + L - 1) / L;
+            ctas += width ? (d.V * nchunk + width - 1) / width : nchunk;
+        }
+        const double t = (double)((ctas + nsm - 1) / nsm) * (work / ctas + halo);
+        if (L == 1 || t < cost) {
+            best = L;
+            cost = t;
+        }
+    }
+    return best;
+}
+
 int plan_fused(clv_engine *e) {
     const char *env = std::getenv("CLV_FUSED");
     if (env && env[0] == '0') return CLV_OK;
@@ -837,12 +867,10 @@ int plan_fused(clv_engine *e) {
     else CK(setup_fused<float>(probe, &per_sm));
     if (per_sm < 1) return CLV_OK;
     e->fused_ctas_per_sm = per_sm;
-    // chunk length: about two waves of CTAs; a batch too small to fill the GPU takes
-    // one imaginary time per CTA (its halo work runs on otherwise idle SMs)
+    // chunk length: the halo of a chunk is the filter of psi(tau0 - 1) and its reads
     long long total_slices = 0;
     for (auto &d : e->chains_h) total_slices += d.nt;
-    const long long target = 2LL * per_sm * nsm;
-    int L = (int)std::max<long long>(1, (total_slices + target - 1) / target);
+    int L = choose_chunk(e, nsm, 0, 0.6);
     if (const char *cl = std::getenv("CLV_CHUNK")) L = std::max(1, atoi(cl));
     e->fused_ln_static = std::getenv("CLV_NO_STATIC_PLAN") ? 0 : ln;
     e->withhold_copy = std::getenv("CLV_TEST_WITHHOLD_COPY") != nullptr;
@@ -1121,13 +1149,11 @@ int plan_tiled(clv_engine *e) {
     if (e->precision == CLV_PREC_F64) CK(setup_tiled<double>(e->model, &occ));
     else CK(setup_tiled<float>(e->model, &occ));
     if (occ < 1) return CLV_OK;
-    // imaginary-time chunk: about one wave of CTAs, 8..64 times per CTA (longer
-    // chunks amortise the halo slice and the prologue; clv_autotune refines it);
-    // fewer for problems too small to fill the GPU
+    // chunk length: the halo of a chunk is the reads of one imaginary time, which the FP32
+    // kernel, bound by memory, pays in full (3D 64^3: 1.04 ms with 16 times a chunk, 1.00 with 64)
     long long tile_taus = 0;
     for (auto &d : e->chains_h) tile_taus += ((long long)d.V * d.nt + 255) / 256;
-    const long long Lw = tile_taus / ((long long)occ * nsm);
-    int L = (int)(Lw >= 8 ? std::min<long long>(64, Lw) : std::max<long long>(1, Lw));
+    int L = choose_chunk(e, nsm, 256, e->precision == CLV_PREC_F32 ? 2.0 : 0.6);
     if (const char *cl = std::getenv("CLV_CHUNK")) L = std::max(1, atoi(cl));
     e->task_capacity = (size_t)tile_taus;  // chunks of one imaginary time
     build_tiled_tasks(e, L);
