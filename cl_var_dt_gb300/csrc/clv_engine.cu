@@ -54,14 +54,14 @@ bool factorize(int n, int *fac, int &nf) {
     return n == 1;
 }
 
-// In-place plan of the tile filter: as few radices of 2 .. 16 as the length allows, the most
+// In-place plan of the tile filter: as few radices of 2 .. most as the length allows, the most
 // even such split, larger ones first.
-bool tile_factors(int n, int *fac, int &nf) {
+bool tile_factors(int n, int most, int *fac, int &nf) {
     static const int radices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
     if (n <= 1) return false;
     for (int want = 1; want <= kMaxTileFactors; ++want) {
         int best[kMaxTileFactors], cur[kMaxTileFactors], sum = 1 << 30;
-        auto search = [&](auto &&self, int rest, int depth, int most) -> void {
+        auto search = [&](auto &&self, int rest, int depth, int top) -> void {
             if (depth == want) {
                 int s = 0;
                 for (int i = 0; i < want; ++i) s += cur[i];
@@ -72,12 +72,12 @@ bool tile_factors(int n, int *fac, int &nf) {
                 return;
             }
             for (int r : radices)
-                if (r <= most && rest % r == 0) {
+                if (r <= top && rest % r == 0) {
                     cur[depth] = r;
                     self(self, rest / r, depth + 1, r);
                 }
         };
-        search(search, n, 0, 16);
+        search(search, n, 0, most);
         if (sum < (1 << 30)) {
             nf = want;
             std::copy(best, best + want, fac);
@@ -315,7 +315,8 @@ int build_tables(clv_engine *e) {
             table(&ax.efilt32, e32);
             // the tile filter's plan, and the filters in the order its forward passes leave
             // the frequencies: position sum_p q_p (L_p / R_p) holds sum_p q_p (R_0 ... R_{p-1})
-            if (!tile_factors(n, ax.tfac, ax.tnf)) ax.tnf = 0;
+            if (!tile_factors(n, e->precision == CLV_PREC_F64 ? tile_radix_max<double>() : tile_radix_max<float>(), ax.tfac, ax.tnf))
+                ax.tnf = 0;
             if (ax.tnf) {
                 std::vector<double> tf64(n), te64(n);
                 for (int i = 0; i < n; ++i) {
@@ -330,6 +331,10 @@ int build_tables(clv_engine *e) {
                     te64[i] = e64[k];
                 }
                 std::vector<float> tf32(tf64.begin(), tf64.end()), te32(te64.begin(), te64.end());
+                for (int k = 0; k < n; ++k) {
+                    ax.fmax = std::max(ax.fmax, std::fabs(f64[k]));
+                    ax.efmax = std::max(ax.efmax, e64[k]);
+                }
                 table(&ax.tfilt64, tf64);
                 table(&ax.tfilt32, tf32);
                 table(&ax.tefilt64, te64);
@@ -558,7 +563,7 @@ int run_groups(clv_engine *e, const std::vector<clv_engine::AxisGroup> &groups, 
             A.accumulate = energy && g.axis > 0;
             A.strided = g.strided;
             if (g.plane) CK(launch_plane_filter<R>(A, e->stream));
-            else CK(launch_axis_filter<R>(A, e->stream));
+            else if constexpr (sizeof(R) == 4) CK(launch_axis_filter<R>(A, e->stream));
         }
         if (trail) CK(trail->mark(e->stream));
     }
@@ -918,8 +923,11 @@ clv_engine::AxisGroup &tile_group(const clv_engine *e, std::vector<clv_engine::A
     return groups.back();
 }
 
-size_t tile_smem(const clv_engine *e, int elems, int nsum, int rows) {
-    return (size_t)(elems + nsum) * e->elem_bytes + (size_t)(nsum + rows) * (e->elem_bytes / 2) + 16;
+// tile, twiddles, filters, the rows' shares of summed filters, the groups' scales (FP64:
+// five words each)
+size_t tile_smem(const clv_engine *e, int elems, int nsum, int rows, int groups) {
+    return (size_t)(elems + nsum) * e->elem_bytes + (size_t)(nsum + rows) * (e->elem_bytes / 2) +
+           (e->precision == CLV_PREC_F64 ? 5 * (size_t)groups * sizeof(unsigned) : 0) + 16;
 }
 
 int tile_plan(clv_engine *e, const TileFilterPlan &p) {
@@ -955,7 +963,8 @@ int add_tile_slices(clv_engine *e, int c, bool energy, std::vector<clv_engine::A
     p.tile_elems = (ns * rows1 * p.pitch + 1) / 2 * 2;
     const int id = tile_plan(e, p);
     auto &g = tile_group(e, groups, 0, p.naxes == 1 ? d.axis[p.axis[0]].n : 0, p.naxes > 1, p.tile_elems,
-                         tile_smem(e, p.tile_elems, nsum, ns * rows1));
+                         tile_smem(e, p.tile_elems, nsum, ns * rows1,
+                                   p.naxes == 1 ? ns * d.V / d.axis[p.axis[0]].n : ns));
     for (int k = 0; k < d.ncomp; ++k)
         for (int t = 0; t < d.nt; t += ns)
             g.ttasks.push_back({c, id, k * d.nt + t, 0, std::min(ns, d.nt - t) * rows1, cols});
@@ -984,7 +993,7 @@ int add_tile_axis(clv_engine *e, int c, int a, bool energy, std::vector<clv_engi
         p.gstride = ax.inner;
         p.tile_elems = (n * p.pitch + 1) / 2 * 2;
         const int id = tile_plan(e, p);
-        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, n));
+        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, 0, W));
         for (int sl = 0; sl < d.ncomp * d.nt; ++sl)
             for (int hi = 0; hi < lines / ax.inner; ++hi)
                 for (int l = 0; l < ax.inner; l += W)
@@ -995,7 +1004,7 @@ int add_tile_axis(clv_engine *e, int c, int a, bool energy, std::vector<clv_engi
         p.pitch = n | 1;
         p.tile_elems = (W * p.pitch + 1) / 2 * 2;
         const int id = tile_plan(e, p);
-        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, W));
+        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, 0, W));
         for (int sl = 0; sl < d.ncomp * d.nt; ++sl)
             for (int l = 0; l < lines; l += W)
                 g.ttasks.push_back({c, id, sl, l * n, std::min(W, lines - l), n});
@@ -1069,12 +1078,13 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
                 continue;
             }
             const int n = ax.n, lines = d.V / n;
-            const bool ct = axis_compile_time_plan(n);
-            if (!ct) {
+            // (FP64 always: the tile filter's integer lines against butterflies bound by the FP64
+            // pipe, k_tile.cuh)
+            if (esz == 16 || !axis_compile_time_plan(n)) {
                 if (int rc = add_tile_axis(e, c, a, energy, groups)) return rc;
                 continue;
             }
-            const int W = esz == 8 ? axis_tile_lines<float>(n) : axis_tile_lines<double>(n);
+            const int W = axis_tile_lines<float>(n);
             int gi = -1;
             for (int g = 0; g < (int)groups.size(); ++g)
                 if (!groups[g].plane && !groups[g].tile && groups[g].axis == a && groups[g].n == n) gi = g;
@@ -1088,8 +1098,7 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
                 g.smem = axis_smem_bytes(n, W, esz);
                 if (g.smem + 1024 > (size_t)dev_smem) return CLV_OK;
                 int occ = 0;
-                if (e->precision == CLV_PREC_F64) CK(setup_axis_filter<double>(n, g.smem, &occ));
-                else CK(setup_axis_filter<float>(n, g.smem, &occ));
+                CK(setup_axis_filter<float>(n, g.smem, &occ));
                 if (occ < 1) return CLV_OK;
                 groups.push_back(std::move(g));
                 gi = (int)groups.size() - 1;
@@ -1116,8 +1125,8 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
     for (auto &g : groups)
         if (g.tile) {
             int occ = 0;
-            if (e->precision == CLV_PREC_F64) CK(setup_tile_filter<double>(g.smem, &occ));
-            else CK(setup_tile_filter<float>(g.smem, &occ));
+            if (e->precision == CLV_PREC_F64) CK(setup_tile_filter<double>(g.smem, g.threads, &occ));
+            else CK(setup_tile_filter<float>(g.smem, g.threads, &occ));
             if (occ < 1) return CLV_OK;
         }
     std::stable_sort(groups.begin(), groups.end(),

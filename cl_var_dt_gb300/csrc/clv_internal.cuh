@@ -12,7 +12,7 @@ namespace clv {
 
 constexpr int kMaxFactors = 16;
 constexpr int kMaxComp = 4;
-constexpr int kMaxTileFactors = 4;  // 2048 = 16 16 8
+constexpr int kMaxTileFactors = 5;  // 1875 = 5 5 5 5 3
 
 // Precision traits: R is the arithmetic type of the bulk field work.
 template <class R> struct Cx;
@@ -65,6 +65,7 @@ struct AxisDev {
     int tfac[kMaxTileFactors];
     const double *tfilt64, *tefilt64;
     const float *tfilt32, *tefilt32;
+    double fmax, efmax;  // largest magnitudes of the two filters (fft_int.cuh)
 };
 
 // Per-chain constants (device copy, read-only during steps).

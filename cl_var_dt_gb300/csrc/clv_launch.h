@@ -264,13 +264,16 @@ struct LaunchTileFilter {
     int threads;        // 128, 256 for tiles above kTileWide elements
     size_t smem_bytes;
 };
+// Largest radix of its passes: FP64 stops at 10, whose 10 elements of four words leave room
+// for five CTAs per SM (16: 168 registers, three CTAs; 128-site lines 568 against 530 us).
+template <class R> __host__ __device__ constexpr int tile_radix_max() { return sizeof(R) == 4 ? 16 : 10; }
 // Elements of a tile of lines, of a whole slice kept on chip (several CTAs per SM), and
 // where a CTA takes 256 threads instead of 128.
 template <class R> __host__ __device__ constexpr int tile_target() { return sizeof(R) == 4 ? 4096 : 2048; }
 template <class R> __host__ __device__ constexpr int tile_slice_max() { return sizeof(R) == 4 ? 12288 : 6144; }
 template <class R> __host__ __device__ constexpr int tile_wide() { return sizeof(R) == 4 ? 6144 : 3072; }
 template <class R> cudaError_t launch_tile_filter(const LaunchTileFilter &L, cudaStream_t s);
-template <class R> cudaError_t setup_tile_filter(size_t smem_bytes, int *ctas_per_sm);
+template <class R> cudaError_t setup_tile_filter(size_t smem_bytes, int threads, int *ctas_per_sm);
 
 // Step over precomputed kinetic terms: the chain's imaginary times are split into nchunk
 // chunks, and its (chunk, site) pairs, flattened, are taken 256 at a time; every thread

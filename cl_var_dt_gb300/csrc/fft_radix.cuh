@@ -7,9 +7,16 @@
 // runtime direction.
 #pragma once
 
+#include <type_traits>
+
 #include "clv_internal.cuh"
+#include "fft_int.cuh"
 
 namespace clv {
+
+// A butterfly's real constant in the arithmetic type: itself, or with 62 fraction bits.
+template <class R> __host__ __device__ constexpr R kconst(double c) { return (R)c; }
+template <> __host__ __device__ constexpr long long kconst<long long>(double c) { return (long long)(c * 4611686018427387904.0); }
 
 // S * i * z for a compile-time direction S
 template <int S, class C2>
@@ -60,6 +67,11 @@ __device__ __forceinline__ double2 vscale(double s, double2 z) { return make_dou
 __device__ __forceinline__ float2 vmul(float2 z, float2 w) { return cmul(z, w); }
 __device__ __forceinline__ double2 vmul(double2 z, double2 w) {
     return make_double2(__fma_rn(z.x, w.x, -__dmul_rn(z.y, w.y)), __fma_rn(z.x, w.y, __dmul_rn(z.y, w.x)));
+}
+// z conj(w)
+template <class C2> __device__ __forceinline__ C2 vmulc(C2 z, C2 w) {
+    w.y = -w.y;
+    return vmul(z, w);
 }
 // p = e + s z and m = e - s z for a real constant s
 __device__ __forceinline__ void vaxpy2(float2 e, float s, float2 z, float2 &p, float2 &m) {
@@ -146,7 +158,7 @@ struct Radix<C2, 8> {
     template <int S>
     static __device__ __forceinline__ void finish(C2 *a, const C2 *e, const C2 *o) {
         using R = decltype(a[0].x);
-        const R h = (R)0.70710678118654752440;
+        const R h = kconst<R>(0.70710678118654752440);
         // twiddles exp(S 2 pi i q/8), q = 1, 2, 3: h t1, S i, h t3
         C2 t1, t3;
         if (S < 0) {
@@ -168,6 +180,7 @@ struct Radix<C2, 8> {
 };
 
 // z * w for a constant w = (wr, wi)
+__device__ __forceinline__ I2 cmulc(I2 z, long long wr, long long wi) { return vmul(z, WCplx{wsplit(wr), wsplit(wi)}); }
 template <class C2, class R>
 __device__ __forceinline__ C2 cmulc(C2 z, R wr, R wi) {
     C2 w;
@@ -183,8 +196,8 @@ struct Radix<C2, 16> {
     template <int S>
     static __device__ __forceinline__ void run(C2 *a) {
         using R = decltype(a[0].x);
-        const R c = (R)0.92387953251128675613, s = (R)0.38268343236508977173;
-        const R h = (R)0.70710678118654752440;
+        const R c = kconst<R>(0.92387953251128675613), s = kconst<R>(0.38268343236508977173);
+        const R h = kconst<R>(0.70710678118654752440);
         const R sg = (R)S;
         C2 y[4][4];
 #pragma unroll
@@ -222,9 +235,16 @@ struct Radix<C2, 3> {
     template <int S>
     static __device__ __forceinline__ void run(C2 *a) {
         using R = decltype(a[0].x);
-        const R half = (R)0.5, s3 = (R)0.86602540378443864676;
+        const R half = kconst<R>(0.5), s3 = kconst<R>(0.86602540378443864676);
         const C2 t1 = vadd(a[1], a[2]), t2 = vsub(a[1], a[2]);
-        C2 m; m.x = fma_rn<R>(-half, t1.x, a[0].x); m.y = fma_rn<R>(-half, t1.y, a[0].y);
+        C2 m;
+        if constexpr (std::is_same_v<R, long long>) {
+            m.x = a[0].x - (t1.x >> 1);
+            m.y = a[0].y - (t1.y >> 1);
+        } else {
+            m.x = fma_rn<R>(-half, t1.x, a[0].x);
+            m.y = fma_rn<R>(-half, t1.y, a[0].y);
+        }
         a[0] = vadd(a[0], t1);
         if constexpr (sizeof(R) == 8) {
             vaxpy2(m, s3, times_si<S>(t2), a[1], a[2]);
@@ -272,8 +292,8 @@ struct Radix<C2, 5> {
     template <int S>
     static __device__ __forceinline__ void run(C2 *a) {
         using R = decltype(a[0].x);
-        const R c1 = (R)0.30901699437494742410, c2 = (R)-0.80901699437494742410;
-        const R s1 = (R)0.95105651629515357212, s2 = (R)0.58778525229247312917;
+        const R c1 = kconst<R>(0.30901699437494742410), c2 = kconst<R>(-0.80901699437494742410);
+        const R s1 = kconst<R>(0.95105651629515357212), s2 = kconst<R>(0.58778525229247312917);
         const C2 t1 = vadd(a[1], a[4]), t2 = vadd(a[2], a[3]);
         const C2 t3 = vsub(a[1], a[4]), t4 = vsub(a[2], a[3]);
         C2 b1, b2, q1, q2;
@@ -341,8 +361,8 @@ struct Radix<C2, 9> {
     static __device__ __forceinline__ void run(C2 *a) {
         using R = decltype(a[0].x);
         // W9^m = (cos(2 pi m / 9), S sin(2 pi m / 9)), m = 1, 2, 4
-        const R c[3] = {(R)0.76604444311897803520, (R)0.17364817766693034885, (R)-0.93969262078590838405};
-        const R s[3] = {(R)(S * 0.64278760968653932632), (R)(S * 0.98480775301220805937), (R)(S * 0.34202014332566873304)};
+        const R c[3] = {kconst<R>(0.76604444311897803520), kconst<R>(0.17364817766693034885), kconst<R>(-0.93969262078590838405)};
+        const R s[3] = {kconst<R>(S * 0.64278760968653932632), kconst<R>(S * 0.98480775301220805937), kconst<R>(S * 0.34202014332566873304)};
         C2 y[3][3];
 #pragma unroll
         for (int n2 = 0; n2 < 3; ++n2) {
@@ -413,7 +433,7 @@ struct Radix<C2, 64> {
                 const int m = n2 * k1;
                 if (m == 0) y[n2][k1] = t[k1];
                 else if (m == 16) y[n2][k1] = times_si<S>(t[k1]);
-                else y[n2][k1] = cmulc(t[k1], (R)cos64(m), (R)(S * sin64(m)));
+                else y[n2][k1] = cmulc(t[k1], kconst<R>(cos64(m)), kconst<R>(S * sin64(m)));
             }
         }
 #pragma unroll

@@ -1,5 +1,6 @@
-// k_axis.cu -- kinetic filter along one axis for slices too large for the
-// fused step kernel (2D 128 x 128, 3D 64^3, long 1D lines).
+// k_axis.cu -- FP32 kinetic filter along one axis of slices that neither the plane filter nor
+// the tile filter's whole slices hold, for lines of 32, 64, 96, 128, 256 and 512 sites (the
+// x axis of 64^3).  FP64 takes the tile filter, whose butterflies run on the integer pipes.
 //
 // The kinetic factor is separable over the axes (the reference's -px^2 filter
 // acts on x only; the spin-1 factor exp(-eps k^2/2) is a product over axes), so
@@ -35,7 +36,6 @@ namespace clv {
 
 template <class R>
 __device__ __forceinline__ const R *efilt_of(const AxisDev &ax);
-template <> __device__ __forceinline__ const double *efilt_of<double>(const AxisDev &ax) { return ax.efilt64; }
 template <> __device__ __forceinline__ const float *efilt_of<float>(const AxisDev &ax) { return ax.efilt32; }
 
 // ----------------------------------------------------------- CTA-wide passes
@@ -334,8 +334,6 @@ cudaError_t launch_axis_filter(const LaunchAxis &L, cudaStream_t s) {
 }
 
 template cudaError_t setup_axis_filter<float>(int, size_t, int *);
-template cudaError_t setup_axis_filter<double>(int, size_t, int *);
 template cudaError_t launch_axis_filter<float>(const LaunchAxis &, cudaStream_t);
-template cudaError_t launch_axis_filter<double>(const LaunchAxis &, cudaStream_t);
 
 }  // namespace clv

@@ -16,9 +16,15 @@
 // pitch) and across them; the divisions are multiplications by a reciprocal that the
 // thread computes once per pass.
 //
-// Bound by the passes over shared memory and the latency between their barriers.  Against
-// the one-warp-per-line plans that these lengths had (a 60-site line gave a warp 15
-// butterflies of radix 4): see plan_tiled for the paths and figures.
+// FP64 lines run in block floating point on the integer pipes (fft_int.cuh): a pass over the
+// raw tile finds every line's largest component (every slice's, when several axes are
+// filtered), the first pass converts as it reads and the last one converts back as it
+// writes.  128-site lines, 4 components x 128 x 128 x 128 imaginary times, both fields: 1.37
+// (butterflies on the FP64 pipe, at its rate) -> 0.53 ms; 48-site lines of 48 x 40 x 36 x 24:
+// 0.93 -> 0.37 ms.  Bound by integer issue (46 % of the ALU) and instruction fetch.
+//
+// FP32 is bound by instruction issue (61 %, 170 instructions an element, a third of them
+// addresses) and the latency between its barriers.  64 ragged chains, 1.6 M sites: 78 us.
 #pragma once
 
 #include "clv_internal.cuh"
@@ -52,15 +58,46 @@ struct TileLines {
     }
 };
 
-enum { TILE_DIF = 0, TILE_MID = 1, TILE_DIT = 2 };
+// Arithmetic of the tile's passes: element type, twiddle and filter types.
+template <class R> struct TileMath;
+template <> struct TileMath<float> { using E = float2; using W = float2; using F = float; };
+template <> struct TileMath<double> { using E = I2; using W = WCplx; using F = long long; };
+
+// FP64: the lines' scale.  Line l belongs to group l / lines per group; of each group, raw: the
+// high word of the largest component as the doubles came in; cur, next: of the largest one
+// after the pass before this one and after this one (zero: cleared for the pass after);
+// exps: the shifts so far.  first: the pass reads doubles; last: it writes them.  eg: the
+// filters' power of two.
+struct TileScale {
+    unsigned *raw, *cur, *next, *zero;
+    int *exps;
+    FastDiv group;
+    int ng, eg;
+    bool first, last;
+    __device__ __forceinline__ void advance() {
+        unsigned *t = cur;
+        cur = next; next = zero; zero = t;
+        first = false;
+    }
+};
+
+enum { TILE_DIF = 0, TILE_MID = 1, TILE_DIT = 2, TILE_MAX = 3 };
+
+__host__ __device__ constexpr int ceil_log2(int n) { return n <= 1 ? 0 : 1 + ceil_log2((n + 1) / 2); }
 
 // One pass of radix R over the tile.  TILE_DIF: forward pass of span L (S = L / R), twiddles
 // after the butterfly unless S = 1.  TILE_MID: the last forward pass, the filter (f in the
 // passes' order of frequencies, plus the line's share fo of the other axes when it is not
-// null), the first inverse pass.  TILE_DIT: the inverse of TILE_DIF.
-template <class C2, class RR, int R, int KIND>
-__device__ __forceinline__ void tile_pass(C2 *t, const TileLines &g, int L, int S, const C2 *tw, const RR *f,
-                                          const RR *fo) {
+// null), the first inverse pass.  TILE_DIT: the inverse of TILE_DIF.  TILE_MAX (FP64): the
+// largest component of every group.
+template <class RR, int R, int KIND>
+__device__ __forceinline__ void tile_pass(typename Cx<RR>::T *t, const TileLines &g, int L, int S,
+                                          const typename TileMath<RR>::W *tw, const typename TileMath<RR>::F *f,
+                                          const typename TileMath<RR>::F *fo, const TileScale &sc) {
+    using C2 = typename Cx<RR>::T;
+    using E = typename TileMath<RR>::E;
+    constexpr bool kInt = sizeof(RR) == 8;
+    constexpr int LR = ceil_log2(R);
     const int NB = g.NL * (g.n / R), ts = g.n / L;
     const FastDiv dS(S);
     const int st = S * g.es;
@@ -69,56 +106,114 @@ __device__ __forceinline__ void tile_pass(C2 *t, const TileLines &g, int L, int 
         const int j = g.dNL.div(b), l = b - j * g.NL;
         const int blk = KIND == TILE_MID ? j : dS.div(j), k = KIND == TILE_MID ? 0 : j - blk * S;
         C2 *p = t + g.base(l) + (blk * L + k) * g.es;
-        C2 v[R];
+        if constexpr (KIND == TILE_MAX) {
+            if constexpr (kInt) {
+                unsigned mx = 0;
 #pragma unroll
-        for (int m = 0; m < R; ++m) v[m] = p[m * st];
-        if constexpr (KIND == TILE_DIF) {
-            Radix<C2, R>::template run<-1>(v);
-            if (S > 1) {
-                const int step = k * ts;
-#pragma unroll
-                for (int q = 1; q < R; ++q) v[q] = vmul(v[q], tw[q * step]);
-            }
-        } else if constexpr (KIND == TILE_DIT) {
-            if (S > 1) {
-                const int step = k * ts;
-#pragma unroll
-                for (int q = 1; q < R; ++q) {
-                    C2 w = tw[q * step];
-                    w.y = -w.y;
-                    v[q] = vmul(v[q], w);
+                for (int m = 0; m < R; ++m) {
+                    const unsigned v = mag_bits(p[m * st]);
+                    mx = v > mx ? v : mx;
                 }
+                atomicMax(&sc.raw[sc.group.div(l)], mx);
             }
-            Radix<C2, R>::template run<1>(v);
         } else {
-            Radix<C2, R>::template run<-1>(v);
-            const RR o = fo ? fo[l] : (RR)0;
-            RR h[R];
+            E v[R];
+            int gr = 0;
+            if constexpr (kInt) {
+                gr = sc.group.div(l);
+                if (sc.first) {
+                    const int em = (int)(sc.raw[gr] >> 20);
 #pragma unroll
-            for (int q = 0; q < R; ++q) h[q] = f[blk * R + q] + o;
-            radix_scaled<C2, R, 1>(v, h);
+                    for (int m = 0; m < R; ++m) {
+                        const double2 d = p[m * st];
+                        v[m] = I2{to_fixed(d.x, em, LR), to_fixed(d.y, em, LR)};
+                    }
+                } else {
+                    const int sh = ishift_for(sc.cur[gr], LR);
+#pragma unroll
+                    for (int m = 0; m < R; ++m) v[m] = ishift(*reinterpret_cast<const I2 *>(p + m * st), sh);
+                }
+            } else {
+#pragma unroll
+                for (int m = 0; m < R; ++m) v[m] = p[m * st];
+            }
+            if constexpr (KIND == TILE_DIF) {
+                Radix<E, R>::template run<-1>(v);
+                if (S > 1) {
+                    const int step = k * ts;
+#pragma unroll
+                    for (int q = 1; q < R; ++q) v[q] = vmul(v[q], tw[q * step]);
+                }
+            } else if constexpr (KIND == TILE_DIT) {
+                if (S > 1) {
+                    const int step = k * ts;
+#pragma unroll
+                    for (int q = 1; q < R; ++q) v[q] = vmulc(v[q], tw[q * step]);
+                }
+                Radix<E, R>::template run<1>(v);
+            } else {
+                Radix<E, R>::template run<-1>(v);
+                typename TileMath<RR>::F o = 0;
+                if (fo) o = fo[l];
+#pragma unroll
+                for (int q = 0; q < R; ++q) {
+                    if constexpr (kInt) v[q] = ifilter<LR>(f[blk * R + q] + o, v[q]);
+                    else v[q] = vscale(f[blk * R + q] + o, v[q]);
+                }
+                Radix<E, R>::template run<1>(v);
+            }
+            if constexpr (kInt) {
+                if (KIND != TILE_DIF && sc.last) {
+                    const int em = (int)(sc.raw[gr] >> 20);
+                    const int e = sc.eg + sc.exps[gr] + (KIND == TILE_MID ? LR : 0) +
+                                  (sc.first ? LR : ishift_for(sc.cur[gr], LR));
+#pragma unroll
+                    for (int m = 0; m < R; ++m) p[m * st] = make_double2(from_fixed(v[m].x, em, e), from_fixed(v[m].y, em, e));
+                } else {
+                    unsigned mx = 0;
+#pragma unroll
+                    for (int m = 0; m < R; ++m) {
+                        const unsigned u = imag_bits(v[m]);
+                        mx = u > mx ? u : mx;
+                        *reinterpret_cast<I2 *>(p + m * st) = v[m];
+                    }
+                    atomicMax(&sc.next[gr], mx);
+                }
+            } else {
+#pragma unroll
+                for (int m = 0; m < R; ++m) p[m * st] = v[m];
+            }
         }
-#pragma unroll
-        for (int m = 0; m < R; ++m) p[m * st] = v[m];
+    }
+    if constexpr (kInt && KIND != TILE_MAX) {
+        if (!sc.last)  // (the last pass reads exps)
+            for (int i = threadIdx.x; i < sc.ng; i += blockDim.x) {
+                sc.exps[i] += (KIND == TILE_MID ? LR : 0) + (sc.first ? LR : ishift_for(sc.cur[i], LR));
+                sc.zero[i] = 0;
+            }
     }
     __syncthreads();
 }
 
-template <class C2, class RR, int KIND>
-__device__ __forceinline__ void tile_pass_any(int R, C2 *t, const TileLines &g, int L, int S, const C2 *tw, const RR *f,
-                                              const RR *fo) {
+template <class RR, int KIND>
+__device__ __forceinline__ void tile_pass_any(int R, typename Cx<RR>::T *t, const TileLines &g, int L, int S,
+                                              const typename TileMath<RR>::W *tw, const typename TileMath<RR>::F *f,
+                                              const typename TileMath<RR>::F *fo, const TileScale &sc) {
     switch (R) {
-        case 2: tile_pass<C2, RR, 2, KIND>(t, g, L, S, tw, f, fo); break;
-        case 3: tile_pass<C2, RR, 3, KIND>(t, g, L, S, tw, f, fo); break;
-        case 4: tile_pass<C2, RR, 4, KIND>(t, g, L, S, tw, f, fo); break;
-        case 5: tile_pass<C2, RR, 5, KIND>(t, g, L, S, tw, f, fo); break;
-        case 6: tile_pass<C2, RR, 6, KIND>(t, g, L, S, tw, f, fo); break;
-        case 8: tile_pass<C2, RR, 8, KIND>(t, g, L, S, tw, f, fo); break;
-        case 9: tile_pass<C2, RR, 9, KIND>(t, g, L, S, tw, f, fo); break;
-        case 10: tile_pass<C2, RR, 10, KIND>(t, g, L, S, tw, f, fo); break;
-        case 12: tile_pass<C2, RR, 12, KIND>(t, g, L, S, tw, f, fo); break;
-        case 15: tile_pass<C2, RR, 15, KIND>(t, g, L, S, tw, f, fo); break;
-        default: tile_pass<C2, RR, 16, KIND>(t, g, L, S, tw, f, fo); break;
+        case 2: tile_pass<RR, 2, KIND>(t, g, L, S, tw, f, fo, sc); break;
+        case 3: tile_pass<RR, 3, KIND>(t, g, L, S, tw, f, fo, sc); break;
+        case 4: tile_pass<RR, 4, KIND>(t, g, L, S, tw, f, fo, sc); break;
+        case 5: tile_pass<RR, 5, KIND>(t, g, L, S, tw, f, fo, sc); break;
+        case 6: tile_pass<RR, 6, KIND>(t, g, L, S, tw, f, fo, sc); break;
+        case 8: tile_pass<RR, 8, KIND>(t, g, L, S, tw, f, fo, sc); break;
+        case 9: tile_pass<RR, 9, KIND>(t, g, L, S, tw, f, fo, sc); break;
+        case 10: tile_pass<RR, 10, KIND>(t, g, L, S, tw, f, fo, sc); break;
+        default:
+            if constexpr (tile_radix_max<RR>() >= 16) {
+                if (R == 12) tile_pass<RR, 12, KIND>(t, g, L, S, tw, f, fo, sc);
+                else if (R == 15) tile_pass<RR, 15, KIND>(t, g, L, S, tw, f, fo, sc);
+                else tile_pass<RR, 16, KIND>(t, g, L, S, tw, f, fo, sc);
+            }
     }
 }
 
@@ -141,9 +236,22 @@ __device__ __forceinline__ void copy_async(C2 *s, const C2 *g) {
                  : "memory");
 }
 
-template <class R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) tile_filter_kernel(const LaunchTileFilter A) {
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+// least e with x <= 2^e, x > 0 finite and normal
+__device__ __forceinline__ int exp_above(double x) {
+    const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
+    return e + (((hi & 0xfffff) | __double2loint(x)) != 0);
+}
+
+// TH threads: 128, or 256 for the large slices.
+template <class R, int TH>
+__global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5 : 2)) tile_filter_kernel(const LaunchTileFilter A) {
     using C2 = typename Cx<R>::T;
+    using W = typename TileMath<R>::W;
+    using F = typename TileMath<R>::F;
+    constexpr bool kInt = sizeof(R) == 8;
+    static_assert(sizeof(W) == sizeof(C2) && sizeof(F) == sizeof(R), "tables take the elements' sizes");
     extern __shared__ __align__(128) unsigned char smem[];
     const int bid = A.nfields == 2 ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const int field = A.nfields == 2 ? (int)(blockIdx.x & 1) : 0;
@@ -151,9 +259,9 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) tile_filter_kerne
     const TileFilterPlan &P = A.plans[task.plan];
     const ChainDev &ch = A.chains[task.chain];
     const int rows = task.rows, cols = task.cols, PZ = P.pitch, nax = P.naxes;
-    const bool energy = A.filter != 0;
+    const bool energy = A.filter != 0, summed = energy && nax > 1;
     C2 *tile = reinterpret_cast<C2 *>(smem);
-    C2 *tw0 = tile + P.tile_elems;
+    W *tw0 = reinterpret_cast<W *>(tile + P.tile_elems);
     const long long off = ch.off + (long long)task.slice * ch.V + task.off;
     const C2 *src = reinterpret_cast<const C2 *>(field ? A.src1 : A.src0) + off;
     C2 *dst = reinterpret_cast<C2 *>(field ? A.dst1 : A.dst0) + off;
@@ -171,8 +279,20 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) tile_filter_kerne
     // frequencies, the component constant folded into the first axis' one
     int nsum = 0;
     for (int a = 0; a < nax; ++a) nsum += ch.axis[P.axis[a]].n;
-    R *f0 = reinterpret_cast<R *>(tw0 + nsum);
+    F *f0 = reinterpret_cast<F *>(tw0 + nsum);
+    F *fo = f0 + nsum;  // summed filters: the rows' shares of the other axes
+    TileScale sc{nullptr, nullptr, nullptr, nullptr, nullptr, FastDiv(1), 0, 0, false, false};
     {
+        // FP64: the filters relative to the power of two at or above their largest value (of
+        // each axis, or of the sum)
+        if constexpr (kInt) {
+            if (summed) {
+                double most = 0, n = 1;
+                for (int a = 0; a < nax; ++a) n *= ch.axis[P.axis[a]].n;
+                for (int a = 0; a < nax; ++a) most += ch.axis[P.axis[a]].efmax * (ch.axis[P.axis[a]].n / n);
+                sc.eg = exp_above(most);
+            }
+        }
         int o = 0;
         for (int a = 0; a < nax; ++a) {
             const AxisDev &ax = ch.axis[P.axis[a]];
@@ -184,64 +304,105 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) tile_filter_kerne
             if (energy)
                 for (int b = 0; b < nax; ++b)
                     if (b != a) cst /= (R)ch.axis[P.axis[b]].n;
+            if constexpr (kInt) {
+                int e = sc.eg;
+                if (!summed) {
+                    e = exp_above((energy ? ax.efmax : ax.fmax) * cst);
+                    sc.eg += e;
+                }
+                cst *= pow2(kFiltQ - e);
+            }
             for (int i = threadIdx.x; i < ax.n; i += blockDim.x) {
-                tw0[o + i] = tw[i];
-                f0[o + i] = f[i] * cst;
+                if constexpr (kInt) {
+                    const double2 w = tw[i];
+                    const double q = 4611686018427387904.0;  // 2^62
+                    tw0[o + i] = WCplx{wsplit(__double2ll_rn(w.x * q)), wsplit(__double2ll_rn(w.y * q))};
+                    f0[o + i] = __double2ll_rn(f[i] * cst);
+                } else {
+                    tw0[o + i] = tw[i];
+                    f0[o + i] = f[i] * cst;
+                }
             }
             o += ax.n;
         }
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncthreads();
-    // forward passes of one axis (all of them when `whole`), inverse passes
-    auto forward = [&](const TileLines &g, const AxisDev &ax, const C2 *tw, bool whole) {
-        int L = ax.n;
-        for (int p = 0; p < (whole ? ax.tnf : ax.tnf - 1); ++p) {
-            const int rad = ax.tfac[p];
-            tile_pass_any<C2, R, TILE_DIF>(rad, tile, g, L, L / rad, tw, (const R *)nullptr, (const R *)nullptr);
-            L /= rad;
-        }
-    };
-    auto inverse = [&](const TileLines &g, const AxisDev &ax, const C2 *tw, bool whole) {
-        int S = whole ? 1 : ax.tfac[ax.tnf - 1];
-        for (int p = (whole ? ax.tnf : ax.tnf - 1) - 1; p >= 0; --p) {
-            const int rad = ax.tfac[p];
-            tile_pass_any<C2, R, TILE_DIT>(rad, tile, g, S * rad, S, tw, (const R *)nullptr, (const R *)nullptr);
-            S *= rad;
-        }
-    };
-    // I of axis a: the tile elements (padding aside) between two of its sites
+    // lines of axis a (P.inner: tile elements, padding aside, between two of its sites)
     auto lines = [&](int a) {
         return TileLines(rows, cols, PZ, ch.axis[P.axis[a]].n, P.inner[a] == 0 ? cols : P.inner[a], P.inner[a] == 1);
     };
-    auto middle = [&](const TileLines &g, const AxisDev &ax, const C2 *tw, const R *f, const R *fo) {
-        const int rad = ax.tfac[ax.tnf - 1];
-        tile_pass_any<C2, R, TILE_MID>(rad, tile, g, rad, 1, tw, f, fo);
+    // FP64: one scale per line, or per slice when several axes mix its lines
+    auto group = [&](int a) {
+        if constexpr (kInt) sc.group = FastDiv(nax == 1 ? 1 : ch.V / ch.axis[P.axis[a]].n);
     };
-    if (!energy || nax == 1) {
+    if constexpr (kInt) {
+        sc.ng = nax == 1 ? total / ch.axis[P.axis[0]].n : total / ch.V;
+        sc.raw = reinterpret_cast<unsigned *>(fo + (summed ? rows : 0));
+        sc.cur = sc.raw + sc.ng;
+        sc.next = sc.cur + sc.ng;
+        sc.zero = sc.next + sc.ng;
+        sc.exps = reinterpret_cast<int *>(sc.zero + sc.ng);
+        for (int i = threadIdx.x; i < 5 * sc.ng; i += blockDim.x) sc.raw[i] = 0;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if constexpr (kInt) {
+        const AxisDev &ax = ch.axis[P.axis[0]];
+        group(0);
+        tile_pass_any<R, TILE_MAX>(ax.tfac[0], tile, lines(0), ax.n, ax.n / ax.tfac[0], nullptr, nullptr, nullptr, sc);
+    }
+    // forward passes of one axis (all of them when `whole`), the middle one, the inverse ones
+    auto forward = [&](const TileLines &g, const AxisDev &ax, const W *tw, bool whole) {
+        int L = ax.n;
+        for (int p = 0; p < (whole ? ax.tnf : ax.tnf - 1); ++p) {
+            const int rad = ax.tfac[p];
+            tile_pass_any<R, TILE_DIF>(rad, tile, g, L, L / rad, tw, nullptr, nullptr, sc);
+            sc.advance();
+            L /= rad;
+        }
+    };
+    auto middle = [&](const TileLines &g, const AxisDev &ax, const W *tw, const F *f, const F *fr, bool end) {
+        const int rad = ax.tfac[ax.tnf - 1];
+        sc.last = end && ax.tnf == 1;
+        tile_pass_any<R, TILE_MID>(rad, tile, g, rad, 1, tw, f, fr, sc);
+        sc.advance();
+    };
+    auto inverse = [&](const TileLines &g, const AxisDev &ax, const W *tw, bool whole, bool end) {
+        int S = whole ? 1 : ax.tfac[ax.tnf - 1];
+        for (int p = (whole ? ax.tnf : ax.tnf - 1) - 1; p >= 0; --p) {
+            const int rad = ax.tfac[p];
+            sc.last = end && p == 0;
+            tile_pass_any<R, TILE_DIT>(rad, tile, g, S * rad, S, tw, nullptr, nullptr, sc);
+            sc.advance();
+            S *= rad;
+        }
+    };
+    sc.first = true;
+    if (!summed) {
         // product of the axes' filters: one axis after the other
         int o = 0;
         for (int a = 0; a < nax; ++a) {
             const AxisDev &ax = ch.axis[P.axis[a]];
             const TileLines g = lines(a);
+            group(a);
+            const bool end = a == nax - 1;
             forward(g, ax, tw0 + o, false);
-            middle(g, ax, tw0 + o, f0 + o, nullptr);
-            inverse(g, ax, tw0 + o, false);
+            middle(g, ax, tw0 + o, f0 + o, nullptr, end);
+            inverse(g, ax, tw0 + o, false, end);
             o += ax.n;
         }
     } else {
         // sum of the axes' filters: every axis forward, the sum at each frequency, and back
         // (the last axis is the innermost: its lines are the tile's rows, whose share of the
         // other axes' filters goes into fo)
-        R *fo = f0 + nsum;
         int o = 0;
         for (int a = 0; a + 1 < nax; ++a) {
             const AxisDev &ax = ch.axis[P.axis[a]];
+            group(a);
             forward(lines(a), ax, tw0 + o, true);
             o += ax.n;
         }
         for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-            R v = 0;
+            F v = 0;
             int o2 = 0;
             for (int a = 0; a + 1 < nax; ++a) {
                 const int n = ch.axis[P.axis[a]].n, I = P.inner[a] == 0 ? cols : P.inner[a];
@@ -254,14 +415,16 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) tile_filter_kerne
         {
             const AxisDev &ax = ch.axis[P.axis[nax - 1]];
             const TileLines g = lines(nax - 1);
+            group(nax - 1);
             forward(g, ax, tw0 + o, false);
-            middle(g, ax, tw0 + o, f0 + o, fo);
-            inverse(g, ax, tw0 + o, false);
+            middle(g, ax, tw0 + o, f0 + o, fo, false);
+            inverse(g, ax, tw0 + o, false, false);
         }
         for (int a = nax - 2; a >= 0; --a) {
             const AxisDev &ax = ch.axis[P.axis[a]];
             o -= ax.n;
-            inverse(lines(a), ax, tw0 + o, true);
+            group(a);
+            inverse(lines(a), ax, tw0 + o, true, a == 0);
         }
     }
     const bool acc = A.accumulate != 0;
@@ -269,13 +432,13 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) tile_filter_kerne
         const int r = dc.div(e), c = e - r * cols;
         C2 *d = dst + (long long)r * gs + c;
         const C2 v = tile[r * PZ + c];
-        *d = acc ? vadd(*d, v) : v;
+        *d = acc ? cadd(*d, v) : v;
     }
 }
 
 template <class R>
-cudaError_t setup_tile_filter(size_t smem_bytes, int *ctas_per_sm) {
-    const void *fn = (const void *)tile_filter_kernel<R>;
+cudaError_t setup_tile_filter(size_t smem_bytes, int threads, int *ctas_per_sm) {
+    const void *fn = threads == 128 ? (const void *)tile_filter_kernel<R, 128> : (const void *)tile_filter_kernel<R, 256>;
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, fn);
     if (e != cudaSuccess) return e;
@@ -283,14 +446,15 @@ cudaError_t setup_tile_filter(size_t smem_bytes, int *ctas_per_sm) {
         e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
         if (e != cudaSuccess) return e;
     }
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, 256, smem_bytes);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, threads, smem_bytes);
 }
 
 template <class R>
 cudaError_t launch_tile_filter(const LaunchTileFilter &L, cudaStream_t s) {
     if (L.ntasks == 0) return cudaSuccess;
     void *args[] = {const_cast<LaunchTileFilter *>(&L)};
-    return cudaLaunchKernel((const void *)tile_filter_kernel<R>, dim3(L.nfields * L.ntasks), dim3(L.threads), args, L.smem_bytes, s);
+    const void *fn = L.threads == 128 ? (const void *)tile_filter_kernel<R, 128> : (const void *)tile_filter_kernel<R, 256>;
+    return cudaLaunchKernel(fn, dim3(L.nfields * L.ntasks), dim3(L.threads), args, L.smem_bytes, s);
 }
 
 }  // namespace clv

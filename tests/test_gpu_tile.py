@@ -98,3 +98,67 @@ def test_ref4_tile_filter_equals_line_filter(clv, monkeypatch, shape, prec):
             out.append(e.get_fields(0))
     tol = 1e-13 if prec == "f64" else 2e-6
     assert rel_err(out[0][0], out[1][0]) < tol and rel_err(out[0][1], out[1][1]) < tol
+
+
+@pytest.mark.parametrize("kind", ["fluctuating", "one_site"])
+@pytest.mark.parametrize("shape", [dict(nx=60, nt=8), dict(nx=128, ny=100, nt=2), dict(nx=30, ny=30, nt=4),
+                                   dict(nx=243, nt=6), dict(nx=1500, nt=4), dict(nx=48, ny=20, nz=15, nt=2)],
+                         ids=lambda d: "x".join(str(v) for v in d.values()))
+def test_fp64_filter_to_rounding(clv, shape, kind):
+    """The integer butterflies against long-double transforms: one step with dt = 1, no couplings
+    and no noise gives psi + (kin(tau - 1) - psi).  The kinetic term, the drift and the sum
+    are rounded once each (2^-53 of the field each), the transform adds 2^-55: 4e-16 in the
+    2-norm."""
+    fft = pytest.importorskip("scipy.fft")
+    c = spin1(clv, **shape, mu=0.0, c0=0.0, c1=0.0, q=0.0, K=1e300, dt_max=1.0)
+    rng = np.random.default_rng(3)
+    with clv.Engine(c, model=clv.MODEL_SPIN1, precision=clv.PREC_F64) as e:
+        f = (rng.standard_normal(e.shape(0)) + 1j * rng.standard_normal(e.shape(0))) * 0.3 + 0.5
+        if kind == "one_site":
+            f *= 1e-3
+            f.reshape(3, c.nt, -1)[:, :, 5] = 3.0
+        e.set_fields(0, f, np.conj(f))
+        e.step_with_noise(np.zeros(2 * f.size))
+        got = e.get_fields(0)[0]
+    want = f.astype(np.clongdouble)
+    for a, n in enumerate((c.nx, c.ny, c.nz)):
+        if n > 1:
+            k = np.arange(n)
+            p = np.where(k < n // 2, 2 * np.pi * k / n, -2 * np.pi * (n - k) / n)
+            s = [1] * 5
+            s[2 + a] = n
+            want = fft.ifft(fft.fft(want, axis=2 + a) * np.exp(-c.eps * 0.5 * p * p).reshape(s), axis=2 + a)
+    want = np.roll(want, 1, 1)
+    assert float(np.linalg.norm(np.abs(got - want).ravel().astype(float))) < \
+        4e-16 * float(np.linalg.norm(np.abs(want).ravel().astype(float)))
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("shape", [dict(nx=60, nt=6), dict(nx=30, ny=24, nt=4), dict(nx=100, ny=81, nt=2)],
+                         ids=lambda d: "x".join(str(v) for v in d.values()))
+def test_non_finite_field_flags_its_chain_only(clv, shape, bad, prec):
+    chains = [spin1(clv, seed=3, **shape), spin1(clv, seed=4, **shape)]
+    with clv.Engine(chains, model=clv.MODEL_SPIN1, precision=clv.PREC_F64 if prec == "f64" else clv.PREC_F32) as e:
+        e.init_spin1()
+        psi, psic = e.get_fields(0)
+        e.step(1)
+        want = e.get_fields(1)
+        assert not any(e.chain_flags())
+    with clv.Engine(chains, model=clv.MODEL_SPIN1, precision=clv.PREC_F64 if prec == "f64" else clv.PREC_F32) as e:
+        e.init_spin1()
+        psi[1, 1].flat[7] = bad
+        e.set_fields(0, psi, psic)
+        e.step(1)
+        assert list(e.chain_flags()) == [1, 0]
+        got = e.get_fields(1)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+def test_zero_field_stays_zero(clv):
+    """The reference's zero start: every line of the filter is zero."""
+    c = clv.ChainParams(nx=60, ny=9, nt=6, eps=0.02, G=0.1, mu=-0.5, DT=0.002, seed=7)
+    with clv.Engine(c, model=clv.MODEL_REF4, precision=clv.PREC_F64) as e:
+        assert e.plan()[0] == "tiled"
+        e.step_with_noise(np.zeros(2 * 4 * 60 * 9 * 6))
+        assert all(np.all(f == 0) for f in e.get_fields(0)) and not any(e.chain_flags())
