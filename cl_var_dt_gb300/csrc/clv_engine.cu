@@ -791,13 +791,15 @@ void build_tiled_tasks(clv_engine *e, int L) {
     }
 }
 
-// Imaginary times per CTA of the step kernels: the chunk length whose CTAs, spread over the
-// SMs, finish soonest.  An SM's time is its share of the CTAs times a CTA's length plus the
-// halo that every chunk pays, and the share is a whole number: 192 CTAs on 152 SMs cost as
-// much as 304 (the FP64 reduce pass on 128 x 128 with chunks of 43: 1.11 ms; of 18: 0.78 ms;
-// the FP64 step of 32 chains of 256 x 128 with 320 CTAs: 1.32 ms, with 288: 1.03 ms).  width:
-// sites a CTA takes of a chunk, 0: all of them.
-int choose_chunk(const clv_engine *e, int nsm, int width, double halo) {
+// Imaginary times per CTA of the step kernels: the chunk length whose CTAs, spread over
+// `slots`, finish soonest.  A slot's time is its share of the CTAs times a CTA's length plus
+// the halo that every chunk pays, and the share is a whole number: 192 CTAs on 152 SMs cost as
+// much as 304 (the FP64 reduce pass on 128 x 128 with chunks of 43: 1.11 ms; of 18: 0.75 ms;
+// the FP64 step of 32 chains of 256 x 128 with 320 CTAs: 1.32 ms, with 288: 1.02 ms).  Slots:
+// the SMs for the fused kernel, whose resident CTAs share the SM's issue slots; resident CTAs
+// for the tiled one, bound by memory or, at one per SM, the FP64 pipe (2D 128 x 128, FP32:
+// step kernel 78 us counted in SMs, 70 us).  width: sites a CTA takes of a chunk, 0: all.
+int choose_chunk(const clv_engine *e, int slots, int width, double halo) {
     int tmax = 1;
     double work = 0;
     for (auto &d : e->chains_h) {
@@ -812,7 +814,7 @@ int choose_chunk(const clv_engine *e, int nsm, int width, double halo) {
             const long long nchunk = (d.nt + L - 1) / L;
             ctas += width ? (d.V * nchunk + width - 1) / width : nchunk;
         }
-        const double t = (double)((ctas + nsm - 1) / nsm) * (work / ctas + halo);
+        const double t = (double)((ctas + slots - 1) / slots) * (work / ctas + halo);
         if (L == 1 || t < cost) {
             best = L;
             cost = t;
@@ -1162,7 +1164,7 @@ int plan_tiled(clv_engine *e) {
     // kernel, bound by memory, pays in full (3D 64^3: 1.04 ms with 16 times a chunk, 1.00 with 64)
     long long tile_taus = 0;
     for (auto &d : e->chains_h) tile_taus += ((long long)d.V * d.nt + 255) / 256;
-    int L = choose_chunk(e, nsm, 256, e->precision == CLV_PREC_F32 ? 2.0 : 0.6);
+    int L = choose_chunk(e, occ * nsm, 256, e->precision == CLV_PREC_F32 ? 2.0 : 0.6);
     if (const char *cl = std::getenv("CLV_CHUNK")) L = std::max(1, atoi(cl));
     e->task_capacity = (size_t)tile_taus;  // chunks of one imaginary time
     build_tiled_tasks(e, L);
@@ -1834,11 +1836,6 @@ int clv_autotune(clv_engine *e, int trial_steps, char *report, int capacity) {
             if (e->fused) {
                 for (int tma : {1, 0}) {
                     if (tma && !e->fused_aligned) continue;
-                    // FP64 lines of 256 without bulk copies filter the ends of a chunk on
-                    // warp pairs, whose radix-4 passes round differently (1e-16)
-                    if (!tma && e->fused_aligned && e->precision == CLV_PREC_F64 && e->fused_ln_static == 256 &&
-                        e->dt_rule == CLV_DT_K_OVER_MAX)
-                        continue;
                     for (int ln : {e->fused_ln_static, 0}) {
                         for (int sd : {0, 1}) {
                             if (sd && e->dt_rule != CLV_DT_REF_MEANMAX) continue;

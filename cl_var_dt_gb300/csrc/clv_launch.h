@@ -186,10 +186,11 @@ __host__ __device__ inline int pass_twiddle_source(int n, int e, bool *conj) {
 }
 
 // Shared memory of the fused kernel before its slots: barriers (64 B), the
-// twiddle and filter tables of tab_n entries, the per-pass twiddles of the
-// compile-time plan of ln-site lines (ln > 0), rounded up to 128 B.
+// twiddle and filter tables of tab_n entries (FP64: a filter table per component, its
+// constant folded in), the per-pass twiddles of the compile-time plan of ln-site lines
+// (ln > 0), rounded up to 128 B.
 __host__ __device__ constexpr int fused_ptw_offset(int tab_n, int esz) {
-    return (64 + tab_n * (esz + esz / 2) + 15) / 16 * 16;
+    return (64 + tab_n * (esz + esz / 2 * (esz == 16 ? kMaxComp : 1)) + 15) / 16 * 16;
 }
 __host__ __device__ constexpr int fused_tab_bytes(int tab_n, int esz, int ln) {
     return (fused_ptw_offset(tab_n, esz) + (ln > 0 ? tw_entries(ln) : 0) * esz + 127) / 128 * 128;

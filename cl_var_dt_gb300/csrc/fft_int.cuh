@@ -135,6 +135,20 @@ __device__ __forceinline__ double from_fixed(long long v, int emax, int e) {
     if (be < 1 || be > 2045) b = be < 1 ? 0 : 0x7ff0000000000000ull;
     return __longlong_as_double((long long)(v < 0 ? b | 0x8000000000000000ull : b));
 }
+// 2^e as a double, -1022 <= e <= 1023
+__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
+// least e with x <= 2^e, x > 0 finite and normal
+__device__ __forceinline__ int exp_above(double x) {
+    const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
+    return e + (((hi & 0xfffff) | __double2loint(x)) != 0);
+}
+// Table entries: a twiddle, and a filter value relative to 2^e.
+__device__ __forceinline__ WCplx twiddle_fixed(double2 w) {
+    const double q = 4611686018427387904.0;  // 2^62
+    return WCplx{wsplit(__double2ll_rn(w.x * q)), wsplit(__double2ll_rn(w.y * q))};
+}
+__device__ __forceinline__ long long filter_fixed(double f, int e) { return __double2ll_rn(f * pow2(kFiltQ - e)); }
+
 // Exponent word of the largest component, for a line's maximum.
 __device__ __forceinline__ unsigned mag_bits(double2 z) {
     const unsigned a = (unsigned)__double2hiint(z.x) & 0x7fffffffu, b = (unsigned)__double2hiint(z.y) & 0x7fffffffu;

@@ -210,123 +210,201 @@ static_assert(tw_mid_off(256) == 56 && tw_inv_off(256, 1) == 248 && tw_inv_off(2
               tw_entries(256) == 500, "pass tables of 256");
 static_assert(tw_entries(128) == 56 + 64 + 14 + 112 && tw_entries(64) == 56 + 56, "pass-table sizes");
 
-// Contiguous-line filter of a length known at run time (the plan without per-pass tables).
-template <class C2, class RR>
-__device__ __forceinline__ void line_filter_1d(const C2 *src, C2 *X, C2 *Y, int n, const C2 *tw, const RR *f, RR cst,
-                                               int lane) {
-    switch (n) {
-        case 64: warp_line_filter_ct<C2, RR, 64>(src, X, Y, tw, f, cst, lane); break;
-        case 128: warp_line_filter_ct<C2, RR, 128>(src, X, Y, tw, f, cst, lane); break;
-        default: warp_line_filter_ct<C2, RR, 256>(src, X, Y, tw, f, cst, lane); break;
-    }
-}
-
-// ------------------------------- lines split over a group of NT = 32 G threads
-// At FP64 the pipe's throughput per SM sub-partition is the bound, and one warp
-// per line keeps only as many sub-partitions busy as there are lines.  A group of
-// G warps shares one line of N = 4^k sites: radix-4 Stockham passes (N / 4
-// butterflies each, one or more per thread), the group's threads synchronised by
-// the named barrier `id` between passes.  Same contract and padded layouts as
-// warp_line_filter_ct; twiddles from the length-N table exp(-2 pi i m / N).
-template <int NT>
-__device__ __forceinline__ void group_sync(int id) {
-    if constexpr (NT == 32) __syncwarp();
-    else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(NT) : "memory");
-}
-
-template <class C2, int N, int NS, int S, bool PS, bool PD, int NT>
-__device__ __forceinline__ void g4_pass(const C2 *s, C2 *d, const C2 *tw, int t) {
-    constexpr int nR = N / 4, tstep = N / (NS * 4);
+// ----------------------------------------------- FP64 lines on the integer pipes
+// The passes of warp_line_filter_ct in block floating point (fft_int.cuh): the warp that owns
+// the line reduces its largest component after every pass with one instruction.  On the FP64
+// pipe the filters were two thirds of the FP64 step: 32 chains of 256 x 128 1.02 -> 0.78 ms,
+// one chain of 64 x 64 in the step loop 22.8 -> 17.8 us.
+struct LineScale {
+    unsigned mx;  // high word of the largest component after the last pass
+    int e;        // shifts so far
+};
+// One pass: butterflies of radix R, twiddles before them (NS > 1).  KIND 0: src holds doubles
+// (the first pass); 1: integers; 2: the middle pass (filter, inverse butterfly; src integers
+// unless it is the only pass); 3: the last pass, which writes doubles.  S: direction.
+template <int N, int R, int NS, int S, bool PS, bool PD, bool PT, int KIND>
+__device__ __forceinline__ void int_pass(const double2 *s, double2 *d, const WCplx *tw, const long long *f, int eg,
+                                         unsigned &raw, LineScale &sc, int lane) {
+    constexpr int nR = N / R, tstep = N / (NS * R), LR = R == 8 ? 3 : (R == 4 ? 2 : 1);
+    constexpr int REP = (nR + 31) / 32;
+    const int sh = KIND == 0 ? LR : ((64 - __clz((int)sc.mx) + LR - kTop) > 0 ? 64 - __clz((int)sc.mx) + LR - kTop : 0);
+    sc.e += sh + (KIND == 2 ? LR : 0);
+    if constexpr (KIND == 0) {
+        unsigned mx = 0;
 #pragma unroll
-    for (int jj = 0; jj < (nR + NT - 1) / NT; ++jj) {
-        const int j = t + NT * jj;
-        if (nR % NT != 0 && j >= nR) break;
+        for (int i = 0; i < N / 32; ++i) {
+            const unsigned m = mag_bits(s[lane + 32 * i]);
+            mx = m > mx ? m : mx;
+        }
+        raw = __reduce_max_sync(0xffffffffu, mx);
+    }
+    const int em = (int)(raw >> 20);
+    unsigned mx = 0;
+#pragma unroll 1
+    for (int jj = 0; jj < REP; ++jj) {
+        const int j = lane + 32 * jj;
+        if (nR % 32 != 0 && j >= nR) break;
         const int k = j & (NS - 1);
-        const C2 *sl = s + (PS ? padi(j) : j);
-        C2 v[4];
+        const double2 *sl = s + (PS ? padi(j) : j);
+        I2 v[R];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            C2 x = sl[PS ? padi(r * nR) : r * nR];
-            if (NS > 1 && r > 0) {
-                C2 w = tw[k * r * tstep];
-                if (S > 0) w.y = -w.y;
-                x = vmul(x, w);
+        for (int r = 0; r < R; ++r) {
+            const double2 *p = sl + (PS ? padi(r * nR) : r * nR);
+            if constexpr (KIND == 0) {
+                const double2 x = *p;
+                v[r] = I2{to_fixed(x.x, em, LR), to_fixed(x.y, em, LR)};
+            } else {
+                v[r] = ishift(*reinterpret_cast<const I2 *>(p), sh);
+                if (NS > 1 && r > 0) {
+                    if constexpr (PT) v[r] = vmul(v[r], tw[(r - 1) * NS + k]);
+                    else if constexpr (S > 0 && KIND != 2) v[r] = vmulc(v[r], tw[k * r * tstep]);
+                    else v[r] = vmul(v[r], tw[k * r * tstep]);
+                }
             }
-            v[r] = x;
         }
-        Radix<C2, 4>::template run<S>(v);
-        const int o = (j / NS) * NS * 4 + k;
-        C2 *dl = d + (PD ? padi(o) : o);
+        Radix<I2, R>::template run<KIND == 2 ? -1 : S>(v);
+        if constexpr (KIND == 2) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) dl[PD ? padi(q * NS) : q * NS] = v[q];
-    }
-}
-
-template <class C2, class RR, int N, bool PS, int NT>
-__device__ __forceinline__ void g4_mid(const C2 *s, C2 *d, const C2 *tw, const RR *f, RR cst, int t) {
-    constexpr int nR = N / 4;
-#pragma unroll
-    for (int jj = 0; jj < (nR + NT - 1) / NT; ++jj) {
-        const int j = t + NT * jj;
-        if (nR % NT != 0 && j >= nR) break;
-        const C2 *sl = s + (PS ? padi(j) : j);
-        C2 v[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            C2 x = sl[PS ? padi(r * nR) : r * nR];
-            if (nR > 1 && r > 0) x = vmul(x, tw[j * r]);
-            v[r] = x;
+            for (int q = 0; q < R; ++q) v[q] = ifilter<LR>(f[j + q * nR], v[q]);
+            Radix<I2, R>::template run<1>(v);
         }
-        Radix<C2, 4>::template run<-1>(v);
-        RR g[4];
+        const int o = KIND == 2 ? j * R : (j / NS) * NS * R + k;
+        double2 *dl = d + (PD ? padi(o) : o);
+        constexpr int st = KIND == 2 ? 1 : NS;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) g[q] = f[j + q * nR] * cst;
-        radix_scaled<C2, 4, 1>(v, g);
-        C2 *dl = d + padi(j * 4);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) dl[q] = v[q];
+        for (int q = 0; q < R; ++q) {
+            double2 *p = dl + (PD ? padi(q * st) : q * st);
+            if constexpr (KIND == 3) {
+                *p = make_double2(from_fixed(v[q].x, em, eg + sc.e), from_fixed(v[q].y, em, eg + sc.e));
+            } else {
+                const unsigned m = imag_bits(v[q]);
+                mx = m > mx ? m : mx;
+                *reinterpret_cast<I2 *>(p) = v[q];
+            }
+        }
     }
+    if constexpr (KIND != 3) sc.mx = __reduce_max_sync(0xffffffffu, mx);
+    __syncwarp();
 }
 
-template <class C2, int N, int P, int NS, int NT>
-__device__ __forceinline__ void g4_fwd(const C2 *&cur, C2 *&nxt, C2 *&oth, const C2 *tw, int t, int id) {
-    if constexpr (NS * 4 < N) {  // every forward pass but the last (done by g4_mid)
-        g4_pass<C2, N, NS, -1, (P > 0), true, NT>(cur, nxt, tw, t);
-        group_sync<NT>(id);
+template <int N, int P, int NS, bool PT>
+__device__ __forceinline__ void int_fwd(const double2 *&cur, double2 *&nxt, double2 *&oth, const WCplx *tw, unsigned &raw,
+                                        LineScale &sc, int lane) {
+    if constexpr (P < p2_nfac(N) - 1) {
+        constexpr int R = p2_fac(N, P);
+        int_pass<N, R, NS, -1, (P > 0), true, PT, (P == 0 ? 0 : 1)>(cur, nxt, PT ? tw + tw_fwd_off(N, P) : tw, nullptr, 0, raw,
+                                                                   sc, lane);
         cur = nxt;
-        C2 *x = nxt; nxt = oth; oth = x;
-        g4_fwd<C2, N, P + 1, NS * 4, NT>(cur, nxt, oth, tw, t, id);
+        double2 *t = nxt; nxt = oth; oth = t;
+        int_fwd<N, P + 1, NS * R, PT>(cur, nxt, oth, tw, raw, sc, lane);
     }
 }
 
-template <class C2, int N, int NS, int NT>
-__device__ __forceinline__ void g4_inv(const C2 *&cur, C2 *&nxt, C2 *&oth, const C2 *tw, int t, int id) {
-    if constexpr (NS < N) {
-        constexpr bool last = NS * 4 == N;  // writes the dense result
-        g4_pass<C2, N, NS, 1, true, !last, NT>(cur, nxt, tw, t);
-        group_sync<NT>(id);
+template <int N, int P, int NS, bool PT>
+__device__ __forceinline__ void int_inv(const double2 *&cur, double2 *&nxt, double2 *&oth, const WCplx *tw, int eg,
+                                        unsigned &raw, LineScale &sc, int lane) {
+    if constexpr (P >= 0) {
+        constexpr int R = p2_fac(N, P);
+        int_pass<N, R, NS, 1, true, (P > 0), PT, (P > 0 ? 1 : 3)>(cur, nxt, PT ? tw + tw_inv_off(N, P) : tw, nullptr, eg, raw,
+                                                                 sc, lane);
         cur = nxt;
-        C2 *x = nxt; nxt = oth; oth = x;
-        g4_inv<C2, N, NS * 4, NT>(cur, nxt, oth, tw, t, id);
+        double2 *t = nxt; nxt = oth; oth = t;
+        int_inv<N, P - 1, NS * R, PT>(cur, nxt, oth, tw, eg, raw, sc, lane);
     }
 }
 
-// N = 4^k, k >= 2: src (dense, read only by the first pass) -> out = X (dense); Y scratch.
-template <class C2, class RR, int N, int NT>
-__device__ __forceinline__ void group_line_filter4(const C2 *src, C2 *X, C2 *Y, const C2 *tw, const RR *f,
-                                                   RR cst, int t, int id) {
-    static_assert(N >= 16 && (N & (N - 1)) == 0 && (N & 0x55555555) != 0, "N = 4^k");
-    // passes: (k - 1) forward, the middle one, (k - 1) inverse = 2k - 1 in all, alternating
-    // X, Y, X, ... from X, so the last (k - 1 odd or even) lands in X when 2k - 1 is odd
-    const C2 *cur = src;
-    C2 *nxt = X, *oth = Y;
-    g4_fwd<C2, N, 0, 1, NT>(cur, nxt, oth, tw, t, id);
-    g4_mid<C2, RR, N, true, NT>(cur, nxt, tw, f, cst, t);
-    group_sync<NT>(id);
+// Same contract as warp_line_filter_ct; f: the component's filter in fixed point relative to
+// 2^eg.
+template <int N, bool PT>
+__device__ __forceinline__ void warp_line_filter_int(const double2 *src, double2 *X, double2 *Y, const WCplx *tw,
+                                                     const long long *f, int eg, int lane) {
+    constexpr int NF = p2_nfac(N), RL = p2_fac(N, NF - 1);
+    static_assert(NF >= 2, "lines of 64 or more sites");
+    const double2 *cur = src;
+    double2 *nxt = X, *oth = Y;
+    unsigned raw = 0;
+    LineScale sc{0, 0};
+    int_fwd<N, 0, 1, PT>(cur, nxt, oth, tw, raw, sc, lane);
+    int_pass<N, RL, N / RL, 1, true, true, PT, 2>(cur, nxt, PT ? tw + tw_mid_off(N) : tw, f, eg, raw, sc, lane);
     cur = nxt;
-    { C2 *x = nxt; nxt = oth; oth = x; }
-    g4_inv<C2, N, 4, NT>(cur, nxt, oth, tw, t, id);
+    { double2 *t = nxt; nxt = oth; oth = t; }
+    int_inv<N, NF - 2, RL, PT>(cur, nxt, oth, tw, eg, raw, sc, lane);
 }
+
+// The line filter of a CTA's warps: tables in shared memory and the call for one line.  N: the
+// compile-time length (per-pass twiddles twT), 0: n at run time (64, 128 or 256; length-n
+// twiddles twS).
+template <class R, int N>
+struct LineFilter;
+template <int N>
+struct LineFilter<float, N> {
+    const float2 *twS, *twT;
+    const float *fS;
+    int n;
+    // fills the tables at smem + 64 (layout fused_ptw_offset); ends without a barrier
+    __device__ __forceinline__ LineFilter(unsigned char *smem, const ChainDev &ch, int n_, int, int) : n(N ? N : n_) {
+        float2 *tw = reinterpret_cast<float2 *>(smem + 64), *pt = reinterpret_cast<float2 *>(smem + fused_ptw_offset(n, 8));
+        float *f = reinterpret_cast<float *>(smem + 64 + n * sizeof(float2));
+        const AxisDev &ax = ch.axis[0];
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            tw[i] = ax.tw32[i];
+            f[i] = ax.filt32[i];
+        }
+        if constexpr (N > 0)
+            for (int i = threadIdx.x; i < tw_entries(N); i += blockDim.x) pt[i] = ax.ptw32[i];
+        twS = tw; twT = pt; fS = f;
+    }
+    // kinetic term of component c's line: src (read only) -> X, scratch Y
+    __device__ __forceinline__ void run(const ChainDev &ch, bool wc, int c, const float2 *src, float2 *X, float2 *Y,
+                                        int lane) const {
+        const float cst = wc ? (float)ch.comp_const[c] : 1.0f;
+        if constexpr (N > 0) {
+            warp_line_filter_ct<float2, float, N, true>(src, X, Y, twT, fS, cst, lane);
+        } else {
+            switch (n) {
+                case 64: warp_line_filter_ct<float2, float, 64>(src, X, Y, twS, fS, cst, lane); break;
+                case 128: warp_line_filter_ct<float2, float, 128>(src, X, Y, twS, fS, cst, lane); break;
+                default: warp_line_filter_ct<float2, float, 256>(src, X, Y, twS, fS, cst, lane); break;
+            }
+        }
+    }
+};
+template <int N>
+struct LineFilter<double, N> {
+    const WCplx *twS, *twT;
+    const long long *fS;
+    int n;
+    __device__ __forceinline__ LineFilter(unsigned char *smem, const ChainDev &ch, int n_, int ncomp, int kinetic)
+        : n(N ? N : n_) {
+        WCplx *tw = reinterpret_cast<WCplx *>(smem + 64), *pt = reinterpret_cast<WCplx *>(smem + fused_ptw_offset(n, 16));
+        long long *f = reinterpret_cast<long long *>(smem + 64 + n * sizeof(WCplx));
+        const AxisDev &ax = ch.axis[0];
+        if constexpr (N == 0)
+            for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = twiddle_fixed(ax.tw64[i]);
+        for (int c = 0; c < ncomp; ++c) {
+            const double cst = kinetic == CLV_KIN_EXP ? ch.comp_const[c] : 1.0;
+            const int e = exp_above(ax.fmax * cst);
+            for (int i = threadIdx.x; i < n; i += blockDim.x) f[c * n + i] = filter_fixed(ax.filt64[i] * cst, e);
+        }
+        if constexpr (N > 0)
+            for (int i = threadIdx.x; i < tw_entries(N); i += blockDim.x) pt[i] = twiddle_fixed(ax.ptw64[i]);
+        twS = tw; twT = pt; fS = f;
+    }
+    __device__ __forceinline__ void run(const ChainDev &ch, bool wc, int c, const double2 *src, double2 *X, double2 *Y,
+                                        int lane) const {
+        const int eg = exp_above(ch.axis[0].fmax * (wc ? ch.comp_const[c] : 1.0));
+        const long long *f = fS + c * n;
+        if constexpr (N > 0) {
+            warp_line_filter_int<N, true>(src, X, Y, twT, f, eg, lane);
+        } else {
+            switch (n) {
+                case 64: warp_line_filter_int<64, false>(src, X, Y, twS, f, eg, lane); break;
+                case 128: warp_line_filter_int<128, false>(src, X, Y, twS, f, eg, lane); break;
+                default: warp_line_filter_int<256, false>(src, X, Y, twS, f, eg, lane); break;
+            }
+        }
+    }
+};
 
 template <class R>
 __device__ __forceinline__ const typename Cx<R>::T *tw_of(const AxisDev &ax);
@@ -379,9 +457,6 @@ fused_step_kernel(const LaunchFused A) {
     const int V = LN ? LN : ch.V, T = ch.nt, cs = LN ? padded_line(LN) : A.comp_stride;
     const int TV = T * V;  // elements of one component of the chain
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem);  // NPS + NQS barriers
-    C2 *twS = reinterpret_cast<C2 *>(smem + 64);
-    R *fS = reinterpret_cast<R *>(smem + 64 + A.tab_n * sizeof(C2));
-    C2 *twT = reinterpret_cast<C2 *>(smem + fused_ptw_offset(A.tab_n, (int)sizeof(C2)));  // LN > 0
     // slot geometry: compile-time for 1D lines of LN sites (the host's formulas, tables of
     // the one filtered axis), so slot addresses are constant offsets
     const int tab_bytes = LN ? fused_tab_bytes(LN, (int)sizeof(C2), LN) : A.tab_bytes;
@@ -411,19 +486,7 @@ fused_step_kernel(const LaunchFused A) {
         for (int i = 0; i < NPS + NQS; ++i) mbar_init(&bars[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // shared copies of the twiddle and filter tables
-    {
-        const C2 *tw = tw_of<R>(ch.axis[0]);
-        const R *f = filt_of<R>(ch.axis[0]);
-        for (int i = threadIdx.x; i < V; i += blockDim.x) {
-            twS[i] = tw[i];
-            fS[i] = f[i];
-        }
-        if constexpr (LN > 0) {
-            const C2 *pt = ptw_of<R>(ch.axis[0]);
-            for (int i = threadIdx.x; i < tw_entries(LN); i += blockDim.x) twT[i] = pt[i];
-        }
-    }
+    const LineFilter<R, LN> lines(smem, ch, V, NC, A.kinetic);  // shared twiddle and filter tables
     __syncthreads();
 
     uint32_t phase = 0, pending = 0;
@@ -466,47 +529,18 @@ fused_step_kernel(const LaunchFused A) {
     const int last_psi = MODEL == CLV_MODEL_REF4 ? tau1 : tau1 - 1;  // last psi time read
     C2 Pp[NC], Kp[NC], Qc[NC];  // psi(tau-1), kin(tau-1), psibar(tau)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = FAST ? 8 : blockDim.x >> 5;
-    // 1D chains: one warp per line (2 NC lines); the remaining warps draw the
-    // Philox noise of the imaginary time into shared memory meanwhile: at FP32 every
-    // component (2 % faster than leaving the third component's block to each site's
-    // thread in the drift phase); at FP64, whose Box-Muller transforms are costly, the
-    // first pair only (8 % faster than all three).
-    constexpr int SMEM_PAIRS = (NC == 3 && sizeof(R) == 8) ? 1 : (NC + 1) / 2;
+    // One warp per line (2 NC lines); the remaining warps draw the Philox noise of the
+    // imaginary time into shared memory meanwhile.
+    constexpr int SMEM_PAIRS = (NC + 1) / 2;
     const bool noise_smem =
         writes && (FAST || A.noise == CLV_NOISE_PHILOX) && 2 * NC < nwarps;
     const bool wc = A.kinetic == CLV_KIN_EXP;
-    // kinetic filter of component c of a 1D slice: src (read only) -> X, scratch Y
-    auto line1d = [&](const C2 *src, C2 *X, C2 *Y, int c) {
-        const R cst = wc ? (R)ch.comp_const[c] : (R)1;
-        if constexpr (LN > 0) warp_line_filter_ct<C2, R, LN, true>(src + c * cs, X + c * cs, Y + c * cs, twT, fS, cst, lane);
-        else line_filter_1d<C2, R>(src + c * cs, X + c * cs, Y + c * cs, V, twS, fS, cst, lane);
-    };
-    // FP64 lines of 256 sites when a CTA filters at most four lines per imaginary time
-    // (the chunks split by field and component halves of the few-CTA problems, e.g. the
-    // reference's own 256 x 32 lattice): two warps per line, so all four SM
-    // sub-partitions' FP64 pipes share the filter instead of one per line.
-    constexpr bool kPairLines = sizeof(R) == 8 && LN == 256 && !FAST;
     // Filter the lines of `mask` (bit job * NC + c: job 0 = psi of src0 -> X0, job 1 =
-    // psibar of src1 -> X1): warp pairs when they fit, else one warp per line.
+    // psibar of src1 -> X1), one warp per line.
     auto filter_lines = [&](int mask, const C2 *src0, C2 *X0, C2 *Y0, const C2 *src1, C2 *X1, C2 *Y1) {
-        const int nl = __popc(mask);
-        if (kPairLines && 2 * nl <= nwarps) {
-            const int g = warp >> 1;
-            if (g < nl) {
-                int m = mask;
-                for (int i = 0; i < g; ++i) m &= m - 1;
-                const int bit = __ffs(m) - 1, job = bit >= NC, c = bit - job * NC;
-                const R cst = wc ? (R)ch.comp_const[c] : (R)1;
-                if constexpr (kPairLines)
-                    group_line_filter4<C2, R, LN, 64>((job ? src1 : src0) + c * cs, (job ? X1 : X0) + c * cs,
-                                                      (job ? Y1 : Y0) + c * cs, twS, fS, cst,
-                                                      threadIdx.x & 63, 1 + g);
-            }
-            return;
-        }
-        if (warp < 2 * NC) {
+        if (warp < 2 * NC && ((mask >> warp) & 1)) {
             const int job = warp >= NC, c = warp - job * NC;
-            if ((mask >> warp) & 1) line1d(job ? src1 : src0, job ? X1 : X0, job ? Y1 : Y0, c);
+            lines.run(ch, wc, c, (job ? src1 : src0) + c * cs, (job ? X1 : X0) + c * cs, (job ? Y1 : Y0) + c * cs, lane);
         }
     };
 
@@ -570,7 +604,7 @@ fused_step_kernel(const LaunchFused A) {
         {
             // kin(tau) -> part0, kinbar(tau+1) -> part1; the field slots stay intact
             // (kin(tau) only feeds the next imaginary time: the chunk's last skips it)
-            if (warp < 2 * NC || (kPairLines && !noise_smem)) {
+            if (warp < 2 * NC) {
                 const int own_lines = cmask & ((1 << NC) - 1);
                 filter_lines(((do_psi && tau + 1 < tau1) ? own_lines : 0) | (do_bar ? own_lines << NC : 0),
                              slot(sp), part0, ybuf0, slot(sq), part1, ybuf1);

@@ -78,7 +78,6 @@ __global__ void __launch_bounds__(256, 1) loop_step_kernel(const LaunchLoop A) {
     constexpr int NC = MODEL == CLV_MODEL_REF4 ? 4 : 3;
     constexpr int CS = padded_line(LN);
     constexpr int SLOT = fused_slot_stride(NC, LN, (int)sizeof(C2));
-    constexpr bool kPairLines = sizeof(R) == 8 && LN == 256;  // as the fused kernel (non-production)
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ double s_dt;
 
@@ -94,22 +93,10 @@ __global__ void __launch_bounds__(256, 1) loop_step_kernel(const LaunchLoop A) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, s = threadIdx.x;
     const bool leader = task.part == 0;  // advances the chain's ChainState
 
-    C2 *twS = reinterpret_cast<C2 *>(smem + 64);
-    R *fS = reinterpret_cast<R *>(smem + 64 + LN * sizeof(C2));
-    C2 *twT = reinterpret_cast<C2 *>(smem + fused_ptw_offset(LN, (int)sizeof(C2)));
     C2 *slots = reinterpret_cast<C2 *>(smem + fused_tab_bytes(LN, (int)sizeof(C2), LN));
     C2 *sPm = slots, *sPc = slots + SLOT, *sPp = slots + 2 * SLOT, *sQc = slots + 3 * SLOT,
        *sQp = slots + 4 * SLOT, *sX = slots + 5 * SLOT, *sY = slots + 6 * SLOT;
-    {
-        const AxisDev &ax = ch.axis[0];
-        const C2 *tw = tw_of<R>(ax), *pt = ptw_of<R>(ax);
-        const R *f = filt_of<R>(ax);
-        for (int i = threadIdx.x; i < LN; i += blockDim.x) {
-            twS[i] = tw[i];
-            fS[i] = f[i];
-        }
-        for (int i = threadIdx.x; i < tw_entries(LN); i += blockDim.x) twT[i] = pt[i];
-    }
+    const LineFilter<R, LN> lines(smem, ch, LN, NC, A.kinetic);
     const bool wc = A.kinetic == CLV_KIN_EXP;
     const DriftConsts<R> dk(ch);
     const uint64_t seed = ch.seed, nstep0 = __ldcg(&st->step);
@@ -119,9 +106,7 @@ __global__ void __launch_bounds__(256, 1) loop_step_kernel(const LaunchLoop A) {
     // draw the CTA's half of the unit normals meanwhile
     const int own_lines = cmask & ((1 << NC) - 1);
     const int mask = do_psi ? own_lines : own_lines << NC;
-    const int nl = __popc(mask);
-    const bool pair = kPairLines && 2 * nl <= 8;
-    const int used = pair ? (1 << (2 * nl)) - 1 : (mask & 0xFF);
+    const int used = mask & 0xFF;
     const int idle = ~used & 0xFF;
     const bool noise_warp = (idle >> warp) & 1;
     const int nthr = __popc(idle) * 32, tn = __popc(idle & ((1 << warp) - 1)) * 32 + lane;
@@ -176,21 +161,9 @@ __global__ void __launch_bounds__(256, 1) loop_step_kernel(const LaunchLoop A) {
         //    kinbar(tau+1)) into sX; unit normals by the idle warps
         {
             const C2 *src = do_psi ? sPm : sQp;
-            if (pair) {
-                const int g = warp >> 1;
-                if (g < nl) {
-                    int m = mask;
-                    for (int i = 0; i < g; ++i) m &= m - 1;
-                    const int bit = __ffs(m) - 1, c = bit - (bit >= NC ? NC : 0);
-                    const R cst = wc ? (R)ch.comp_const[c] : (R)1;
-                    if constexpr (kPairLines)
-                        group_line_filter4<C2, R, LN, 64>(src + c * CS, sX + c * CS, sY + c * CS, twS, fS, cst,
-                                                          threadIdx.x & 63, 1 + g);
-                }
-            } else if ((mask >> warp) & 1) {
+            if ((mask >> warp) & 1) {
                 const int c = warp - (warp >= NC ? NC : 0);
-                const R cst = wc ? (R)ch.comp_const[c] : (R)1;
-                warp_line_filter_ct<C2, R, LN, true>(src + c * CS, sX + c * CS, sY + c * CS, twT, fS, cst, lane);
+                lines.run(ch, wc, c, src + c * CS, sX + c * CS, sY + c * CS, lane);
             }
             if (noise_warp)
                 for (int x = n0 + tn; x < n1; x += nthr) draw(x, nstep);

@@ -236,14 +236,6 @@ __device__ __forceinline__ void copy_async(C2 *s, const C2 *g) {
                  : "memory");
 }
 
-// 2^e as a double, -1022 <= e <= 1023
-__device__ __forceinline__ double pow2(int e) { return __hiloint2double((e + 1023) << 20, 0); }
-// least e with x <= 2^e, x > 0 finite and normal
-__device__ __forceinline__ int exp_above(double x) {
-    const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
-    return e + (((hi & 0xfffff) | __double2loint(x)) != 0);
-}
-
 // TH threads: 128, or 256 for the large slices.
 template <class R, int TH>
 __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5 : 2)) tile_filter_kernel(const LaunchTileFilter A) {
@@ -314,9 +306,7 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
             }
             for (int i = threadIdx.x; i < ax.n; i += blockDim.x) {
                 if constexpr (kInt) {
-                    const double2 w = tw[i];
-                    const double q = 4611686018427387904.0;  // 2^62
-                    tw0[o + i] = WCplx{wsplit(__double2ll_rn(w.x * q)), wsplit(__double2ll_rn(w.y * q))};
+                    tw0[o + i] = twiddle_fixed(tw[i]);
                     f0[o + i] = __double2ll_rn(f[i] * cst);
                 } else {
                     tw0[o + i] = tw[i];
