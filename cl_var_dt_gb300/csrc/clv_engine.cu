@@ -167,10 +167,11 @@ struct clv_engine {
     double *noise_d = nullptr;
     std::vector<SiteTask> site_tasks_h, obs_tasks_h;
     SiteTask *site_tasks = nullptr, *obs_tasks = nullptr;
-    std::vector<ObsTask> s1obs_tasks_h;   // spin-1 observables
-    ObsTask *s1obs_tasks = nullptr;
-    double *s1obs_partials = nullptr;
-    unsigned int *s1obs_arrive = nullptr;
+    std::vector<ObsTask> obs_pairs_h;     // observables
+    ObsTask *obs_pairs = nullptr;
+    double *obs_partials = nullptr, *obs_scratch = nullptr;
+    long long obs_scratch_n = 0;          // doubles (reference model)
+    unsigned int *obs_arrive = nullptr;
     std::vector<LineTask> line_tasks_h[3];
     LineTask *line_tasks[3] = {nullptr, nullptr, nullptr};
     int max_bundle[3] = {0, 0, 0};
@@ -217,12 +218,23 @@ struct clv_engine {
         return CLV_OK;
     }
 
-    LaunchSites sites(bool obs = false) const {
+    LaunchObs obs() const {
+        LaunchObs L{};
+        L.chains = chains_d;
+        L.tasks = obs_pairs;
+        L.ntasks = (int)obs_pairs_h.size();
+        L.psi = psi();
+        L.psic = psic();
+        L.partials = obs_partials;
+        return L;
+    }
+
+    LaunchSites sites() const {
         LaunchSites L{};
         L.chains = chains_d;
         L.state = state_d;
-        L.tasks = obs ? obs_tasks : site_tasks;
-        L.ntasks = obs ? (int)obs_tasks_h.size() : (int)site_tasks_h.size();
+        L.tasks = site_tasks;
+        L.ntasks = (int)site_tasks_h.size();
         L.model = model;
         L.dt_rule = dt_rule;
         L.noise = noise;
@@ -252,6 +264,8 @@ int build_tables(clv_engine *e) {
         std::memcpy(p.bytes.data(), vec.data(), p.bytes.size());
         pend.push_back(std::move(p));
     };
+    long long all_sites = 0;
+    for (auto &p : e->params) all_sites += (long long)p.nx * p.ny * p.nz * p.nt;
     for (int c = 0; c < nch; ++c) {
         const clv_chain_params &p = e->params[c];
         ChainDev &d = e->chains_h[c];
@@ -363,15 +377,18 @@ int build_tables(clv_engine *e) {
         d.site_nblocks = (nsites + kSiteBlock - 1) / kSiteBlock;
         for (int b = 0; b < d.site_nblocks; ++b) e->site_tasks_h.push_back({c, b * kSiteBlock});
         for (int b = 0; b < (d.V + 255) / 256; ++b) e->obs_tasks_h.push_back({c, b * 256});
-        // spin-1 observables: 256 sites x chunks of at most 16 imaginary times
+        // observables: (chunk, site) pairs, chunks of at most 16 imaginary times (spin-1, whose
+        // threads sum in the working precision), fewer where that leaves SMs idle
         {
-            const int nchunk = (p.nt + 15) / 16;
-            d.obs_block0 = (int)e->s1obs_tasks_h.size();
-            for (int k = 0; k < nchunk; ++k)
-                for (int b = 0; b < (d.V + 255) / 256; ++b)
-                    e->s1obs_tasks_h.push_back({c, b * 256, (int)((long long)p.nt * k / nchunk),
-                                                (int)((long long)p.nt * (k + 1) / nchunk)});
-            d.obs_nblocks = (int)e->s1obs_tasks_h.size() - d.obs_block0;
+            const long long per = all_sites / (2LL * 256 * e->num_sms);
+            const int L = (int)std::max<long long>(1, std::min<long long>(e->model == CLV_MODEL_REF4 ? 64 : 16, per));
+            d.obs_nchunk = (p.nt + L - 1) / L;
+            d.obs_block0 = (int)e->obs_pairs_h.size();
+            d.obs_scr = e->obs_scratch_n;
+            const long long pairs = (long long)d.V * d.obs_nchunk;
+            e->obs_scratch_n += 3 * pairs;
+            for (long long f = 0; f < pairs; f += 256) e->obs_pairs_h.push_back({c, (int)f});
+            d.obs_nblocks = (int)e->obs_pairs_h.size() - d.obs_block0;
         }
         // line tasks per axis
         const int budget = e->precision == CLV_PREC_F64 ? kMaxBundleElems64 : kMaxBundleElems32;
@@ -1033,7 +1050,7 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
         // slice) under the exponential kinetic factor, a product over the axes: one
         // plane-filter launch instead of two axis launches
         int pa = -1;
-        if (!energy && e->kinetic == CLV_KIN_EXP && !std::getenv("CLV_NO_PLANE")) {
+        if ((energy || e->kinetic == CLV_KIN_EXP) && !std::getenv("CLV_NO_PLANE")) {
             const int n1 = d.axis[1].n, n2 = d.axis[2].n;
             pa = n2 <= 1 ? (d.axis[0].n == n1 ? 0 : -1) : (n1 == n2 ? 1 : -1);
             const int pn = pa >= 0 ? d.axis[pa].n : 0;
@@ -1041,8 +1058,8 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
             if (pn == 32 || pn == 64 || pn == 96 || pn == 128) {
                 const size_t sm = plane_smem_bytes(pn, esz);
                 if (sm + 1024 <= (size_t)dev_smem) {
-                    if (e->precision == CLV_PREC_F64) CK(setup_plane_filter<double>(pn, sm, &occ));
-                    else CK(setup_plane_filter<float>(pn, sm, &occ));
+                    if (e->precision == CLV_PREC_F64) CK(setup_plane_filter<double>(pn, energy, sm, &occ));
+                    else CK(setup_plane_filter<float>(pn, energy, sm, &occ));
                 }
             }
             if (occ < 1) pa = -1;
@@ -1069,7 +1086,7 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
                     g.pitch = plane_pitch(n);
                     g.W = 1;
                     g.plane = 1;
-                    g.with_const = a == 0;
+                    g.with_const = !energy && a == 0;
                     g.smem = plane_smem_bytes(n, esz);
                     groups.push_back(std::move(g));
                     gi = (int)groups.size() - 1;
@@ -1305,9 +1322,10 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
         (rc = e->alloc(&e->site_tasks, e->site_tasks_h.size() * sizeof(SiteTask))) ||
         (rc = e->alloc(&e->obs_tasks, e->obs_tasks_h.size() * sizeof(SiteTask))) ||
         (rc = e->alloc(&e->partials, e->site_tasks_h.size() * sizeof(double2))) ||
-        (rc = e->alloc(&e->s1obs_tasks, std::max<size_t>(1, e->s1obs_tasks_h.size()) * sizeof(ObsTask))) ||
-        (rc = e->alloc(&e->s1obs_partials, std::max<size_t>(1, e->s1obs_tasks_h.size()) * 8 * sizeof(double))) ||
-        (rc = e->alloc(&e->s1obs_arrive, nch * sizeof(unsigned int))) ||
+        (rc = e->alloc(&e->obs_pairs, e->obs_pairs_h.size() * sizeof(ObsTask))) ||
+        (rc = e->alloc(&e->obs_partials, e->obs_pairs_h.size() * 8 * sizeof(double))) ||
+        (rc = e->alloc(&e->obs_scratch, e->model == CLV_MODEL_REF4 ? e->obs_scratch_n * sizeof(double) : 0)) ||
+        (rc = e->alloc(&e->obs_arrive, nch * sizeof(unsigned int))) ||
         (rc = e->alloc(&e->accF, std::max(1, e->acc_F_total) * sizeof(double))) ||
         (rc = e->alloc(&e->accN, nch * 5 * sizeof(double))) ||
         (rc = e->alloc(&e->samples, (size_t)e->sample_cap * nch * 8 * sizeof(double))) ||
@@ -1351,8 +1369,8 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
     if ((ce = up(e->chains_d, e->chains_h.data(), nch * sizeof(ChainDev))) != cudaSuccess ||
         (ce = up(e->site_tasks, e->site_tasks_h.data(), e->site_tasks_h.size() * sizeof(SiteTask))) != cudaSuccess ||
         (ce = up(e->obs_tasks, e->obs_tasks_h.data(), e->obs_tasks_h.size() * sizeof(SiteTask))) != cudaSuccess ||
-        (ce = up(e->s1obs_tasks, e->s1obs_tasks_h.data(), e->s1obs_tasks_h.size() * sizeof(ObsTask))) != cudaSuccess ||
-        (ce = cudaMemset(e->s1obs_arrive, 0, nch * sizeof(unsigned int))) != cudaSuccess)
+        (ce = up(e->obs_pairs, e->obs_pairs_h.data(), e->obs_pairs_h.size() * sizeof(ObsTask))) != cudaSuccess ||
+        (ce = cudaMemset(e->obs_arrive, 0, nch * sizeof(unsigned int))) != cudaSuccess)
         return bail(fail(CLV_ERR_CUDA, cudaGetErrorString(ce)));
     for (int a = 0; a < 3; ++a)
         if (!e->line_tasks_h[a].empty() &&
@@ -1685,9 +1703,14 @@ int clv_evaluate(clv_engine *e) {
     CK(cudaSetDevice(e->device));
     const int nch = (int)e->params.size();
     if (e->model == CLV_MODEL_REF4) {
-        LaunchSites L = e->sites(true);
-        if (e->precision == CLV_PREC_F64) CK(launch_obs_ref<double>(L, e->accF, e->accN, e->stream));
-        else CK(launch_obs_ref<float>(L, e->accF, e->accN, e->stream));
+        LaunchObs L = e->obs();
+        L.sites = e->obs_tasks;
+        L.nsites = (int)e->obs_tasks_h.size();
+        L.scratch = e->obs_scratch;
+        L.accF = e->accF;
+        L.accN = e->accN;
+        if (e->precision == CLV_PREC_F64) CK(launch_obs_ref<double>(L, e->stream));
+        else CK(launch_obs_ref<float>(L, e->stream));
     } else {
         if (e->sample_count == e->sample_cap) {
             // move the full sample buffer to the host and start over
@@ -1712,15 +1735,9 @@ int clv_evaluate(clv_engine *e) {
                          : run_kinetic<float>(e, e->psi(), nullptr, e->kin, nullptr, 1, 1);
             if (rc) return rc;
         }
-        LaunchObs L{};
-        L.chains = e->chains_d;
-        L.tasks = e->s1obs_tasks;
-        L.ntasks = (int)e->s1obs_tasks_h.size();
-        L.psi = e->psi();
-        L.psic = e->psic();
+        LaunchObs L = e->obs();
         L.tpsi = e->kin;
-        L.partials = e->s1obs_partials;
-        L.arrive = e->s1obs_arrive;
+        L.arrive = e->obs_arrive;
         L.samples = e->samples;
         L.slot = e->sample_count;
         L.nchains = nch;

@@ -83,7 +83,9 @@ struct ChainDev {
     int site_block0, site_nblocks; // range of this chain's blocks in site-parallel kernels
     int fused_block0, fused_nblocks; // range of this chain's CTAs in the fused step kernel
     int obs_off;                   // offset of this chain's F-profile accumulators
-    int obs_block0, obs_nblocks;   // range of this chain's CTAs in the spin-1 observables
+    int obs_block0, obs_nblocks;   // range of this chain's CTAs in the observables
+    int obs_nchunk;                // its chunks of imaginary time there
+    long long obs_scr;             // offset of its (chunk, site) profile sums (three arrays of nchunk V)
 };
 
 // Per-chain mutable step state (device).
@@ -120,12 +122,11 @@ struct FusedTask {
     int cmask;  // components this CTA filters, drifts, updates and stores (bit c); 0: all
 };
 
-// A CTA's share of the spin-1 observables: 256 spatial sites from site0 of one
-// chain over imaginary times [tau0, tau1).
+// A CTA's share of the observables: 256 consecutive (chunk, site) pairs of one chain, the
+// imaginary times split into ChainDev::obs_nchunk chunks.
 struct ObsTask {
     int chain;
-    int site0;
-    int tau0, tau1;
+    int flat0;
 };
 
 // A CTA's share of the kinetic line filter: lines [line0, line0+nlines) of one

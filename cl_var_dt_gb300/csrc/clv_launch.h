@@ -327,7 +327,7 @@ __host__ __device__ constexpr size_t plane_smem_bytes(int n, size_t esz) {
     return plane_tab_bytes(n, esz) + (size_t)n * plane_pitch(n) * esz;
 }
 template <class R> cudaError_t launch_plane_filter(const LaunchAxis &L, cudaStream_t s);
-template <class R> cudaError_t setup_plane_filter(int n, size_t smem_bytes, int *ctas_per_sm);
+template <class R> cudaError_t setup_plane_filter(int n, int energy, size_t smem_bytes, int *ctas_per_sm);
 template <class R> cudaError_t launch_tiled(const LaunchTiled &L, cudaStream_t s);
 template <class R> cudaError_t setup_tiled(int model, int *ctas_per_sm);
 // Axis filter geometry, lines of 32, 64, 96, 128, 256 and 512 sites.  Lines per tile
@@ -368,19 +368,22 @@ template <class R> cudaError_t launch_set_mean_field(const LaunchSites &L, int f
                                                      double im, cudaStream_t s);
 template <class R> cudaError_t launch_init_spin1(const LaunchSites &L, double amp, double sigma,
                                                  cudaStream_t s);
-template <class R> cudaError_t launch_obs_ref(const LaunchSites &L, double *accF, double *accN,
-                                              cudaStream_t s);
-// Spin-1 observables: CTA = 256 spatial sites of one chain x imaginary times [tau0, tau1).
+// Observables (k_obs.cu); reference model: the (chunk, site) sums, then their reduction.
 struct LaunchObs {
     const ChainDev *chains;
     const ObsTask *tasks;
     int ntasks;
+    const SiteTask *sites;  // reference model: 256 sites of one chain per CTA of the reduction
+    int nsites;
     const void *psi, *psic, *tpsi;
     double *partials;       // 8 per task
     unsigned int *arrive;   // per chain, zero between launches
     double *samples;        // [slot][chain][8]
     int slot, nchains;
+    double *scratch;        // reference model: profile sums of every (chunk, site)
+    double *accF, *accN;
 };
+template <class R> cudaError_t launch_obs_ref(const LaunchObs &L, cudaStream_t s);
 template <class R> cudaError_t launch_obs_spin1(const LaunchObs &L, cudaStream_t s);
 // complex128 boundary layout <-> engine precision (same element order)
 template <class R> cudaError_t launch_import(void *dst, const double2 *src, long long n,

@@ -114,8 +114,9 @@ struct InPlace {
 
     // The last forward pass (span R_last, no twiddles), the filter f at each output's
     // frequency, and the first inverse pass, in registers.
-    template <class C2, class RR>
-    static __device__ __forceinline__ void mid(C2 *t, int LS, int ES, const RR *f) {
+    // fo: a share per line added to the filter (sum of two axes' filters), or null.
+    template <class C2, class RR, bool SUM = false>
+    static __device__ __forceinline__ void mid(C2 *t, int LS, int ES, const RR *f, const RR *fo = nullptr) {
         constexpr int nR = N / RL, NB = NL * nR, PER = (NB + T - 1) / T;
 #pragma unroll(U)
         for (int p = 0; p < PER; ++p) {
@@ -130,11 +131,12 @@ struct InPlace {
             if constexpr (sizeof(RR) == 8) {
                 RR g[RL];
 #pragma unroll
-                for (int q = 0; q < RL; ++q) g[q] = f[fj + q * nR];
+                for (int q = 0; q < RL; ++q) g[q] = SUM ? f[fj + q * nR] + fo[l] : f[fj + q * nR];
                 radix_scaled<C2, RL, 1>(v, g);
             } else {  // (value by value: the FP32 planes run at their register caps)
+                const RR o = SUM ? fo[l] : (RR)0;
 #pragma unroll
-                for (int q = 0; q < RL; ++q) v[q] = vscale(f[fj + q * nR], v[q]);
+                for (int q = 0; q < RL; ++q) v[q] = vscale(SUM ? f[fj + q * nR] + o : f[fj + q * nR], v[q]);
                 Radix<C2, RL>::template run<1>(v);
             }
 #pragma unroll
@@ -193,6 +195,31 @@ struct InPlace {
             __syncthreads();
             inv<C2, P - 1, P_END>(t, LS, ES, tw);
         }
+    }
+
+    // Frequency at position i after all forward passes.
+    template <int P = 0, int W = 1>
+    static __device__ __forceinline__ int freq(int i) {
+        if constexpr (P >= NF) {
+            return 0;
+        } else {
+            constexpr int S = span(P + 1);
+            const int q = i / S;
+            return q * W + freq<P + 1, W * Plan::fac(N, P)>(i - q * S);
+        }
+    }
+    // Transform of all lines to digit-reversed frequencies (from forward pass P on) and back.
+    template <class C2, int P>
+    static __device__ __forceinline__ void forward(C2 *t, int LS, int ES, const C2 *tw) {
+        if constexpr (P < NF) {
+            dif<C2, P>(t, LS, ES, tw);
+            __syncthreads();
+            forward<C2, P + 1>(t, LS, ES, tw);
+        }
+    }
+    template <class C2>
+    static __device__ __forceinline__ void backward(C2 *t, int LS, int ES, const C2 *tw) {
+        inv<C2, NF - 1>(t, LS, ES, tw);
     }
 
     // Filter all NL lines of the tile along their axis, in place, from forward pass P0
