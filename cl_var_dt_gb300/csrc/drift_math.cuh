@@ -45,14 +45,14 @@ template <class R, class C2> __device__ __forceinline__ C2 xmsub(C2 s, C2 a, C2 
 // Per-chain constants of the drift in the working precision, loaded once per CTA.
 template <class R>
 struct DriftConsts {
-    R eps, pre, g2, c0, c1, ec0, ec1;
+    R eps, pre, g2, ec0, ec1;
     R mu[4];
+    bool scaled;  // a_x is not 1 (a product with 1 is left out)
     __device__ __forceinline__ explicit DriftConsts(const ChainDev &ch) {
         eps = (R)ch.eps;
         pre = (R)ch.a_x;
         g2 = (R)(2 * ch.G);
-        c0 = (R)ch.c0;
-        c1 = (R)ch.c1;
+        scaled = pre != (R)1;
         ec0 = (R)(ch.eps * ch.c0);  // spin-1: eps c0 and eps c1 (the drift's prefactors)
         ec1 = (R)(ch.eps * ch.c1);
         mu[0] = (R)(ch.mu + ch.P + ch.Q);
@@ -72,7 +72,7 @@ struct DriftConsts {
 //   t_0 = S k_0 + b_3 D,  t_1 = S k_1 - b_2 D,  t_2 = S k_2 - b_1 D,  t_3 = S k_3 + b_0 D
 // (the reference adds three densities and one exchange product per component; the
 // density it leaves out is b_{3-a} k_{3-a}, whose product with k_a is D's second term).
-// 87 FP64 operations per field instead of 144 in the component-wise form: the
+// 80 FP64 operations per field (88 when a_x is not 1) instead of 144 in the component-wise form: the
 // reference model's reduce pass is bound by the FP64 pipe (2 operations per clock and SM):
 // 1.73 -> 1.17 ms on 128 x 128 x 128 imaginary times.
 template <class R, class C2>
@@ -103,8 +103,9 @@ __device__ __forceinline__ void drift_ref4_vals(const DriftConsts<R> &k, const C
             m.y = S.y;
             C2 in = xmadd<R>(km[a], m, pm[a]);
             in = (a == 0 || a == 3) ? xmadd<R>(in, cc[3 - a], D) : xmsub<R>(in, cc[3 - a], D);
-            K[a].x = mul_rn<R>(pre, fma_rn<R>(eps, in.x, add_rn<R>(pm[a].x, -pc[a].x)));
-            K[a].y = mul_rn<R>(pre, fma_rn<R>(eps, in.y, add_rn<R>(pm[a].y, -pc[a].y)));
+            K[a].x = fma_rn<R>(eps, in.x, add_rn<R>(pm[a].x, -pc[a].x));
+            K[a].y = fma_rn<R>(eps, in.y, add_rn<R>(pm[a].y, -pc[a].y));
+            if (k.scaled) K[a] = xscale<R>(pre, K[a]);
         }
     }
     if (which & 2) {
@@ -119,8 +120,9 @@ __device__ __forceinline__ void drift_ref4_vals(const DriftConsts<R> &k, const C
             in.y = fma_rn<R>(mu[a], pp[a].y, kp[a].y);
             in = xmadd<R>(in, S, cp[a]);
             in = (a == 0 || a == 3) ? xmadd<R>(in, pc[3 - a], D) : xmsub<R>(in, pc[3 - a], D);
-            Kc[a].x = mul_rn<R>(pre, fma_rn<R>(eps, in.x, add_rn<R>(cp[a].x, -cc[a].x)));
-            Kc[a].y = mul_rn<R>(pre, fma_rn<R>(eps, in.y, add_rn<R>(cp[a].y, -cc[a].y)));
+            Kc[a].x = fma_rn<R>(eps, in.x, add_rn<R>(cp[a].x, -cc[a].x));
+            Kc[a].y = fma_rn<R>(eps, in.y, add_rn<R>(cp[a].y, -cc[a].y));
+            if (k.scaled) Kc[a] = xscale<R>(pre, Kc[a]);
         }
     }
 }
@@ -186,21 +188,13 @@ __device__ __forceinline__ R abs2(C2 z) {
     return fma_rn<R>(z.x, z.x, mul_rn<R>(z.y, z.y));
 }
 
-// psi + dt K + z, rounded step by step as the reference's kernels do
-// (multiply_by_timestep, add_noise, summation); conj = 1 adds conj(z).  FP32,
-// which has no counterpart in the reference to match bit for bit, rounds dt K + z
-// once (fused multiply-add).
+// psi + dt K + z (multiply_by_timestep, add_noise, summation); conj = 1 adds conj(z).  dt K + z
+// is rounded once (fused multiply-add).
 template <class R, class C2>
 __device__ __forceinline__ C2 langevin_update(C2 p, C2 K, R dt, C2 z, bool conj) {
     C2 o;
-    const R zy = conj ? -z.y : z.y;
-    if constexpr (sizeof(R) == 4) {
-        o.x = __fadd_rn(p.x, __fmaf_rn(K.x, dt, z.x));
-        o.y = __fadd_rn(p.y, __fmaf_rn(K.y, dt, zy));
-    } else {
-        o.x = add_rn<R>(p.x, add_rn<R>(mul_rn<R>(K.x, dt), z.x));
-        o.y = add_rn<R>(p.y, add_rn<R>(mul_rn<R>(K.y, dt), zy));
-    }
+    o.x = add_rn<R>(p.x, fma_rn<R>(K.x, dt, z.x));
+    o.y = add_rn<R>(p.y, fma_rn<R>(K.y, dt, conj ? -z.y : z.y));
     return o;
 }
 
