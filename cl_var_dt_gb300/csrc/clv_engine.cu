@@ -129,7 +129,7 @@ struct clv_engine {
     bool fused_split = false;  // psi and psibar in separate CTAs (build_fused_tasks)
     // step loop (k_loop.cu): resident CTAs of the loop kernel per SM (0: not available)
     int loop_per_sm = 0;
-    unsigned int *loop_sync = nullptr;  // grid barrier counter and abort flag
+    unsigned int *loop_sync = nullptr;  // the step loop's arrival flags and abort flag
     void *loop_noise = nullptr;         // a step's unit normals (field layout), allocated for problems it fits
     // tiled path (slices too large for the fused kernel): per-axis filter
     // launches grouped by (axis, line length), then the tau-streaming step
@@ -643,7 +643,8 @@ int enqueue_loop(clv_engine *e, int nsteps, EventTrail *trail, int *done = nullp
     if (done) *done = 0;
     while (nsteps > 0) {
         const int n = std::min(nsteps, 1 << 16);
-        CK(cudaMemsetAsync(e->loop_sync, 0, 2 * sizeof(unsigned int), e->stream));
+        const size_t ntasks = e->fused_tasks_h.size();
+        CK(cudaMemsetAsync(e->loop_sync, 0, (2 * ntasks + 1) * sizeof(unsigned int), e->stream));
         if (trail) CK(trail->mark(e->stream));
         LaunchLoop L{};
         L.chains = e->chains_d;
@@ -660,8 +661,9 @@ int enqueue_loop(clv_engine *e, int nsteps, EventTrail *trail, int *done = nullp
         L.from = e->cur;
         L.noise = e->loop_noise;
         L.partials = e->fused_partials;
+        L.part_stride = (int)e->task_capacity;
         L.bar = e->loop_sync;
-        L.abort = reinterpret_cast<int *>(e->loop_sync + 1);
+        L.abort = reinterpret_cast<int *>(e->loop_sync + 2 * ntasks);
         L.withhold = e->withhold_copy;
         const cudaError_t le = launch_loop<R>(L, e->stream);
         if (le == cudaErrorCooperativeLaunchTooLarge) {
@@ -1314,7 +1316,7 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
         (rc = e->alloc(&e->kin, fb)) || (rc = e->alloc(&e->kinc, fb_scratch)) ||
         (rc = e->alloc(&e->drift, fb_drift)) || (rc = e->alloc(&e->driftc, fb_drift)) ||
         (rc = e->alloc(&e->fused_tasks, (e->fused ? nparts : 1) * sizeof(FusedTask))) ||
-        (rc = e->alloc(&e->fused_partials, nparts * sizeof(double2))) ||
+        (rc = e->alloc(&e->fused_partials, (e->loop_per_sm > 0 ? 2 : 1) * nparts * sizeof(double2))) ||
         (rc = e->alloc(&e->tile_tasks, (e->tiled ? nparts : 1) * sizeof(TileTask))) ||
         (rc = e->alloc(&e->stage, 2 * e->max_chain_elems * sizeof(double2))) ||
         (rc = e->alloc(&e->chains_d, nch * sizeof(ChainDev))) ||
@@ -1329,7 +1331,7 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
         (rc = e->alloc(&e->accF, std::max(1, e->acc_F_total) * sizeof(double))) ||
         (rc = e->alloc(&e->accN, nch * 5 * sizeof(double))) ||
         (rc = e->alloc(&e->samples, (size_t)e->sample_cap * nch * 8 * sizeof(double))) ||
-        (rc = e->alloc(&e->loop_sync, 2 * sizeof(unsigned int))))
+        (rc = e->alloc(&e->loop_sync, (e->loop_per_sm > 0 ? 2 * nparts + 1 : 1) * sizeof(unsigned int))))
         return bail(rc);
     {
         // the step loop's normals: for problems whose split tasks of one imaginary time

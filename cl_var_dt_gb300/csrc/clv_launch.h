@@ -84,9 +84,10 @@ struct LaunchLoop {
     int from;             // buffer set the first step reads
     void *noise;          // unit normals of the current step (field layout), exchanged by the CTA pairs
     double2 *partials;
-    unsigned int *bar;    // grid barrier arrivals, zero at launch
-    int *abort;           // set when a barrier wait gives up, zero at launch
-    int withhold;         // failure-detection test: CTA 0 never arrives at the first barrier
+    int part_stride;      // partials of odd steps follow those of even ones
+    unsigned int *bar;    // arrival flags, zero at launch: the first of a step per CTA, then the second
+    int *abort;           // set when a wait gives up, zero at launch
+    int withhold;         // failure-detection test: CTA 0 never arrives
 };
 
 // Compile-time plans of power-of-two lines: factor order 8, 8, ..., then 4 or 2
@@ -187,13 +188,13 @@ __host__ __device__ inline int pass_twiddle_source(int n, int e, bool *conj) {
 
 // Shared memory of the fused kernel before its slots: barriers (64 B), the
 // twiddle and filter tables of tab_n entries (FP64: a filter table per component, its
-// constant folded in), the per-pass twiddles of the compile-time plan of ln-site lines
-// (ln > 0), rounded up to 128 B.
+// constant folded in), at FP32 the per-pass twiddles of the compile-time plan of ln-site
+// lines (ln > 0), rounded up to 128 B.
 __host__ __device__ constexpr int fused_ptw_offset(int tab_n, int esz) {
     return (64 + tab_n * (esz + esz / 2 * (esz == 16 ? kMaxComp : 1)) + 15) / 16 * 16;
 }
 __host__ __device__ constexpr int fused_tab_bytes(int tab_n, int esz, int ln) {
-    return (fused_ptw_offset(tab_n, esz) + (ln > 0 ? tw_entries(ln) : 0) * esz + 127) / 128 * 128;
+    return (fused_ptw_offset(tab_n, esz) + (ln > 0 && esz == 8 ? tw_entries(ln) : 0) * esz + 127) / 128 * 128;
 }
 
 // Elements of a padded FFT scratch line of n sites (one spare element per 16, even).

@@ -211,125 +211,180 @@ static_assert(tw_mid_off(256) == 56 && tw_inv_off(256, 1) == 248 && tw_inv_off(2
 static_assert(tw_entries(128) == 56 + 64 + 14 + 112 && tw_entries(64) == 56 + 56, "pass-table sizes");
 
 // ----------------------------------------------- FP64 lines on the integer pipes
-// The passes of warp_line_filter_ct in block floating point (fft_int.cuh): the warp that owns
-// the line reduces its largest component after every pass with one instruction.  On the FP64
-// pipe the filters were two thirds of the FP64 step: 32 chains of 256 x 128 1.02 -> 0.78 ms,
-// one chain of 64 x 64 in the step loop 22.8 -> 17.8 us.
-struct LineScale {
-    unsigned mx;  // high word of the largest component after the last pass
-    int e;        // shifts so far
-};
-// One pass: butterflies of radix R, twiddles before them (NS > 1).  KIND 0: src holds doubles
-// (the first pass); 1: integers; 2: the middle pass (filter, inverse butterfly; src integers
-// unless it is the only pass); 3: the last pass, which writes doubles.  S: direction.
-template <int N, int R, int NS, int S, bool PS, bool PD, bool PT, int KIND>
-__device__ __forceinline__ void int_pass(const double2 *s, double2 *d, const WCplx *tw, const long long *f, int eg,
-                                         unsigned &raw, LineScale &sc, int lane) {
-    constexpr int nR = N / R, tstep = N / (NS * R), LR = R == 8 ? 3 : (R == 4 ? 2 : 1);
-    constexpr int REP = (nR + 31) / 32;
-    const int sh = KIND == 0 ? LR : ((64 - __clz((int)sc.mx) + LR - kTop) > 0 ? 64 - __clz((int)sc.mx) + LR - kTop : 0);
-    sc.e += sh + (KIND == 2 ? LR : 0);
-    if constexpr (KIND == 0) {
-        unsigned mx = 0;
-#pragma unroll
-        for (int i = 0; i < N / 32; ++i) {
-            const unsigned m = mag_bits(s[lane + 32 * i]);
-            mx = m > mx ? m : mx;
+// Filter of one contiguous line of N = 64, 128 or 256 sites in block floating point
+// (fft_int.cuh) by NT = 32 threads of a warp or 64 of two: Stockham passes of radix 4 (N = 128:
+// the middle pass of radix 2), one reduction of the line's largest component after each.  The
+// passes of a direction are one loop: unrolled radix-8 passes, executed once per line, spent
+// most of their time fetching instructions (a 256-site line of the step loop 15400 clocks).
+// The result does not depend on NT.
+template <int NT>
+__device__ __forceinline__ void group_sync(int id) {
+    if constexpr (NT == 32) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(NT) : "memory");
+}
+
+template <int N, int NT>
+struct IntLine {
+    static constexpr int LOG = N == 64 ? 6 : (N == 128 ? 7 : 8);
+    static constexpr int K4 = (LOG - 1) / 2, RL = N >> (2 * K4);  // forward radix-4 passes, the middle radix
+    static constexpr int NB = N / 4, REP = (NB + NT - 1) / NT;
+    static_assert((N == 64 || N == 128 || N == 256) && (RL == 2 || RL == 4), "lines of 64, 128 or 256 sites");
+
+    int t, id;
+    unsigned *slots;  // NT = 64: four words of shared memory of the group
+    int par;
+    unsigned mx;      // high word of the line's largest component
+    int e;            // shifts so far
+
+    // largest of the group's values, after everything it wrote to shared memory is visible
+    __device__ __forceinline__ unsigned reduce(unsigned m) {
+        m = __reduce_max_sync(0xffffffffu, m);
+        if constexpr (NT == 32) {
+            __syncwarp();
+        } else {
+            if ((t & 31) == 0) slots[2 * par + (t >> 5)] = m;
+            group_sync<NT>(id);
+            const unsigned a = slots[2 * par], b = slots[2 * par + 1];
+            m = a > b ? a : b;
+            par ^= 1;
         }
-        raw = __reduce_max_sync(0xffffffffu, mx);
+        return m;
     }
-    const int em = (int)(raw >> 20);
-    unsigned mx = 0;
-#pragma unroll 1
-    for (int jj = 0; jj < REP; ++jj) {
-        const int j = lane + 32 * jj;
-        if (nR % 32 != 0 && j >= nR) break;
-        const int k = j & (NS - 1);
-        const double2 *sl = s + (PS ? padi(j) : j);
-        I2 v[R];
+    __device__ __forceinline__ void track(unsigned &m, const I2 &v) {
+        const unsigned u = imag_bits(v);
+        m = u > m ? u : m;
+    }
+
+    // src (doubles, read only) -> X (doubles), scratch Y; tw: length-N table, f: the component's
+    // filter relative to 2^eg
+    __device__ __forceinline__ void run(const double2 *src, double2 *X, double2 *Y, const WCplx *tw, const long long *f,
+                                        int eg) {
+        par = 0;
+        unsigned m = 0;
+        double2 d[REP][4];
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const double2 *p = sl + (PS ? padi(r * nR) : r * nR);
-            if constexpr (KIND == 0) {
-                const double2 x = *p;
-                v[r] = I2{to_fixed(x.x, em, LR), to_fixed(x.y, em, LR)};
-            } else {
-                v[r] = ishift(*reinterpret_cast<const I2 *>(p), sh);
-                if (NS > 1 && r > 0) {
-                    if constexpr (PT) v[r] = vmul(v[r], tw[(r - 1) * NS + k]);
-                    else if constexpr (S > 0 && KIND != 2) v[r] = vmulc(v[r], tw[k * r * tstep]);
-                    else v[r] = vmul(v[r], tw[k * r * tstep]);
+        for (int i = 0; i < REP; ++i) {
+            const int j = t + NT * i;
+            if (NB % NT == 0 || j < NB)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    d[i][r] = src[j + r * NB];
+                    const unsigned u = mag_bits(d[i][r]);
+                    m = u > m ? u : m;
+                }
+        }
+        const int em = (int)(reduce(m) >> 20);
+        e = 2;
+        m = 0;
+#pragma unroll
+        for (int i = 0; i < REP; ++i) {
+            const int j = t + NT * i;
+            if (NB % NT == 0 || j < NB) {
+                I2 v[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) v[r] = I2{to_fixed(d[i][r].x, em, 2), to_fixed(d[i][r].y, em, 2)};
+                Radix<I2, 4>::template run<-1>(v);
+                I2 *o = reinterpret_cast<I2 *>(X);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    track(m, v[q]);
+                    o[padi(4 * j + q)] = v[q];
                 }
             }
         }
-        Radix<I2, R>::template run<KIND == 2 ? -1 : S>(v);
-        if constexpr (KIND == 2) {
-#pragma unroll
-            for (int q = 0; q < R; ++q) v[q] = ifilter<LR>(f[j + q * nR], v[q]);
-            Radix<I2, R>::template run<1>(v);
+        mx = reduce(m);
+        const I2 *cur = reinterpret_cast<const I2 *>(X);
+        I2 *nxt = reinterpret_cast<I2 *>(Y), *oth = reinterpret_cast<I2 *>(X);
+        auto swap = [&]() {
+            cur = nxt;
+            I2 *x = nxt;
+            nxt = oth;
+            oth = x;
+        };
+#pragma unroll 1
+        for (int p = 1; p < K4; ++p) {
+            pass<-1, false>(cur, nxt, tw, 2 * p, 0, 0);
+            swap();
         }
-        const int o = KIND == 2 ? j * R : (j / NS) * NS * R + k;
-        double2 *dl = d + (PD ? padi(o) : o);
-        constexpr int st = KIND == 2 ? 1 : NS;
+        middle(cur, nxt, tw, f);
+        swap();
+#pragma unroll 1
+        for (int p = 0; p < K4 - 1; ++p) {
+            pass<1, false>(cur, nxt, tw, LOG - 2 * K4 + 2 * p, 0, 0);
+            swap();
+        }
+        pass<1, true>(cur, nxt, tw, LOG - 2, em, eg);
+    }
+
+    // Radix-4 pass at stride NS = 2^ls; LAST: writes doubles, dense.
+    template <int S, bool LAST>
+    __device__ __forceinline__ void pass(const I2 *s, I2 *dst, const WCplx *tw, int ls, int em, int eg) {
+        const int sh = ishift_for(mx, 2);
+        e += sh;
+        unsigned m = 0;
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-            double2 *p = dl + (PD ? padi(q * st) : q * st);
-            if constexpr (KIND == 3) {
-                *p = make_double2(from_fixed(v[q].x, em, eg + sc.e), from_fixed(v[q].y, em, eg + sc.e));
-            } else {
-                const unsigned m = imag_bits(v[q]);
-                mx = m > mx ? m : mx;
-                *reinterpret_cast<I2 *>(p) = v[q];
+        for (int i = 0; i < REP; ++i) {
+            const int j = t + NT * i;
+            if (NB % NT == 0 || j < NB) {
+                const int k = j & ((1 << ls) - 1);
+                const I2 *sl = s + padi(j);
+                I2 v[4];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    v[r] = ishift(sl[padi(r * NB)], sh);
+                    if (r > 0) {
+                        const WCplx w = tw[(k * r) << (LOG - 2 - ls)];
+                        v[r] = S < 0 ? vmul(v[r], w) : vmulc(v[r], w);
+                    }
+                }
+                Radix<I2, 4>::template run<S>(v);
+                const int o = ((j >> ls) << (ls + 2)) + k;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if constexpr (LAST) {
+                        reinterpret_cast<double2 *>(dst)[o + (q << ls)] =
+                            make_double2(from_fixed(v[q].x, em, eg + e), from_fixed(v[q].y, em, eg + e));
+                    } else {
+                        track(m, v[q]);
+                        dst[padi(o + (q << ls))] = v[q];
+                    }
+                }
             }
         }
+        if constexpr (LAST) group_sync<NT>(id);
+        else mx = reduce(m);
     }
-    if constexpr (KIND != 3) sc.mx = __reduce_max_sync(0xffffffffu, mx);
-    __syncwarp();
-}
 
-template <int N, int P, int NS, bool PT>
-__device__ __forceinline__ void int_fwd(const double2 *&cur, double2 *&nxt, double2 *&oth, const WCplx *tw, unsigned &raw,
-                                        LineScale &sc, int lane) {
-    if constexpr (P < p2_nfac(N) - 1) {
-        constexpr int R = p2_fac(N, P);
-        int_pass<N, R, NS, -1, (P > 0), true, PT, (P == 0 ? 0 : 1)>(cur, nxt, PT ? tw + tw_fwd_off(N, P) : tw, nullptr, 0, raw,
-                                                                   sc, lane);
-        cur = nxt;
-        double2 *t = nxt; nxt = oth; oth = t;
-        int_fwd<N, P + 1, NS * R, PT>(cur, nxt, oth, tw, raw, sc, lane);
+    // Last forward pass, filter, first inverse pass.
+    __device__ __forceinline__ void middle(const I2 *s, I2 *dst, const WCplx *tw, const long long *f) {
+        constexpr int LR = RL == 4 ? 2 : 1, NM = N / RL, REPM = (NM + NT - 1) / NT;
+        const int sh = ishift_for(mx, LR);
+        e += sh + LR;
+        unsigned m = 0;
+#pragma unroll
+        for (int i = 0; i < REPM; ++i) {
+            const int j = t + NT * i;
+            if (NM % NT == 0 || j < NM) {
+                I2 v[RL];
+#pragma unroll
+                for (int r = 0; r < RL; ++r) {
+                    v[r] = ishift(s[padi(j + r * NM)], sh);
+                    if (r > 0) v[r] = vmul(v[r], tw[j * r]);
+                }
+                Radix<I2, RL>::template run<-1>(v);
+#pragma unroll
+                for (int q = 0; q < RL; ++q) v[q] = ifilter<LR>(f[j + q * NM], v[q]);
+                Radix<I2, RL>::template run<1>(v);
+#pragma unroll
+                for (int q = 0; q < RL; ++q) {
+                    track(m, v[q]);
+                    dst[padi(j * RL + q)] = v[q];
+                }
+            }
+        }
+        mx = reduce(m);
     }
-}
-
-template <int N, int P, int NS, bool PT>
-__device__ __forceinline__ void int_inv(const double2 *&cur, double2 *&nxt, double2 *&oth, const WCplx *tw, int eg,
-                                        unsigned &raw, LineScale &sc, int lane) {
-    if constexpr (P >= 0) {
-        constexpr int R = p2_fac(N, P);
-        int_pass<N, R, NS, 1, true, (P > 0), PT, (P > 0 ? 1 : 3)>(cur, nxt, PT ? tw + tw_inv_off(N, P) : tw, nullptr, eg, raw,
-                                                                 sc, lane);
-        cur = nxt;
-        double2 *t = nxt; nxt = oth; oth = t;
-        int_inv<N, P - 1, NS * R, PT>(cur, nxt, oth, tw, eg, raw, sc, lane);
-    }
-}
-
-// Same contract as warp_line_filter_ct; f: the component's filter in fixed point relative to
-// 2^eg.
-template <int N, bool PT>
-__device__ __forceinline__ void warp_line_filter_int(const double2 *src, double2 *X, double2 *Y, const WCplx *tw,
-                                                     const long long *f, int eg, int lane) {
-    constexpr int NF = p2_nfac(N), RL = p2_fac(N, NF - 1);
-    static_assert(NF >= 2, "lines of 64 or more sites");
-    const double2 *cur = src;
-    double2 *nxt = X, *oth = Y;
-    unsigned raw = 0;
-    LineScale sc{0, 0};
-    int_fwd<N, 0, 1, PT>(cur, nxt, oth, tw, raw, sc, lane);
-    int_pass<N, RL, N / RL, 1, true, true, PT, 2>(cur, nxt, PT ? tw + tw_mid_off(N) : tw, f, eg, raw, sc, lane);
-    cur = nxt;
-    { double2 *t = nxt; nxt = oth; oth = t; }
-    int_inv<N, NF - 2, RL, PT>(cur, nxt, oth, tw, eg, raw, sc, lane);
-}
+};
 
 // The line filter of a CTA's warps: tables in shared memory and the call for one line.  N: the
 // compile-time length (per-pass twiddles twT), 0: n at run time (64, 128 or 256; length-n
@@ -355,8 +410,10 @@ struct LineFilter<float, N> {
         twS = tw; twT = pt; fS = f;
     }
     // kinetic term of component c's line: src (read only) -> X, scratch Y
+    template <int NT = 32>
     __device__ __forceinline__ void run(const ChainDev &ch, bool wc, int c, const float2 *src, float2 *X, float2 *Y,
-                                        int lane) const {
+                                        int lane, int = 0) const {
+        static_assert(NT == 32, "FP32 lines take one warp");
         const float cst = wc ? (float)ch.comp_const[c] : 1.0f;
         if constexpr (N > 0) {
             warp_line_filter_ct<float2, float, N, true>(src, X, Y, twT, fS, cst, lane);
@@ -371,36 +428,48 @@ struct LineFilter<float, N> {
 };
 template <int N>
 struct LineFilter<double, N> {
-    const WCplx *twS, *twT;
+    const WCplx *twS;
     const long long *fS;
+    unsigned *slots;  // four words for each of four 64-thread groups
     int n;
     __device__ __forceinline__ LineFilter(unsigned char *smem, const ChainDev &ch, int n_, int ncomp, int kinetic)
         : n(N ? N : n_) {
-        WCplx *tw = reinterpret_cast<WCplx *>(smem + 64), *pt = reinterpret_cast<WCplx *>(smem + fused_ptw_offset(n, 16));
+        WCplx *tw = reinterpret_cast<WCplx *>(smem + 64);
         long long *f = reinterpret_cast<long long *>(smem + 64 + n * sizeof(WCplx));
         const AxisDev &ax = ch.axis[0];
-        if constexpr (N == 0)
-            for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = twiddle_fixed(ax.tw64[i]);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = twiddle_fixed(ax.tw64[i]);
         for (int c = 0; c < ncomp; ++c) {
             const double cst = kinetic == CLV_KIN_EXP ? ch.comp_const[c] : 1.0;
             const int e = exp_above(ax.fmax * cst);
             for (int i = threadIdx.x; i < n; i += blockDim.x) f[c * n + i] = filter_fixed(ax.filt64[i] * cst, e);
         }
-        if constexpr (N > 0)
-            for (int i = threadIdx.x; i < tw_entries(N); i += blockDim.x) pt[i] = twiddle_fixed(ax.ptw64[i]);
-        twS = tw; twT = pt; fS = f;
+        __shared__ unsigned sl[16];
+        slots = sl;
+        twS = tw; fS = f;
     }
+    template <int LEN, int NT>
+    __device__ __forceinline__ void line(const double2 *src, double2 *X, double2 *Y, const long long *f, int eg, int t,
+                                         int g) const {
+        IntLine<LEN, NT> l;
+        l.t = t;
+        l.id = 1 + g;
+        l.slots = slots + 4 * g;
+        l.run(src, X, Y, twS, f, eg);
+    }
+    // kinetic term of component c's line by thread t of NT: src (read only) -> X, scratch Y; g: the
+    // group's number when NT = 64
+    template <int NT = 32>
     __device__ __forceinline__ void run(const ChainDev &ch, bool wc, int c, const double2 *src, double2 *X, double2 *Y,
-                                        int lane) const {
+                                        int t, int g = 0) const {
         const int eg = exp_above(ch.axis[0].fmax * (wc ? ch.comp_const[c] : 1.0));
         const long long *f = fS + c * n;
         if constexpr (N > 0) {
-            warp_line_filter_int<N, true>(src, X, Y, twT, f, eg, lane);
+            line<N, NT>(src, X, Y, f, eg, t, g);
         } else {
             switch (n) {
-                case 64: warp_line_filter_int<64, false>(src, X, Y, twS, f, eg, lane); break;
-                case 128: warp_line_filter_int<128, false>(src, X, Y, twS, f, eg, lane); break;
-                default: warp_line_filter_int<256, false>(src, X, Y, twS, f, eg, lane); break;
+                case 64: line<64, NT>(src, X, Y, f, eg, t, g); break;
+                case 128: line<128, NT>(src, X, Y, f, eg, t, g); break;
+                default: line<256, NT>(src, X, Y, f, eg, t, g); break;
             }
         }
     }
@@ -536,8 +605,23 @@ fused_step_kernel(const LaunchFused A) {
         writes && (FAST || A.noise == CLV_NOISE_PHILOX) && 2 * NC < nwarps;
     const bool wc = A.kinetic == CLV_KIN_EXP;
     // Filter the lines of `mask` (bit job * NC + c: job 0 = psi of src0 -> X0, job 1 =
-    // psibar of src1 -> X1), one warp per line.
+    // psibar of src1 -> X1), one warp per line; FP64 lines of 256 on two warps when they fit
+    // (the chunks split by field and component halves of the few-CTA problems).
+    constexpr bool kPairLines = sizeof(R) == 8 && LN == 256 && !FAST;
     auto filter_lines = [&](int mask, const C2 *src0, C2 *X0, C2 *Y0, const C2 *src1, C2 *X1, C2 *Y1) {
+        if constexpr (kPairLines) {
+            const int nl = __popc(mask), g = warp >> 1;
+            if (2 * nl <= nwarps) {
+                if (g < nl) {
+                    int m = mask;
+                    for (int i = 0; i < g; ++i) m &= m - 1;
+                    const int bit = __ffs(m) - 1, job = bit >= NC, c = bit - job * NC;
+                    lines.template run<64>(ch, wc, c, (job ? src1 : src0) + c * cs, (job ? X1 : X0) + c * cs,
+                                           (job ? Y1 : Y0) + c * cs, threadIdx.x & 63, g);
+                }
+                return;
+            }
+        }
         if (warp < 2 * NC && ((mask >> warp) & 1)) {
             const int job = warp >= NC, c = warp - job * NC;
             lines.run(ch, wc, c, (job ? src1 : src0) + c * cs, (job ? X1 : X0) + c * cs, (job ? Y1 : Y0) + c * cs, lane);
@@ -604,7 +688,7 @@ fused_step_kernel(const LaunchFused A) {
         {
             // kin(tau) -> part0, kinbar(tau+1) -> part1; the field slots stay intact
             // (kin(tau) only feeds the next imaginary time: the chunk's last skips it)
-            if (warp < 2 * NC) {
+            if (warp < 2 * NC || (kPairLines && !noise_smem)) {
                 const int own_lines = cmask & ((1 << NC) - 1);
                 filter_lines(((do_psi && tau + 1 < tau1) ? own_lines : 0) | (do_bar ? own_lines << NC : 0),
                              slot(sp), part0, ybuf0, slot(sq), part1, ybuf1);
