@@ -413,6 +413,35 @@ __host__ __device__ constexpr double cos64(int m) {
 }
 __host__ __device__ constexpr double sin64(int m) { return cos64((m + 48) & 63); }  // cos(2 pi (m - 16) / 64)
 
+// 32 = 4 x 8: x[8 n1 + n2] -> radix 4 over n1 (index k1), twiddle W32^(n2 k1), radix 8 over
+// n2 (index k2) -> X[k1 + 4 k2].
+template <class C2>
+struct Radix<C2, 32> {
+    template <int S>
+    static __device__ __forceinline__ void run(C2 *a) {
+        using R = decltype(a[0].x);
+        C2 y[4][8];
+#pragma unroll
+        for (int n2 = 0; n2 < 8; ++n2) {
+            C2 t[4] = {a[n2], a[8 + n2], a[16 + n2], a[24 + n2]};
+            Radix<C2, 4>::template run<S>(t);
+#pragma unroll
+            for (int k1 = 0; k1 < 4; ++k1) {
+                const int m = 2 * n2 * k1;
+                if (m == 0) y[k1][n2] = t[k1];
+                else if (m == 16) y[k1][n2] = times_si<S>(t[k1]);
+                else y[k1][n2] = cmulc(t[k1], kconst<R>(cos64(m)), kconst<R>(S * sin64(m)));
+            }
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < 4; ++k1) {
+            Radix<C2, 8>::template run<S>(y[k1]);
+#pragma unroll
+            for (int k2 = 0; k2 < 8; ++k2) a[k1 + 4 * k2] = y[k1][k2];
+        }
+    }
+};
+
 // 64 = 8 x 8: x[8 n1 + n2] -> radix 8 over n1 (index k1), twiddle W64^(n2 k1), radix 8
 // over n2 (index k2) -> X[k1 + 8 k2], W64 = exp(S 2 pi i / 64); the twiddles are
 // compile-time constants.  For a thread that holds a whole 64-site line in registers.

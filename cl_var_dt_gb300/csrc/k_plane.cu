@@ -13,7 +13,8 @@
 // The first pass (along the slower axis, whose lines are columns) reads its
 // butterflies straight from global memory, 32 consecutive columns a warp; the
 // plane is written back from shared memory in row order.  FP32 planes of 64 take
-// one thread per line instead, the line in registers (plane_lines_in_registers).
+// one thread per line instead, the line in registers (plane_lines_in_registers), FP32
+// planes of 128 2D blocks of it (plane_blocks_128).
 // The plane is read once and written once: half the traffic of the two axis
 // launches it replaces.
 #include "clv_internal.cuh"
@@ -31,8 +32,7 @@ __host__ __device__ constexpr int plane_first_group(int n, int esz) {
 }
 
 // Butterflies of a pass unrolled together: all of a thread's (at most 8) for the FP64
-// planes of 96 (one CTA per SM), else one at a time, streamed (several resident CTAs;
-// on the FP32 planes of 128 the streamed passes measured 4-6 % faster than unrolled).
+// planes of 96 (one CTA per SM), else one at a time, streamed (several resident CTAs).
 __host__ __device__ constexpr int plane_unroll(int n, int esz) { return n == 96 && esz == 16 ? 8 : 1; }
 
 // Two-radix line plans of the plane (clv_launch.h plane_fac).
@@ -95,6 +95,125 @@ __device__ __forceinline__ void plane_lines_in_registers(const LaunchAxis &A) {
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) dst[i * N + l] = tile[i * PL + l];
+}
+
+// FP32 planes of 128: a plane fills an SM's shared memory, so one CTA runs and every access
+// to the tile counts.  32 elements per thread in 2D blocks: columns 8 x 16, rows 4 x 32, with
+// the columns' last inverse pass (8 rows) and the rows' first forward pass (4 columns) done
+// on one 8 x 4 block, the first pass read from and the last written to global memory: 8 shared
+// accesses an element and four barriers instead of the in-place passes' 12 and six.  In
+// the blocks a thread's twiddles serve all its rows or columns.  768 planes (one chain, 3
+// components x 128 slices x 2 fields): 96.5 us in place -> 78 us (floor 30).
+//   A  columns forward, radix 8:  rows k + 16 m of column c                  -> tile
+//   B  columns middle, radix 16:  rows 16 j + m                              tile
+//   C  columns inverse, radix 8 and rows forward, radix 4: rows k + 16 m, columns l + 32 n  tile
+//   D  rows middle, radix 32:     columns 32 q + i of row r                  tile
+//   E  rows inverse, radix 4:     columns l + 32 n of 8 rows                 -> global
+__device__ __forceinline__ void plane_blocks_128(const LaunchAxis &A) {
+    using C2 = float2;
+    constexpr int N = 128, PL = plane_pitch(N);
+    extern __shared__ __align__(128) unsigned char smem[];
+    const AxisTask task = A.tasks[blockIdx.x >> 1];
+    const int field = (int)(blockIdx.x & 1);
+    const ChainDev &ch = A.chains[task.chain];
+    const AxisDev &axr = ch.axis[A.axis], &axc = ch.axis[A.axis + 1];
+    C2 *tw = reinterpret_cast<C2 *>(smem);
+    float *fr = reinterpret_cast<float *>(smem + N * sizeof(C2));
+    float *fc = fr + N;
+    C2 *tile = reinterpret_cast<C2 *>(smem + plane_tab_bytes(N, sizeof(C2)));
+    const long long soff = ch.off + (long long)task.slice * ch.V + (long long)task.l0 * (N * N);
+    const C2 *src = reinterpret_cast<const C2 *>(field ? A.src1 : A.src0) + soff;
+    C2 *dst = reinterpret_cast<C2 *>(field ? A.dst1 : A.dst0) + soff;
+    const int c = threadIdx.x & 127, g = threadIdx.x >> 7, l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    {
+        C2 v[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[i][m] = src[(g + 4 * i + 16 * m) * N + c];
+        if (threadIdx.x < N) {
+            tw[c] = axc.tw32[c];
+            fr[c] = axr.filt32[c];
+            fc[c] = axc.filt32[c] * (A.with_const ? (float)ch.comp_const[task.slice / ch.nt] : 1.0f);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int k = g + 4 * i;
+            Radix<C2, 8>::run<-1>(v[i]);
+            tile[k * PL + c] = v[i][0];
+#pragma unroll
+            for (int q = 1; q < 8; ++q) tile[(k + 16 * q) * PL + c] = vmul(v[i][q], tw[q * k]);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int j = g + 4 * i;
+        C2 *t = tile + j * 16 * PL + c;
+        C2 v[16];
+#pragma unroll
+        for (int m = 0; m < 16; ++m) v[m] = t[m * PL];
+        Radix<C2, 16>::run<-1>(v);
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = vscale(fr[j + 8 * q], v[q]);
+        Radix<C2, 16>::run<1>(v);
+#pragma unroll
+        for (int m = 0; m < 16; ++m) t[m * PL] = v[m];
+    }
+    __syncthreads();
+    {
+        C2 *t = tile + w * PL + l;
+        C2 v[4][8];
+#pragma unroll
+        for (int m = 0; m < 8; ++m)
+#pragma unroll
+            for (int n = 0; n < 4; ++n) v[n][m] = t[16 * m * PL + 32 * n];
+#pragma unroll
+        for (int m = 1; m < 8; ++m) {
+            const C2 x = tw[m * w];
+#pragma unroll
+            for (int n = 0; n < 4; ++n) v[n][m] = vmulc(v[n][m], x);
+        }
+#pragma unroll
+        for (int n = 0; n < 4; ++n) Radix<C2, 8>::run<1>(v[n]);
+        const C2 x1 = tw[l], x2 = tw[2 * l], x3 = tw[3 * l];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            C2 u[4] = {v[0][m], v[1][m], v[2][m], v[3][m]};
+            Radix<C2, 4>::run<-1>(u);
+            C2 *o = t + 16 * m * PL;
+            o[0] = u[0];
+            o[32] = vmul(u[1], x1);
+            o[64] = vmul(u[2], x2);
+            o[96] = vmul(u[3], x3);
+        }
+    }
+    __syncthreads();
+    {
+        C2 *t = tile + c * PL + 32 * g;  // row c, columns 32 g ...
+        C2 v[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = t[i];
+        Radix<C2, 32>::run<-1>(v);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = vscale(fc[g + 4 * i], v[i]);
+        Radix<C2, 32>::run<1>(v);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) t[i] = v[i];
+    }
+    __syncthreads();
+    const C2 x1 = tw[l], x2 = tw[2 * l], x3 = tw[3 * l];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = w + 16 * i;
+        const C2 *t = tile + r * PL + l;
+        C2 u[4] = {t[0], vmulc(t[32], x1), vmulc(t[64], x2), vmulc(t[96], x3)};
+        Radix<C2, 4>::run<1>(u);
+        C2 *o = dst + r * N + l;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) o[32 * n] = u[n];
+    }
 }
 
 // In-place passes over the plane in shared memory (inplace_fft.cuh).
@@ -262,6 +381,7 @@ template <class R, int N>
 __global__ void __launch_bounds__(plane_threads(N, (int)sizeof(R) * 2), plane_min_ctas(N, (int)sizeof(R) * 2))
 plane_filter_kernel(const LaunchAxis A) {
     if constexpr (plane_line_per_thread(N, (int)sizeof(R) * 2)) plane_lines_in_registers<R, N>(A);
+    else if constexpr (N == 128 && sizeof(R) == 4) plane_blocks_128(A);
     else plane_in_place<R, N>(A);
 }
 
