@@ -140,6 +140,7 @@ struct clv_engine {
         int tile = 0;   // 1: tile filter (k_tile.cuh), tasks in ttasks; n = 0 when lengths differ
         int threads = 128;
         int whole = 0;  // tile filter over whole slices
+        int resident = 0;  // plane filter: CTAs the GPU holds
         std::vector<TileFilterTask> ttasks;
         TileFilterTask *td = nullptr;
         int strided = 1;  // every chain's lines of this axis are neighbours in memory (stride > 1)
@@ -579,6 +580,7 @@ int run_groups(clv_engine *e, const std::vector<clv_engine::AxisGroup> &groups, 
             A.filter = energy;
             A.accumulate = energy && g.axis > 0;
             A.strided = g.strided;
+            A.resident = g.resident;
             if (g.plane) CK(launch_plane_filter<R>(A, e->stream));
             else if constexpr (sizeof(R) == 4) CK(launch_axis_filter<R>(A, e->stream));
         }
@@ -1051,12 +1053,11 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
         // square planes of side 32 to 128 (a 2D slice, or the (y, z) planes of a 3D
         // slice) under the exponential kinetic factor, a product over the axes: one
         // plane-filter launch instead of two axis launches
-        int pa = -1;
+        int pa = -1, occ = 0;
         if ((energy || e->kinetic == CLV_KIN_EXP) && !std::getenv("CLV_NO_PLANE")) {
             const int n1 = d.axis[1].n, n2 = d.axis[2].n;
             pa = n2 <= 1 ? (d.axis[0].n == n1 ? 0 : -1) : (n1 == n2 ? 1 : -1);
             const int pn = pa >= 0 ? d.axis[pa].n : 0;
-            int occ = 0;
             if (pn == 32 || pn == 64 || pn == 96 || pn == 128) {
                 const size_t sm = plane_smem_bytes(pn, esz);
                 if (sm + 1024 <= (size_t)dev_smem) {
@@ -1088,6 +1089,7 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
                     g.pitch = plane_pitch(n);
                     g.W = 1;
                     g.plane = 1;
+                    g.resident = occ * e->num_sms;
                     g.with_const = !energy && a == 0;
                     g.smem = plane_smem_bytes(n, esz);
                     groups.push_back(std::move(g));

@@ -233,6 +233,7 @@ struct LaunchAxis {
     int filter;      // 0: kinetic filter, 1: kinetic-energy filter k^2/2 (normalised)
     int accumulate;  // 1: dst += filtered (sum over axes of one-axis operators)
     int strided;     // every task's lines are neighbours in memory (axis stride > 1)
+    int resident;    // CTAs the GPU holds (plane filter)
 };
 
 // Tile filter (k_tile.cuh): a tile of one field -- whole slices, or a strided or

@@ -46,6 +46,15 @@ __host__ __device__ constexpr int plane_min_ctas(int n, int esz) {
     return esz == 8 ? (n == 32 ? 8 : (n == 64 ? 6 : (n == 96 ? 3 : 1))) : (n == 32 ? 4 : (n == 64 ? 3 : 1));
 }
 
+// The filter's planes in blocks (plane_blocks): its threads and CTAs per SM.
+__host__ __device__ constexpr bool plane_in_blocks(int n, int esz) { return esz == 8 && (n == 96 || n == 128); }
+__host__ __device__ constexpr int filter_threads(int n, int esz) {
+    return plane_in_blocks(n, esz) && n == 96 ? 192 : plane_threads(n, esz);
+}
+__host__ __device__ constexpr int filter_min_ctas(int n, int esz) {
+    return plane_in_blocks(n, esz) && n == 96 ? 2 : plane_min_ctas(n, esz);
+}
+
 // One thread per line with the whole line in registers (FP32 planes of 64): thread l
 // loads column l straight from global memory (a warp: 32 consecutive columns), runs the
 // 64-point transform, the filter and the inverse in registers and writes the column into
@@ -97,122 +106,157 @@ __device__ __forceinline__ void plane_lines_in_registers(const LaunchAxis &A) {
     for (int i = 0; i < N; ++i) dst[i * N + l] = tile[i * PL + l];
 }
 
-// FP32 planes of 128: a plane fills an SM's shared memory, so one CTA runs and every access
-// to the tile counts.  32 elements per thread in 2D blocks: columns 8 x 16, rows 4 x 32, with
-// the columns' last inverse pass (8 rows) and the rows' first forward pass (4 columns) done
-// on one 8 x 4 block, the first pass read from and the last written to global memory: 8 shared
-// accesses an element and four barriers instead of the in-place passes' 12 and six.  In
-// the blocks a thread's twiddles serve all its rows or columns.  768 planes (one chain, 3
-// components x 128 slices x 2 fields): 96.5 us in place -> 78 us (floor 30).
-//   A  columns forward, radix 8:  rows k + 16 m of column c                  -> tile
-//   B  columns middle, radix 16:  rows 16 j + m                              tile
-//   C  columns inverse, radix 8 and rows forward, radix 4: rows k + 16 m, columns l + 32 n  tile
-//   D  rows middle, radix 32:     columns 32 q + i of row r                  tile
-//   E  rows inverse, radix 4:     columns l + 32 n of 8 rows                 -> global
-__device__ __forceinline__ void plane_blocks_128(const LaunchAxis &A) {
+// FP32 planes of 96 and 128: few CTAs fill an SM's shared memory, so every access to the tile
+// counts.  2D blocks in registers: columns 8 x CB, rows RA x RB, with the columns' last inverse
+// pass (8 rows) and the rows' first forward pass (RA columns) done on one 8 x RA block, the
+// first pass read from and the last written to global memory: 8 shared accesses an element and
+// four barriers instead of the in-place passes' 12 and six.  In the blocks a thread's
+// twiddles serve all its rows or columns.
+//   A  columns forward, radix 8:  rows k + CB m of column c                  -> tile
+//   B  columns middle, radix CB:  rows CB j + m                              tile
+//   C  columns inverse, radix 8 and rows forward, radix RA: rows k + CB m, columns l + RB n  tile
+//   D  rows middle, radix RB:     columns RB q + i of row r                  tile
+//   E  rows inverse, radix RA:    columns l + RB n of 8 rows                 -> global
+// 768 planes of 128 (one chain, 3 components x 128 slices x 2 fields): 96.5 us in place -> 76
+// us (floor 30); 3840 planes of 96: 463 -> 422 us (floor 250).  Blocks of 128 (512 threads, one
+// CTA) prefetch the plane that follows on the SM into L2 (940 -> 902 us for 3840 planes); of 96
+// (192 threads, two CTAs that overlap) do not (422 -> 447 us).
+template <int N>
+struct PlaneBlocks {
+    static constexpr int CB = N / 8, RA = N == 128 ? 4 : 6, RB = N / RA, T = CB * RB, G = T / N, RPT = T / RB;
+    static constexpr int NA = CB / G, NB = 8 / G, ND = RA / G, NE = N / RPT;
+};
+
+template <int N>
+__device__ __forceinline__ void plane_blocks(const LaunchAxis &A) {
     using C2 = float2;
-    constexpr int N = 128, PL = plane_pitch(N);
+    using P = PlaneBlocks<N>;
+    constexpr int PL = plane_pitch(N), CB = P::CB, RA = P::RA, RB = P::RB, G = P::G;
     extern __shared__ __align__(128) unsigned char smem[];
-    const AxisTask task = A.tasks[blockIdx.x >> 1];
-    const int field = (int)(blockIdx.x & 1);
-    const ChainDev &ch = A.chains[task.chain];
-    const AxisDev &axr = ch.axis[A.axis], &axc = ch.axis[A.axis + 1];
     C2 *tw = reinterpret_cast<C2 *>(smem);
     float *fr = reinterpret_cast<float *>(smem + N * sizeof(C2));
     float *fc = fr + N;
     C2 *tile = reinterpret_cast<C2 *>(smem + plane_tab_bytes(N, sizeof(C2)));
-    const long long soff = ch.off + (long long)task.slice * ch.V + (long long)task.l0 * (N * N);
-    const C2 *src = reinterpret_cast<const C2 *>(field ? A.src1 : A.src0) + soff;
-    C2 *dst = reinterpret_cast<C2 *>(field ? A.dst1 : A.dst0) + soff;
-    const int c = threadIdx.x & 127, g = threadIdx.x >> 7, l = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int c = threadIdx.x % N, g = threadIdx.x / N, l = threadIdx.x % RB, w = threadIdx.x / RB;
+    C2 v[P::NA][8];
+    C2 *dst;
+    auto load = [&](int t) {
+        const AxisTask task = A.tasks[t >> 1];
+        const ChainDev &ch = A.chains[task.chain];
+        const long long off = ch.off + (long long)task.slice * ch.V + (long long)task.l0 * (N * N);
+        const C2 *src = reinterpret_cast<const C2 *>(t & 1 ? A.src1 : A.src0) + off + c;
+#pragma unroll
+        for (int i = 0; i < P::NA; ++i)
+#pragma unroll
+            for (int m = 0; m < 8; ++m) v[i][m] = src[(g + G * i + CB * m) * N];
+    };
+    const int t = blockIdx.x;
+    load(t);
+    if (threadIdx.x < N) tw[c] = A.chains[A.tasks[t >> 1].chain].axis[A.axis + 1].tw32[c];
+    __syncthreads();
     {
-        C2 v[4][8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int m = 0; m < 8; ++m) v[i][m] = src[(g + 4 * i + 16 * m) * N + c];
+        const AxisTask task = A.tasks[t >> 1];
+        const ChainDev &ch = A.chains[task.chain];
+        dst = reinterpret_cast<C2 *>(t & 1 ? A.dst1 : A.dst0) + ch.off + (long long)task.slice * ch.V +
+              (long long)task.l0 * (N * N);
         if (threadIdx.x < N) {
-            tw[c] = axc.tw32[c];
-            fr[c] = axr.filt32[c];
-            fc[c] = axc.filt32[c] * (A.with_const ? (float)ch.comp_const[task.slice / ch.nt] : 1.0f);
+            fr[c] = ch.axis[A.axis].filt32[c];
+            fc[c] = ch.axis[A.axis + 1].filt32[c] * (A.with_const ? (float)ch.comp_const[task.slice / ch.nt] : 1.0f);
         }
-        __syncthreads();
+    }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int k = g + 4 * i;
-            Radix<C2, 8>::run<-1>(v[i]);
-            tile[k * PL + c] = v[i][0];
+    for (int i = 0; i < P::NA; ++i) {
+        const int k = g + G * i;
+        Radix<C2, 8>::run<-1>(v[i]);
+        tile[k * PL + c] = v[i][0];
 #pragma unroll
-            for (int q = 1; q < 8; ++q) tile[(k + 16 * q) * PL + c] = vmul(v[i][q], tw[q * k]);
-        }
+        for (int q = 1; q < 8; ++q) tile[(k + CB * q) * PL + c] = vmul(v[i][q], tw[q * k]);
+    }
+    // the plane that follows on this SM, into L2
+    if (const int tn = t + A.resident; N == 128 && tn < 2 * A.ntasks) {
+        const AxisTask task = A.tasks[tn >> 1];
+        const ChainDev &ch = A.chains[task.chain];
+        const long long off = ch.off + (long long)task.slice * ch.V + (long long)task.l0 * (N * N);
+        const C2 *src = reinterpret_cast<const C2 *>(tn & 1 ? A.src1 : A.src0) + off;
+        for (int i = threadIdx.x * 16; i < N * N; i += P::T * 16) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + i));
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int j = g + 4 * i;
-        C2 *t = tile + j * 16 * PL + c;
-        C2 v[16];
+    for (int i = 0; i < P::NB; ++i) {
+        const int j = g + G * i;
+        C2 *x = tile + j * CB * PL + c;
+        C2 u[CB];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) v[m] = t[m * PL];
-        Radix<C2, 16>::run<-1>(v);
+        for (int m = 0; m < CB; ++m) u[m] = x[m * PL];
+        Radix<C2, CB>::template run<-1>(u);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] = vscale(fr[j + 8 * q], v[q]);
-        Radix<C2, 16>::run<1>(v);
+        for (int q = 0; q < CB; ++q) u[q] = vscale(fr[j + 8 * q], u[q]);
+        Radix<C2, CB>::template run<1>(u);
 #pragma unroll
-        for (int m = 0; m < 16; ++m) t[m * PL] = v[m];
+        for (int m = 0; m < CB; ++m) x[m * PL] = u[m];
     }
     __syncthreads();
     {
-        C2 *t = tile + w * PL + l;
-        C2 v[4][8];
+        C2 *x = tile + w * PL + l;
+        C2 b[RA][8];
 #pragma unroll
         for (int m = 0; m < 8; ++m)
 #pragma unroll
-            for (int n = 0; n < 4; ++n) v[n][m] = t[16 * m * PL + 32 * n];
+            for (int n = 0; n < RA; ++n) b[n][m] = x[CB * m * PL + RB * n];
 #pragma unroll
         for (int m = 1; m < 8; ++m) {
-            const C2 x = tw[m * w];
+            const C2 z = tw[m * w];
 #pragma unroll
-            for (int n = 0; n < 4; ++n) v[n][m] = vmulc(v[n][m], x);
+            for (int n = 0; n < RA; ++n) b[n][m] = vmulc(b[n][m], z);
         }
 #pragma unroll
-        for (int n = 0; n < 4; ++n) Radix<C2, 8>::run<1>(v[n]);
-        const C2 x1 = tw[l], x2 = tw[2 * l], x3 = tw[3 * l];
+        for (int n = 0; n < RA; ++n) Radix<C2, 8>::run<1>(b[n]);
+        C2 z[RA];
+#pragma unroll
+        for (int n = 1; n < RA; ++n) z[n] = tw[n * l];
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
-            C2 u[4] = {v[0][m], v[1][m], v[2][m], v[3][m]};
-            Radix<C2, 4>::run<-1>(u);
-            C2 *o = t + 16 * m * PL;
+            C2 u[RA];
+#pragma unroll
+            for (int n = 0; n < RA; ++n) u[n] = b[n][m];
+            Radix<C2, RA>::template run<-1>(u);
+            C2 *o = x + CB * m * PL;
             o[0] = u[0];
-            o[32] = vmul(u[1], x1);
-            o[64] = vmul(u[2], x2);
-            o[96] = vmul(u[3], x3);
+#pragma unroll
+            for (int n = 1; n < RA; ++n) o[RB * n] = vmul(u[n], z[n]);
         }
     }
     __syncthreads();
-    {
-        C2 *t = tile + c * PL + 32 * g;  // row c, columns 32 g ...
-        C2 v[32];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = t[i];
-        Radix<C2, 32>::run<-1>(v);
+    for (int i = 0; i < P::ND; ++i) {
+        const int q = g + G * i;
+        C2 *x = tile + c * PL + RB * q;  // row c
+        C2 u[RB];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = vscale(fc[g + 4 * i], v[i]);
-        Radix<C2, 32>::run<1>(v);
+        for (int m = 0; m < RB; ++m) u[m] = x[m];
+        Radix<C2, RB>::template run<-1>(u);
 #pragma unroll
-        for (int i = 0; i < 32; ++i) t[i] = v[i];
+        for (int m = 0; m < RB; ++m) u[m] = vscale(fc[q + RA * m], u[m]);
+        Radix<C2, RB>::template run<1>(u);
+#pragma unroll
+        for (int m = 0; m < RB; ++m) x[m] = u[m];
     }
     __syncthreads();
-    const C2 x1 = tw[l], x2 = tw[2 * l], x3 = tw[3 * l];
+    C2 z[RA];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = w + 16 * i;
-        const C2 *t = tile + r * PL + l;
-        C2 u[4] = {t[0], vmulc(t[32], x1), vmulc(t[64], x2), vmulc(t[96], x3)};
-        Radix<C2, 4>::run<1>(u);
+    for (int n = 1; n < RA; ++n) z[n] = tw[n * l];
+#pragma unroll
+    for (int i = 0; i < P::NE; ++i) {
+        const int r = w + P::RPT * i;
+        const C2 *x = tile + r * PL + l;
+        C2 u[RA];
+        u[0] = x[0];
+#pragma unroll
+        for (int n = 1; n < RA; ++n) u[n] = vmulc(x[RB * n], z[n]);
+        Radix<C2, RA>::template run<1>(u);
         C2 *o = dst + r * N + l;
 #pragma unroll
-        for (int n = 0; n < 4; ++n) o[32 * n] = u[n];
+        for (int n = 0; n < RA; ++n) o[RB * n] = u[n];
     }
 }
 
@@ -378,10 +422,10 @@ plane_energy_kernel(const LaunchAxis A) {
 // (the x index of a 3D slice, 0 for 2D)}; blockIdx.x % 2 selects the field.
 // Axes A.axis (rows, the slower one) and A.axis + 1 (columns, contiguous).
 template <class R, int N>
-__global__ void __launch_bounds__(plane_threads(N, (int)sizeof(R) * 2), plane_min_ctas(N, (int)sizeof(R) * 2))
+__global__ void __launch_bounds__(filter_threads(N, (int)sizeof(R) * 2), filter_min_ctas(N, (int)sizeof(R) * 2))
 plane_filter_kernel(const LaunchAxis A) {
     if constexpr (plane_line_per_thread(N, (int)sizeof(R) * 2)) plane_lines_in_registers<R, N>(A);
-    else if constexpr (N == 128 && sizeof(R) == 4) plane_blocks_128(A);
+    else if constexpr (plane_in_blocks(N, (int)sizeof(R) * 2)) plane_blocks<N>(A);
     else plane_in_place<R, N>(A);
 }
 
@@ -407,7 +451,9 @@ cudaError_t setup_plane_filter(int n, int energy, size_t smem_bytes, int *ctas_p
     if (!fn) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     if (e != cudaSuccess) return e;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, plane_threads(n, (int)sizeof(R) * 2), smem_bytes);
+    const int esz = (int)sizeof(R) * 2;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, energy ? plane_threads(n, esz) : filter_threads(n, esz),
+                                                         smem_bytes);
 }
 
 template <class R>
@@ -416,7 +462,10 @@ cudaError_t launch_plane_filter(const LaunchAxis &L, cudaStream_t s) {
     const void *fn = plane_kernel_ptr<R>(L.n, L.filter);
     if (!fn) return cudaErrorInvalidValue;
     void *args[] = {(void *)&L};
-    return cudaLaunchKernel(fn, dim3(L.nfields * L.ntasks), dim3(plane_threads(L.n, (int)sizeof(R) * 2)), args, L.smem_bytes, s);
+    const int esz = (int)sizeof(R) * 2, blocks = L.nfields * L.ntasks;
+    if (L.filter || !plane_in_blocks(L.n, esz))
+        return cudaLaunchKernel(fn, dim3(blocks), dim3(plane_threads(L.n, esz)), args, L.smem_bytes, s);
+    return cudaLaunchKernel(fn, dim3(blocks), dim3(filter_threads(L.n, esz)), args, L.smem_bytes, s);
 }
 
 template cudaError_t setup_plane_filter<float>(int, int, size_t, int *);
