@@ -118,6 +118,7 @@ struct clv_engine {
     // two-pass (reference dt rule) fused steps: the reduce pass stores the drift and a
     // streaming update applies it, instead of a second filter + drift pass
     bool store_drift = false;
+    bool draw_in_reduce = false;  // tiled: the reduce pass draws the normals of the stored-drift update
     std::vector<FusedTask> fused_tasks_h;
     FusedTask *fused_tasks = nullptr;
     double2 *fused_partials = nullptr;
@@ -126,6 +127,7 @@ struct clv_engine {
     size_t fused_smem = 0;
     int fused_ctas_per_sm = 0;
     int num_sms = 0;
+    long long all_sites = 0;  // site count over chains and imaginary times
     bool fused_split = false;  // psi and psibar in separate CTAs (build_fused_tasks)
     // step loop (k_loop.cu): resident CTAs of the loop kernel per SM (0: not available)
     int loop_per_sm = 0;
@@ -265,7 +267,8 @@ int build_tables(clv_engine *e) {
         std::memcpy(p.bytes.data(), vec.data(), p.bytes.size());
         pend.push_back(std::move(p));
     };
-    long long all_sites = 0;
+    long long &all_sites = e->all_sites;
+    all_sites = 0;
     for (auto &p : e->params) all_sites += (long long)p.nx * p.ny * p.nz * p.nt;
     for (int c = 0; c < nch; ++c) {
         const clv_chain_params &p = e->params[c];
@@ -533,6 +536,7 @@ LaunchTiled tiled_launch(const clv_engine *e, int from, int mode, bool ext) {
     L.noise_buf = e->noise_d;
     L.drift_out = (mode == FUSED_MAXONLY && e->store_drift) ? e->drift : nullptr;
     L.driftc_out = (mode == FUSED_MAXONLY && e->store_drift) ? e->driftc : nullptr;
+    L.draw = mode == FUSED_MAXONLY && e->draw_in_reduce && !ext;
     return L;
 }
 
@@ -601,17 +605,19 @@ int enqueue_tiled(clv_engine *e, bool external_noise, EventTrail *trail, int fro
         L.only_rejected = 1;
         CK(launch_tiled<R>(L, e->stream));
     } else {
-        CK(launch_tiled<R>(tiled_launch(e, from, FUSED_MAXONLY, external_noise), e->stream));
+        const LaunchTiled reduce = tiled_launch(e, from, FUSED_MAXONLY, external_noise);
+        CK(launch_tiled<R>(reduce, e->stream));
         if (trail) CK(trail->mark(e->stream));
         if (e->store_drift) {
             // the stored drift applied by the site-parallel update, which draws its noise
-            // while the reduce pass runs (programmatic launch)
+            // while the reduce pass runs (programmatic launch) unless that pass drew it
             LaunchSites L = e->sites();
             L.psi = e->fld[from][0];
             L.psic = e->fld[from][1];
             L.psi_w = e->fld[from ^ 1][0];
             L.psic_w = e->fld[from ^ 1][1];
             L.noise = external_noise ? CLV_NOISE_EXTERNAL : CLV_NOISE_PHILOX;
+            L.drawn = reduce.draw;
             L.pdl = !std::getenv("CLV_NO_PDL");
             CK(launch_update<R>(L, e->stream));
         } else {
@@ -1177,25 +1183,33 @@ int plan_tiled(clv_engine *e) {
         e->axis_groups = std::move(groups);
         return CLV_OK;
     }
-    int occ = 0;
-    if (e->precision == CLV_PREC_F64) CK(setup_tiled<double>(e->model, &occ));
-    else CK(setup_tiled<float>(e->model, &occ));
-    if (occ < 1) return CLV_OK;
-    // chunk length: the halo of a chunk is the reads of one imaginary time, which the FP32
-    // kernel, bound by memory, pays in full (3D 64^3: 1.04 ms with 16 times a chunk, 1.00 with 64)
-    long long tile_taus = 0;
-    for (auto &d : e->chains_h) tile_taus += ((long long)d.V * d.nt + 255) / 256;
-    int L = choose_chunk(e, occ * nsm, 256, e->precision == CLV_PREC_F32 ? 2.0 : 0.6);
-    if (const char *cl = std::getenv("CLV_CHUNK")) L = std::max(1, atoi(cl));
-    e->task_capacity = (size_t)tile_taus;  // chunks of one imaginary time
-    build_tiled_tasks(e, L);
-    e->axis_groups = std::move(groups);
-    e->speculate = !(std::getenv("CLV_NO_SPECULATE"));
     // reference rule at FP64, where arithmetic is scarce: the reduce pass stores the drift
     // and the update applies it, instead of a second drift pass
     e->store_drift = e->dt_rule == CLV_DT_REF_MEANMAX && e->precision == CLV_PREC_F64;
     if (const char *sd = std::getenv("CLV_STORE_DRIFT"))
         e->store_drift = e->dt_rule == CLV_DT_REF_MEANMAX && sd[0] == '1';
+    // Where that pass fills the GPU for a while it is bound by the FP64 pipe, so it also draws
+    // the normals (integer pipes) into the buffer that the update overwrites: 128 x 128 x 128,
+    // reduce 672 -> 745 us and update 397 -> 190 us.  A short one is bound by latencies, and the
+    // update draws them beside it (160 000 sites, 4 blocks an SM: 186 us a step, 200 drawn here).
+    e->draw_in_reduce = e->store_drift && e->precision == CLV_PREC_F64 && e->all_sites >= 16LL * 256 * nsm;
+    int occ = 0;
+    if (e->precision == CLV_PREC_F64) CK(setup_tiled<double>(e->model, e->draw_in_reduce, &occ));
+    else CK(setup_tiled<float>(e->model, 0, &occ));
+    if (occ < 1) return CLV_OK;
+    // chunk length: the halo of a chunk is the reads of one imaginary time, which the FP32
+    // kernel, bound by memory, pays in full (3D 64^3: 1.04 ms with 16 times a chunk, 1.00 with 64)
+    long long tile_taus = 0;
+    for (auto &d : e->chains_h) tile_taus += ((long long)d.V * d.nt + 255) / 256;
+    // (a reduce pass bound by the FP64 pipe: CTAs that share an SM share its pipe, and the halo
+    // costs it one density)
+    int L = e->draw_in_reduce ? choose_chunk(e, nsm, 256, 0.15)
+                              : choose_chunk(e, occ * nsm, 256, e->precision == CLV_PREC_F32 ? 2.0 : 0.6);
+    if (const char *cl = std::getenv("CLV_CHUNK")) L = std::max(1, atoi(cl));
+    e->task_capacity = (size_t)tile_taus;  // chunks of one imaginary time
+    build_tiled_tasks(e, L);
+    e->axis_groups = std::move(groups);
+    e->speculate = !(std::getenv("CLV_NO_SPECULATE"));
     e->tiled = true;
     return CLV_OK;
 }

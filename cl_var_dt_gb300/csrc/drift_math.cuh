@@ -74,15 +74,59 @@ struct DriftConsts {
 // density it leaves out is b_{3-a} k_{3-a}, whose product with k_a is D's second term).
 // 80 FP64 operations per field (88 when a_x is not 1) instead of 144 in the component-wise form: the
 // reference model's reduce pass is bound by the FP64 pipe (2 operations per clock and SM):
-// 1.73 -> 1.17 ms on 128 x 128 x 128 imaginary times.
+// 1.73 -> 1.17 ms on 128 x 128 x 128 imaginary times.  S is the same for both fields'
+// drifts of one (psi(tau), psibar(tau+1)) pair, always formed psi first: the streaming
+// kernel computes it once and carries it (18 operations fewer).
 template <class R, class C2>
-__device__ __forceinline__ void ref4_contact(R g2, const C2 *k, const C2 *b, C2 &S, C2 &D) {
-    S = xmul<R>(k[0], b[0]);
+__device__ __forceinline__ C2 ref4_density(R g2, const C2 *psi, const C2 *bar) {
+    C2 S = xmul<R>(psi[0], bar[0]);
 #pragma unroll
-    for (int a = 1; a < 4; ++a) S = xmadd<R>(S, k[a], b[a]);
-    D = xmsub<R>(xmul<R>(k[1], k[2]), k[0], k[3]);
-    S = xscale<R>(-g2, S);
-    D = xscale<R>(-g2, D);
+    for (int a = 1; a < 4; ++a) S = xmadd<R>(S, psi[a], bar[a]);
+    return xscale<R>(-g2, S);
+}
+template <class R, class C2>
+__device__ __forceinline__ C2 ref4_exchange(R g2, const C2 *k) {
+    return xscale<R>(-g2, xmsub<R>(xmul<R>(k[1], k[2]), k[0], k[3]));
+}
+
+// S: ref4_density of (pm, cc).
+template <class R, class C2>
+__device__ __forceinline__ void drift_ref4_psi(const DriftConsts<R> &k, C2 S, const C2 *pm, const C2 *pc,
+                                               const C2 *cc, const C2 *km, C2 *K, int cmask = 0xF) {
+    const C2 D = ref4_exchange<R>(k.g2, pm);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        if (!((cmask >> a) & 1)) continue;
+        C2 m;
+        m.x = add_rn<R>(k.mu[a], S.x);
+        m.y = S.y;
+        C2 in = xmadd<R>(km[a], m, pm[a]);
+        in = (a == 0 || a == 3) ? xmadd<R>(in, cc[3 - a], D) : xmsub<R>(in, cc[3 - a], D);
+        K[a].x = fma_rn<R>(k.eps, in.x, add_rn<R>(pm[a].x, -pc[a].x));
+        K[a].y = fma_rn<R>(k.eps, in.y, add_rn<R>(pm[a].y, -pc[a].y));
+        if (k.scaled) K[a] = xscale<R>(k.pre, K[a]);
+    }
+}
+
+// S: ref4_density of (pc, cp).
+template <class R, class C2>
+__device__ __forceinline__ void drift_ref4_bar(const DriftConsts<R> &k, C2 S, const C2 *pc, const C2 *pp, const C2 *cc,
+                                               const C2 *cp, const C2 *kp, C2 *Kc, int cmask = 0xF) {
+    const C2 D = ref4_exchange<R>(k.g2, cp);
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        if (!((cmask >> a) & 1)) continue;
+        // the chemical-potential term of the conjugate drift multiplies psi(tau+1)
+        // (Propagator_without_cutoff.cu:71,88,105,122)
+        C2 in;
+        in.x = fma_rn<R>(k.mu[a], pp[a].x, kp[a].x);
+        in.y = fma_rn<R>(k.mu[a], pp[a].y, kp[a].y);
+        in = xmadd<R>(in, S, cp[a]);
+        in = (a == 0 || a == 3) ? xmadd<R>(in, pc[3 - a], D) : xmsub<R>(in, pc[3 - a], D);
+        Kc[a].x = fma_rn<R>(k.eps, in.x, add_rn<R>(cp[a].x, -cc[a].x));
+        Kc[a].y = fma_rn<R>(k.eps, in.y, add_rn<R>(cp[a].y, -cc[a].y));
+        if (k.scaled) Kc[a] = xscale<R>(k.pre, Kc[a]);
+    }
 }
 
 template <class R, class C2>
@@ -90,41 +134,8 @@ __device__ __forceinline__ void drift_ref4_vals(const DriftConsts<R> &k, const C
                                                 const C2 *pp, const C2 *cc, const C2 *cp,
                                                 const C2 *km, const C2 *kp, C2 *K, C2 *Kc, int which = 3,
                                                 int cmask = 0xF) {
-    const R *mu = k.mu;
-    const R pre = k.pre, eps = k.eps;
-    C2 S, D;
-    if (which & 1) {
-        ref4_contact<R>(k.g2, pm, cc, S, D);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            if (!((cmask >> a) & 1)) continue;
-            C2 m;
-            m.x = add_rn<R>(mu[a], S.x);
-            m.y = S.y;
-            C2 in = xmadd<R>(km[a], m, pm[a]);
-            in = (a == 0 || a == 3) ? xmadd<R>(in, cc[3 - a], D) : xmsub<R>(in, cc[3 - a], D);
-            K[a].x = fma_rn<R>(eps, in.x, add_rn<R>(pm[a].x, -pc[a].x));
-            K[a].y = fma_rn<R>(eps, in.y, add_rn<R>(pm[a].y, -pc[a].y));
-            if (k.scaled) K[a] = xscale<R>(pre, K[a]);
-        }
-    }
-    if (which & 2) {
-        ref4_contact<R>(k.g2, cp, pc, S, D);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            if (!((cmask >> a) & 1)) continue;
-            // the chemical-potential term of the conjugate drift multiplies psi(tau+1)
-            // (Propagator_without_cutoff.cu:71,88,105,122)
-            C2 in;
-            in.x = fma_rn<R>(mu[a], pp[a].x, kp[a].x);
-            in.y = fma_rn<R>(mu[a], pp[a].y, kp[a].y);
-            in = xmadd<R>(in, S, cp[a]);
-            in = (a == 0 || a == 3) ? xmadd<R>(in, pc[3 - a], D) : xmsub<R>(in, pc[3 - a], D);
-            Kc[a].x = fma_rn<R>(eps, in.x, add_rn<R>(cp[a].x, -cc[a].x));
-            Kc[a].y = fma_rn<R>(eps, in.y, add_rn<R>(cp[a].y, -cc[a].y));
-            if (k.scaled) Kc[a] = xscale<R>(pre, Kc[a]);
-        }
-    }
+    if (which & 1) drift_ref4_psi<R>(k, ref4_density<R>(k.g2, pm, cc), pm, pc, cc, km, K, cmask);
+    if (which & 2) drift_ref4_bar<R>(k, ref4_density<R>(k.g2, pc, cp), pc, pp, cc, cp, kp, Kc, cmask);
 }
 
 // Spin-1 model.  Of one (bar, ket) pair the contact potential V = c0/2 n^2 + c1/2 (Fz^2 +

@@ -3,9 +3,9 @@
 // (k_axis.cu writes kin = e^{-eps H_kin} psi and kinbar for all imaginary times).
 //
 // A thread owns one spatial site of one chain over a chunk of imaginary times
-// [tau0, tau1) and streams through it; a CTA takes 256 consecutive (chunk, site) pairs.  psi(tau-1), psi(tau),
-// kin(tau-1) and psibar(tau) are carried in registers from the previous tau;
-// each iteration loads psi(tau+1), psibar(tau+1), kin(tau) and kinbar(tau+1),
+// [tau0, tau1) and streams through it; a CTA takes 256 consecutive (chunk, site) pairs.  psi(tau-1), psi(tau)
+// and psibar(tau) are carried in registers from the previous tau;
+// each iteration loads psi(tau+1), psibar(tau+1), kin(tau-1) and kinbar(tau+1),
 // prefetched one tau ahead, so every array is read once per step (plus one halo
 // slice per CTA).  Drift (Propagator_without_cutoff.cu:1-129 for the reference
 // model; the spin-1 drift otherwise), the step-rule reduction, the noise
@@ -36,14 +36,16 @@ __device__ __forceinline__ void normal_pair(uint64_t seed, uint32_t chain, uint6
 }
 
 
-// One task: 256 consecutive (chunk, site) pairs of one chain.
-template <class R, int MODEL>
+// One task: 256 consecutive (chunk, site) pairs of one chain.  REDUCE: the reduce pass that
+// stores the drift and the step's unit normals (tiled_reduce_kernel).
+template <class R, int MODEL, bool REDUCE>
 __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask task) {
     using C2 = typename Cx<R>::T;
     constexpr int NC = MODEL == CLV_MODEL_REF4 ? 4 : 3;
     const ChainDev &ch = A.chains[task.chain];
     ChainState *st = A.state + task.chain;
-    if (A.mode == FUSED_APPLY && A.only_rejected && st->accepted) return;  // uniform per CTA
+    const int mode = REDUCE ? FUSED_MAXONLY : A.mode;
+    if (mode == FUSED_APPLY && A.only_rejected && st->accepted) return;  // uniform per CTA
 
     const int V = ch.V, T = ch.nt;
     const int flat = task.flat0 + threadIdx.x;
@@ -55,12 +57,13 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
     const C2 *gkinc = reinterpret_cast<const C2 *>(A.kinc) + ch.off;
     C2 *opsi = reinterpret_cast<C2 *>(A.psi_out) + ch.off;
     C2 *opsic = reinterpret_cast<C2 *>(A.psic_out) + ch.off;
-    const bool writes = A.mode != FUSED_MAXONLY;
+    const bool writes = mode != FUSED_MAXONLY;
 
     R dt = 0;
     uint64_t nstep = 0;
-    if (A.mode == FUSED_SPEC) { dt = (R)ch.dt_max; nstep = st->step; }
-    else if (A.mode == FUSED_APPLY) { dt = (R)st->dt; nstep = st->noise_step; }
+    if (mode == FUSED_SPEC) dt = (R)ch.dt_max;
+    if (mode != FUSED_APPLY) nstep = st->step;
+    else { dt = (R)st->dt; nstep = st->noise_step; }
     const R sd = (R)sqrt((double)dt);
 
     auto at = [&](int c, int tau) -> long long {
@@ -69,17 +72,18 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
     };
     const DriftConsts<R> dk(ch);
     const int tau0 = (int)((long long)T * chunk / task.nchunk), tau1 = (int)((long long)T * (chunk + 1) / task.nchunk);
-    // carried: psi(tau-1), kin(tau-1), psibar(tau), psi(tau)
-    C2 Pp[NC], Kp[NC], Qc[NC], Pc[NC];
-    Spin1Link<C2> Bm;  // spin-1: the pair (psibar(tau), psi(tau-1)), carried
-    // prefetched for the next tau: psi(tau+1), psibar(tau+1), kin(tau), kinbar(tau+1)
+    // carried: psi(tau-1), psibar(tau), psi(tau) and the pair (psibar(tau), psi(tau-1))
+    C2 Pp[NC], Qc[NC], Pc[NC];
+    Spin1Link<C2> Bm;
+    C2 Sm;
+    // prefetched for the next tau: psi(tau+1), psibar(tau+1), kin(tau-1), kinbar(tau+1)
     C2 nP[NC], nQ[NC], nK[NC], nKc[NC];
     auto load_next = [&](int tau) {
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             nP[c] = gpsi[at(c, tau + 1)];
             nQ[c] = gpsic[at(c, tau + 1)];
-            nK[c] = gkin[at(c, tau)];
+            nK[c] = gkin[at(c, tau - 1)];
             nKc[c] = gkinc[at(c, tau + 1)];
         }
     };
@@ -87,12 +91,12 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
             Pp[c] = gpsi[at(c, tau0 - 1)];
-            Kp[c] = gkin[at(c, tau0 - 1)];
             Qc[c] = gpsic[at(c, tau0)];
             Pc[c] = gpsi[at(c, tau0)];
         }
         if constexpr (MODEL == CLV_MODEL_SPIN1) Bm = spin1_link<R>(dk, Qc, Pp);
-        load_next(tau0);
+        else Sm = ref4_density<R>(dk.g2, Pp, Qc);
+        if (!REDUCE) load_next(tau0);
     }
 
     R mxr = 0, smr = 0;
@@ -101,20 +105,22 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
     const int ref_rule = A.dt_rule == CLV_DT_REF_MEANMAX;
     if (act) {
         for (int tau = tau0; tau < tau1; ++tau) {
-            C2 vpp[NC], vcp[NC], kt[NC], kp[NC];
+            if (REDUCE) load_next(tau);
+            C2 vpp[NC], vcp[NC], km[NC], kp[NC];
 #pragma unroll
-            for (int c = 0; c < NC; ++c) { vpp[c] = nP[c]; vcp[c] = nQ[c]; kt[c] = nK[c]; kp[c] = nKc[c]; }
-            if (tau + 1 < tau1) load_next(tau + 1);
+            for (int c = 0; c < NC; ++c) { vpp[c] = nP[c]; vcp[c] = nQ[c]; km[c] = nK[c]; kp[c] = nKc[c]; }
+            if (!REDUCE && tau + 1 < tau1) load_next(tau + 1);
             C2 K[NC], Kc[NC];
-            if constexpr (MODEL == CLV_MODEL_REF4)
-                drift_ref4_vals<R>(dk, Pp, Pc, vpp, Qc, vcp, Kp, kp, K, Kc);
-            else
-            {
-                spin1_drift_psi<R>(Bm, Pp, Pc, Kp, K);
+            if constexpr (MODEL == CLV_MODEL_REF4) {
+                drift_ref4_psi<R>(dk, Sm, Pp, Pc, Qc, km, K);
+                Sm = ref4_density<R>(dk.g2, Pc, vcp);
+                drift_ref4_bar<R>(dk, Sm, Pc, vpp, Qc, vcp, kp, Kc);
+            } else {
+                spin1_drift_psi<R>(Bm, Pp, Pc, km, K);
                 Bm = spin1_link<R>(dk, vcp, Pc);
                 spin1_drift_bar<R>(Bm, vcp, Qc, kp, Kc);
             }
-            if (A.mode == FUSED_MAXONLY && A.drift_out) {
+            if (REDUCE || (mode == FUSED_MAXONLY && A.drift_out)) {
                 // the stored-drift update reads the drift instead of a second drift pass
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
@@ -123,8 +129,8 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
                     reinterpret_cast<C2 *>(A.driftc_out)[ch.off + gi] = Kc[c];
                 }
             }
-            if (A.mode != FUSED_APPLY) {
-                if (ref_rule) {
+            if (mode != FUSED_APPLY) {
+                if (REDUCE || ref_rule) {
                     const R a0 = abs_drift(K[0]);
                     mxr = max_nan(mxr, a0);
                     smr += a0;
@@ -134,10 +140,10 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
                     for (int c = 0; c < NC; ++c) mxr = max_nan(mxr, max_nan(abs2<R>(K[c]), abs2<R>(Kc[c])));
                 }
             }
-            if (writes) {
+            if (writes || REDUCE) {
                 const uint32_t site = (uint32_t)(tau * V + s);
                 C2 z[NC];
-                if (A.noise == CLV_NOISE_PHILOX) {
+                if (REDUCE || A.noise == CLV_NOISE_PHILOX) {
 #pragma unroll
                     for (int c = 0; c < NC; c += 2) {
                         if (c + 1 < NC) {
@@ -157,6 +163,10 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
                 }
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
+                    if (!writes) {
+                        opsi[((long long)c * T + tau) * V + s] = z[c];
+                        continue;
+                    }
                     C2 zz;
                     zz.x = mul_rn<R>(sd, z[c].x);
                     zz.y = mul_rn<R>(sd, z[c].y);
@@ -169,12 +179,11 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
             for (int c = 0; c < NC; ++c) {
                 Pp[c] = Pc[c];
                 Pc[c] = vpp[c];
-                Kp[c] = kt[c];
                 Qc[c] = vcp[c];
             }
         }
     }
-    if (A.mode == FUSED_APPLY) return;
+    if (mode == FUSED_APPLY) return;
 
     // chain-wide reduction: partial per CTA, the last CTA of the chain finishes the step
     double mx = (double)mxr, sm = (double)smr;
@@ -213,8 +222,8 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
         st->t += dtn;
         st->noise_step = st->step;
         st->step += 1;
-        st->accepted = (A.mode == FUSED_SPEC && dtn == ch.dt_max) ? 1 : 0;
-        if (!st->accepted) st->rejected += (A.mode == FUSED_SPEC);
+        st->accepted = (mode == FUSED_SPEC && dtn == ch.dt_max) ? 1 : 0;
+        if (!st->accepted) st->rejected += (mode == FUSED_SPEC);
         st->arrive = 0;
     }
 }
@@ -226,28 +235,41 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) tiled_step_kernel
     // a stored-drift update launched programmatically after this reduce pass may start
     // drawing its noise now; it waits for this grid's end before it reads the results
     asm volatile("griddepcontrol.launch_dependents;");
-    tiled_task<R, MODEL>(A, A.tasks[blockIdx.x]);
+    tiled_task<R, MODEL, false>(A, A.tasks[blockIdx.x]);
+}
+
+// The reference rule's reduce pass at FP64 that also draws the step's unit normals: the drift
+// keeps the FP64 pipe busy and the normals the integer pipes, so one warp's drift covers
+// another's normals.  The loads are not prefetched: 128 registers, two CTAs an SM instead of one
+// (128 x 128 x 128: 672 us for the drift alone, 745 with the normals; the FP64 operations 510).
+template <int MODEL>
+__global__ void __launch_bounds__(256, 2) tiled_reduce_kernel(const LaunchTiled A) {
+    tiled_task<double, MODEL, true>(A, A.tasks[blockIdx.x]);
+}
+
+template <class R>
+static const void *tiled_kernel_ptr(int model, int draw) {
+    const bool ref4 = model == CLV_MODEL_REF4;
+    if constexpr (sizeof(R) == 8) {
+        if (draw) return ref4 ? (const void *)tiled_reduce_kernel<CLV_MODEL_REF4> : (const void *)tiled_reduce_kernel<CLV_MODEL_SPIN1>;
+    }
+    return ref4 ? (const void *)tiled_step_kernel<R, CLV_MODEL_REF4> : (const void *)tiled_step_kernel<R, CLV_MODEL_SPIN1>;
 }
 
 template <class R>
 cudaError_t launch_tiled(const LaunchTiled &L, cudaStream_t s) {
     if (L.ntasks == 0) return cudaSuccess;
-    if (L.model == CLV_MODEL_REF4)
-        tiled_step_kernel<R, CLV_MODEL_REF4><<<L.ntasks, 256, 0, s>>>(L);
-    else
-        tiled_step_kernel<R, CLV_MODEL_SPIN1><<<L.ntasks, 256, 0, s>>>(L);
-    return cudaGetLastError();
+    void *args[] = {(void *)&L};
+    return cudaLaunchKernel(tiled_kernel_ptr<R>(L.model, L.draw), dim3(L.ntasks), dim3(256), args, 0, s);
 }
 
 template <class R>
-cudaError_t setup_tiled(int model, int *ctas_per_sm) {
-    const void *fn = model == CLV_MODEL_REF4 ? (const void *)tiled_step_kernel<R, CLV_MODEL_REF4>
-                                             : (const void *)tiled_step_kernel<R, CLV_MODEL_SPIN1>;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, 256, 0);
+cudaError_t setup_tiled(int model, int draw, int *ctas_per_sm) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, tiled_kernel_ptr<R>(model, draw), 256, 0);
 }
 
-template cudaError_t setup_tiled<float>(int, int *);
-template cudaError_t setup_tiled<double>(int, int *);
+template cudaError_t setup_tiled<float>(int, int, int *);
+template cudaError_t setup_tiled<double>(int, int, int *);
 template cudaError_t launch_tiled<float>(const LaunchTiled &, cudaStream_t);
 template cudaError_t launch_tiled<double>(const LaunchTiled &, cudaStream_t);
 
