@@ -966,8 +966,50 @@ int tile_plan(clv_engine *e, const TileFilterPlan &p) {
     return (int)e->tile_plans_h.size() - 1;
 }
 
-// Whole slices of chain c: tiles of consecutive imaginary times of one component, about
-// tile_target elements (one slice when it is larger).
+// Slices of chain d per tile: about tile_target elements (one slice when it is larger), with
+// two exceptions.
+//   * A problem whose tiles of that size would leave three quarters of the CTAs' places empty
+//     takes smaller ones, down to an eighth (8 to 32 sites a side, 13 700 sites: step 21.3 ->
+//     17.5 us; below that the launch gets longer again).
+//   * Slices of which four at most fit, all alike (long lines), take the count with the fewest
+//     elements and table entries to go through in all waves: their few CTAs per SM are bound
+//     by the latency of their passes, and a wave that is nearly empty costs a full one
+//     (FP64, 1536 sites x 64: one line a tile, 1.1 waves, 149 us; two, one wave, 119 us;
+//     143 chains of 1152, FP32: three lines 657 us, two 594 us, one 745 us).
+int slices_per_tile(const clv_engine *e, const ChainDev &d, int nsum, int rows1, int pitch, bool energy) {
+    const bool f64 = e->elem_bytes == 16;
+    const int base = f64 ? tile_target<double>() : tile_target<float>();
+    const int most = f64 ? tile_slice_max<double>() : tile_slice_max<float>();
+    const int wide = f64 ? tile_wide<double>() : tile_wide<float>();
+    auto resident = [&](int elems, size_t smem) {
+        const int by_regs = f64 ? (elems >= wide ? 2 : 5) : (elems >= wide ? 3 : 6);
+        return std::min(by_regs, std::max(1, (int)((size_t)(228 << 10) / (smem + 1024))));
+    };
+    const double total = (double)e->all_sites * d.ncomp * (energy ? 1 : 2);  // elements
+    bool alike = base / d.V <= 4;
+    for (auto &o : e->chains_h) alike = alike && o.V == d.V && o.axis[0].n == d.axis[0].n && o.axis[1].n == d.axis[1].n;
+    if (alike) {
+        int best = 1;
+        double cost = 0;
+        for (int ns = 1; ns <= std::max(1, std::min(d.nt, most / d.V)); ++ns) {
+            const int elems = ns * rows1 * pitch;
+            const size_t smem = tile_smem(e, elems, nsum, ns * rows1, ns * rows1);
+            double tiles = 0;
+            for (auto &o : e->chains_h) tiles += (double)d.ncomp * ((o.nt + ns - 1) / ns) * (energy ? 1 : 2);
+            const double t = std::ceil(tiles / ((double)resident(elems, smem) * e->num_sms)) * (ns * d.V + nsum);
+            if (ns == 1 || t <= cost) {
+                best = ns;
+                cost = t;
+            }
+        }
+        return best;
+    }
+    const double share = total / ((f64 ? 5 : 6) * (double)e->num_sms);
+    const int target = share < base / 4 ? std::max(base / 8, (int)share) : base;
+    return std::max(1, std::min(d.nt, target / d.V));
+}
+
+// Whole slices of chain c: tiles of consecutive imaginary times of one component.
 int add_tile_slices(clv_engine *e, int c, bool energy, std::vector<clv_engine::AxisGroup> &groups) {
     const ChainDev &d = e->chains_h[c];
     int last = 0;
@@ -987,8 +1029,7 @@ int add_tile_slices(clv_engine *e, int c, bool energy, std::vector<clv_engine::A
     }
     p.pitch = cols | 1;
     p.with_const = !energy && e->kinetic == CLV_KIN_EXP;
-    const int target = e->elem_bytes == 8 ? tile_target<float>() : tile_target<double>();
-    const int ns = std::max(1, std::min(d.nt, target / d.V));
+    const int ns = slices_per_tile(e, d, nsum, rows1, p.pitch, energy);
     p.tile_elems = (ns * rows1 * p.pitch + 1) / 2 * 2;
     const int id = tile_plan(e, p);
     auto &g = tile_group(e, groups, 0, p.naxes == 1 ? d.axis[p.axis[0]].n : 0, p.naxes > 1, p.tile_elems,
