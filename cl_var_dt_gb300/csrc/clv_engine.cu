@@ -118,6 +118,7 @@ struct clv_engine {
     // two-pass (reference dt rule) fused steps: the reduce pass stores the drift and a
     // streaming update applies it, instead of a second filter + drift pass
     bool store_drift = false;
+    bool tiled_lean = false;      // tiled, FP64: enough sites for two CTAs an SM (k_tiled.cu)
     bool draw_in_reduce = false;  // tiled: the reduce pass draws the normals of the stored-drift update
     std::vector<FusedTask> fused_tasks_h;
     FusedTask *fused_tasks = nullptr;
@@ -536,6 +537,7 @@ LaunchTiled tiled_launch(const clv_engine *e, int from, int mode, bool ext) {
     L.noise_buf = e->noise_d;
     L.drift_out = (mode == FUSED_MAXONLY && e->store_drift) ? e->drift : nullptr;
     L.driftc_out = (mode == FUSED_MAXONLY && e->store_drift) ? e->driftc : nullptr;
+    L.lean = e->tiled_lean;
     L.draw = mode == FUSED_MAXONLY && e->draw_in_reduce && !ext;
     return L;
 }
@@ -1233,10 +1235,14 @@ int plan_tiled(clv_engine *e) {
     // the normals (integer pipes) into the buffer that the update overwrites: 128 x 128 x 128,
     // reduce 672 -> 745 us and update 397 -> 190 us.  A short one is bound by latencies, and the
     // update draws them beside it (160 000 sites, 4 blocks an SM: 186 us a step, 200 drawn here).
-    e->draw_in_reduce = e->store_drift && e->precision == CLV_PREC_F64 && e->all_sites >= 16LL * 256 * nsm;
+    // A step kernel that draws beside its drift takes the same two CTAs an SM from 8 blocks on
+    // (0.57 M sites, 14: 301 -> 229 us; 0.096 M, 2: 57 us, 70 in that form).
+    const long long blocks = e->all_sites / 256;
+    e->draw_in_reduce = e->store_drift && e->precision == CLV_PREC_F64 && blocks >= 16LL * nsm;
+    e->tiled_lean = e->precision == CLV_PREC_F64 && blocks >= 8LL * nsm;
     int occ = 0;
-    if (e->precision == CLV_PREC_F64) CK(setup_tiled<double>(e->model, e->draw_in_reduce, &occ));
-    else CK(setup_tiled<float>(e->model, 0, &occ));
+    if (e->precision == CLV_PREC_F64) CK(setup_tiled<double>(e->model, e->tiled_lean, e->draw_in_reduce, &occ));
+    else CK(setup_tiled<float>(e->model, 0, 0, &occ));
     if (occ < 1) return CLV_OK;
     // chunk length: the halo of a chunk is the reads of one imaginary time, which the FP32
     // kernel, bound by memory, pays in full (3D 64^3: 1.04 ms with 16 times a chunk, 1.00 with 64)

@@ -302,6 +302,7 @@ struct LaunchTiled {
     double2 *partials;
     const double *noise_buf;
     void *drift_out, *driftc_out;  // MAXONLY: also store K, Kbar here (field layout), or null
+    int lean;                      // FP64: no loads ahead, two CTAs an SM
     int draw;                      // MAXONLY: also store the step's unit normals in psi_out
 };
 
@@ -333,7 +334,7 @@ __host__ __device__ constexpr size_t plane_smem_bytes(int n, size_t esz) {
 template <class R> cudaError_t launch_plane_filter(const LaunchAxis &L, cudaStream_t s);
 template <class R> cudaError_t setup_plane_filter(int n, int energy, size_t smem_bytes, int *ctas_per_sm);
 template <class R> cudaError_t launch_tiled(const LaunchTiled &L, cudaStream_t s);
-template <class R> cudaError_t setup_tiled(int model, int draw, int *ctas_per_sm);
+template <class R> cudaError_t setup_tiled(int model, int lean, int draw, int *ctas_per_sm);
 // Axis filter geometry, lines of 32, 64, 96, 128, 256 and 512 sites.  Lines per tile
 // (FP32; half at FP64): 64 for 32, 32 for 64, 16 for 96 and 128, 8 for 256 and 512, so that a
 // radix-8 pass has about a butterfly for each of the 256 threads and a tile with

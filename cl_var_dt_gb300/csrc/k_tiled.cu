@@ -36,9 +36,12 @@ __device__ __forceinline__ void normal_pair(uint64_t seed, uint32_t chain, uint6
 }
 
 
-// One task: 256 consecutive (chunk, site) pairs of one chain.  REDUCE: the reduce pass that
-// stores the drift and the step's unit normals (tiled_reduce_kernel).
-template <class R, int MODEL, bool REDUCE>
+// One task: 256 consecutive (chunk, site) pairs of one chain.  LEAN (large FP64 problems): an
+// imaginary time's loads are not issued one ahead, which leaves two CTAs an SM their
+// registers, so that one warp's drift (FP64 pipe) covers another's normals (integer pipes):
+// 45 spin-1 chains of up to 27 x 20 sites, 0.57 M sites: 301 -> 229 us.  REDUCE: the reduce
+// pass that stores the drift and the step's unit normals (tiled_reduce_kernel).
+template <class R, int MODEL, bool LEAN, bool REDUCE>
 __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask task) {
     using C2 = typename Cx<R>::T;
     constexpr int NC = MODEL == CLV_MODEL_REF4 ? 4 : 3;
@@ -96,7 +99,7 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
         }
         if constexpr (MODEL == CLV_MODEL_SPIN1) Bm = spin1_link<R>(dk, Qc, Pp);
         else Sm = ref4_density<R>(dk.g2, Pp, Qc);
-        if (!REDUCE) load_next(tau0);
+        if (!LEAN) load_next(tau0);
     }
 
     R mxr = 0, smr = 0;
@@ -105,11 +108,11 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
     const int ref_rule = A.dt_rule == CLV_DT_REF_MEANMAX;
     if (act) {
         for (int tau = tau0; tau < tau1; ++tau) {
-            if (REDUCE) load_next(tau);
+            if (LEAN) load_next(tau);
             C2 vpp[NC], vcp[NC], km[NC], kp[NC];
 #pragma unroll
             for (int c = 0; c < NC; ++c) { vpp[c] = nP[c]; vcp[c] = nQ[c]; km[c] = nK[c]; kp[c] = nKc[c]; }
-            if (!REDUCE && tau + 1 < tau1) load_next(tau + 1);
+            if (!LEAN && tau + 1 < tau1) load_next(tau + 1);
             C2 K[NC], Kc[NC];
             if constexpr (MODEL == CLV_MODEL_REF4) {
                 drift_ref4_psi<R>(dk, Sm, Pp, Pc, Qc, km, K);
@@ -230,46 +233,46 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
 
 // One CTA per task.  (Persistent CTAs walking the task list measured slower:
 // every task start exposes its first loads, which resident CTAs otherwise hide.)
-template <class R, int MODEL>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) tiled_step_kernel(const LaunchTiled A) {
+template <class R, int MODEL, bool LEAN>
+__global__ void __launch_bounds__(256, LEAN || sizeof(R) == 4 ? 2 : 1) tiled_step_kernel(const LaunchTiled A) {
     // a stored-drift update launched programmatically after this reduce pass may start
     // drawing its noise now; it waits for this grid's end before it reads the results
     asm volatile("griddepcontrol.launch_dependents;");
-    tiled_task<R, MODEL, false>(A, A.tasks[blockIdx.x]);
+    tiled_task<R, MODEL, LEAN, false>(A, A.tasks[blockIdx.x]);
 }
 
 // The reference rule's reduce pass at FP64 that also draws the step's unit normals: the drift
-// keeps the FP64 pipe busy and the normals the integer pipes, so one warp's drift covers
-// another's normals.  The loads are not prefetched: 128 registers, two CTAs an SM instead of one
+// keeps the FP64 pipe busy and the normals the integer pipes
 // (128 x 128 x 128: 672 us for the drift alone, 745 with the normals; the FP64 operations 510).
 template <int MODEL>
 __global__ void __launch_bounds__(256, 2) tiled_reduce_kernel(const LaunchTiled A) {
-    tiled_task<double, MODEL, true>(A, A.tasks[blockIdx.x]);
+    tiled_task<double, MODEL, true, true>(A, A.tasks[blockIdx.x]);
 }
 
 template <class R>
-static const void *tiled_kernel_ptr(int model, int draw) {
+static const void *tiled_kernel_ptr(int model, int lean, int draw) {
     const bool ref4 = model == CLV_MODEL_REF4;
     if constexpr (sizeof(R) == 8) {
         if (draw) return ref4 ? (const void *)tiled_reduce_kernel<CLV_MODEL_REF4> : (const void *)tiled_reduce_kernel<CLV_MODEL_SPIN1>;
+        if (lean && !ref4) return (const void *)tiled_step_kernel<R, CLV_MODEL_SPIN1, true>;
     }
-    return ref4 ? (const void *)tiled_step_kernel<R, CLV_MODEL_REF4> : (const void *)tiled_step_kernel<R, CLV_MODEL_SPIN1>;
+    return ref4 ? (const void *)tiled_step_kernel<R, CLV_MODEL_REF4, false> : (const void *)tiled_step_kernel<R, CLV_MODEL_SPIN1, false>;
 }
 
 template <class R>
 cudaError_t launch_tiled(const LaunchTiled &L, cudaStream_t s) {
     if (L.ntasks == 0) return cudaSuccess;
     void *args[] = {(void *)&L};
-    return cudaLaunchKernel(tiled_kernel_ptr<R>(L.model, L.draw), dim3(L.ntasks), dim3(256), args, 0, s);
+    return cudaLaunchKernel(tiled_kernel_ptr<R>(L.model, L.lean, L.draw), dim3(L.ntasks), dim3(256), args, 0, s);
 }
 
 template <class R>
-cudaError_t setup_tiled(int model, int draw, int *ctas_per_sm) {
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, tiled_kernel_ptr<R>(model, draw), 256, 0);
+cudaError_t setup_tiled(int model, int lean, int draw, int *ctas_per_sm) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, tiled_kernel_ptr<R>(model, lean, draw), 256, 0);
 }
 
-template cudaError_t setup_tiled<float>(int, int, int *);
-template cudaError_t setup_tiled<double>(int, int, int *);
+template cudaError_t setup_tiled<float>(int, int, int, int *);
+template cudaError_t setup_tiled<double>(int, int, int, int *);
 template cudaError_t launch_tiled<float>(const LaunchTiled &, cudaStream_t);
 template cudaError_t launch_tiled<double>(const LaunchTiled &, cudaStream_t);
 
