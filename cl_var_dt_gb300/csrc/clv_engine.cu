@@ -359,20 +359,17 @@ int build_tables(clv_engine *e) {
                 table(&ax.tefilt64, te64);
                 table(&ax.tefilt32, te32);
             }
-            // per-pass twiddles of the fused kernel's compile-time line plans, from the
-            // same rounded values
+            // per-pass twiddles of the fused kernel's FP32 line plans, from the same rounded
+            // values
             if (n == 64 || n == 128 || n == 256 || n == 512) {
                 const int ne = tw_entries(n);
-                std::vector<double2> p64(ne);
                 std::vector<float2> p32(ne);
                 for (int i = 0; i < ne; ++i) {
                     bool conj = false;
                     const int m = pass_twiddle_source(n, i, &conj);
-                    p64[i] = tw64[m];
                     p32[i] = tw32[m];
-                    if (conj) { p64[i].y = -p64[i].y; p32[i].y = -p32[i].y; }
+                    if (conj) p32[i].y = -p32[i].y;
                 }
-                table(&ax.ptw64, p64);
                 table(&ax.ptw32, p32);
             }
         }

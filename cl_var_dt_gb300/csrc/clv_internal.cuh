@@ -55,9 +55,8 @@ struct AxisDev {
     const float *filt32;
     const double *efilt64; // kinetic-energy filter k^2/2 / n (spin-1 observables)
     const float *efilt32;
-    // per-pass twiddle tables of the fused kernel's power-of-two line plans
+    // per-pass twiddles of the fused kernel's FP32 power-of-two line plans
     // (layout tw_*_off, n = 64 ... 512); null for other lengths
-    const double2 *ptw64;
     const float2 *ptw32;
     // in-place plan of the tile filter (k_tile.cuh): radices 2 .. 16, and the two filters in
     // its order of frequencies (position i after the forward passes)

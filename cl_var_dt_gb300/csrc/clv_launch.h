@@ -42,8 +42,6 @@ struct LaunchSites {
     void *drift, *driftc;
     double2 *partials;        // one (max, sum) per CTA
     const double *noise_buf;  // external noise (reference ind_rand layout)
-    double *acc;              // observable accumulators
-    int acc_slot;
     int pdl;                  // update: programmatic launch (may start while the previous kernel runs)
     int drawn;                // update: psi_w holds the unit normals
 };

@@ -6,7 +6,7 @@
 // in shared memory by TMA bulk copies (cp.async.bulk + mbarrier), prefetched
 // two slices ahead.  For every tau the CTA
 //   1. applies the kinetic filter to psi(tau) and psibar(tau+1) in shared
-//      memory (Stockham FFT per axis, real filter, inverse FFT);
+//      memory (FFT of the line, real filter, inverse FFT; FP64 in integers, IntLine);
 //   2. computes the drift K(tau), Kbar(tau) of every site from the resident
 //      slices psi(tau-1), psi(tau), psi(tau+1), psibar(tau), psibar(tau+1) and the
 //      kinetic terms kin(tau-1), kinbar(tau+1);
@@ -479,10 +479,6 @@ template <class R>
 __device__ __forceinline__ const typename Cx<R>::T *tw_of(const AxisDev &ax);
 template <> __device__ __forceinline__ const double2 *tw_of<double>(const AxisDev &ax) { return ax.tw64; }
 template <> __device__ __forceinline__ const float2 *tw_of<float>(const AxisDev &ax) { return ax.tw32; }
-template <class R>
-__device__ __forceinline__ const typename Cx<R>::T *ptw_of(const AxisDev &ax);
-template <> __device__ __forceinline__ const double2 *ptw_of<double>(const AxisDev &ax) { return ax.ptw64; }
-template <> __device__ __forceinline__ const float2 *ptw_of<float>(const AxisDev &ax) { return ax.ptw32; }
 template <class R>
 __device__ __forceinline__ const R *filt_of(const AxisDev &ax);
 template <> __device__ __forceinline__ const double *filt_of<double>(const AxisDev &ax) { return ax.filt64; }
