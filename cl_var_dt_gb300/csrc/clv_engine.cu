@@ -495,6 +495,7 @@ LaunchFused fused_launch(const clv_engine *e, int from, int mode, bool ext) {
     L.only_rejected = 0;
     L.use_tma = e->use_tma;
     L.withhold = e->withhold_copy && mode != FUSED_APPLY;
+    L.alone = L.ntasks <= e->num_sms;
     L.drift_out = (mode == FUSED_MAXONLY && e->store_drift) ? e->drift : nullptr;
     L.driftc_out = (mode == FUSED_MAXONLY && e->store_drift) ? e->driftc : nullptr;
     L.psi_in = e->fld[from][0];
@@ -895,6 +896,7 @@ int plan_fused(clv_engine *e) {
     probe.model = e->model;
     probe.ln = ln;
     probe.smem_bytes = smem;
+    probe.slot_stride = stride;
     int per_sm = 0;
     if (e->precision == CLV_PREC_F64) CK(setup_fused<double>(probe, &per_sm));
     else CK(setup_fused<float>(probe, &per_sm));
@@ -903,7 +905,11 @@ int plan_fused(clv_engine *e) {
     // chunk length: the halo of a chunk is the filter of psi(tau0 - 1) and its reads
     long long total_slices = 0;
     for (auto &d : e->chains_h) total_slices += d.nt;
-    int L = choose_chunk(e, nsm, 0, 0.6);
+    // (CTAs that share an SM share its issue slots; the FP64 spin-1 form of two CTAs an SM waits
+    // on its own latencies, so a wave takes both, and a start costs 1.6 imaginary times)
+    const bool two = e->precision == CLV_PREC_F64 && e->model == CLV_MODEL_SPIN1 &&
+                     e->dt_rule == CLV_DT_K_OVER_MAX && ln > 0 && per_sm > 1;
+    int L = two ? choose_chunk(e, per_sm * nsm, 0, 1.6) : choose_chunk(e, nsm, 0, 0.6);
     if (const char *cl = std::getenv("CLV_CHUNK")) L = std::max(1, atoi(cl));
     e->fused_ln_static = std::getenv("CLV_NO_STATIC_PLAN") ? 0 : ln;
     e->withhold_copy = std::getenv("CLV_TEST_WITHHOLD_COPY") != nullptr;
@@ -1879,6 +1885,7 @@ static int apply_plan(clv_engine *e, int L, int tma, int ln, int sd) {
             probe.model = e->model;
             probe.ln = ln;
             probe.smem_bytes = e->fused_smem;
+            probe.slot_stride = e->slot_stride;
             int per_sm = 0;
             if (e->precision == CLV_PREC_F64) CK(setup_fused<double>(probe, &per_sm));
             else CK(setup_fused<float>(probe, &per_sm));

@@ -32,6 +32,8 @@
 #include "drift_math.cuh"
 #include "fft_radix.cuh"
 
+#include <type_traits>
+
 namespace clv {
 
 // ------------------------------------------------------------ TMA / mbarrier
@@ -223,7 +225,9 @@ __device__ __forceinline__ void group_sync(int id) {
     else asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(NT) : "memory");
 }
 
-template <int N, int NT>
+// INPLACE: every pass reads its elements, waits for the group and writes them back, without the
+// scratch line.
+template <int N, int NT, bool INPLACE = false>
 struct IntLine {
     static constexpr int LOG = N == 64 ? 6 : (N == 128 ? 7 : 8);
     static constexpr int K4 = (LOG - 1) / 2, RL = N >> (2 * K4);  // forward radix-4 passes, the middle radix
@@ -294,7 +298,7 @@ struct IntLine {
         }
         mx = reduce(m);
         const I2 *cur = reinterpret_cast<const I2 *>(X);
-        I2 *nxt = reinterpret_cast<I2 *>(Y), *oth = reinterpret_cast<I2 *>(X);
+        I2 *nxt = reinterpret_cast<I2 *>(INPLACE ? X : Y), *oth = reinterpret_cast<I2 *>(X);
         auto swap = [&]() {
             cur = nxt;
             I2 *x = nxt;
@@ -322,6 +326,15 @@ struct IntLine {
         const int sh = ishift_for(mx, 2);
         e += sh;
         unsigned m = 0;
+        I2 u[REP][4];
+        if constexpr (INPLACE) {
+#pragma unroll
+            for (int i = 0; i < REP; ++i)
+                if (const int j = t + NT * i; NB % NT == 0 || j < NB)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) u[i][r] = s[padi(j) + padi(r * NB)];
+            group_sync<NT>(id);
+        }
 #pragma unroll
         for (int i = 0; i < REP; ++i) {
             const int j = t + NT * i;
@@ -331,7 +344,7 @@ struct IntLine {
                 I2 v[4];
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    v[r] = ishift(sl[padi(r * NB)], sh);
+                    v[r] = ishift(INPLACE ? u[i][r] : sl[padi(r * NB)], sh);
                     if (r > 0) {
                         const WCplx w = tw[(k * r) << (LOG - 2 - ls)];
                         v[r] = S < 0 ? vmul(v[r], w) : vmulc(v[r], w);
@@ -361,6 +374,15 @@ struct IntLine {
         const int sh = ishift_for(mx, LR);
         e += sh + LR;
         unsigned m = 0;
+        I2 u[REPM][RL];
+        if constexpr (INPLACE) {
+#pragma unroll
+            for (int i = 0; i < REPM; ++i)
+                if (const int j = t + NT * i; NM % NT == 0 || j < NM)
+#pragma unroll
+                    for (int r = 0; r < RL; ++r) u[i][r] = s[padi(j + r * NM)];
+            group_sync<NT>(id);
+        }
 #pragma unroll
         for (int i = 0; i < REPM; ++i) {
             const int j = t + NT * i;
@@ -368,7 +390,7 @@ struct IntLine {
                 I2 v[RL];
 #pragma unroll
                 for (int r = 0; r < RL; ++r) {
-                    v[r] = ishift(s[padi(j + r * NM)], sh);
+                    v[r] = ishift(INPLACE ? u[i][r] : s[padi(j + r * NM)], sh);
                     if (r > 0) v[r] = vmul(v[r], tw[j * r]);
                 }
                 Radix<I2, RL>::template run<-1>(v);
@@ -410,7 +432,7 @@ struct LineFilter<float, N> {
         twS = tw; twT = pt; fS = f;
     }
     // kinetic term of component c's line: src (read only) -> X, scratch Y
-    template <int NT = 32>
+    template <int NT = 32, bool INPLACE = false>
     __device__ __forceinline__ void run(const ChainDev &ch, bool wc, int c, const float2 *src, float2 *X, float2 *Y,
                                         int lane, int = 0) const {
         static_assert(NT == 32, "FP32 lines take one warp");
@@ -447,10 +469,10 @@ struct LineFilter<double, N> {
         slots = sl;
         twS = tw; fS = f;
     }
-    template <int LEN, int NT>
+    template <int LEN, int NT, bool INPLACE>
     __device__ __forceinline__ void line(const double2 *src, double2 *X, double2 *Y, const long long *f, int eg, int t,
                                          int g) const {
-        IntLine<LEN, NT> l;
+        IntLine<LEN, NT, INPLACE> l;
         l.t = t;
         l.id = 1 + g;
         l.slots = slots + 4 * g;
@@ -458,18 +480,18 @@ struct LineFilter<double, N> {
     }
     // kinetic term of component c's line by thread t of NT: src (read only) -> X, scratch Y; g: the
     // group's number when NT = 64
-    template <int NT = 32>
+    template <int NT = 32, bool INPLACE = false>
     __device__ __forceinline__ void run(const ChainDev &ch, bool wc, int c, const double2 *src, double2 *X, double2 *Y,
                                         int t, int g = 0) const {
         const int eg = exp_above(ch.axis[0].fmax * (wc ? ch.comp_const[c] : 1.0));
         const long long *f = fS + c * n;
         if constexpr (N > 0) {
-            line<N, NT>(src, X, Y, f, eg, t, g);
+            line<N, NT, INPLACE>(src, X, Y, f, eg, t, g);
         } else {
             switch (n) {
-                case 64: line<64, NT>(src, X, Y, f, eg, t, g); break;
-                case 128: line<128, NT>(src, X, Y, f, eg, t, g); break;
-                default: line<256, NT>(src, X, Y, f, eg, t, g); break;
+                case 64: line<64, NT, INPLACE>(src, X, Y, f, eg, t, g); break;
+                case 128: line<128, NT, INPLACE>(src, X, Y, f, eg, t, g); break;
+                default: line<256, NT, INPLACE>(src, X, Y, f, eg, t, g); break;
             }
         }
     }
@@ -493,11 +515,15 @@ template <> __device__ __forceinline__ const float *filt_of<float>(const AxisDev
 // Per-site state carried in registers across imaginary times: psi(tau-1),
 // kin(tau-1), psibar(tau).
 
-template <class R, int MODEL, int LN, bool FAST = false>
+// TWO: the production variant of the FP64 spin-1 model where there is more than one CTA for an
+// SM: lines filtered in place and registers for two CTAs an SM.  One CTA's 8 warps issue on 21 %
+// of the clocks, waiting on their own arithmetic; two overlap (32 chains of 256 x 128: 771 -> 477
+// us a step).  With an SM to itself a CTA is 3 % faster with all the registers.
+template <class R, int MODEL, int LN, bool FAST = false, bool TWO = false>
 // FP64 1D lines off the production variant (the reference's step rule on few CTAs):
 // registers capped at two CTAs' worth, so that the programmatic update's CTAs (its
 // noise drawn while this pass runs) fit beside this kernel's on every SM.
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : ((LN > 0 && !FAST) ? 2 : 1))
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : (LN > 0 && (TWO || !FAST) ? 2 : 1))
 fused_step_kernel(const LaunchFused A) {
     using C2 = typename Cx<R>::T;
     constexpr int NC = MODEL == CLV_MODEL_REF4 ? 4 : 3;
@@ -531,7 +557,7 @@ fused_step_kernel(const LaunchFused A) {
     // slots 0..NPS-1: psi ring; NPS..NPS+NQS-1: psibar ring; then the kinetic
     // results of the two fields, two FFT scratch buffers and the noise of one tau
     C2 *part0 = slot(NPS + NQS), *part1 = slot(NPS + NQS + 1);
-    C2 *ybuf0 = slot(NPS + NQS + 2), *ybuf1 = slot(NPS + NQS + 3), *nzbuf = slot(NPS + NQS + 4);
+    C2 *ybuf0 = slot(NPS + NQS + 2), *ybuf1 = slot(NPS + NQS + 3), *nzbuf = slot(NPS + NQS + (TWO ? 2 : 4));
     const C2 *gpsi = reinterpret_cast<const C2 *>(A.psi_in) + ch.off;
     const C2 *gpsic = reinterpret_cast<const C2 *>(A.psic_in) + ch.off;
     C2 *opsi = reinterpret_cast<C2 *>(A.psi_out) + ch.off;
@@ -620,7 +646,7 @@ fused_step_kernel(const LaunchFused A) {
         }
         if (warp < 2 * NC && ((mask >> warp) & 1)) {
             const int job = warp >= NC, c = warp - job * NC;
-            lines.run(ch, wc, c, (job ? src1 : src0) + c * cs, (job ? X1 : X0) + c * cs, (job ? Y1 : Y0) + c * cs, lane);
+            lines.template run<32, TWO>(ch, wc, c, (job ? src1 : src0) + c * cs, (job ? X1 : X0) + c * cs, (job ? Y1 : Y0) + c * cs, lane);
         }
     };
 
@@ -892,21 +918,24 @@ fused_step_kernel(const LaunchFused A) {
     }
 }
 
-// Kernel pointer of one instantiation (defined in k_fused_<precision>_<model>.cu).
+// Kernel pointer of one instantiation (defined in k_fused_<precision>_<model>.cu); two: the
+// TWO form of the production variant (FP64 spin-1).
 void *fused_kernel_f32_ref4(int ln, bool fast);
 void *fused_kernel_f32_spin1(int ln, bool fast);
 void *fused_kernel_f64_ref4(int ln, bool fast);
-void *fused_kernel_f64_spin1(int ln, bool fast);
+void *fused_kernel_f64_spin1(int ln, bool fast, bool two);
 
-template <class R, int MODEL>
-void *fused_fn(int ln, bool fast) {
+template <class R, int MODEL, bool HAS_TWO = false>
+void *fused_fn(int ln, bool fast, bool two = false) {
+    auto of = [&](auto len) {
+        constexpr int LN = decltype(len)::value;
+        if (fast && two) return (void *)fused_step_kernel<R, MODEL, LN, true, HAS_TWO>;
+        return fast ? (void *)fused_step_kernel<R, MODEL, LN, true> : (void *)fused_step_kernel<R, MODEL, LN>;
+    };
     switch (ln) {
-        case 64: return fast ? (void *)fused_step_kernel<R, MODEL, 64, true>
-                             : (void *)fused_step_kernel<R, MODEL, 64>;
-        case 128: return fast ? (void *)fused_step_kernel<R, MODEL, 128, true>
-                              : (void *)fused_step_kernel<R, MODEL, 128>;
-        case 256: return fast ? (void *)fused_step_kernel<R, MODEL, 256, true>
-                              : (void *)fused_step_kernel<R, MODEL, 256>;
+        case 64: return of(std::integral_constant<int, 64>{});
+        case 128: return of(std::integral_constant<int, 128>{});
+        case 256: return of(std::integral_constant<int, 256>{});
         default: break;
     }
     return (void *)fused_step_kernel<R, MODEL, 0>;
