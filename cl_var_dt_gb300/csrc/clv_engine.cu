@@ -850,6 +850,33 @@ int choose_chunk(const clv_engine *e, int slots, int width, double halo) {
     return best;
 }
 
+bool tiled_off() {
+    const char *env = std::getenv("CLV_TILED");
+    return env && env[0] == '0';
+}
+
+// 1D batches of ln-site lines that the tiled path steps faster than the fused one (us a step,
+// fused / tiled; chains x sites x imaginary times).  The fused step saves the kinetic term's way
+// through HBM, but filters with a warp per line; the tile filter fills its warps whatever
+// the lines, and the tiled step overlaps noise and drift over more of them.
+//   * FP32 under the reference's rule, whose second pass filters once more (the step loop's
+//     small problems aside): 3 x 64 x 32 27 / 23, 8 x 256 x 64 47 / 38, 120 x 128 x 100 275 / 177.
+//   * FP64 from three blocks of sites an SM on, lines of 64 and, under the reference's rule,
+//     of 256: reference model 40 x 64 x 64 212 / 158, 120 x 256 x 100 2669 / 2172; spin-1 40 x 64
+//     x 64 159 / 122.  Others stay: reference model 120 x 128 x 100 1056 / 1113; 8 x 64 x 64
+//     64 / 64; spin-1 40 x 128 x 64 201 / 219, 40 x 256 x 64 328 / 384.
+//   * FP32, K/max rule: lines of 64 from 16 blocks an SM on (120 x 64 x 100 84 / 69; 40 x 64 x 64
+//     28 / 28; 120 x 128 x 100 104 / 113).
+bool tiled_is_faster(const clv_engine *e, int ln) {
+    const bool ref_rule = e->dt_rule == CLV_DT_REF_MEANMAX;
+    const long long per_sm = e->all_sites / (256LL * e->num_sms);
+    if (e->precision == CLV_PREC_F64) return per_sm >= 3 && (ln == 64 || (ln == 256 && ref_rule));
+    if (!ref_rule) return ln == 64 && per_sm >= 16;
+    long long slices = 0;
+    for (auto &d : e->chains_h) slices += d.nt;
+    return 2 * slices > (long long)e->loop_per_sm * e->num_sms;
+}
+
 int plan_fused(clv_engine *e) {
     const char *env = std::getenv("CLV_FUSED");
     if (env && env[0] == '0') return CLV_OK;
@@ -874,6 +901,14 @@ int plan_fused(clv_engine *e) {
     for (auto &d : e->chains_h)
         if (d.ny != 1 || d.nz != 1 || d.nx != ln) ln = 0;
     if (ln != 64 && ln != 128 && ln != 256) return CLV_OK;
+    // the step loop's resident CTAs per SM
+    int coop = 0;
+    CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->device));
+    if (coop && !std::getenv("CLV_NO_STATIC_PLAN")) {
+        if (e->precision == CLV_PREC_F64) CK(setup_loop<double>(e->model, ln, &e->loop_per_sm));
+        else CK(setup_loop<float>(e->model, ln, &e->loop_per_sm));
+    }
+    if (!env && !tiled_off() && tiled_is_faster(e, ln)) return CLV_OK;
     if (std::getenv("CLV_NO_STATIC_PLAN")) ln = 0;
     const int tab_n = vmax;  // twiddles and filter of the lines
     const int tab_bytes = fused_tab_bytes(tab_n, (int)esz, ln);
@@ -920,15 +955,6 @@ int plan_fused(clv_engine *e) {
     e->fused_aligned = aligned;
     e->task_capacity = 4 * (size_t)total_slices;  // chunks of one imaginary time, split twice
     e->fused = true;
-    // the step loop's resident CTAs per SM (1D lines of a compile-time length)
-    if (ln > 0) {
-        int coop = 0;
-        CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, e->device));
-        if (coop) {
-            if (e->precision == CLV_PREC_F64) CK(setup_loop<double>(e->model, ln, &e->loop_per_sm));
-            else CK(setup_loop<float>(e->model, ln, &e->loop_per_sm));
-        }
-    }
     build_fused_tasks(e, L);
     return CLV_OK;
 }
