@@ -37,9 +37,10 @@ sys.path.insert(0, REPO)
 SEED = 20261203
 METRIC = "site-updates/s"
 # FP64 flops of one site-update of the batched workload's FP64 step (2 DFMA + DADD + DMUL,
-# ncu counters of fused_step_kernel<double, SPIN1, 1, 256, FAST> on 16 chains:
-# profiles/fp64_step_spin1_batched_1d256.md)
-FP64_FLOPS_PER_SITE_UPDATE = 1024.6
+# ncu counters of fused_step_kernel<double, SPIN1, 256, FAST, TWO> on 32 chains:
+# profiles/fp64_step_spin1_batched_1d256.md): drift, update and step rule; the line filters and
+# the noise run on the integer pipes
+FP64_FLOPS_PER_SITE_UPDATE = 255.4
 
 
 def workload(name, nchains=None):
@@ -459,7 +460,7 @@ def run_ours(args):
     v64 = world * sites * f64["steps"] / (f64["ms"] / 1e3) if f64 else None
     fp64_roof = None
     if f64:
-        # the FP64 step is bound by the FP64 pipe: flops per site-update (ncu count) over the
+        # the FP64 pipe's share of the FP64 step: flops per site-update (ncu count) over the
         # device's DFMA rate measured here (clv_measure_peaks)
         fp64_peak, fp32_peak = clv.measure_peaks(local)
         ach = FP64_FLOPS_PER_SITE_UPDATE * v64 / world / 1e12

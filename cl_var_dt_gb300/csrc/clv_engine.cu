@@ -869,6 +869,10 @@ bool tiled_off() {
 //     28 / 28; 120 x 128 x 100 104 / 113).
 bool tiled_is_faster(const clv_engine *e, int ln) {
     const bool ref_rule = e->dt_rule == CLV_DT_REF_MEANMAX;
+    // its two more field-sized arrays (and the stored drift's) have to fit
+    size_t room = 0, all = 0;
+    if (cudaMemGetInfo(&room, &all) != cudaSuccess) return false;
+    if ((double)e->all_sites * e->ncomp * e->elem_bytes * 8 > 0.95 * (double)room) return false;
     const long long per_sm = e->all_sites / (256LL * e->num_sms);
     if (e->precision == CLV_PREC_F64) return per_sm >= 3 && (ln == 64 || (ln == 256 && ref_rule));
     if (!ref_rule) return ln == 64 && per_sm >= 16;

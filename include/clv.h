@@ -176,9 +176,10 @@ int clv_load_checkpoint(clv_engine *e, const char *path);
 int clv_device_bytes(clv_engine *e, size_t *bytes);
 
 /* The kernel plan the engine chose for a step, as a NUL-terminated string
- * "<path>:<phase>,<phase>,...": path "fused" (every slice in shared memory),
- * "tiled" (axis filters, then the streaming step) or "unfused" (line filters,
- * drift, update); the phases in the order clv_step_timed reports them. */
+ * "<path>:<phase>,<phase>,...": path "fused" (1D lines of 64, 128 or 256 in shared
+ * memory, or the step loop), "tiled" (filters by tile, plane or axis, then the streaming
+ * step) or "unfused" (filters, drift, update); the phases in the order clv_step_timed
+ * reports them. */
 int clv_get_plan(clv_engine *e, char *buf, int capacity);
 
 /* Autotuner: times trial_steps steps of each candidate plan of the engine's path
