@@ -1001,17 +1001,29 @@ int tile_plan(clv_engine *e, const TileFilterPlan &p) {
     return (int)e->tile_plans_h.size() - 1;
 }
 
-// Slices of chain d per tile: about tile_target elements (one slice when it is larger), with
-// two exceptions.
+// Shared elements between the rows of a tile with `lines` lines along rows of n.  A phase of a
+// warp's access (16 elements at FP32, 8 at FP64) takes the lines of the tile at as many
+// neighbouring positions as fit: an odd pitch keeps it free of conflicts when one position of
+// that many lines does, else an odd multiple of the positions does.
+int tile_pitch(const clv_engine *e, int n, int lines) {
+    int g = e->elem_bytes == 8 ? 16 : 8;
+    for (int l = 1; l < lines && g > 1; l *= 2) g /= 2;
+    return g == 1 ? n | 1 : (n + g - 1) / g * g + ((n + g - 1) / g % 2 ? 0 : g);
+}
+
+// Slices of chain d per tile: about tile_target elements (one slice when it is larger), lines in
+// a number that a phase of a warp's access divides evenly when one is near, with two exceptions.
 //   * A problem whose tiles of that size would leave three quarters of the CTAs' places empty
 //     takes smaller ones, down to an eighth (8 to 32 sites a side, 13 700 sites: step 21.3 ->
 //     17.5 us; below that the launch gets longer again).
-//   * Slices of which four at most fit, all alike (long lines), take the count with the fewest
-//     elements and table entries to go through in all waves: their few CTAs per SM are bound
-//     by the latency of their passes, and a wave that is nearly empty costs a full one
-//     (FP64, 1536 sites x 64: one line a tile, 1.1 waves, 149 us; two, one wave, 119 us;
-//     143 chains of 1152, FP32: three lines 657 us, two 594 us, one 745 us).
-int slices_per_tile(const clv_engine *e, const ChainDev &d, int nsum, int rows1, int pitch, bool energy) {
+//   * Few slices a tile, all chains alike (long lines).  FP32 lines: eight, four or two, whichever
+//     first leaves two CTAs an SM and fills the GPU (4 x 1500 x 96: two lines 71 us a step, eight
+//     52; 143 chains of 1152: 615, 541 with four, 490; 60 x 960 x 96: 501, 424, 374: the tables
+//     of a tile cost as much as a line).  FP64, bound by its passes, and 2D or 3D slices: the
+//     fewest elements and table entries to go through in all waves, a tile of 256 threads at
+//     twice the pace (FP64, 1536 x 64: one line a tile, 1.1 waves, 149 us; two, one wave, 119 us;
+//     6 x 675, 431 -> 410 us; 40 x 720 x 64, two lines 1270 us, eight 1120).
+int slices_per_tile(const clv_engine *e, const ChainDev &d, int nsum, int rows1, int cols, bool energy) {
     const bool f64 = e->elem_bytes == 16;
     const int base = f64 ? tile_target<double>() : tile_target<float>();
     const int most = f64 ? tile_slice_max<double>() : tile_slice_max<float>();
@@ -1021,27 +1033,48 @@ int slices_per_tile(const clv_engine *e, const ChainDev &d, int nsum, int rows1,
         return std::min(by_regs, std::max(1, (int)((size_t)(228 << 10) / (smem + 1024))));
     };
     const double total = (double)e->all_sites * d.ncomp * (energy ? 1 : 2);  // elements
-    bool alike = base / d.V <= 4;
+    bool alike = base / d.V <= (f64 || rows1 > 1 ? 4 : 10);
     for (auto &o : e->chains_h) alike = alike && o.V == d.V && o.axis[0].n == d.axis[0].n && o.axis[1].n == d.axis[1].n;
     if (alike) {
+        const int last = std::max(1, std::min(d.nt, most / d.V));
+        auto of = [&](int ns, double &tiles) {
+            const int elems = ns * rows1 * tile_pitch(e, cols, ns * rows1);
+            tiles = 0;
+            for (auto &o : e->chains_h) tiles += (double)d.ncomp * ((o.nt + ns - 1) / ns) * (energy ? 1 : 2);
+            return resident(elems, tile_smem(e, elems, nsum, ns * rows1, ns * rows1));
+        };
+        double tiles = 0;
+        if (!f64 && rows1 == 1) {
+            for (int ns = 8; ns > 1; ns /= 2)
+                if (ns <= last && of(ns, tiles) >= 2 && tiles >= 1.4 * e->num_sms) return ns;
+            return 1;
+        }
         int best = 1;
         double cost = 0;
-        for (int ns = 1; ns <= std::max(1, std::min(d.nt, most / d.V)); ++ns) {
-            const int elems = ns * rows1 * pitch;
-            const size_t smem = tile_smem(e, elems, nsum, ns * rows1, ns * rows1);
-            double tiles = 0;
-            for (auto &o : e->chains_h) tiles += (double)d.ncomp * ((o.nt + ns - 1) / ns) * (energy ? 1 : 2);
-            const double t = std::ceil(tiles / ((double)resident(elems, smem) * e->num_sms)) * (ns * d.V + nsum);
-            if (ns == 1 || t <= cost) {
+        for (int ns = 1; ns <= last; ++ns) {
+            const int places = of(ns, tiles) * e->num_sms;
+            const bool line = rows1 == 1, full = tiles >= places;
+            const double t = std::ceil(tiles / places) * (ns * d.V + (line ? 0.72 : 1.0) * nsum) /
+                             (line && ns * d.V >= wide ? (full ? 2 : 1.7) : 1);
+            if (ns == 1 || t <= (line && full ? 1.05 : 1) * cost) {
                 best = ns;
-                cost = t;
+                cost = ns == 1 ? t : std::min(t, cost);
             }
         }
         return best;
     }
     const double share = total / ((f64 ? 5 : 6) * (double)e->num_sms);
     const int target = share < base / 4 ? std::max(base / 8, (int)share) : base;
-    return std::max(1, std::min(d.nt, target / d.V));
+    int ns = std::max(1, target / d.V);
+    if (rows1 == 1) {
+        // lines: a power of two, or a multiple of a phase's lines, when one is near
+        const int m = f64 ? 8 : 16;
+        int r = ns >= m ? (ns + m / 2) / m * m : ns;
+        if (r * d.V * 15 > 16 * target) r = ns / m * m;
+        while (r < m && (r & (r - 1))) r &= r - 1;
+        if (ns < 2 * m ? 5 * r >= 4 * ns : 10 * r >= 9 * ns) ns = r;
+    }
+    return std::min(d.nt, ns);
 }
 
 // Whole slices of chain c: tiles of consecutive imaginary times of one component.
@@ -1062,9 +1095,9 @@ int add_tile_slices(clv_engine *e, int c, bool energy, std::vector<clv_engine::A
         p.inner[p.naxes++] = d.axis[a].inner;
         nsum += d.axis[a].n;
     }
-    p.pitch = cols | 1;
     p.with_const = !energy && e->kinetic == CLV_KIN_EXP;
-    const int ns = slices_per_tile(e, d, nsum, rows1, p.pitch, energy);
+    const int ns = slices_per_tile(e, d, nsum, rows1, cols, energy);
+    p.pitch = tile_pitch(e, cols, ns * rows1);
     p.tile_elems = (ns * rows1 * p.pitch + 1) / 2 * 2;
     const int id = tile_plan(e, p);
     auto &g = tile_group(e, groups, 0, p.naxes == 1 ? d.axis[p.axis[0]].n : 0, p.naxes > 1, p.tile_elems,
@@ -1106,7 +1139,7 @@ int add_tile_axis(clv_engine *e, int c, int a, bool energy, std::vector<clv_engi
     } else {
         const int W = std::max(1, std::min(lines, target / n));
         p.inner[0] = 1;
-        p.pitch = n | 1;
+        p.pitch = tile_pitch(e, n, W);
         p.tile_elems = (W * p.pitch + 1) / 2 * 2;
         const int id = tile_plan(e, p);
         auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, 0, W));

@@ -243,7 +243,7 @@ struct TileFilterPlan {
     int axis[3];        // in the order of processing
     int inner[3];       // tile elements (padding aside) between two sites of the axis; 1: the
                         // rows' own axis, 0: the task's columns (a strided tile)
-    int pitch;          // shared elements between rows (odd)
+    int pitch;          // shared elements between rows (tile_pitch)
     int gstride;        // global elements between rows, 0: rows follow one another
     int with_const;     // multiply the component constant
     int tile_elems;     // shared elements of a full tile

@@ -2,7 +2,7 @@
 // length 2^a 3^b 5^c, whole small slices, and strided or contiguous tiles of large ones.
 //
 // A task is a tile of one field held in shared memory: `rows` rows of `cols` elements at
-// an odd pitch.  It is one of
+// a pitch without bank conflicts (tile_pitch).  It is one of
 //   * whole slices: consecutive (component, imaginary time) slices of a chain, rows along
 //     the innermost axis; every filtered axis is transformed while the slice is on chip, so
 //     a 2D or 3D slice is read and written once;
@@ -12,8 +12,8 @@
 // frequencies, decimation in time; see inplace_fft.cuh) with a plan of two or three
 // radices of 2 .. 16 that the host chose for the length: 60 = 10 x 6 takes three passes
 // over shared memory.  Butterfly b of a pass is butterfly b / NL of line b mod NL, so a
-// warp works on 32 lines at a time however short they are, conflict-free along rows (odd
-// pitch) and across them; the divisions are multiplications by a reciprocal that the
+// warp works on 32 lines at a time however short they are, conflict-free along rows and
+// across them; the divisions are multiplications by a reciprocal that the
 // thread computes once per pass.
 //
 // FP64 lines run in block floating point on the integer pipes (fft_int.cuh): a pass over the
