@@ -1293,8 +1293,11 @@ int plan_tiled(clv_engine *e) {
         return CLV_OK;
     }
     // reference rule at FP64, where arithmetic is scarce: the reduce pass stores the drift
-    // and the update applies it, instead of a second drift pass
-    e->store_drift = e->dt_rule == CLV_DT_REF_MEANMAX && e->precision == CLV_PREC_F64;
+    // and the update applies it, instead of a second drift pass; at FP32 in problems bound by
+    // latencies, whose update starts on its noise beside the pass (11 chains of 64 sites, 21 800
+    // sites: 23 -> 21.5 us a step; 0.43 M sites 68 -> 74, which keep the second pass)
+    e->store_drift = e->dt_rule == CLV_DT_REF_MEANMAX &&
+                     (e->precision == CLV_PREC_F64 || e->all_sites < 2LL * 256 * nsm);
     if (const char *sd = std::getenv("CLV_STORE_DRIFT"))
         e->store_drift = e->dt_rule == CLV_DT_REF_MEANMAX && sd[0] == '1';
     // Where that pass fills the GPU for a while it is bound by the FP64 pipe, so it also draws
