@@ -175,6 +175,7 @@ struct clv_engine {
     ObsTask *obs_pairs = nullptr;
     double *obs_partials = nullptr, *obs_scratch = nullptr;
     long long obs_scratch_n = 0;          // doubles (reference model)
+    bool obs_group = false;               // 16 pairs a CTA (k_obs.cu)
     unsigned int *obs_arrive = nullptr;
     std::vector<LineTask> line_tasks_h[3];
     LineTask *line_tasks[3] = {nullptr, nullptr, nullptr};
@@ -379,17 +380,20 @@ int build_tables(clv_engine *e) {
         d.site_nblocks = (nsites + kSiteBlock - 1) / kSiteBlock;
         for (int b = 0; b < d.site_nblocks; ++b) e->site_tasks_h.push_back({c, b * kSiteBlock});
         for (int b = 0; b < (d.V + 255) / 256; ++b) e->obs_tasks_h.push_back({c, b * 256});
-        // observables: (chunk, site) pairs, chunks of at most 16 imaginary times (spin-1, whose
-        // threads sum in the working precision), fewer where that leaves SMs idle
+        // observables: (chunk, site) pairs, chunks of at most 16 imaginary times for spin-1, whose
+        // threads sum in the working precision, fewer where that leaves SMs idle; FP32 samples of
+        // small problems keep the 16 (and their rounding) and take a thread per imaginary time
         {
             const long long per = all_sites / (2LL * 256 * e->num_sms);
-            const int L = (int)std::max<long long>(1, std::min<long long>(e->model == CLV_MODEL_REF4 ? 64 : 16, per));
+            const bool ref4 = e->model == CLV_MODEL_REF4;
+            e->obs_group = !ref4 && e->precision == CLV_PREC_F32 && per < 4;
+            const int L = e->obs_group ? 16 : (int)std::max<long long>(1, std::min<long long>(ref4 ? 64 : 16, per));
             d.obs_nchunk = (p.nt + L - 1) / L;
             d.obs_block0 = (int)e->obs_pairs_h.size();
             d.obs_scr = e->obs_scratch_n;
             const long long pairs = (long long)d.V * d.obs_nchunk;
             e->obs_scratch_n += 3 * pairs;
-            for (long long f = 0; f < pairs; f += 256) e->obs_pairs_h.push_back({c, (int)f});
+            for (long long f = 0; f < pairs; f += e->obs_group ? 16 : 256) e->obs_pairs_h.push_back({c, (int)f});
             d.obs_nblocks = (int)e->obs_pairs_h.size() - d.obs_block0;
         }
         // line tasks per axis
@@ -1871,6 +1875,7 @@ int clv_evaluate(clv_engine *e) {
         }
         LaunchObs L = e->obs();
         L.tpsi = e->kin;
+        L.group = e->obs_group;
         L.arrive = e->obs_arrive;
         L.samples = e->samples;
         L.slot = e->sample_count;

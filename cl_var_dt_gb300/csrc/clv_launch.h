@@ -386,6 +386,7 @@ struct LaunchObs {
     int slot, nchains;
     double *scratch;        // reference model: profile sums of every (chunk, site)
     double *accF, *accN;
+    int group;  // spin-1, FP32: 16 pairs a CTA, a thread per imaginary time
 };
 template <class R> cudaError_t launch_obs_ref(const LaunchObs &L, cudaStream_t s);
 template <class R> cudaError_t launch_obs_spin1(const LaunchObs &L, cudaStream_t s);

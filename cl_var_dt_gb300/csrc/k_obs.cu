@@ -29,8 +29,8 @@ __device__ __forceinline__ long long oidx(const ChainDev &ch, int c, int tau, in
 struct ObsRange {
     int s, tau0, tau1;
     bool act;
-    __device__ __forceinline__ ObsRange(const ChainDev &ch, const ObsTask &task) {
-        const int flat = task.flat0 + threadIdx.x, k = flat / ch.V;
+    __device__ __forceinline__ ObsRange(const ChainDev &ch, const ObsTask &task, int pair) {
+        const int flat = task.flat0 + pair, k = flat / ch.V;
         s = flat - k * ch.V;
         act = k < ch.obs_nchunk;
         tau0 = (int)((long long)ch.nt * k / ch.obs_nchunk);
@@ -72,7 +72,7 @@ obs_ref_kernel(const ChainDev *__restrict__ chains, const ObsTask *__restrict__ 
     __shared__ double sh[8][4];
     const ObsTask task = tasks[blockIdx.x];
     const ChainDev &ch = chains[task.chain];
-    const ObsRange o(ch, task);
+    const ObsRange o(ch, task, threadIdx.x);
     double n[4] = {0, 0, 0, 0}, fx = 0, fy = 0;
     if (o.act) {
 #pragma unroll 2
@@ -187,7 +187,10 @@ cudaError_t launch_obs_ref(const LaunchObs &L, cudaStream_t s) {
 // range, then in FP64 across the CTA (one partial of the 8 sums per CTA); the
 // chain's last CTA adds its partials (no atomics on the sums, the same result for every
 // run) and writes the sample.
-template <class R>
+// GROUP (FP32, few pairs): 16 pairs by 16 threads, one imaginary time each; a thread then adds
+// a pair's values in the order and precision of the streaming form, whose sums it repeats bit
+// for bit (one chain of 256 x 32: an evaluation 28 us streaming, @@ so).
+template <class R, bool GROUP>
 __global__ void __launch_bounds__(256)
 obs_spin1_kernel(const ChainDev *__restrict__ chains, const ObsTask *__restrict__ tasks,
                  const typename Cx<R>::T *__restrict__ psi, const typename Cx<R>::T *__restrict__ psic,
@@ -198,13 +201,14 @@ obs_spin1_kernel(const ChainDev *__restrict__ chains, const ObsTask *__restrict_
     __shared__ int am_last;
     const ObsTask task = tasks[blockIdx.x];
     const ChainDev &ch = chains[task.chain];
-    const ObsRange o(ch, task);
-    const int s = o.s;
+    const ObsRange o(ch, task, GROUP ? threadIdx.x & 15 : threadIdx.x);
+    const int s = o.s, mine = o.tau0 + (int)(threadIdx.x >> 4);
+    const int from = GROUP ? mine : o.tau0, to = GROUP ? min(mine + 1, o.tau1) : o.tau1;
     R acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (o.act) {
         const R r2 = (R)1.41421356237309504880, q = (R)ch.q, c0h = (R)(0.5 * ch.c0),
                 c1h = (R)(0.5 * ch.c1);
-        for (int tau = o.tau0; tau < o.tau1; ++tau) {
+        for (int tau = from; tau < to; ++tau) {
             const int tp = tau == ch.nt - 1 ? 0 : tau + 1;
             C2 bar[3], ket[3], tk[3];
 #pragma unroll
@@ -226,18 +230,35 @@ obs_spin1_kernel(const ChainDev *__restrict__ chains, const ObsTask *__restrict_
             acc[4] += F2.x; acc[5] += F2.y; acc[6] += e.x; acc[7] += e.y;
         }
     }
-    // FP64 above the thread: warp shuffles, then the CTA's 8 warps in order
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double part[8];
+    if constexpr (GROUP) {
+        __shared__ R val[8][16][16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) part[i] = (double)acc[i];
-    const double sum = warp_sums<8>(part);
-    if (lane % 4 == 0) sh[warp][lane / 4] = sum;
-    __syncthreads();
-    if (threadIdx.x < 8) {
-        double v = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += sh[w][threadIdx.x];
-        partials[(size_t)blockIdx.x * 8 + threadIdx.x] = v;
+        for (int i = 0; i < 8; ++i) val[i][threadIdx.x >> 4][threadIdx.x & 15] = acc[i];
+        __syncthreads();
+        const int i = threadIdx.x >> 4, p = threadIdx.x & 15;
+        if (i < 8) {
+            R t = 0;
+            if (o.act)
+                for (int j = 0; j < o.tau1 - o.tau0; ++j) t += val[i][j][p];
+            double v = (double)t;
+#pragma unroll
+            for (int b = 8; b > 0; b >>= 1) v += __shfl_xor_sync(0xffffffffu, v, b);
+            if (p == 0) partials[(size_t)blockIdx.x * 8 + i] = v;
+        }
+    } else {
+        // FP64 above the thread: warp shuffles, then the CTA's 8 warps in order
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double part[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) part[i] = (double)acc[i];
+        const double sum = warp_sums<8>(part);
+        if (lane % 4 == 0) sh[warp][lane / 4] = sum;
+        __syncthreads();
+        if (threadIdx.x < 8) {
+            double v = 0.0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += sh[w][threadIdx.x];
+            partials[(size_t)blockIdx.x * 8 + threadIdx.x] = v;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -257,9 +278,12 @@ template <class R>
 cudaError_t launch_obs_spin1(const LaunchObs &L, cudaStream_t s) {
     using C2 = typename Cx<R>::T;
     if (L.ntasks == 0) return cudaSuccess;
-    obs_spin1_kernel<R><<<L.ntasks, 256, 0, s>>>(L.chains, L.tasks, (const C2 *)L.psi, (const C2 *)L.psic,
-                                                 (const C2 *)L.tpsi, L.partials, L.arrive, L.samples,
-                                                 L.slot, L.nchains);
+    auto run = [&](auto kern) {
+        kern<<<L.ntasks, 256, 0, s>>>(L.chains, L.tasks, (const C2 *)L.psi, (const C2 *)L.psic, (const C2 *)L.tpsi,
+                                      L.partials, L.arrive, L.samples, L.slot, L.nchains);
+    };
+    if (sizeof(R) == 4 && L.group) run(obs_spin1_kernel<R, sizeof(R) == 4>);
+    else run(obs_spin1_kernel<R, false>);
     return cudaGetLastError();
 }
 

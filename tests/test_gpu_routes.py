@@ -148,3 +148,16 @@ def test_reference_observables_by_chunks(clv, oracle, nx, ny, nt):
     want_F, want_n = oracle.ref_observables(p, a, b)
     # (the engine reports means over the imaginary times, and over the sites for the densities)
     assert rel_err(n, want_n / nt / (nx * ny)) < TOL["f64"] and rel_err(F, want_F / nt) < TOL["f64"]
+
+
+# few pairs (a thread per imaginary time) with chunks that end inside a CTA, and streaming
+@pytest.mark.parametrize("nx,ny,nt", [(64, 1, 16), (30, 1, 25), (24, 9, 33), (128, 128, 40)])
+def test_spin1_samples_at_fp32(clv, oracle, nx, ny, nt):
+    c = spin1(clv, nx=nx, ny=ny, nt=nt)
+    p = oracle.spin1_params(nx=nx, ny=ny, nt=nt, eps=c.eps, mu=c.mu, c0=c.c0, c1=c.c1, q=c.q, Kc=c.K, dt_max=c.dt_max)
+    with clv.Engine(c, model=clv.MODEL_SPIN1, precision=clv.PREC_F32) as e:
+        e.init_spin1()
+        e.evaluate()
+        psi, psic = e.get_fields(0)
+        want, got = oracle.spin1_observables(p, psi, psic), e.spin1_samples(0)[0]
+    assert np.max(np.abs(got - want)) < TOL["f32"] * max(1.0, float(np.max(np.abs(want))))
