@@ -132,7 +132,8 @@ CLV_HD uint64_t neg2log_fixed(uint32_t x, int &ex) {
     // |ln(1 + r)| = w 2^-(62 + s) with |r| normalised first, so that a tiny r keeps its bits
     const bool neg = r < 0;
     const uint64_t ra = neg ? 0 - (uint64_t)r : (uint64_t)r;
-    const int s = lead64(ra | 1);                           // >= 7
+    // (its least magnitude but 0 is 2^22; the bit set here bounds the shift below at r = 0, whose w is 0)
+    const int s = lead64(ra | 256);                         // 7 .. 55
     const uint64_t w = umulhi64(ra << s, P);
     // sum in units of 2^-62 for e = 32 (a sum below 1.39), of 2^-58 else (below 46)
     const int sh = e == 32 ? 0 : 4;

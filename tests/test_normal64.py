@@ -60,3 +60,12 @@ def test_normal64_to_the_last_place(normals, words):
         ulp = np.spacing(np.abs(w).astype(np.float64))
         assert np.all(g[w == 0] == 0)
         assert np.max(np.abs(g.astype(np.longdouble) - w) / ulp) < 0.75
+
+
+def test_no_undefined_behaviour(tmp_path):
+    """Shifts and sums of every edge word (the word 0, whose remainder is exactly 0, among them)."""
+    exe = str(tmp_path / "normal64")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-DNORMAL64_MAIN", "-fsanitize=undefined", "-fno-sanitize-recover=all",
+                    os.path.join(HERE, "normal64_harness.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe] + [str(v) for v in EDGE], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
