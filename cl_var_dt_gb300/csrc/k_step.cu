@@ -234,10 +234,14 @@ update_drawn_kernel(const ChainDev *__restrict__ chains, const ChainState *__res
     const int n = ch.V * ch.nt, site = task.site0 + threadIdx.x, a = blockIdx.y;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (a >= ch.ncomp) return;
+    // (threads past the chain's end load nothing: psi_o is written below)
     const bool in = site < n;
-    const long long i = ch.off + (long long)a * n + (in ? site : 0);
-    const C2 p = psi[i], pb = psic[i], k = drift[i], kb = driftc[i];
-    C2 z = psi_o[i];
+    const long long i = ch.off + (long long)a * n + site;
+    C2 p = mk<C2>(0.0, 0.0), pb = p, k = p, kb = p, z = p;
+    if (in) {
+        p = psi[i]; pb = psic[i]; k = drift[i]; kb = driftc[i];
+        z = psi_o[i];
+    }
     const double2 dts = step_size(&state[task.chain]);
     if (!in) return;
     const R dt = (R)dts.x, sd = (R)dts.y;

@@ -102,6 +102,18 @@ def test_normals_drawn_in_the_reduce_pass(clv, monkeypatch, shapes):
     against_separate_kernels(clv, monkeypatch, chains, clv.MODEL_REF4, "f64", "tiled")
 
 
+def test_drawn_normals_give_the_update_kernels_bits(clv, monkeypatch):
+    """A chain whose last block of 128 sites is partly empty (20 x 21 sites, 127 times), alone (the
+    update draws its normals) and beside a chain that fills the GPU (the reduce pass draws them)."""
+    monkeypatch.setenv("CLV_CHUNK", "8")   # the mean's order of summation
+    small, large = ref4(clv, nx=20, ny=21, nt=127), ref4(clv, nx=128, ny=128, nt=48, seed=9)
+    start = start_of([small, large])
+    alone, ai, _ = one_step(clv, [small], clv.MODEL_REF4, "f64", start[:1])
+    both, bi, _ = one_step(clv, [small, large], clv.MODEL_REF4, "f64", start)
+    assert ai["dt"][0] == bi["dt"][0]
+    assert np.array_equal(alone[0][0], both[0][0]) and np.array_equal(alone[0][1], both[0][1])
+
+
 def test_fp64_spin1_with_two_ctas_an_sm_tiled(clv, monkeypatch):
     chains = [spin1(clv, nx=27, ny=20, nt=64 + i, mu=0.5 + 0.1 * i, seed=5 + i) for i in range(10)]
     against_separate_kernels(clv, monkeypatch, chains, clv.MODEL_SPIN1, "f64", "tiled")
