@@ -103,10 +103,10 @@ def test_normals_drawn_in_the_reduce_pass(clv, monkeypatch, shapes):
 
 
 def test_drawn_normals_give_the_update_kernels_bits(clv, monkeypatch):
-    """A chain whose last block of 128 sites is partly empty (20 x 21 sites, 127 times), alone (the
+    """A chain whose last block of 128 sites is partly empty (20 x 27 sites, 127 times), alone (the
     update draws its normals) and beside a chain that fills the GPU (the reduce pass draws them)."""
     monkeypatch.setenv("CLV_CHUNK", "8")   # the mean's order of summation
-    small, large = ref4(clv, nx=20, ny=21, nt=127), ref4(clv, nx=128, ny=128, nt=48, seed=9)
+    small, large = ref4(clv, nx=20, ny=27, nt=127), ref4(clv, nx=128, ny=128, nt=48, seed=9)
     start = start_of([small, large])
     alone, ai, _ = one_step(clv, [small], clv.MODEL_REF4, "f64", start[:1])
     both, bi, _ = one_step(clv, [small, large], clv.MODEL_REF4, "f64", start)
