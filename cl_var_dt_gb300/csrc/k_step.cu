@@ -145,12 +145,15 @@ cudaError_t launch_drift(const LaunchSites &L, cudaStream_t s) {
 
 // --------------------------------------------------------------- update
 // dt and sqrt(dt) of a chain, by one thread of the block: an FP64 root in every thread (0.2 a
-// clock and SM) is half of an update's time (128 x 128 x 128, FP64: 276 -> 190 us).
+// clock and SM) is half of an update's time (128 x 128 x 128, FP64: 276 -> 190 us).  The root
+// is of dt in the working precision, as in the apply passes and the step loop: at FP32 the
+// root of the FP64 value rounds to another float for one dt in eight.
+template <class R>
 __device__ __forceinline__ double2 step_size(const ChainState *st) {
     __shared__ double2 d;
     if (threadIdx.x == 0) {
-        const double dt = __ldcg(&st->dt);
-        d = make_double2(dt, sqrt(dt));
+        const R dt = (R)__ldcg(&st->dt);
+        d = make_double2((double)dt, sqrt((double)dt));
     }
     __syncthreads();
     return d;
@@ -194,7 +197,7 @@ update_kernel(const ChainDev *__restrict__ chains, const ChainState *__restrict_
     };
     if (early) draw(pre);
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the reduce pass is complete and visible
-    const double2 dts = step_size(stc);
+    const double2 dts = step_size<R>(stc);
     if (!in) return;
     const uint64_t nstep = __ldcg(&stc->noise_step);
     if (nstep != pre) draw(nstep);
@@ -242,7 +245,7 @@ update_drawn_kernel(const ChainDev *__restrict__ chains, const ChainState *__res
         p = psi[i]; pb = psic[i]; k = drift[i]; kb = driftc[i];
         z = psi_o[i];
     }
-    const double2 dts = step_size(&state[task.chain]);
+    const double2 dts = step_size<R>(&state[task.chain]);
     if (!in) return;
     const R dt = (R)dts.x, sd = (R)dts.y;
     z.x = mul_rn<R>(sd, z.x);

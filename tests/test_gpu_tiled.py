@@ -216,3 +216,25 @@ def test_tiled_stored_drift_equals_apply_pass(clv, env, shape):
     (a, ia), (b, ib) = out
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
     assert np.array_equal(ia["dt"], ib["dt"]) and np.array_equal(ia["t"], ib["t"])
+
+
+@pytest.mark.parametrize("shape", [dict(nx=64, ny=32, nt=8), dict(nx=60, nt=9)], ids=["2d", "1d"])
+def test_tiled_stored_drift_equals_apply_pass_fp32(clv, env, shape):
+    """The same at FP32 over 60 steps, that is, 60 step sizes: the stored-drift update takes the
+    root of the step size rounded to FP32, as the apply pass does (one size in eight has
+    another root when it is taken in FP64)."""
+    env(CLV_FUSED="0")
+    c = clv.ChainParams(**shape, eps=0.02, a_x=1.0, G=0.1, Q=0.02, P=0.05, mu=-0.5, DT=0.002, seed=7)
+    out = []
+    for sd in ("1", "0"):
+        env(CLV_STORE_DRIFT=sd)
+        with clv.Engine(c, model=clv.MODEL_REF4, precision=clv.PREC_F32) as e:
+            assert e.plan()[1][-1] == ("stored_drift_update" if sd == "1" else "tiled_apply")
+            rng = np.random.default_rng(2)
+            f = (rng.standard_normal(e.shape(0)) + 1j * rng.standard_normal(e.shape(0))) * 0.3 + 0.5
+            e.set_fields(0, f, np.conj(f))
+            e.step(60)
+            out.append((e.get_fields(0), e.step_info()))
+    (a, ia), (b, ib) = out
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    assert np.array_equal(ia["dt"], ib["dt"]) and np.array_equal(ia["t"], ib["t"])
