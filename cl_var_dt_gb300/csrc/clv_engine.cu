@@ -2002,7 +2002,7 @@ int clv_autotune(clv_engine *e, int trial_steps, char *report, int capacity) {
                     }
                 }
             } else {
-                cands.push_back({L, 0, 0, 0, 0.f});
+                cands.push_back({L, 0, 0, e->store_drift, 0.f});
             }
         }
         // the trials run real steps: keep the state and restore it after each

@@ -57,3 +57,13 @@ def test_autotune_without_a_tunable_plan(clv):
     with clv.Engine(chains(clv, nx=2048, nt=4), model=clv.MODEL_SPIN1) as e:
         assert e.plan()[0] == "unfused"
         assert "no tunable plan" in e.autotune(2)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_autotune_reports_a_tiled_plan_that_stores_its_drift(clv, prec):
+    c = clv.ChainParams(nx=30, ny=24, nt=8, eps=0.02, G=0.1, mu=-0.5, DT=0.002, seed=7)
+    with clv.Engine(c, model=clv.MODEL_REF4, precision=clv.PREC_F64 if prec == "f64" else clv.PREC_F32) as e:
+        assert e.plan() == ("tiled", e.plan()[1]) and e.plan()[1][-1] == "stored_drift_update"
+        rep = e.autotune(1)
+        assert all("stored_drift=1" in line for line in rep.splitlines()), rep
+        assert e.plan()[1][-1] == "stored_drift_update"
