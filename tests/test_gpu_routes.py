@@ -173,3 +173,31 @@ def test_spin1_samples_at_fp32(clv, oracle, nx, ny, nt):
         psi, psic = e.get_fields(0)
         want, got = oracle.spin1_observables(p, psi, psic), e.spin1_samples(0)[0]
     assert np.max(np.abs(got - want)) < TOL["f32"] * max(1.0, float(np.max(np.abs(want))))
+
+
+# a thread sums all imaginary times of its site (one chunk)
+@pytest.mark.parametrize("nt,kind", [(24, "condensate"), (64, "random")])
+def test_reference_profiles_round_once_a_time(clv, nt, kind):
+    """F_x, F_y, F_z against extended precision.  A running sum over nt times rounds once a time
+    at its own size: a variance of u^2 / 3 times its square, u = 2^-53, which for a random walk
+    adds up to nt / 6 of the result's (a condensate's sum: nt / 9); a time's eight products add
+    8 / 3 of their own."""
+    c = ref4(clv, nx=300, ny=270, nt=nt)
+    rng = np.random.default_rng(4)
+    amp = 0.4 if kind == "condensate" else 0.0
+    a, b = (amp + 0.2 * (rng.standard_normal((4, nt, 300, 270, 1)) + 1j * rng.standard_normal((4, nt, 300, 270, 1)))
+            for _ in range(2))
+    with clv.Engine(c, model=clv.MODEL_REF4, precision=clv.PREC_F64) as e:
+        e.set_fields(0, a, b)
+        e.evaluate()
+        n, F = e.ref_observables(0)
+    sites = rng.choice(300 * 270, 4000, replace=False)
+    k = a.reshape(4, nt, -1)[:, :, sites].astype(np.clongdouble)
+    m = np.roll(b.reshape(4, nt, -1)[:, :, sites].astype(np.clongdouble), -1, 1)
+    t20, t02, t31, t13 = m[2] * k[0], m[0] * k[2], m[3] * k[1], m[1] * k[3]
+    d = m * k
+    want = np.stack([(t20 + t02 + t31 + t13).real, -(t20 - t02 + t31 - t13).imag, (d[0] + d[1] - d[2] - d[3]).real]).sum(1)
+    err = F.reshape(3, -1)[:, sites] * np.longdouble(nt) - want
+    rms = np.sqrt((err ** 2).sum(1) / (want ** 2).sum(1)).astype(float)
+    # (the mean over the times divides once more: another third)
+    assert np.all(rms < 2.0 ** -53 * np.sqrt(nt / 6 + 9 / 3)), rms
