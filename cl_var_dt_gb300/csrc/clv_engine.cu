@@ -380,14 +380,16 @@ int build_tables(clv_engine *e) {
         d.site_nblocks = (nsites + kSiteBlock - 1) / kSiteBlock;
         for (int b = 0; b < d.site_nblocks; ++b) e->site_tasks_h.push_back({c, b * kSiteBlock});
         for (int b = 0; b < (d.V + 255) / 256; ++b) e->obs_tasks_h.push_back({c, b * 256});
-        // observables: (chunk, site) pairs, chunks of at most 16 imaginary times for spin-1, whose
-        // threads sum in the working precision, fewer where that leaves SMs idle; FP32 samples of
-        // small problems keep the 16 (and their rounding) and take a thread per imaginary time
+        // observables: (chunk, site) pairs, chunks of at most 64 imaginary times for the reference
+        // model and 16 for spin-1 at FP64, fewer where that leaves SMs idle.  Spin-1 at FP32, whose
+        // threads sum in FP32, takes 16 whatever the batch, so that a chain's sample does not
+        // depend on the chains beside it; small problems take a thread per imaginary time
         {
             const long long per = all_sites / (2LL * 256 * e->num_sms);
             const bool ref4 = e->model == CLV_MODEL_REF4;
             e->obs_group = !ref4 && e->precision == CLV_PREC_F32 && per < 4;
-            const int L = e->obs_group ? 16 : (int)std::max<long long>(1, std::min<long long>(ref4 ? 64 : 16, per));
+            const int L = !ref4 && e->precision == CLV_PREC_F32
+                              ? 16 : (int)std::max<long long>(1, std::min<long long>(ref4 ? 64 : 16, per));
             d.obs_nchunk = (p.nt + L - 1) / L;
             d.obs_block0 = (int)e->obs_pairs_h.size();
             d.obs_scr = e->obs_scratch_n;

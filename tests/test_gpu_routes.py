@@ -201,3 +201,22 @@ def test_reference_profiles_round_once_a_time(clv, nt, kind):
     rms = np.sqrt((err ** 2).sum(1) / (want ** 2).sum(1)).astype(float)
     # (the mean over the times divides once more: another third)
     assert np.all(rms < 2.0 ** -53 * np.sqrt(nt / 6 + 9 / 3)), rms
+
+
+def test_spin1_sample_does_not_depend_on_the_batch(clv):
+    """A chain's FP32 sample alone, in a batch of 0.5 and of 1.5 million sites: the same FP32 sums
+    of 16 imaginary times, added in FP64 (5 000 of them: 5 000 2^-53 of the sum of magnitudes at
+    the very most)."""
+    c = spin1(clv, nx=60, nt=50)
+    rng = np.random.default_rng(6)
+    f = 0.6 + 0.1 * (rng.standard_normal((3, 50, 60, 1, 1)) + 1j * rng.standard_normal((3, 50, 60, 1, 1)))
+    got = []
+    for more in (0, 7, 23):
+        with clv.Engine([c] + [spin1(clv, nx=512, nt=128, seed=i) for i in range(more)], model=clv.MODEL_SPIN1,
+                        precision=clv.PREC_F32) as e:
+            e.init_spin1()
+            e.set_fields(0, f, np.conj(f))
+            e.evaluate()
+            got.append(e.spin1_samples(0)[0])
+    for g in got[1:]:
+        assert np.max(np.abs(g - got[0])) < 1e-12 * np.max(np.abs(got[0])), (got[0], g)
