@@ -68,40 +68,57 @@ struct DriftConsts {
 // cmask: the components a whose K[a], Kc[a] are computed (bit a; CTA-uniform).
 //
 // The contact term of component a with the multiplied field k and the other field b is,
-// with S = sum_c k_c b_c and D = k_1 k_2 - k_0 k_3,
-//   t_0 = S k_0 + b_3 D,  t_1 = S k_1 - b_2 D,  t_2 = S k_2 - b_1 D,  t_3 = S k_3 + b_0 D
-// (the reference adds three densities and one exchange product per component; the
-// density it leaves out is b_{3-a} k_{3-a}, whose product with k_a is D's second term).
-// 80 FP64 operations per field (88 when a_x is not 1) instead of 144 in the component-wise form: the
-// reference model's reduce pass is bound by the FP64 pipe (2 operations per clock and SM):
-// 1.73 -> 1.17 ms on 128 x 128 x 128 imaginary times.  S is the same for both fields'
-// drifts of one (psi(tau), psibar(tau+1)) pair, always formed psi first: the streaming
-// kernel computes it once and carries it (18 operations fewer).
+// with n_c = k_c b_c, E_a = sum of n_c over c != 3 - a, and k_p k_q the two components beside
+// a and 3 - a,
+//   t_a = E_a k_a + b_{3-a} k_p k_q
+// (the reference's three densities and exchange product, its exchange product of one pair
+// shared by both of the pair's components).  E_a is summed without n_{3-a}: taken out of the
+// sum of all four it would leave that density's rounding in t_a, which is the whole of it
+// where component 3 - a is far above the others.  106 FP64 operations per field (114 when a_x
+// is not 1) instead of 144 in the component-wise form: the reference model's reduce pass is
+// bound by the FP64 pipe (2 operations per clock and SM).  The E_a are the same for both
+// fields' drifts of one (psi(tau), psibar(tau+1)) pair, always formed psi first: the streaming
+// kernel computes them once and carries them (40 operations fewer).
+template <class C2>
+struct Ref4Density {
+    C2 E[4];  // -2G E_a
+};
 template <class R, class C2>
-__device__ __forceinline__ C2 ref4_density(R g2, const C2 *psi, const C2 *bar) {
-    C2 S = xmul<R>(psi[0], bar[0]);
+__device__ __forceinline__ Ref4Density<C2> ref4_density(R g2, const C2 *psi, const C2 *bar, int cmask = 0xF) {
+    Ref4Density<C2> d;
 #pragma unroll
-    for (int a = 1; a < 4; ++a) S = xmadd<R>(S, psi[a], bar[a]);
-    return xscale<R>(-g2, S);
+    for (int h = 0; h < 2; ++h) {  // components 0 and 1 share n_0 + n_1, 2 and 3 n_2 + n_3
+        if (!((cmask >> (2 * h)) & 3)) continue;
+        const C2 both = xmadd<R>(xmul<R>(psi[2 * h], bar[2 * h]), psi[2 * h + 1], bar[2 * h + 1]);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int a = 2 * h + u, c = (a + 2) & 3;  // 0, 1, 2, 3: the third density is n_2, n_3, n_0, n_1
+            d.E[a] = xscale<R>(-g2, xmadd<R>(both, psi[c], bar[c]));
+        }
+    }
+    return d;
 }
+// -2G k_1 k_2 (components 0 and 3) and -2G k_0 k_3 (1 and 2)
 template <class R, class C2>
-__device__ __forceinline__ C2 ref4_exchange(R g2, const C2 *k) {
-    return xscale<R>(-g2, xmsub<R>(xmul<R>(k[1], k[2]), k[0], k[3]));
+__device__ __forceinline__ void ref4_exchange(R g2, const C2 *k, C2 *D) {
+    D[0] = xscale<R>(-g2, xmul<R>(k[1], k[2]));
+    D[1] = xscale<R>(-g2, xmul<R>(k[0], k[3]));
 }
 
 // S: ref4_density of (pm, cc).
 template <class R, class C2>
-__device__ __forceinline__ void drift_ref4_psi(const DriftConsts<R> &k, C2 S, const C2 *pm, const C2 *pc,
+__device__ __forceinline__ void drift_ref4_psi(const DriftConsts<R> &k, const Ref4Density<C2> &S, const C2 *pm, const C2 *pc,
                                                const C2 *cc, const C2 *km, C2 *K, int cmask = 0xF) {
-    const C2 D = ref4_exchange<R>(k.g2, pm);
+    C2 D[2];
+    ref4_exchange<R>(k.g2, pm, D);
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
         if (!((cmask >> a) & 1)) continue;
         C2 m;
-        m.x = add_rn<R>(k.mu[a], S.x);
-        m.y = S.y;
+        m.x = add_rn<R>(k.mu[a], S.E[a].x);
+        m.y = S.E[a].y;
         C2 in = xmadd<R>(km[a], m, pm[a]);
-        in = (a == 0 || a == 3) ? xmadd<R>(in, cc[3 - a], D) : xmsub<R>(in, cc[3 - a], D);
+        in = xmadd<R>(in, cc[3 - a], D[a == 0 || a == 3 ? 0 : 1]);
         K[a].x = fma_rn<R>(k.eps, in.x, add_rn<R>(pm[a].x, -pc[a].x));
         K[a].y = fma_rn<R>(k.eps, in.y, add_rn<R>(pm[a].y, -pc[a].y));
         if (k.scaled) K[a] = xscale<R>(k.pre, K[a]);
@@ -110,9 +127,10 @@ __device__ __forceinline__ void drift_ref4_psi(const DriftConsts<R> &k, C2 S, co
 
 // S: ref4_density of (pc, cp).
 template <class R, class C2>
-__device__ __forceinline__ void drift_ref4_bar(const DriftConsts<R> &k, C2 S, const C2 *pc, const C2 *pp, const C2 *cc,
-                                               const C2 *cp, const C2 *kp, C2 *Kc, int cmask = 0xF) {
-    const C2 D = ref4_exchange<R>(k.g2, cp);
+__device__ __forceinline__ void drift_ref4_bar(const DriftConsts<R> &k, const Ref4Density<C2> &S, const C2 *pc, const C2 *pp,
+                                               const C2 *cc, const C2 *cp, const C2 *kp, C2 *Kc, int cmask = 0xF) {
+    C2 D[2];
+    ref4_exchange<R>(k.g2, cp, D);
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
         if (!((cmask >> a) & 1)) continue;
@@ -121,8 +139,8 @@ __device__ __forceinline__ void drift_ref4_bar(const DriftConsts<R> &k, C2 S, co
         C2 in;
         in.x = fma_rn<R>(k.mu[a], pp[a].x, kp[a].x);
         in.y = fma_rn<R>(k.mu[a], pp[a].y, kp[a].y);
-        in = xmadd<R>(in, S, cp[a]);
-        in = (a == 0 || a == 3) ? xmadd<R>(in, pc[3 - a], D) : xmsub<R>(in, pc[3 - a], D);
+        in = xmadd<R>(in, S.E[a], cp[a]);
+        in = xmadd<R>(in, pc[3 - a], D[a == 0 || a == 3 ? 0 : 1]);
         Kc[a].x = fma_rn<R>(k.eps, in.x, add_rn<R>(cp[a].x, -cc[a].x));
         Kc[a].y = fma_rn<R>(k.eps, in.y, add_rn<R>(cp[a].y, -cc[a].y));
         if (k.scaled) Kc[a] = xscale<R>(k.pre, Kc[a]);
@@ -134,8 +152,8 @@ __device__ __forceinline__ void drift_ref4_vals(const DriftConsts<R> &k, const C
                                                 const C2 *pp, const C2 *cc, const C2 *cp,
                                                 const C2 *km, const C2 *kp, C2 *K, C2 *Kc, int which = 3,
                                                 int cmask = 0xF) {
-    if (which & 1) drift_ref4_psi<R>(k, ref4_density<R>(k.g2, pm, cc), pm, pc, cc, km, K, cmask);
-    if (which & 2) drift_ref4_bar<R>(k, ref4_density<R>(k.g2, pc, cp), pc, pp, cc, cp, kp, Kc, cmask);
+    if (which & 1) drift_ref4_psi<R>(k, ref4_density<R>(k.g2, pm, cc, cmask), pm, pc, cc, km, K, cmask);
+    if (which & 2) drift_ref4_bar<R>(k, ref4_density<R>(k.g2, pc, cp, cmask), pc, pp, cc, cp, kp, Kc, cmask);
 }
 
 // Spin-1 model.  Of one (bar, ket) pair the contact potential V = c0/2 n^2 + c1/2 (Fz^2 +

@@ -78,7 +78,7 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
     // carried: psi(tau-1), psibar(tau), psi(tau) and the pair (psibar(tau), psi(tau-1))
     C2 Pp[NC], Qc[NC], Pc[NC];
     Spin1Link<C2> Bm;
-    C2 Sm;
+    Ref4Density<C2> Sm;
     // prefetched for the next tau: psi(tau+1), psibar(tau+1), kin(tau-1), kinbar(tau+1)
     C2 nP[NC], nQ[NC], nK[NC], nKc[NC];
     auto load_next = [&](int tau) {
