@@ -19,6 +19,7 @@
 
 #include "clv_internal.cuh"
 #include "clv_launch.h"
+#include "tile_plan.h"
 
 using namespace clv;
 
@@ -52,39 +53,6 @@ bool factorize(int n, int *fac, int &nf) {
     while (n % 3 == 0 && nf < kMaxFactors) { fac[nf++] = 3; n /= 3; }
     while (n % 5 == 0 && nf < kMaxFactors) { fac[nf++] = 5; n /= 5; }
     return n == 1;
-}
-
-// In-place plan of the tile filter: as few radices of 2 .. most as the length allows, the most
-// even such split, larger ones first.
-bool tile_factors(int n, int most, int *fac, int &nf) {
-    static const int radices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
-    if (n <= 1) return false;
-    for (int want = 1; want <= kMaxTileFactors; ++want) {
-        int best[kMaxTileFactors], cur[kMaxTileFactors], sum = 1 << 30;
-        auto search = [&](auto &&self, int rest, int depth, int top) -> void {
-            if (depth == want) {
-                int s = 0;
-                for (int i = 0; i < want; ++i) s += cur[i];
-                if (rest == 1 && s < sum) {
-                    sum = s;
-                    std::copy(cur, cur + want, best);
-                }
-                return;
-            }
-            for (int r : radices)
-                if (r <= top && rest % r == 0) {
-                    cur[depth] = r;
-                    self(self, rest / r, depth + 1, r);
-                }
-        };
-        search(search, n, 0, most);
-        if (sum < (1 << 30)) {
-            nf = want;
-            std::copy(best, best + want, fac);
-            return true;
-        }
-    }
-    return false;
 }
 
 }  // namespace
@@ -334,21 +302,15 @@ int build_tables(clv_engine *e) {
             table(&ax.efilt64, e64);
             table(&ax.efilt32, e32);
             // the tile filter's plan, and the filters in the order its forward passes leave
-            // the frequencies: position sum_p q_p (L_p / R_p) holds sum_p q_p (R_0 ... R_{p-1})
+            // the frequencies
             if (!tile_factors(n, e->precision == CLV_PREC_F64 ? tile_radix_max<double>() : tile_radix_max<float>(), ax.tfac, ax.tnf))
                 ax.tnf = 0;
             if (ax.tnf) {
+                const std::vector<int> order = tile_order(n, ax.tfac, ax.tnf);
                 std::vector<double> tf64(n), te64(n);
                 for (int i = 0; i < n; ++i) {
-                    int rest = i, L = n, w = 1, k = 0;
-                    for (int p = 0; p < ax.tnf; ++p) {
-                        L /= ax.tfac[p];
-                        k += rest / L * w;
-                        rest %= L;
-                        w *= ax.tfac[p];
-                    }
-                    tf64[i] = f64[k];
-                    te64[i] = e64[k];
+                    tf64[i] = f64[order[i]];
+                    te64[i] = e64[order[i]];
                 }
                 std::vector<float> tf32(tf64.begin(), tf64.end()), te32(te64.begin(), te64.end());
                 for (int k = 0; k < n; ++k) {
@@ -1007,16 +969,6 @@ int tile_plan(clv_engine *e, const TileFilterPlan &p) {
     return (int)e->tile_plans_h.size() - 1;
 }
 
-// Shared elements between the rows of a tile with `lines` lines along rows of n.  A phase of a
-// warp's access (16 elements at FP32, 8 at FP64) takes the lines of the tile at as many
-// neighbouring positions as fit: an odd pitch keeps it free of conflicts when one position of
-// that many lines does, else an odd multiple of the positions does.
-int tile_pitch(const clv_engine *e, int n, int lines) {
-    int g = e->elem_bytes == 8 ? 16 : 8;
-    for (int l = 1; l < lines && g > 1; l *= 2) g /= 2;
-    return g == 1 ? n | 1 : (n + g - 1) / g * g + ((n + g - 1) / g % 2 ? 0 : g);
-}
-
 // Slices of chain d per tile: about tile_target elements (one slice when it is larger), lines in
 // a number that a phase of a warp's access divides evenly when one is near, with two exceptions.
 //   * A problem whose tiles of that size would leave three quarters of the CTAs' places empty
@@ -1044,7 +996,7 @@ int slices_per_tile(const clv_engine *e, const ChainDev &d, int nsum, int rows1,
     if (alike) {
         const int last = std::max(1, std::min(d.nt, most / d.V));
         auto of = [&](int ns, double &tiles) {
-            const int elems = ns * rows1 * tile_pitch(e, cols, ns * rows1);
+            const int elems = ns * rows1 * tile_pitch(e->elem_bytes, cols, ns * rows1);
             tiles = 0;
             for (auto &o : e->chains_h) tiles += (double)d.ncomp * ((o.nt + ns - 1) / ns) * (energy ? 1 : 2);
             return resident(elems, tile_smem(e, elems, nsum, ns * rows1, ns * rows1));
@@ -1103,7 +1055,7 @@ int add_tile_slices(clv_engine *e, int c, bool energy, std::vector<clv_engine::A
     }
     p.with_const = !energy && e->kinetic == CLV_KIN_EXP;
     const int ns = slices_per_tile(e, d, nsum, rows1, cols, energy);
-    p.pitch = tile_pitch(e, cols, ns * rows1);
+    p.pitch = tile_pitch(e->elem_bytes, cols, ns * rows1);
     p.tile_elems = (ns * rows1 * p.pitch + 1) / 2 * 2;
     const int id = tile_plan(e, p);
     auto &g = tile_group(e, groups, 0, p.naxes == 1 ? d.axis[p.axis[0]].n : 0, p.naxes > 1, p.tile_elems,
@@ -1145,7 +1097,7 @@ int add_tile_axis(clv_engine *e, int c, int a, bool energy, std::vector<clv_engi
     } else {
         const int W = std::max(1, std::min(lines, target / n));
         p.inner[0] = 1;
-        p.pitch = tile_pitch(e, n, W);
+        p.pitch = tile_pitch(e->elem_bytes, n, W);
         p.tile_elems = (W * p.pitch + 1) / 2 * 2;
         const int id = tile_plan(e, p);
         auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, 0, W));

@@ -239,8 +239,7 @@ struct Radix<C2, 3> {
         const C2 t1 = vadd(a[1], a[2]), t2 = vsub(a[1], a[2]);
         C2 m;
         if constexpr (std::is_same_v<R, long long>) {
-            m.x = a[0].x - (t1.x >> 1);
-            m.y = a[0].y - (t1.y >> 1);
+            m = vsub(a[0], ihalf(t1));
         } else {
             m.x = fma_rn<R>(-half, t1.x, a[0].x);
             m.y = fma_rn<R>(-half, t1.y, a[0].y);

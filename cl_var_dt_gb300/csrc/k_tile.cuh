@@ -228,13 +228,21 @@ template <> __device__ __forceinline__ const float *tile_filt<float>(const AxisD
     return energy ? ax.tefilt32 : ax.tfilt32;
 }
 
-// Global to shared without registers (8 or 16 bytes per thread).
+// Global to shared without registers (8 or 16 bytes per thread), and the wait for it.
+#if defined(__CUDACC__)
 template <class C2>
 __device__ __forceinline__ void copy_async(C2 *s, const C2 *g) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((uint32_t)__cvta_generic_to_shared(s)), "l"(g),
                  "n"((int)sizeof(C2))
                  : "memory");
 }
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+#else  // host build of the tests
+template <class C2> inline void copy_async(C2 *s, const C2 *g) { *s = *g; }
+inline void copy_async_commit() {}
+inline void copy_async_wait() {}
+#endif
 
 // TH threads: 128, or 256 for the large slices.
 template <class R, int TH>
@@ -266,7 +274,7 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
         const int r = dc.div(e), c = e - r * cols;
         copy_async(tile + r * PZ + c, src + (long long)r * gs + c);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    copy_async_commit();
     // tables of the filtered axes: twiddles, then the filters in the passes' order of
     // frequencies, the component constant folded into the first axis' one
     int nsum = 0;
@@ -333,7 +341,7 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
         sc.exps = reinterpret_cast<int *>(sc.zero + sc.ng);
         for (int i = threadIdx.x; i < 5 * sc.ng; i += blockDim.x) sc.raw[i] = 0;
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    copy_async_wait();
     __syncthreads();
     if constexpr (kInt) {
         const AxisDev &ax = ch.axis[P.axis[0]];
