@@ -297,6 +297,7 @@ int build_tables(clv_engine *e) {
             std::vector<float> f32(f64.begin(), f64.end()), e32(e64.begin(), e64.end());
             table(&ax.tw64, tw64);
             table(&ax.tw32, tw32);
+            if (e->precision == CLV_PREC_F64) table(&ax.tw62, fixed_twiddles(n));
             table(&ax.filt64, f64);
             table(&ax.filt32, f32);
             table(&ax.efilt64, e64);

@@ -51,6 +51,7 @@ struct AxisDev {
     int fac[kMaxFactors];  // radix of each Stockham pass
     const double2 *tw64;   // exp(-2 pi i k/n), k < n
     const float2 *tw32;
+    const void *tw62;      // the same with 62 fraction bits (WCplx; FP64 engines, fft_int.cuh)
     const double *filt64;  // kinetic filter f[k], k < n (normalisation folded in)
     const float *filt32;
     const double *efilt64; // kinetic-energy filter k^2/2 / n (spin-1 observables)

@@ -151,11 +151,7 @@ __device__ __forceinline__ int exp_above(double x) {
     const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
     return e + (((hi & 0xfffff) | __double2loint(x)) != 0);
 }
-// Table entries: a twiddle, and a filter value relative to 2^e.
-__device__ __forceinline__ WCplx twiddle_fixed(double2 w) {
-    const double q = 4611686018427387904.0;  // 2^62
-    return WCplx{wsplit(__double2ll_rn(w.x * q)), wsplit(__double2ll_rn(w.y * q))};
-}
+// Table entry: a filter value relative to 2^e.
 __device__ __forceinline__ long long filter_fixed(double f, int e) { return __double2ll_rn(f * pow2(kFiltQ - e)); }
 
 // Exponent word of the largest component, for a line's maximum.

@@ -14,9 +14,12 @@
 
 namespace clv {
 
-// A butterfly's real constant in the arithmetic type: itself, or with 62 fraction bits.
-template <class R> __host__ __device__ constexpr R kconst(double c) { return (R)c; }
-template <> __host__ __device__ constexpr long long kconst<long long>(double c) { return (long long)(c * 4611686018427387904.0); }
+// A butterfly's real constant in the arithmetic type: itself, or with 62 fraction bits (lo: what
+// the double c leaves of it).
+template <class R> __host__ __device__ constexpr R kconst(double c, double lo = 0.0) { return (R)c; }
+template <> __host__ __device__ constexpr long long kconst<long long>(double c, double lo) {
+    return (long long)(c * 4611686018427387904.0) + (long long)(lo * 4611686018427387904.0 + (lo < 0 ? -0.5 : 0.5));
+}
 
 // S * i * z for a compile-time direction S
 template <int S, class C2>
@@ -158,7 +161,7 @@ struct Radix<C2, 8> {
     template <int S>
     static __device__ __forceinline__ void finish(C2 *a, const C2 *e, const C2 *o) {
         using R = decltype(a[0].x);
-        const R h = kconst<R>(0.70710678118654752440);
+        const R h = kconst<R>(0.70710678118654752440, -4.833646656726457e-17);
         // twiddles exp(S 2 pi i q/8), q = 1, 2, 3: h t1, S i, h t3
         C2 t1, t3;
         if (S < 0) {
@@ -235,7 +238,7 @@ struct Radix<C2, 3> {
     template <int S>
     static __device__ __forceinline__ void run(C2 *a) {
         using R = decltype(a[0].x);
-        const R half = kconst<R>(0.5), s3 = kconst<R>(0.86602540378443864676);
+        const R half = kconst<R>(0.5), s3 = kconst<R>(0.86602540378443864676, 5.017542110903451e-17);
         const C2 t1 = vadd(a[1], a[2]), t2 = vsub(a[1], a[2]);
         C2 m;
         if constexpr (std::is_same_v<R, long long>) {
@@ -291,8 +294,8 @@ struct Radix<C2, 5> {
     template <int S>
     static __device__ __forceinline__ void run(C2 *a) {
         using R = decltype(a[0].x);
-        const R c1 = kconst<R>(0.30901699437494742410), c2 = kconst<R>(-0.80901699437494742410);
-        const R s1 = kconst<R>(0.95105651629515357212), s2 = kconst<R>(0.58778525229247312917);
+        const R c1 = kconst<R>(0.30901699437494742410, -2.716057601841253e-17), c2 = kconst<R>(-0.80901699437494742410, 2.716057601841253e-17);
+        const R s1 = kconst<R>(0.95105651629515357212, 4.09345009000873e-17), s2 = kconst<R>(0.58778525229247312917, -7.93475083819002e-18);
         const C2 t1 = vadd(a[1], a[4]), t2 = vadd(a[2], a[3]);
         const C2 t3 = vsub(a[1], a[4]), t4 = vsub(a[2], a[3]);
         C2 b1, b2, q1, q2;
@@ -360,8 +363,8 @@ struct Radix<C2, 9> {
     static __device__ __forceinline__ void run(C2 *a) {
         using R = decltype(a[0].x);
         // W9^m = (cos(2 pi m / 9), S sin(2 pi m / 9)), m = 1, 2, 4
-        const R c[3] = {kconst<R>(0.76604444311897803520), kconst<R>(0.17364817766693034885), kconst<R>(-0.93969262078590838405)};
-        const R s[3] = {kconst<R>(S * 0.64278760968653932632), kconst<R>(S * 0.98480775301220805937), kconst<R>(S * 0.34202014332566873304)};
+        const R c[3] = {kconst<R>(0.76604444311897803520, 2.1750711742081045e-17), kconst<R>(0.17364817766693034885, -1.0090493350843633e-17), kconst<R>(-0.93969262078590838405, 4.385093284002042e-17)};
+        const R s[3] = {kconst<R>(S * 0.64278760968653932632, S * -3.659607900790949e-17), kconst<R>(S * 0.98480775301220805937, S * 3.905108875799298e-17), kconst<R>(S * 0.34202014332566873304, S * 2.0136016534644645e-17)};
         C2 y[3][3];
 #pragma unroll
         for (int n2 = 0; n2 < 3; ++n2) {

@@ -459,7 +459,7 @@ struct LineFilter<double, N> {
         WCplx *tw = reinterpret_cast<WCplx *>(smem + 64);
         long long *f = reinterpret_cast<long long *>(smem + 64 + n * sizeof(WCplx));
         const AxisDev &ax = ch.axis[0];
-        for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = twiddle_fixed(ax.tw64[i]);
+        for (int i = threadIdx.x; i < n; i += blockDim.x) tw[i] = static_cast<const WCplx *>(ax.tw62)[i];
         for (int c = 0; c < ncomp; ++c) {
             const double cst = kinetic == CLV_KIN_EXP ? ch.comp_const[c] : 1.0;
             const int e = exp_above(ax.fmax * cst);

@@ -217,8 +217,8 @@ __device__ __forceinline__ void tile_pass_any(int R, typename Cx<RR>::T *t, cons
     }
 }
 
-template <class R> __device__ __forceinline__ const typename Cx<R>::T *tile_tw(const AxisDev &ax);
-template <> __device__ __forceinline__ const double2 *tile_tw<double>(const AxisDev &ax) { return ax.tw64; }
+template <class R> __device__ __forceinline__ const typename TileMath<R>::W *tile_tw(const AxisDev &ax);
+template <> __device__ __forceinline__ const WCplx *tile_tw<double>(const AxisDev &ax) { return static_cast<const WCplx *>(ax.tw62); }
 template <> __device__ __forceinline__ const float2 *tile_tw<float>(const AxisDev &ax) { return ax.tw32; }
 template <class R> __device__ __forceinline__ const R *tile_filt(const AxisDev &ax, int energy);
 template <> __device__ __forceinline__ const double *tile_filt<double>(const AxisDev &ax, int energy) {
@@ -296,7 +296,7 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
         int o = 0;
         for (int a = 0; a < nax; ++a) {
             const AxisDev &ax = ch.axis[P.axis[a]];
-            const C2 *tw = tile_tw<R>(ax);
+            const W *tw = tile_tw<R>(ax);
             const R *f = tile_filt<R>(ax, energy);
             // energy: sum of the axes' k^2/2; each axis' table carries 1/n, and the sum over
             // axes of a slice's transforms needs the product of all 1/n on every term
@@ -313,13 +313,9 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
                 cst *= pow2(kFiltQ - e);
             }
             for (int i = threadIdx.x; i < ax.n; i += blockDim.x) {
-                if constexpr (kInt) {
-                    tw0[o + i] = twiddle_fixed(tw[i]);
-                    f0[o + i] = __double2ll_rn(f[i] * cst);
-                } else {
-                    tw0[o + i] = tw[i];
-                    f0[o + i] = f[i] * cst;
-                }
+                tw0[o + i] = tw[i];
+                if constexpr (kInt) f0[o + i] = __double2ll_rn(f[i] * cst);
+                else f0[o + i] = f[i] * cst;
             }
             o += ax.n;
         }

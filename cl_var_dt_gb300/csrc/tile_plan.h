@@ -1,11 +1,12 @@
 // tile_plan.h -- host side of the tile filter's plans (k_tile.cuh): radices, the order of
-// frequencies that they leave, the tile's pitch.
+// frequencies that they leave, the tile's pitch; the twiddles of the integer lines.
 #pragma once
 
 #include <algorithm>
 #include <vector>
 
 #include "clv_internal.cuh"
+#include "fft_int.cuh"
 
 namespace clv {
 
@@ -57,6 +58,40 @@ inline std::vector<int> tile_order(int n, const int *fac, int nf) {
         order[i] = k;
     }
     return order;
+}
+
+// exp(-2 pi i k / n), k < n, with 62 fraction bits.  Rounded doubles would carry 2^-54 of an
+// element into every product, which is the whole error of a line with one site far above the
+// others.  Taylor series in 96 fraction bits of the angle from the nearest multiple of pi / 4
+// (integers: the same table on every host).
+inline std::vector<WCplx> fixed_twiddles(int n) {
+    using u128 = unsigned __int128;
+    using i128 = __int128;
+    auto mul = [](i128 a, i128 b) {  // |a|, |b| <= 2^96
+        const u128 x = a < 0 ? -(u128)a : (u128)a, y = b < 0 ? -(u128)b : (u128)b, m = ((u128)1 << 48) - 1;
+        const u128 p = (x >> 48) * (y >> 48) + (((x >> 48) * (y & m) + (x & m) * (y >> 48)) >> 48);
+        return (a < 0) != (b < 0) ? -(i128)p : (i128)p;
+    };
+    const i128 one = (i128)1 << 96, twopi = ((i128)0x6487ED511ull << 64) | 0x0B4611A62633145Cull;
+    std::vector<WCplx> tw(n);
+    for (int k = 0; k < n; ++k) {
+        const int o = (8 * k + n / 2) / n;                         // nearest multiple of pi / 4
+        const i128 t = twopi * (8 * k - o * n) / (8 * n);
+        i128 c = 0, s = 0, term = one;
+        for (int j = 1; term != 0; j += 2) {                       // cos, sin of t, |t| <= pi / 8
+            c += term;
+            term = mul(term, t) / j;
+            s += term;
+            term = -mul(term, t) / (j + 1);
+        }
+        const i128 h = ((i128)0xB504F333ull << 64) | 0xF9DE6484597D89B3ull;  // sqrt(1/2)
+        const i128 d = mul(h, c - s), e = mul(h, c + s);
+        // angle o pi / 4 + t
+        const i128 x[8] = {c, d, -s, -e, -c, -d, s, e}, y[8] = {s, e, c, d, -s, -e, -c, -d};
+        auto round = [](i128 v) { return (long long)((v + ((i128)1 << 33)) >> 34); };
+        tw[k] = WCplx{wsplit(round(x[o & 7])), wsplit(round(-y[o & 7]))};
+    }
+    return tw;
 }
 
 // Shared elements between the rows of a tile with `lines` lines along rows of n.  A phase of a

@@ -118,3 +118,25 @@ def test_no_site_is_worse_than_the_others(lib, n, kind):
     x, f = field("condensate", 200, (n,)), [filter_of(kind, n)]
     _, site = errors(integer(lib, x, f), exact(x, f))
     assert site.max() < 1.3 * np.sqrt((site ** 2).mean()), site.argmax()
+
+
+@pytest.mark.parametrize("n", [2, 3, 8, 27, 48, 125, 900, 1875, 2048])
+def test_twiddles_to_62_bits(lib, n):
+    """Half a unit of rounding and 2^-80 of the series; 2^-2 units of the extended reference."""
+    tab = np.empty((n, 2), np.int64)
+    lib.fixed_twiddle_table(n, ptr(tab))
+    c, s = dft(n, -1)
+    got = tab.astype(LD)
+    want = np.stack([c[1 % n], s[1 % n]], 1) * LD(2) ** 62
+    assert np.abs(got - want).max() < 0.76
+
+
+@pytest.mark.parametrize("kind", ["exp", "k2"])
+@pytest.mark.parametrize("n", [9, 60, 192, 480, 729, 1152, 1728])
+def test_one_site_far_above_the_others(lib, n, kind):
+    """No further off than FP64 butterflies, at the worst site and in the 2-norm: with one site a
+    thousand times the others every product of it carries its factor's error."""
+    x, f = field("one_site", 48, (n,)), [filter_of(kind, n)]
+    want = exact(x, f)
+    (norm, site), (norm64, site64) = errors(integer(lib, x, f), want), errors(butterflies(lib, x, f), want)
+    assert norm < norm64 and site.max() < site64.max()

@@ -20,6 +20,13 @@ extern "C" void tile_frequencies(int n, int most, int *out) {
     std::copy(o.begin(), o.end(), out);
 }
 
+extern "C" void fixed_twiddle_table(int n, long long *out) {
+    for (const WCplx &w : fixed_twiddles(n)) {
+        *out++ = (long long)w.x.h * 4294967296ll + w.x.l;
+        *out++ = (long long)w.y.h * 4294967296ll + w.y.l;
+    }
+}
+
 static std::vector<double2> twiddles(int n) {
     std::vector<double2> tw(n);
     for (int k = 0; k < n; ++k) {
@@ -41,7 +48,7 @@ extern "C" int tile_filter(const int *dims, int axes, int ns, int energy, double
     ch.ncomp = 1;
     ch.comp_const[0] = cst;
     TileFilterPlan P{};
-    std::vector<double2> tw[3];
+    std::vector<WCplx> tw[3];
     std::vector<double> f[3];
     int last = 0, nsum = 0;
     for (int a = 0, o = 0; a < 3; ++a) {
@@ -51,7 +58,7 @@ extern "C" int tile_filter(const int *dims, int axes, int ns, int energy, double
         if (dims[a] > 1) last = a;
         if (dims[a] <= 1 || a >= axes) continue;
         if (!tile_factors(ax.n, tile_radix_max<double>(), ax.tfac, ax.tnf)) return 0;
-        tw[a] = twiddles(ax.n);
+        tw[a] = fixed_twiddles(ax.n);
         const std::vector<int> order = tile_order(ax.n, ax.tfac, ax.tnf);
         f[a].resize(ax.n);
         double most = 0;
@@ -60,7 +67,7 @@ extern "C" int tile_filter(const int *dims, int axes, int ns, int energy, double
             most = std::max(most, std::fabs(f[a][i]));
         }
         o += ax.n;
-        ax.tw64 = tw[a].data();
+        ax.tw62 = tw[a].data();
         ax.tfilt64 = ax.tefilt64 = f[a].data();
         ax.fmax = ax.efmax = most;
         P.axis[P.naxes] = a;
