@@ -8,10 +8,10 @@
 // inverse in integers, and is converted back.
 //
 // * Block floating point: a pass of radix R first shifts its line by the bits that keep R
-//   times the largest component below 2^62 (kTop), which the pass before it has found;
-//   the first pass' input is scaled to that.  The shifts add up per line.  The middle pass
-//   shifts its product with the filter by ceil(log2 R), for the inverse butterfly whose
-//   inputs it has only in registers.
+//   times the largest component, which the pass before it has found, below 2^62.25; the first
+//   pass' input is scaled to that.  The shifts add up per line.  The middle pass shifts its
+//   product with the filter by ceil(log2 R), for the inverse butterfly whose inputs it has
+//   only in registers.
 // * Twiddles carry 62 fraction bits, filters 60 relative to the power of two at or above
 //   their largest value; products are rounded (a bias of half a unit at every frequency
 //   would add up at the line's first site).
@@ -101,16 +101,29 @@ __device__ __forceinline__ I2 ishift(I2 z, int s) {
     return I2{(z.x + (half - ((int)z.y & any))) >> s, (z.y + (half - ((int)z.x & any))) >> s};
 }
 __device__ __forceinline__ I2 ihalf(I2 z) { return I2{(z.x + ((int)z.y & 1)) >> 1, (z.y + ((int)z.x & 1)) >> 1}; }
-// High words of the magnitudes (a line's largest component), and the shift that keeps
-// 2^lr times a component of that high word below 2^kTop.
+// High word of the magnitude of a line's largest component.
 __device__ __forceinline__ unsigned imag_bits(I2 z) {
     const int a = (int)(z.x >> 32), b = (int)(z.y >> 32);
     const unsigned u = (unsigned)(a ^ (a >> 31)), v = (unsigned)(b ^ (b >> 31));
     return u > v ? u : v;
 }
-__device__ __forceinline__ int ishift_for(unsigned mag, int lr) {
-    const int s = 64 - __clz((int)mag) + lr - kTop;
-    return s > 0 ? s : 0;
+// Shifts before a butterfly of R inputs: the least that keeps R times a component below
+// 2^62.25, so that the outputs, of up to sqrt(2) times that, keep within 63 bits and their
+// products with twiddles too (imul's cross products: 2^30.75 2^31.5 + 2^31.5 2^30 < 2^63).
+// Counting R as the next power of two, and the component too, would leave up to two bits of the 62 unused
+// in every pass: a condensate fills them all at one frequency, and what it leaves to the others
+// is their precision (lines of 729 and 900 sites: 1.3 times the FP64 butterflies' error, now 0.7).
+// ishift_for: of a component with the high word mag; ifirst_for: of a double with the high
+// word raw, which to_fixed puts in [2^61, 2^62).
+__device__ __forceinline__ int ishift_for(unsigned mag, int r) {
+    const unsigned long long t = (unsigned long long)(mag + 1u) * (unsigned)r;  // units of 2^32
+    const int s = 33 - __clzll((long long)t);                                   // t >> s in [2^30, 2^31)
+    return s < 0 ? 0 : s + ((t >> s) > 1276901416ull);                          // 2^30.25
+}
+__device__ __forceinline__ int ifirst_for(unsigned raw, int r) {
+    const unsigned t = ((raw & 0xfffffu) + 0x100001u) * (unsigned)r;  // units of 2^41
+    const int s = 10 - __clz((int)t);                                 // t >> s in [2^21, 2^22)
+    return s + ((t >> s) > 2493948u);                                 // 2^21.25
 }
 // product with a filter value (kFiltQ fraction bits), shifted by another S <= 4 bits
 template <int S>

@@ -277,8 +277,9 @@ struct IntLine {
                     m = u > m ? u : m;
                 }
         }
-        const int em = (int)(reduce(m) >> 20);
-        e = 2;
+        const unsigned raw = reduce(m);
+        const int em = (int)(raw >> 20);
+        e = ifirst_for(raw, 4);
         m = 0;
 #pragma unroll
         for (int i = 0; i < REP; ++i) {
@@ -286,7 +287,7 @@ struct IntLine {
             if (NB % NT == 0 || j < NB) {
                 I2 v[4];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) v[r] = I2{to_fixed(d[i][r].x, em, 2), to_fixed(d[i][r].y, em, 2)};
+                for (int r = 0; r < 4; ++r) v[r] = I2{to_fixed(d[i][r].x, em, e), to_fixed(d[i][r].y, em, e)};
                 Radix<I2, 4>::template run<-1>(v);
                 I2 *o = reinterpret_cast<I2 *>(X);
 #pragma unroll
@@ -323,7 +324,7 @@ struct IntLine {
     // Radix-4 pass at stride NS = 2^ls; LAST: writes doubles, dense.
     template <int S, bool LAST>
     __device__ __forceinline__ void pass(const I2 *s, I2 *dst, const WCplx *tw, int ls, int em, int eg) {
-        const int sh = ishift_for(mx, 2);
+        const int sh = ishift_for(mx, 4);
         e += sh;
         unsigned m = 0;
         I2 u[REP][4];
@@ -371,7 +372,7 @@ struct IntLine {
     // Last forward pass, filter, first inverse pass.
     __device__ __forceinline__ void middle(const I2 *s, I2 *dst, const WCplx *tw, const long long *f) {
         constexpr int LR = RL == 4 ? 2 : 1, NM = N / RL, REPM = (NM + NT - 1) / NT;
-        const int sh = ishift_for(mx, LR);
+        const int sh = ishift_for(mx, RL);
         e += sh + LR;
         unsigned m = 0;
         I2 u[REPM][RL];

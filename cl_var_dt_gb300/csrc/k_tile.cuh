@@ -122,14 +122,14 @@ __device__ __forceinline__ void tile_pass(typename Cx<RR>::T *t, const TileLines
             if constexpr (kInt) {
                 gr = sc.group.div(l);
                 if (sc.first) {
-                    const int em = (int)(sc.raw[gr] >> 20);
+                    const int em = (int)(sc.raw[gr] >> 20), sf = ifirst_for(sc.raw[gr], R);
 #pragma unroll
                     for (int m = 0; m < R; ++m) {
                         const double2 d = p[m * st];
-                        v[m] = I2{to_fixed(d.x, em, LR), to_fixed(d.y, em, LR)};
+                        v[m] = I2{to_fixed(d.x, em, sf), to_fixed(d.y, em, sf)};
                     }
                 } else {
-                    const int sh = ishift_for(sc.cur[gr], LR);
+                    const int sh = ishift_for(sc.cur[gr], R);
 #pragma unroll
                     for (int m = 0; m < R; ++m) v[m] = ishift(*reinterpret_cast<const I2 *>(p + m * st), sh);
                 }
@@ -166,7 +166,7 @@ __device__ __forceinline__ void tile_pass(typename Cx<RR>::T *t, const TileLines
                 if (KIND != TILE_DIF && sc.last) {
                     const int em = (int)(sc.raw[gr] >> 20);
                     const int e = sc.eg + sc.exps[gr] + (KIND == TILE_MID ? LR : 0) +
-                                  (sc.first ? LR : ishift_for(sc.cur[gr], LR));
+                                  (sc.first ? ifirst_for(sc.raw[gr], R) : ishift_for(sc.cur[gr], R));
 #pragma unroll
                     for (int m = 0; m < R; ++m) p[m * st] = make_double2(from_fixed(v[m].x, em, e), from_fixed(v[m].y, em, e));
                 } else {
@@ -188,7 +188,7 @@ __device__ __forceinline__ void tile_pass(typename Cx<RR>::T *t, const TileLines
     if constexpr (kInt && KIND != TILE_MAX) {
         if (!sc.last)  // (the last pass reads exps)
             for (int i = threadIdx.x; i < sc.ng; i += blockDim.x) {
-                sc.exps[i] += (KIND == TILE_MID ? LR : 0) + (sc.first ? LR : ishift_for(sc.cur[i], LR));
+                sc.exps[i] += (KIND == TILE_MID ? LR : 0) + (sc.first ? ifirst_for(sc.raw[i], R) : ishift_for(sc.cur[i], R));
                 sc.zero[i] = 0;
             }
     }

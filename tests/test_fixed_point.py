@@ -140,3 +140,29 @@ def test_one_site_far_above_the_others(lib, n, kind):
     want = exact(x, f)
     (norm, site), (norm64, site64) = errors(integer(lib, x, f), want), errors(butterflies(lib, x, f), want)
     assert norm < norm64 and site.max() < site64.max()
+
+
+@pytest.mark.parametrize("kind", ["condensate", "wide", "flat"])
+@pytest.mark.parametrize("dims", [(8,), (48,), (60,), (250,), (600,), (729,), (810,), (900,), (1250,), (1875,), (2000,), (2048,),
+                                  (30, 30), (27, 25), (8, 6, 4)], ids=lambda d: "x".join(map(str, d)))
+def test_exponential_filter_against_butterflies(lib, dims, kind):
+    """No further off than FP64 butterflies on a condensate, whose zero mode takes the top bits:
+    plans of one to five radices, lines and slices."""
+    x, f = field(kind, 48, dims), [filter_of("exp", n) for n in dims]
+    want = exact(x, f)
+    (norm, site), (norm64, site64) = errors(integer(lib, x, f), want), errors(butterflies(lib, x, f), want)
+    assert norm < norm64 and site.max() < site64.max()
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 9, 16, 48, 60, 243, 500, 900, 1875])
+def test_single_modes_do_not_overflow(lib, n):
+    """A line that is one mode grows by its whole radix in every pass; amplitudes along the binade
+    and directions of up to sqrt(2) times a component.  An overflow would be an error of the
+    line's size; roundings are 2^-50 of it at most."""
+    k, j = np.arange(min(n, 40))[:, None], np.arange(n)[None, :]
+    for amp in (1.0, 1.2, 1.5, 1.9999999, 2 - 2.0 ** -52):
+        for turn in (1.0, 1j, np.exp(0.25j * np.pi), np.exp(1.0j)):
+            x = amp * turn * np.exp(2j * np.pi * (k * j % n) / n)
+            f = filter_of("exp", n)
+            want = x * (f * n)[k]
+            assert np.abs(integer(lib, x, [f]) - want).max() < 2.0 ** -50 * 2
