@@ -246,6 +246,7 @@ struct TileFilterPlan {
     int pitch;          // shared elements between rows (tile_pitch)
     int gstride;        // global elements between rows, 0: rows follow one another
     int with_const;     // multiply the component constant
+    int based;          // FP64: the filter vanishes at zero frequency (k^2), lines relative to their first site
     int tile_elems;     // shared elements of a full tile
 };
 struct TileFilterTask {

@@ -19,7 +19,10 @@
 // FP64 lines run in block floating point on the integer pipes (fft_int.cuh): a pass over the
 // raw tile finds every line's largest component (every slice's, when several axes are
 // filtered), the first pass converts as it reads and the last one converts back as it
-// writes.  128-site lines, 4 components x 128 x 128 x 128 imaginary times, both fields: 1.37
+// writes.  A filter that vanishes at zero frequency (k^2: the reference's kinetic term and all
+// kinetic energies) does not see a constant, so its lines are taken relative to their first
+// site: a condensate would fill the top bits at a frequency that is then thrown away (lines of 1250
+// sites: 1.6 times the FP64 butterflies' error, now 0.5).  128-site lines, 4 components x 128 x 128 x 128 imaginary times, both fields: 1.37
 // (butterflies on the FP64 pipe, at its rate) -> 0.53 ms; 48-site lines of 48 x 40 x 36 x 24:
 // 0.93 -> 0.37 ms.  Bound by integer issue (46 % of the ALU) and instruction fetch.
 //
@@ -66,11 +69,12 @@ template <> struct TileMath<double> { using E = I2; using W = WCplx; using F = l
 // FP64: the lines' scale.  Line l belongs to group l / lines per group; of each group, raw: the
 // high word of the largest component as the doubles came in; cur, next: of the largest one
 // after the pass before this one and after this one (zero: cleared for the pass after);
-// exps: the shifts so far.  first: the pass reads doubles; last: it writes them.  eg: the
+// exps: the shifts so far; base: its first site, for a filter that vanishes at zero frequency (or null).  first: the pass reads doubles; last: it writes them.  eg: the
 // filters' power of two.
 struct TileScale {
     unsigned *raw, *cur, *next, *zero;
     int *exps;
+    double2 *base;
     FastDiv group;
     int ng, eg;
     bool first, last;
@@ -109,12 +113,18 @@ __device__ __forceinline__ void tile_pass(typename Cx<RR>::T *t, const TileLines
         if constexpr (KIND == TILE_MAX) {
             if constexpr (kInt) {
                 unsigned mx = 0;
+                const int gr = sc.group.div(l);
+                if (sc.base) {
+                    const double2 z0 = sc.base[gr];
+#pragma unroll
+                    for (int m = 0; m < R; ++m) p[m * st] = vsub(p[m * st], z0);
+                }
 #pragma unroll
                 for (int m = 0; m < R; ++m) {
                     const unsigned v = mag_bits(p[m * st]);
                     mx = v > mx ? v : mx;
                 }
-                atomicMax(&sc.raw[sc.group.div(l)], mx);
+                atomicMax(&sc.raw[gr], mx);
             }
         } else {
             E v[R];
@@ -279,9 +289,10 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
     // frequencies, the component constant folded into the first axis' one
     int nsum = 0;
     for (int a = 0; a < nax; ++a) nsum += ch.axis[P.axis[a]].n;
-    F *f0 = reinterpret_cast<F *>(tw0 + nsum);
+    // (FP64, a filter that vanishes at zero frequency: the groups' first sites between them)
+    F *f0 = reinterpret_cast<F *>(tw0 + nsum + (kInt && P.based ? (nax == 1 ? total / ch.axis[P.axis[0]].n : total / ch.V) : 0));
     F *fo = f0 + nsum;  // summed filters: the rows' shares of the other axes
-    TileScale sc{nullptr, nullptr, nullptr, nullptr, nullptr, FastDiv(1), 0, 0, false, false};
+    TileScale sc{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, FastDiv(1), 0, 0, false, false};
     {
         // FP64: the filters relative to the power of two at or above their largest value (of
         // each axis, or of the sum)
@@ -336,12 +347,19 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
         sc.zero = sc.next + sc.ng;
         sc.exps = reinterpret_cast<int *>(sc.zero + sc.ng);
         for (int i = threadIdx.x; i < 5 * sc.ng; i += blockDim.x) sc.raw[i] = 0;
+        if (P.based) sc.base = reinterpret_cast<double2 *>(tw0 + nsum);
     }
     copy_async_wait();
     __syncthreads();
     if constexpr (kInt) {
         const AxisDev &ax = ch.axis[P.axis[0]];
         group(0);
+        if (sc.base) {
+            const TileLines g = lines(0);
+            for (int i = threadIdx.x; i < sc.ng; i += blockDim.x)
+                sc.base[i] = tile[nax == 1 ? g.base(i) : i * (ch.V / cols) * PZ];
+            __syncthreads();
+        }
         tile_pass_any<R, TILE_MAX>(ax.tfac[0], tile, lines(0), ax.n, ax.n / ax.tfac[0], nullptr, nullptr, nullptr, sc);
     }
     // forward passes of one axis (all of them when `whole`), the middle one, the inverse ones

@@ -87,19 +87,13 @@ def dft(n, sign):
 
 
 def exact(x, filters, energy=False):
+    fft = pytest.importorskip("scipy.fft")
     out = np.zeros(x.shape, np.clongdouble) if energy else x.astype(np.clongdouble)
     for a, f in enumerate(filters):
-        n = f.size
-        if n == 1:
-            continue
-        fr, fi = dft(n, -1)
-        # the filter in x space: a real, even or general kernel of the differences of sites
-        kr = (f.astype(LD)[None, :] * fr).sum(1)
-        ki = -(f.astype(LD)[None, :] * fi).sum(1)
-        d = (np.arange(n)[:, None] - np.arange(n)[None, :]) % n
-        y = np.moveaxis(x.astype(np.clongdouble) if energy else out, a + 1, -1)
-        y = y @ (kr[d] + 1j * ki[d]).T.astype(np.clongdouble)
-        y = np.moveaxis(y, -1, a + 1)
+        s = [1] * x.ndim
+        s[a + 1] = f.size
+        y = x.astype(np.clongdouble) if energy else out
+        y = fft.ifft(fft.fft(y, axis=a + 1) * f.astype(LD).reshape(s), axis=a + 1) * f.size
         out = out + y if energy else y
     return out
 
@@ -166,3 +160,39 @@ def test_single_modes_do_not_overflow(lib, n):
             f = filter_of("exp", n)
             want = x * (f * n)[k]
             assert np.abs(integer(lib, x, [f]) - want).max() < 2.0 ** -50 * 2
+
+
+@pytest.mark.parametrize("kind", ["condensate", "wide", "flat"])
+@pytest.mark.parametrize("dims", [(8,), (48,), (60,), (250,), (600,), (729,), (810,), (900,), (1250,), (1875,), (2000,), (2048,),
+                                  (30, 30), (27, 25), (8, 6, 4)], ids=lambda d: "x".join(map(str, d)))
+def test_k2_filters_against_butterflies(lib, dims, kind):
+    """The k^2 filter of lines and the kinetic energy of slices, which throw the condensate away."""
+    energy = len(dims) > 1
+    x, f = field(kind, 48, dims), [filter_of("energy" if energy else "k2", n) for n in dims]
+    want = exact(x, f, energy)
+    # (the kernel takes the product of all 1 / n into every axis of a sum)
+    (norm, site), (norm64, site64) = errors(integer(lib, x, f, energy), want), errors(butterflies(lib, x, f, energy), want)
+    assert norm < norm64 and site.max() < site64.max()
+
+
+@pytest.mark.parametrize("scale", [1e-150, 1.0, 1e150])
+def test_lines_of_one_value(lib, scale):
+    """A constant line under a filter that vanishes at zero frequency gives exact zeros, also beside
+    other lines of the tile."""
+    x = np.ones((6, 60), complex) * (0.3 - 0.7j) * scale
+    x[2:4] = field("condensate", 2, (60,)) * scale
+    got = integer(lib, x, [filter_of("k2", 60)])
+    assert np.all(got[[0, 1, 4, 5]] == 0) and np.all(got[2:4] != 0)
+
+
+@pytest.mark.parametrize("kind", ["exp", "k2"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("site", [0, 7, 59])
+def test_non_finite_lines_are_nan_and_alone(lib, kind, bad, site):
+    x, f = field("wide", 5, (60,)), [filter_of(kind, 60)]
+    want = integer(lib, x, f)
+    y = x.copy()
+    y[2, site] = bad
+    got = integer(lib, y, f)
+    assert np.all(np.isnan(got[2]))
+    assert np.array_equal(got[[0, 1, 3, 4]], want[[0, 1, 3, 4]])

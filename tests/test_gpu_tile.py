@@ -162,3 +162,43 @@ def test_zero_field_stays_zero(clv):
         assert e.plan()[0] == "tiled"
         e.step_with_noise(np.zeros(2 * 4 * 60 * 9 * 6))
         assert all(np.all(f == 0) for f in e.get_fields(0)) and not any(e.chain_flags())
+
+
+# lines of one to five radices at FP64, relative to their first site; strided tiles with a remainder;
+# two-site lines, whose groups of a tile are the most there can be
+@pytest.mark.parametrize("shape", [(2, 1, 1, 9), (48, 1, 1, 5), (729, 1, 1, 3), (810, 1, 1, 3), (900, 1, 1, 2), (1250, 1, 1, 2),
+                                   (1875, 1, 1, 2), (2048, 1, 1, 2), (48, 20, 15, 2), (2, 60, 60, 2), (100, 81, 1, 2)], ids=str)
+def test_ref4_kinetic_term_against_the_oracle(clv, oracle, shape):
+    """(An odd extent has no momentum -k for its last one, so there the direction of the transform
+    counts: the engine's is the oracle's for psibar and on the mirrored lattice for psi.)"""
+    nx, ny, nz, nt = shape
+    c = clv.ChainParams(nx=nx, ny=ny, nz=nz, nt=nt, eps=0.02, a_x=1.0, G=0.1, Q=0.02, P=0.05, mu=-0.5, DT=0.002, seed=7)
+    p = oracle.Params(nx=nx, ny=ny, nz=nz, nt=nt, ncomp=4, eps=c.eps, a_x=c.a_x, mu=c.mu, P=c.P, Q=c.Q, G=c.G, DT=c.DT)
+    rng = np.random.default_rng(5)
+    with clv.Engine(c, model=clv.MODEL_REF4, precision=clv.PREC_F64) as e:
+        f = 0.5 + 0.2 * (rng.standard_normal(e.shape(0)) + 1j * rng.standard_normal(e.shape(0)))
+        e.set_fields(0, f, np.conj(f))
+        zero = np.zeros(2 * f.size)
+        e.step_with_noise(zero)
+        gp, gc = e.get_fields(0)
+        dt = e.step_info()["dt"][0]
+    mirror = (lambda a: np.ascontiguousarray(np.roll(a[:, :, ::-1], 1, 2))) if nx % 2 else (lambda a: a)
+    psi, psic, want, _, _ = oracle.step(p, mirror(f), mirror(np.conj(f)), noise=zero)
+    assert abs(dt - want) <= 1e-12 * want
+    assert rel_err(gp, mirror(psi)) < 1e-12
+    if nx % 2 == 0:
+        assert rel_err(gc, psic) < 1e-12
+
+
+# kinetic energies of whole slices, summed over the axes at FP64, and axis by axis
+@pytest.mark.parametrize("shape", [(729, 1, 1, 3), (1875, 1, 1, 2), (30, 30, 1, 5), (2, 2, 2, 9), (8, 6, 4, 5), (100, 81, 1, 2)],
+                         ids=str)
+def test_spin1_energies_at_fp64(clv, oracle, shape):
+    c = spin1(clv, nx=shape[0], ny=shape[1], nz=shape[2], nt=shape[3])
+    p = oracle_params(oracle, c)
+    with clv.Engine(c, model=clv.MODEL_SPIN1, precision=clv.PREC_F64) as e:
+        e.init_spin1()
+        e.evaluate()
+        psi, psic = e.get_fields(0)
+        want, got = oracle.spin1_observables(p, psi, psic), e.spin1_samples(0)[0]
+    assert np.max(np.abs(got - want)) < 1e-12 * max(1.0, float(np.max(np.abs(want))))
