@@ -67,70 +67,55 @@ struct DriftConsts {
 // Kbar only, 3 = both (a CTA-uniform choice of the kernels that split the fields);
 // cmask: the components a whose K[a], Kc[a] are computed (bit a; CTA-uniform).
 //
-// The contact term of component a with the multiplied field k and the other field b is,
-// with n_c = k_c b_c, E_a = sum of n_c over c != 3 - a, and k_p k_q the two components beside
-// a and 3 - a,
-//   t_a = E_a k_a + b_{3-a} k_p k_q
-// (the reference's three densities and exchange product, its exchange product of one pair
-// shared by both of the pair's components).  E_a is summed without n_{3-a}: taken out of the
-// sum of all four it would leave that density's rounding in t_a, which is the whole of it
-// where component 3 - a is far above the others.  106 FP64 operations per field (114 when a_x
-// is not 1) instead of 144 in the component-wise form: the reference model's reduce pass is
-// bound by the FP64 pipe (2 operations per clock and SM).  The E_a are the same for both
-// fields' drifts of one (psi(tau), psibar(tau+1)) pair, always formed psi first: the streaming
-// kernel computes them once and carries them (40 operations fewer).
+// The contact term of component a with the multiplied field k and the other field b (three
+// densities and an exchange product in the reference) is, with n_01 = k_0 b_0 + k_1 b_1, n_23 the
+// same of 2 and 3, X = k_0 b_2 + k_1 b_3 and Y = k_2 b_0 + k_3 b_1,
+//   t_0 = n_01 k_0 + X k_2,  t_1 = n_01 k_1 + X k_3,  t_2 = n_23 k_2 + Y k_0,  t_3 = n_23 k_3 + Y k_1.
+// For the other field's drift k and b change places, that is, X and Y do, so one set serves both
+// fields' drifts of a (psi(tau), psibar(tau+1)) pair: the streaming kernel computes it once and
+// carries it.  94 FP64 operations per field (102 when a_x is not 1; 20 fewer when carried) instead
+// of 144 in the component-wise form: the reference model's reduce pass is bound by the FP64
+// pipe (2 operations per clock and SM).  No term is added that cancels again: a form with the
+// sum of all four densities, which takes component 3 - a's out of t_a, carries its rounding
+// where that component is far above the others.
 template <class C2>
-struct Ref4Density {
-    C2 E[4];  // -2G E_a
+struct Ref4Pair {
+    C2 n01, n23, X, Y;  // times -2G
 };
+// which: 1 = what K's components of cmask need, 2 = Kbar's, 3 = both (and all components)
 template <class R, class C2>
-__device__ __forceinline__ Ref4Density<C2> ref4_density(R g2, const C2 *psi, const C2 *bar, int cmask = 0xF) {
-    Ref4Density<C2> d;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {  // components 0 and 1 share n_0 + n_1, 2 and 3 n_2 + n_3
-        if (!((cmask >> (2 * h)) & 3)) continue;
-        const C2 both = xmadd<R>(xmul<R>(psi[2 * h], bar[2 * h]), psi[2 * h + 1], bar[2 * h + 1]);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int a = 2 * h + u, c = (a + 2) & 3;  // 0, 1, 2, 3: the third density is n_2, n_3, n_0, n_1
-            d.E[a] = xscale<R>(-g2, xmadd<R>(both, psi[c], bar[c]));
-        }
-    }
-    return d;
-}
-// -2G k_1 k_2 (components 0 and 3) and -2G k_0 k_3 (1 and 2)
-template <class R, class C2>
-__device__ __forceinline__ void ref4_exchange(R g2, const C2 *k, C2 *D) {
-    D[0] = xscale<R>(-g2, xmul<R>(k[1], k[2]));
-    D[1] = xscale<R>(-g2, xmul<R>(k[0], k[3]));
+__device__ __forceinline__ Ref4Pair<C2> ref4_pair(R g2, const C2 *psi, const C2 *bar, int which = 3, int cmask = 0xF) {
+    Ref4Pair<C2> p;
+    const bool lo = (cmask & 3) != 0, hi = (cmask & 12) != 0;
+    auto two = [&](int a, int b, int c, int d) { return xscale<R>(-g2, xmadd<R>(xmul<R>(psi[a], bar[b]), psi[c], bar[d])); };
+    if (lo) p.n01 = two(0, 0, 1, 1);
+    if (hi) p.n23 = two(2, 2, 3, 3);
+    if (which == 3 || (which == 1 ? lo : hi)) p.X = two(0, 2, 1, 3);
+    if (which == 3 || (which == 1 ? hi : lo)) p.Y = two(2, 0, 3, 1);
+    return p;
 }
 
-// S: ref4_density of (pm, cc).
+// p: ref4_pair of (pm, cc).
 template <class R, class C2>
-__device__ __forceinline__ void drift_ref4_psi(const DriftConsts<R> &k, const Ref4Density<C2> &S, const C2 *pm, const C2 *pc,
-                                               const C2 *cc, const C2 *km, C2 *K, int cmask = 0xF) {
-    C2 D[2];
-    ref4_exchange<R>(k.g2, pm, D);
+__device__ __forceinline__ void drift_ref4_psi(const DriftConsts<R> &k, const Ref4Pair<C2> &p, const C2 *pm, const C2 *pc,
+                                               const C2 *km, C2 *K, int cmask = 0xF) {
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
         if (!((cmask >> a) & 1)) continue;
-        C2 m;
-        m.x = add_rn<R>(k.mu[a], S.E[a].x);
-        m.y = S.E[a].y;
+        C2 m = a < 2 ? p.n01 : p.n23;
+        m.x = add_rn<R>(k.mu[a], m.x);
         C2 in = xmadd<R>(km[a], m, pm[a]);
-        in = xmadd<R>(in, cc[3 - a], D[a == 0 || a == 3 ? 0 : 1]);
+        in = xmadd<R>(in, a < 2 ? p.X : p.Y, pm[a ^ 2]);
         K[a].x = fma_rn<R>(k.eps, in.x, add_rn<R>(pm[a].x, -pc[a].x));
         K[a].y = fma_rn<R>(k.eps, in.y, add_rn<R>(pm[a].y, -pc[a].y));
         if (k.scaled) K[a] = xscale<R>(k.pre, K[a]);
     }
 }
 
-// S: ref4_density of (pc, cp).
+// p: ref4_pair of (pc, cp).
 template <class R, class C2>
-__device__ __forceinline__ void drift_ref4_bar(const DriftConsts<R> &k, const Ref4Density<C2> &S, const C2 *pc, const C2 *pp,
-                                               const C2 *cc, const C2 *cp, const C2 *kp, C2 *Kc, int cmask = 0xF) {
-    C2 D[2];
-    ref4_exchange<R>(k.g2, cp, D);
+__device__ __forceinline__ void drift_ref4_bar(const DriftConsts<R> &k, const Ref4Pair<C2> &p, const C2 *pp, const C2 *cc,
+                                               const C2 *cp, const C2 *kp, C2 *Kc, int cmask = 0xF) {
 #pragma unroll
     for (int a = 0; a < 4; ++a) {
         if (!((cmask >> a) & 1)) continue;
@@ -139,8 +124,8 @@ __device__ __forceinline__ void drift_ref4_bar(const DriftConsts<R> &k, const Re
         C2 in;
         in.x = fma_rn<R>(k.mu[a], pp[a].x, kp[a].x);
         in.y = fma_rn<R>(k.mu[a], pp[a].y, kp[a].y);
-        in = xmadd<R>(in, S.E[a], cp[a]);
-        in = xmadd<R>(in, pc[3 - a], D[a == 0 || a == 3 ? 0 : 1]);
+        in = xmadd<R>(in, a < 2 ? p.n01 : p.n23, cp[a]);
+        in = xmadd<R>(in, a < 2 ? p.Y : p.X, cp[a ^ 2]);
         Kc[a].x = fma_rn<R>(k.eps, in.x, add_rn<R>(cp[a].x, -cc[a].x));
         Kc[a].y = fma_rn<R>(k.eps, in.y, add_rn<R>(cp[a].y, -cc[a].y));
         if (k.scaled) Kc[a] = xscale<R>(k.pre, Kc[a]);
@@ -152,8 +137,8 @@ __device__ __forceinline__ void drift_ref4_vals(const DriftConsts<R> &k, const C
                                                 const C2 *pp, const C2 *cc, const C2 *cp,
                                                 const C2 *km, const C2 *kp, C2 *K, C2 *Kc, int which = 3,
                                                 int cmask = 0xF) {
-    if (which & 1) drift_ref4_psi<R>(k, ref4_density<R>(k.g2, pm, cc, cmask), pm, pc, cc, km, K, cmask);
-    if (which & 2) drift_ref4_bar<R>(k, ref4_density<R>(k.g2, pc, cp, cmask), pc, pp, cc, cp, kp, Kc, cmask);
+    if (which & 1) drift_ref4_psi<R>(k, ref4_pair<R>(k.g2, pm, cc, 1, cmask), pm, pc, km, K, cmask);
+    if (which & 2) drift_ref4_bar<R>(k, ref4_pair<R>(k.g2, pc, cp, 2, cmask), pp, cc, cp, kp, Kc, cmask);
 }
 
 // Spin-1 model.  Of one (bar, ket) pair the contact potential V = c0/2 n^2 + c1/2 (Fz^2 +

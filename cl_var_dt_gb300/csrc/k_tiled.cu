@@ -78,7 +78,7 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
     // carried: psi(tau-1), psibar(tau), psi(tau) and the pair (psibar(tau), psi(tau-1))
     C2 Pp[NC], Qc[NC], Pc[NC];
     Spin1Link<C2> Bm;
-    Ref4Density<C2> Sm;
+    Ref4Pair<C2> Sm;
     // prefetched for the next tau: psi(tau+1), psibar(tau+1), kin(tau-1), kinbar(tau+1)
     C2 nP[NC], nQ[NC], nK[NC], nKc[NC];
     auto load_next = [&](int tau) {
@@ -98,7 +98,7 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
             Pc[c] = gpsi[at(c, tau0)];
         }
         if constexpr (MODEL == CLV_MODEL_SPIN1) Bm = spin1_link<R>(dk, Qc, Pp);
-        else Sm = ref4_density<R>(dk.g2, Pp, Qc);
+        else Sm = ref4_pair<R>(dk.g2, Pp, Qc);
         if (!LEAN) load_next(tau0);
     }
 
@@ -115,9 +115,9 @@ __device__ __forceinline__ void tiled_task(const LaunchTiled &A, const TileTask 
             if (!LEAN && tau + 1 < tau1) load_next(tau + 1);
             C2 K[NC], Kc[NC];
             if constexpr (MODEL == CLV_MODEL_REF4) {
-                drift_ref4_psi<R>(dk, Sm, Pp, Pc, Qc, km, K);
-                Sm = ref4_density<R>(dk.g2, Pc, vcp);
-                drift_ref4_bar<R>(dk, Sm, Pc, vpp, Qc, vcp, kp, Kc);
+                drift_ref4_psi<R>(dk, Sm, Pp, Pc, km, K);
+                Sm = ref4_pair<R>(dk.g2, Pc, vcp);
+                drift_ref4_bar<R>(dk, Sm, vpp, Qc, vcp, kp, Kc);
             } else {
                 spin1_drift_psi<R>(Bm, Pp, Pc, km, K);
                 Bm = spin1_link<R>(dk, vcp, Pc);
