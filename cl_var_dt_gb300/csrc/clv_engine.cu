@@ -960,17 +960,17 @@ clv_engine::AxisGroup &tile_group(const clv_engine *e, std::vector<clv_engine::A
     return groups.back();
 }
 
-// A filter that vanishes at zero frequency: the reference's k^2, kinetic energies.
-bool tile_based(const clv_engine *e, bool energy) {
-    return e->precision == CLV_PREC_F64 && (energy || e->kinetic == CLV_KIN_REF_LINEAR_PX);
+// Lines (slices of a sum) of `sites` taken relative to their first site (kBasedSites).
+bool tile_based(const clv_engine *e, bool energy, int sites) {
+    return e->precision == CLV_PREC_F64 && sites > kBasedSites && (energy || e->kinetic == CLV_KIN_REF_LINEAR_PX);
 }
 
 // tile, twiddles, filters, the rows' shares of summed filters, the groups' scales (FP64:
 // five words each, and the first site where the filter vanishes at zero frequency)
-size_t tile_smem(const clv_engine *e, int elems, int nsum, int rows, int groups, bool energy) {
+size_t tile_smem(const clv_engine *e, int elems, int nsum, int rows, int groups, bool based) {
     return (size_t)(elems + nsum) * e->elem_bytes + (size_t)(nsum + rows) * (e->elem_bytes / 2) +
            (e->precision == CLV_PREC_F64 ? 5 * (size_t)groups * sizeof(unsigned) : 0) +
-           (tile_based(e, energy) ? (size_t)groups * sizeof(double2) : 0) + 16;
+           (based ? (size_t)groups * sizeof(double2) : 0) + 16;
 }
 
 int tile_plan(clv_engine *e, const TileFilterPlan &p) {
@@ -1010,7 +1010,7 @@ int slices_per_tile(const clv_engine *e, const ChainDev &d, int nsum, int rows1,
             const int elems = ns * rows1 * tile_pitch(e->elem_bytes, cols, ns * rows1);
             tiles = 0;
             for (auto &o : e->chains_h) tiles += (double)d.ncomp * ((o.nt + ns - 1) / ns) * (energy ? 1 : 2);
-            return resident(elems, tile_smem(e, elems, nsum, ns * rows1, ns * rows1, energy));
+            return resident(elems, tile_smem(e, elems, nsum, ns * rows1, ns * rows1, tile_based(e, energy, d.V)));
         };
         double tiles = 0;
         if (!f64 && rows1 == 1) {
@@ -1065,14 +1065,14 @@ int add_tile_slices(clv_engine *e, int c, bool energy, std::vector<clv_engine::A
         nsum += d.axis[a].n;
     }
     p.with_const = !energy && e->kinetic == CLV_KIN_EXP;
-    p.based = tile_based(e, energy);
+    p.based = tile_based(e, energy, p.naxes == 1 ? d.axis[p.axis[0]].n : d.V);
     const int ns = slices_per_tile(e, d, nsum, rows1, cols, energy);
     p.pitch = tile_pitch(e->elem_bytes, cols, ns * rows1);
     p.tile_elems = (ns * rows1 * p.pitch + 1) / 2 * 2;
     const int id = tile_plan(e, p);
     auto &g = tile_group(e, groups, 0, p.naxes == 1 ? d.axis[p.axis[0]].n : 0, p.naxes > 1, p.tile_elems,
                          tile_smem(e, p.tile_elems, nsum, ns * rows1,
-                                   p.naxes == 1 ? ns * d.V / d.axis[p.axis[0]].n : ns, energy));
+                                   p.naxes == 1 ? ns * d.V / d.axis[p.axis[0]].n : ns, p.based));
     for (int k = 0; k < d.ncomp; ++k)
         for (int t = 0; t < d.nt; t += ns)
             g.ttasks.push_back({c, id, k * d.nt + t, 0, std::min(ns, d.nt - t) * rows1, cols});
@@ -1092,7 +1092,7 @@ int add_tile_axis(clv_engine *e, int c, int a, bool energy, std::vector<clv_engi
     p.naxes = 1;
     p.axis[0] = a;
     p.with_const = !energy && e->kinetic == CLV_KIN_EXP && a == 0;
-    p.based = tile_based(e, energy);
+    p.based = tile_based(e, energy, n);
     if (ax.inner > 1) {
         int W = target / n;
         W = W >= 16 ? W / 16 * 16 : (W >= 8 ? 8 : 4);
@@ -1102,7 +1102,7 @@ int add_tile_axis(clv_engine *e, int c, int a, bool energy, std::vector<clv_engi
         p.gstride = ax.inner;
         p.tile_elems = (n * p.pitch + 1) / 2 * 2;
         const int id = tile_plan(e, p);
-        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, 0, W, energy));
+        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, 0, W, p.based));
         for (int sl = 0; sl < d.ncomp * d.nt; ++sl)
             for (int hi = 0; hi < lines / ax.inner; ++hi)
                 for (int l = 0; l < ax.inner; l += W)
@@ -1113,7 +1113,7 @@ int add_tile_axis(clv_engine *e, int c, int a, bool energy, std::vector<clv_engi
         p.pitch = tile_pitch(e->elem_bytes, n, W);
         p.tile_elems = (W * p.pitch + 1) / 2 * 2;
         const int id = tile_plan(e, p);
-        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, 0, W, energy));
+        auto &g = tile_group(e, groups, a, n, false, p.tile_elems, tile_smem(e, p.tile_elems, n, 0, W, p.based));
         for (int sl = 0; sl < d.ncomp * d.nt; ++sl)
             for (int l = 0; l < lines; l += W)
                 g.ttasks.push_back({c, id, sl, l * n, std::min(W, lines - l), n});

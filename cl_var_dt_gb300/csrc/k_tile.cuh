@@ -69,12 +69,11 @@ template <> struct TileMath<double> { using E = I2; using W = WCplx; using F = l
 // FP64: the lines' scale.  Line l belongs to group l / lines per group; of each group, raw: the
 // high word of the largest component as the doubles came in; cur, next: of the largest one
 // after the pass before this one and after this one (zero: cleared for the pass after);
-// exps: the shifts so far; base: its first site, for a filter that vanishes at zero frequency (or null).  first: the pass reads doubles; last: it writes them.  eg: the
+// exps: the shifts so far.  first: the pass reads doubles; last: it writes them.  eg: the
 // filters' power of two.
 struct TileScale {
     unsigned *raw, *cur, *next, *zero;
     int *exps;
-    double2 *base;
     FastDiv group;
     int ng, eg;
     bool first, last;
@@ -113,18 +112,12 @@ __device__ __forceinline__ void tile_pass(typename Cx<RR>::T *t, const TileLines
         if constexpr (KIND == TILE_MAX) {
             if constexpr (kInt) {
                 unsigned mx = 0;
-                const int gr = sc.group.div(l);
-                if (sc.base) {
-                    const double2 z0 = sc.base[gr];
-#pragma unroll
-                    for (int m = 0; m < R; ++m) p[m * st] = vsub(p[m * st], z0);
-                }
 #pragma unroll
                 for (int m = 0; m < R; ++m) {
                     const unsigned v = mag_bits(p[m * st]);
                     mx = v > mx ? v : mx;
                 }
-                atomicMax(&sc.raw[gr], mx);
+                atomicMax(&sc.raw[sc.group.div(l)], mx);
             }
         } else {
             E v[R];
@@ -292,7 +285,7 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
     // (FP64, a filter that vanishes at zero frequency: the groups' first sites between them)
     F *f0 = reinterpret_cast<F *>(tw0 + nsum + (kInt && P.based ? (nax == 1 ? total / ch.axis[P.axis[0]].n : total / ch.V) : 0));
     F *fo = f0 + nsum;  // summed filters: the rows' shares of the other axes
-    TileScale sc{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, FastDiv(1), 0, 0, false, false};
+    TileScale sc{nullptr, nullptr, nullptr, nullptr, nullptr, FastDiv(1), 0, 0, false, false};
     {
         // FP64: the filters relative to the power of two at or above their largest value (of
         // each axis, or of the sum)
@@ -347,17 +340,31 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
         sc.zero = sc.next + sc.ng;
         sc.exps = reinterpret_cast<int *>(sc.zero + sc.ng);
         for (int i = threadIdx.x; i < 5 * sc.ng; i += blockDim.x) sc.raw[i] = 0;
-        if (P.based) sc.base = reinterpret_cast<double2 *>(tw0 + nsum);
     }
     copy_async_wait();
     __syncthreads();
     if constexpr (kInt) {
         const AxisDev &ax = ch.axis[P.axis[0]];
         group(0);
-        if (sc.base) {
-            const TileLines g = lines(0);
-            for (int i = threadIdx.x; i < sc.ng; i += blockDim.x)
-                sc.base[i] = tile[nax == 1 ? g.base(i) : i * (ch.V / cols) * PZ];
+        if (P.based) {
+            // element e: line (slice of a sum) hi I + (e mod I), whose first one is hi per + (e mod I)
+            double2 *base = reinterpret_cast<double2 *>(tw0 + nsum);
+            const int I = nax > 1 ? 1 : (P.inner[0] == 0 ? cols : P.inner[0]), per = nax > 1 ? ch.V : ax.n * I;
+            const FastDiv dp(per), dI(I);
+            auto at = [&](int e) {
+                const int r = dc.div(e);
+                return tile + r * PZ + (e - r * cols);
+            };
+            for (int i = threadIdx.x; i < sc.ng; i += blockDim.x) {
+                const int hi = dI.div(i);
+                base[i] = *at(hi * per + (i - hi * I));
+            }
+            __syncthreads();
+            for (int e = threadIdx.x; e < total; e += blockDim.x) {
+                const int hi = dp.div(e), lo = e - hi * per;
+                C2 *p = at(e);
+                *p = vsub(*p, base[hi * I + (lo - dI.div(lo) * I)]);
+            }
             __syncthreads();
         }
         tile_pass_any<R, TILE_MAX>(ax.tfac[0], tile, lines(0), ax.n, ax.n / ax.tfac[0], nullptr, nullptr, nullptr, sc);

@@ -76,8 +76,8 @@ extern "C" int tile_filter(const int *dims, int axes, int ns, int energy, double
     }
     const int cols = dims[last], rows = ns * ch.V / cols;
     P.with_const = !energy;
-    // a filter that vanishes at zero frequency
-    P.based = energy || filt[0] == 0.0;
+    // a filter that vanishes at zero frequency, long lines (large slices of a sum)
+    P.based = (P.naxes == 1 ? ch.axis[P.axis[0]].n : ch.V) > kBasedSites && (energy || filt[0] == 0.0);
     P.pitch = tile_pitch(16, cols, rows);
     P.tile_elems = (rows * P.pitch + 1) / 2 * 2;
     if ((size_t)P.tile_elems * 16 + nsum * 24 + rows * 8 + 36 * (size_t)rows * cols > sizeof smem) return 0;
