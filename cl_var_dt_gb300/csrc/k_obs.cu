@@ -7,9 +7,9 @@
 //   numbers are computed in real space here: with the reference's transform
 //   directions, sum_k psibar~(k) psi~(k) = V sum_x psibar(x) psi(x) (Parseval),
 //   so no FFT and no host round trip is needed.  One thread sums a site over a chunk of
-//   imaginary times (34 FP64 operations each; a time's products are summed among themselves
-//   and added to the running sum once: added one by one, each would be rounded at that sum's
-//   size, 2 to 3 times the error), a second kernel adds the chunks in order.
+//   imaginary times (29 FP64 operations each; the products of two times are summed among
+//   themselves and added to the running sum once: added one by one, each would be rounded at
+//   that sum's size, 2 to 3 times the error), a second kernel adds the chunks in order.
 //   Bound by the FP64 pipe on large lattices (4 components, 128^2 x 128: 405 -> 144 us), by
 //   latency on small ones, where a thread per site left one CTA to walk through imaginary
 //   time (256 x 32: 105 -> 33 us).
@@ -76,31 +76,33 @@ obs_ref_kernel(const ChainDev *__restrict__ chains, const ObsTask *__restrict__ 
     const ObsRange o(ch, task, threadIdx.x);
     double n[4] = {0, 0, 0, 0}, fx = 0, fy = 0, fz = 0;
     if (o.act) {
-#pragma unroll 2
-        for (int tau = o.tau0; tau < o.tau1; ++tau) {
-            const int tp = tau == ch.nt - 1 ? 0 : tau + 1;
-            double2 pc[4], cp[4];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const auto u = psi[oidx(ch, a, tau, o.s)];
-                const auto v = psic[oidx(ch, a, tp, o.s)];
-                pc[a] = make_double2(u.x, u.y);
-                cp[a] = make_double2(v.x, v.y);
-            }
+        for (int tau = o.tau0; tau < o.tau1; tau += 2) {
             double x = 0, y = 0, d[4] = {0, 0, 0, 0};
-            add_re(x, cp[2], pc[0]); add_re(x, cp[0], pc[2]);
-            add_re(x, cp[3], pc[1]); add_re(x, cp[1], pc[3]);
-            // Re(i w) = -Im(w) of t20 - t02 + t31 - t13
-            sub_im(y, cp[2], pc[0]); add_im(y, cp[0], pc[2]);
-            sub_im(y, cp[3], pc[1]); add_im(y, cp[1], pc[3]);
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                add_re(d[a], cp[a], pc[a]);
-                n[a] += d[a];
+            for (int u = 0; u < 2; ++u) {
+                const int t = tau + u, tp = t == ch.nt - 1 ? 0 : t + 1;
+                if (t >= o.tau1) break;
+                double2 pc[4], cp[4];
+#pragma unroll
+                for (int a = 0; a < 4; ++a) {
+                    const auto v = psi[oidx(ch, a, t, o.s)];
+                    const auto w = psic[oidx(ch, a, tp, o.s)];
+                    pc[a] = make_double2(v.x, v.y);
+                    cp[a] = make_double2(w.x, w.y);
+                }
+                add_re(x, cp[2], pc[0]); add_re(x, cp[0], pc[2]);
+                add_re(x, cp[3], pc[1]); add_re(x, cp[1], pc[3]);
+                // Re(i w) = -Im(w) of t20 - t02 + t31 - t13
+                sub_im(y, cp[2], pc[0]); add_im(y, cp[0], pc[2]);
+                sub_im(y, cp[3], pc[1]); add_im(y, cp[1], pc[3]);
+#pragma unroll
+                for (int a = 0; a < 4; ++a) add_re(d[a], cp[a], pc[a]);
             }
             fx += x;
             fy += y;
             fz += (d[0] + d[1]) - (d[2] + d[3]);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) n[a] += d[a];
         }
         const long long nv = (long long)ch.obs_nchunk * ch.V;
         double *F = scratch + ch.obs_scr + task.flat0 + threadIdx.x;
