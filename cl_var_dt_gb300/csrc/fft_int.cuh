@@ -15,8 +15,7 @@
 // * Twiddles carry 62 fraction bits, filters 60 relative to the power of two at or above
 //   their largest value; products are rounded (a bias of half a unit at every frequency
 //   would add up at the line's first site).
-// Lines whose largest component is below 2^-895 count as zero; a line with an infinity or
-// NaN is NaN.  Measured against
+// Values below 2^-1022 count as zero; a line with an infinity or NaN is NaN.  Measured against
 // long-double transforms (2-norm of a step's kinetic term): 1.1 to 2.8 10^-16 over lines and
 // slices of 30 to 1500 sites, also with one site a thousand times the others, where FP64
 // butterflies gave 2.2 to 4.1 10^-16.
@@ -135,17 +134,16 @@ __device__ __forceinline__ I2 ifilter(long long f, I2 z) {
 
 // Conversions, by moving bits (a product and a conversion each way on the FP64 pipe measured
 // 3 to 6 % slower).  emax: biased exponent of the line's largest component, which goes to
-// [2^(kTop - 1), 2^kTop) >> s.
+// [2^(kTop - 1), 2^kTop) >> s.  Values below 2^-1022 count as zero.
 __device__ __forceinline__ long long to_fixed(double x, int emax, int s) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const int r = (emax < 128 ? 8192 : emax) - (int)((hi >> 20) & 0x7ffu) + (64 - kTop) + s;
+    const int ex = (int)((hi >> 20) & 0x7ffu), r = (ex ? emax : 8192) - ex + (64 - kTop) + s;
     const unsigned long long m = ((unsigned long long)(0x80000000u | (hi << 11) | (lo >> 21)) << 32) | (lo << 11);
     const unsigned long long v = r > 63 ? 0ull : m >> r;
     return (hi >> 31) ? -(long long)v : (long long)v;
 }
 // The double nearest v 2^e times the unit of to_fixed at s = 0; NaN for a line with an
-// infinity or NaN.  (Zero below, infinity above the normal range: a line's values keep within
-// 2^63 of its largest, which is above 2^-895.)
+// infinity or NaN.  (Zero below, infinity above the normal range.)
 __device__ __forceinline__ double from_fixed(long long v, int emax, int e) {
     if (emax == 0x7ff) return __longlong_as_double(0x7ff8000000000000ll);
     const unsigned long long a = v < 0 ? 0 - (unsigned long long)v : (unsigned long long)v;
@@ -154,7 +152,7 @@ __device__ __forceinline__ double from_fixed(long long v, int emax, int e) {
     const unsigned long long m = a << l;
     const int be = emax + e - l + (64 - kTop);  // biased exponent
     unsigned long long b = ((unsigned long long)(be - 1) << 52) + (m >> 11) + ((m >> 10) & 1);
-    if (be < 1 || be > 2045) b = be < 1 ? 0 : 0x7ff0000000000000ull;
+    if (be < 1 || be > 2046) b = be < 1 ? 0 : 0x7ff0000000000000ull;
     return __longlong_as_double((long long)(v < 0 ? b | 0x8000000000000000ull : b));
 }
 // 2^e as a double, -1022 <= e <= 1023

@@ -196,3 +196,27 @@ def test_non_finite_lines_are_nan_and_alone(lib, kind, bad, site):
     got = integer(lib, y, f)
     assert np.all(np.isnan(got[2]))
     assert np.array_equal(got[[0, 1, 3, 4]], want[[0, 1, 3, 4]])
+
+
+@pytest.mark.parametrize("n", [60, 300])
+@pytest.mark.parametrize("kind", ["exp", "k2"])
+def test_range_of_the_doubles(lib, n, kind):
+    """A line times a power of two gives its result times it, bit for bit, wherever neither leaves the
+    normal numbers: up to the last binade, and down to 2^-1022."""
+    x, f = field("wide", 6, (n,)), [filter_of(kind, n)]
+    want = integer(lib, x, f)
+    low = lambda *a: min(np.abs(v[v != 0]).min() for z in a for v in (z.real, z.imag))
+    high = lambda *a: max(np.abs(v).max() for z in a for v in (z.real, z.imag))
+    # (the first site is subtracted: a difference of sites is a value, too)
+    top = 1023 - int(np.floor(np.log2(max(2 * high(x), high(want)))))
+    bottom = -1022 - int(np.floor(np.log2(min(low(x), low(want), low(x[:, 1:] - x[:, :1])))))
+    for k in (top, top - 1, 900, -850, -900, bottom + 1, bottom):
+        got = integer(lib, np.ldexp(x.real, k) + 1j * np.ldexp(x.imag, k), f)
+        assert np.array_equal(got.real, np.ldexp(want.real, k)) and np.array_equal(got.imag, np.ldexp(want.imag, k)), k
+
+
+def test_last_binade(lib):
+    """Results of the last binade, [2^1023, 2^1024), are not infinite."""
+    x = np.ldexp(1.75, 1023) * np.ones((3, 60), complex)
+    got = integer(lib, x, [filter_of("exp", 60)])
+    assert np.all(np.abs(got.real / x.real - 1) < 2.0 ** -50) and np.all(np.isfinite(got.imag))
