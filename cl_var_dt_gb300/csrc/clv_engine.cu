@@ -15,6 +15,8 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 #include "clv_internal.cuh"
@@ -118,8 +120,19 @@ struct clv_engine {
         size_t smem;
         std::vector<AxisTask> tasks;
         AxisTask *d = nullptr;
+        int ntasks() const { return (int)(tile ? ttasks.size() : tasks.size()); }
+        int chain_of(int i) const { return tile ? ttasks[i].chain : tasks[i].chain; }
     };
     bool tiled = false;
+    // Chains [c0, c1) whose kinetic terms are held at once (tiled path): all of them, or, where
+    // kinbar has no memory, as many at a time as kin holds twice (plan_windows); groups: first
+    // task and count in every launch group
+    struct Window {
+        int c0, c1;
+        long long off, elems;  // of the chains in a field array
+        std::vector<std::pair<int, int>> groups;
+    };
+    std::vector<Window> windows;
     std::vector<TileFilterPlan> tile_plans_h;
     TileFilterPlan *tile_plans = nullptr;
     std::vector<AxisGroup> axis_groups;
@@ -487,12 +500,20 @@ LaunchFused fused_launch(const clv_engine *e, int from, int mode, bool ext) {
     return L;
 }
 
-LaunchTiled tiled_launch(const clv_engine *e, int from, int mode, bool ext) {
+// kin and kinbar of a window's chains, as if of all: kinbar's own array, or behind kin's elements.
+std::pair<void *, void *> window_kin(const clv_engine *e, const clv_engine::Window &w) {
+    if (e->kinc) return {e->kin, e->kinc};
+    char *k = static_cast<char *>(e->kin) - w.off * e->elem_bytes;
+    return {k, k + w.elems * e->elem_bytes};
+}
+
+LaunchTiled tiled_launch(const clv_engine *e, const clv_engine::Window &w, int from, int mode, bool ext) {
     LaunchTiled L{};
     L.chains = e->chains_d;
     L.state = e->state_d;
-    L.tasks = e->tile_tasks;
-    L.ntasks = (int)e->tile_tasks_h.size();
+    const ChainDev &first = e->chains_h[w.c0], &last = e->chains_h[w.c1 - 1];
+    L.tasks = e->tile_tasks + first.fused_block0;
+    L.ntasks = last.fused_block0 + last.fused_nblocks - first.fused_block0;
     L.model = e->model;
     L.dt_rule = e->dt_rule;
     L.noise = ext ? CLV_NOISE_EXTERNAL : CLV_NOISE_PHILOX;
@@ -500,8 +521,7 @@ LaunchTiled tiled_launch(const clv_engine *e, int from, int mode, bool ext) {
     L.only_rejected = 0;
     L.psi_in = e->fld[from][0];
     L.psic_in = e->fld[from][1];
-    L.kin = e->kin;
-    L.kinc = e->kinc;
+    std::tie(L.kin, L.kinc) = window_kin(e, w);
     L.psi_out = e->fld[from ^ 1][0];
     L.psic_out = e->fld[from ^ 1][1];
     L.partials = e->fused_partials;
@@ -515,23 +535,27 @@ LaunchTiled tiled_launch(const clv_engine *e, int from, int mode, bool ext) {
 
 // The launches of a group list.  Kinetic filter (two fields, src1 not null): the groups of
 // axis 0 read the fields, the others continue in kin/kinbar.  Kinetic energy (src1 null):
-// every axis reads src0, the first writes kin and the others add to it.
+// every axis reads src0, the first writes kin and the others add to it.  w: the chains of a
+// window only.
 template <class R>
 int run_groups(clv_engine *e, const std::vector<clv_engine::AxisGroup> &groups, const void *src0, const void *src1,
-               EventTrail *trail = nullptr) {
+               const clv_engine::Window *w = nullptr, EventTrail *trail = nullptr) {
     const bool energy = src1 == nullptr;
-    for (const auto &g : groups) {
-        const void *s0 = (energy || g.axis == 0) ? src0 : e->kin, *s1 = g.axis == 0 ? src1 : e->kinc;
+    const auto kin = w ? window_kin(e, *w) : std::pair<void *, void *>(e->kin, e->kinc);
+    for (size_t i = 0; i < groups.size(); ++i) {
+        const auto &g = groups[i];
+        const void *s0 = (energy || g.axis == 0) ? src0 : kin.first, *s1 = g.axis == 0 ? src1 : kin.second;
+        const int first = w ? w->groups[i].first : 0, count = w ? w->groups[i].second : g.ntasks();
         if (g.tile) {
             LaunchTileFilter T{};
             T.chains = e->chains_d;
             T.plans = e->tile_plans;
-            T.tasks = g.td;
-            T.ntasks = (int)g.ttasks.size();
+            T.tasks = g.td + first;
+            T.ntasks = count;
             T.src0 = s0;
             T.src1 = s1;
-            T.dst0 = e->kin;
-            T.dst1 = e->kinc;
+            T.dst0 = kin.first;
+            T.dst1 = kin.second;
             T.nfields = energy ? 1 : 2;
             T.filter = energy;
             T.accumulate = energy && g.axis > 0;
@@ -541,8 +565,8 @@ int run_groups(clv_engine *e, const std::vector<clv_engine::AxisGroup> &groups, 
         } else {
             LaunchAxis A{};
             A.chains = e->chains_d;
-            A.tasks = g.d;
-            A.ntasks = (int)g.tasks.size();
+            A.tasks = g.d + first;
+            A.ntasks = count;
             A.axis = g.axis;
             A.n = g.n;
             A.W = g.W;
@@ -550,8 +574,8 @@ int run_groups(clv_engine *e, const std::vector<clv_engine::AxisGroup> &groups, 
             A.with_const = g.with_const;
             A.src0 = s0;
             A.src1 = s1;
-            A.dst0 = e->kin;
-            A.dst1 = e->kinc;
+            A.dst0 = kin.first;
+            A.dst1 = kin.second;
             A.smem_bytes = g.smem;
             A.nfields = energy ? 1 : 2;
             A.filter = energy;
@@ -566,25 +590,28 @@ int run_groups(clv_engine *e, const std::vector<clv_engine::AxisGroup> &groups, 
     return CLV_OK;
 }
 
-// Tiled step: kinetic filter axis by axis into kin/kinbar, then the streaming
+// Tiled step of a window's chains: kinetic filter axis by axis into kin/kinbar, then the streaming
 // drift/noise/update kernel (speculative dt with redo, or reduce then apply).
 template <class R>
-int enqueue_tiled(clv_engine *e, bool external_noise, EventTrail *trail, int from) {
-    if (int rc = run_groups<R>(e, e->axis_groups, e->fld[from][0], e->fld[from][1], trail)) return rc;
+int enqueue_window(clv_engine *e, const clv_engine::Window &w, bool external_noise, EventTrail *trail, int from) {
+    if (int rc = run_groups<R>(e, e->axis_groups, e->fld[from][0], e->fld[from][1], &w, trail)) return rc;
     if (e->speculate && e->dt_rule == CLV_DT_K_OVER_MAX) {
-        CK(launch_tiled<R>(tiled_launch(e, from, FUSED_SPEC, external_noise), e->stream));
+        CK(launch_tiled<R>(tiled_launch(e, w, from, FUSED_SPEC, external_noise), e->stream));
         if (trail) CK(trail->mark(e->stream));
-        LaunchTiled L = tiled_launch(e, from, FUSED_APPLY, external_noise);
+        LaunchTiled L = tiled_launch(e, w, from, FUSED_APPLY, external_noise);
         L.only_rejected = 1;
         CK(launch_tiled<R>(L, e->stream));
     } else {
-        const LaunchTiled reduce = tiled_launch(e, from, FUSED_MAXONLY, external_noise);
+        const LaunchTiled reduce = tiled_launch(e, w, from, FUSED_MAXONLY, external_noise);
         CK(launch_tiled<R>(reduce, e->stream));
         if (trail) CK(trail->mark(e->stream));
         if (e->store_drift) {
             // the stored drift applied by the site-parallel update, which draws its noise
             // while the reduce pass runs (programmatic launch) unless that pass drew it
+            const ChainDev &first = e->chains_h[w.c0], &last = e->chains_h[w.c1 - 1];
             LaunchSites L = e->sites();
+            L.tasks += first.site_block0;
+            L.ntasks = last.site_block0 + last.site_nblocks - first.site_block0;
             L.psi = e->fld[from][0];
             L.psic = e->fld[from][1];
             L.psi_w = e->fld[from ^ 1][0];
@@ -594,10 +621,17 @@ int enqueue_tiled(clv_engine *e, bool external_noise, EventTrail *trail, int fro
             L.pdl = !std::getenv("CLV_NO_PDL");
             CK(launch_update<R>(L, e->stream));
         } else {
-            CK(launch_tiled<R>(tiled_launch(e, from, FUSED_APPLY, external_noise), e->stream));
+            CK(launch_tiled<R>(tiled_launch(e, w, from, FUSED_APPLY, external_noise), e->stream));
         }
     }
     if (trail) CK(trail->mark(e->stream));
+    return CLV_OK;
+}
+
+template <class R>
+int enqueue_tiled(clv_engine *e, bool external_noise, EventTrail *trail, int from) {
+    for (const auto &w : e->windows)
+        if (int rc = enqueue_window<R>(e, w, external_noise, trail, from)) return rc;
     return CLV_OK;
 }
 
@@ -706,7 +740,7 @@ int enqueue_step(clv_engine *e, bool external_noise, EventTrail *trail, int from
     // lines beyond the tiled path's: the tile filter, or the line filter where the tile path
     // is switched off (CLV_TILED=0)
     int rc = e->axis_groups.empty() ? run_kinetic<R>(e, e->fld[from][0], e->fld[from][1], e->kin, e->kinc, 0, 2, trail)
-                                    : run_groups<R>(e, e->axis_groups, e->fld[from][0], e->fld[from][1], trail);
+                                    : run_groups<R>(e, e->axis_groups, e->fld[from][0], e->fld[from][1], nullptr, trail);
     if (rc) return rc;
     LaunchSites L = e->sites();
     L.psi = e->fld[from][0];
@@ -1301,6 +1335,56 @@ int plan_tiled(clv_engine *e) {
     return CLV_OK;
 }
 
+// The windows of the tiled path: one, or, without an array for kinbar, runs of chains whose
+// elements kin holds twice.  False when a chain alone is too large for that.
+bool plan_windows(clv_engine *e, bool split) {
+    e->windows.clear();
+    const int nch = (int)e->chains_h.size();
+    const long long most = split ? e->total_elems / 2 : e->total_elems;
+    for (int c = 0; c < nch;) {
+        clv_engine::Window w{};
+        w.c0 = c;
+        w.off = e->chains_h[c].off;
+        for (; c < nch; ++c) {
+            const ChainDev &d = e->chains_h[c];
+            const long long elems = d.off + (long long)d.ncomp * d.nt * d.V - w.off;
+            if (elems > most) break;
+            w.elems = elems;
+        }
+        if (c == w.c0) return false;
+        w.c1 = c;
+        for (const auto &g : e->axis_groups) {  // (tasks are in the order of chains)
+            int first = 0;
+            while (first < g.ntasks() && g.chain_of(first) < w.c0) ++first;
+            int end = first;
+            while (end < g.ntasks() && g.chain_of(end) < w.c1) ++end;
+            w.groups.push_back({first, end - first});
+        }
+        e->windows.push_back(std::move(w));
+    }
+    return true;
+}
+
+// Memory for a call of an engine under way; the tiled path gives kinbar's back for it where there
+// is no other.
+cudaError_t malloc_beside(clv_engine *e, void **p, size_t bytes) {
+    const char *test = std::getenv("CLV_TEST_NO_KINBAR");
+    cudaError_t ce = test && test[0] == '2' && e->kinc ? cudaErrorMemoryAllocation : cudaMalloc(p, bytes);
+    if (ce != cudaErrorMemoryAllocation || !e->tiled || !e->kinc) return ce;
+    cudaGetLastError();
+    if (!plan_windows(e, true)) {
+        plan_windows(e, false);
+        return ce;
+    }
+    e->drop_graphs();
+    if ((ce = cudaStreamSynchronize(e->stream)) != cudaSuccess) return ce;
+    e->allocs.erase(std::find(e->allocs.begin(), e->allocs.end(), e->kinc));
+    e->dev_bytes -= e->total_elems * e->elem_bytes;
+    cudaFree(e->kinc);
+    e->kinc = nullptr;
+    return cudaMalloc(p, bytes);
+}
+
 int check_chain(clv_engine *e, int chain) {
     if (!e) return fail(CLV_ERR_ARG, "null engine");
     if (chain < 0 || chain >= (int)e->params.size()) return fail(CLV_ERR_ARG, "chain out of range");
@@ -1416,7 +1500,7 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
     const int nch = cfg->nchains;
     if ((rc = e->alloc(&e->fld[0][0], fb)) || (rc = e->alloc(&e->fld[0][1], fb)) ||
         (rc = e->alloc(&e->fld[1][0], fb)) || (rc = e->alloc(&e->fld[1][1], fb)) ||
-        (rc = e->alloc(&e->kin, fb)) || (rc = e->alloc(&e->kinc, fb_scratch)) ||
+        (rc = e->alloc(&e->kin, fb)) || (!e->tiled && (rc = e->alloc(&e->kinc, fb_scratch))) ||
         (rc = e->alloc(&e->drift, fb_drift)) || (rc = e->alloc(&e->driftc, fb_drift)) ||
         (rc = e->alloc(&e->fused_tasks, (e->fused ? nparts : 1) * sizeof(FusedTask))) ||
         (rc = e->alloc(&e->fused_partials, (e->loop_per_sm > 0 ? 2 : 1) * nparts * sizeof(double2))) ||
@@ -1455,6 +1539,15 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
                              : e->alloc(&g.d, g.tasks.size() * sizeof(AxisTask))))
                 return bail(rc);
     if ((rc = e->alloc(&e->tile_plans, e->tile_plans_h.size() * sizeof(TileFilterPlan)))) return bail(rc);
+    if (e->tiled) {
+        // A batch that leaves no memory for kinbar steps its chains in windows, with the same bits:
+        // the memory of a step that keeps no kinetic terms but the observables' (5 field arrays
+        // for spin-1, 7 for the reference model at FP64).
+        const char *test = std::getenv("CLV_TEST_NO_KINBAR");  // as if its allocation failed: 1 here, 2 later
+        rc = test && test[0] == '1' ? fail(CLV_ERR_NOMEM, "kinbar withheld by a test") : e->alloc(&e->kinc, fb);
+        cudaGetLastError();  // (a refused allocation is no error of a later launch)
+        if (!plan_windows(e, rc != CLV_OK)) return bail(rc);
+    }
     auto up = [&](void *d, const void *h, size_t b) {
         return cudaMemcpy(d, h, b, cudaMemcpyHostToDevice);
     };
@@ -1553,7 +1646,7 @@ static int copy_fields(clv_engine *e, int c0, int c1, const void *const src_in[2
             e->stage_all = nullptr;
             e->stage_all_elems = 0;
             void *q = nullptr;
-            CK(cudaMalloc(&q, n * sizeof(double2)));
+            CK(malloc_beside(e, &q, n * sizeof(double2)));
             e->stage_all = (double2 *)q;
             e->stage_all_elems = n;
         }
@@ -1737,11 +1830,12 @@ int clv_step_timed(clv_engine *e, float *phase_ms, int capacity, int *nphases) {
         e->cur ^= 1;
     }
     CK(cudaStreamSynchronize(e->stream));
-    const int n = (int)trail.ev.size() - 1;
-    for (int i = 0; i < n && i < capacity; ++i) {
+    // (the windows of a tiled step go through the same phases one after the other)
+    const int all = (int)trail.ev.size() - 1, n = e->tiled ? all / (int)e->windows.size() : all;
+    for (int i = 0; i < all; ++i) {
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, trail.ev[i], trail.ev[i + 1]));
-        if (phase_ms) phase_ms[i] = ms;
+        if (phase_ms && i % n < capacity) phase_ms[i % n] = i < n ? ms : phase_ms[i % n] + ms;
     }
     if (nphases) *nphases = n;
     return CLV_OK;
@@ -1754,7 +1848,7 @@ int clv_step_with_noise(clv_engine *e, const double *noise, int where) {
     CK(cudaSetDevice(e->device));
     if (!e->noise_d) {
         void *p = nullptr;
-        CK(cudaMalloc(&p, e->noise_total * sizeof(double)));
+        CK(malloc_beside(e, &p, e->noise_total * sizeof(double)));
         e->noise_d = (double *)p;
     }
     CK(cudaMemcpyAsync(e->noise_d, noise, e->noise_total * sizeof(double), kind_of(where, true),
@@ -1997,7 +2091,7 @@ int clv_autotune(clv_engine *e, int trial_steps, char *report, int capacity) {
         };
         cudaError_t ce = cudaSuccess;
         for (int f = 0; f < 2 && ce == cudaSuccess; ++f) {
-            ce = cudaMalloc(&save[f], fb);
+            ce = malloc_beside(e, &save[f], fb);
             if (ce == cudaSuccess)
                 ce = cudaMemcpyAsync(save[f], e->fld[cur0][f], fb, cudaMemcpyDeviceToDevice, e->stream);
         }
