@@ -204,6 +204,14 @@ struct clv_engine {
         return CLV_OK;
     }
 
+    template <class T>
+    void release(T **p, size_t bytes) {
+        allocs.erase(std::find(allocs.begin(), allocs.end(), *p));
+        dev_bytes -= bytes;
+        cudaFree(*p);
+        *p = nullptr;
+    }
+
     LaunchObs obs() const {
         LaunchObs L{};
         L.chains = chains_d;
@@ -1351,7 +1359,10 @@ bool plan_windows(clv_engine *e, bool split) {
             if (elems > most) break;
             w.elems = elems;
         }
-        if (c == w.c0) return false;
+        if (c == w.c0) {
+            e->windows.clear();
+            return false;
+        }
         w.c1 = c;
         for (const auto &g : e->axis_groups) {  // (tasks are in the order of chains)
             int first = 0;
@@ -1378,10 +1389,7 @@ cudaError_t malloc_beside(clv_engine *e, void **p, size_t bytes) {
     }
     e->drop_graphs();
     if ((ce = cudaStreamSynchronize(e->stream)) != cudaSuccess) return ce;
-    e->allocs.erase(std::find(e->allocs.begin(), e->allocs.end(), e->kinc));
-    e->dev_bytes -= e->total_elems * e->elem_bytes;
-    cudaFree(e->kinc);
-    e->kinc = nullptr;
+    e->release(&e->kinc, (size_t)e->total_elems * e->elem_bytes);
     return cudaMalloc(p, bytes);
 }
 
@@ -1542,11 +1550,19 @@ int clv_create(const clv_config *cfg, clv_engine **out) {
     if (e->tiled) {
         // A batch that leaves no memory for kinbar steps its chains in windows, with the same bits:
         // the memory of a step that keeps no kinetic terms but the observables' (5 field arrays
-        // for spin-1, 7 for the reference model at FP64).
+        // for spin-1, 7 for the reference model at FP64).  Where one chain holds more than half of
+        // the elements the stored drift gives its two arrays, also with the same bits.
         const char *test = std::getenv("CLV_TEST_NO_KINBAR");  // as if its allocation failed: 1 here, 2 later
         rc = test && test[0] == '1' ? fail(CLV_ERR_NOMEM, "kinbar withheld by a test") : e->alloc(&e->kinc, fb);
         cudaGetLastError();  // (a refused allocation is no error of a later launch)
-        if (!plan_windows(e, rc != CLV_OK)) return bail(rc);
+        if (rc && !plan_windows(e, true) && e->store_drift) {
+            e->release(&e->drift, fb);
+            e->release(&e->driftc, fb);
+            e->store_drift = e->draw_in_reduce = false;
+            rc = e->alloc(&e->kinc, fb);
+        }
+        if (!rc) plan_windows(e, false);
+        else if (e->windows.empty()) return bail(rc);
     }
     auto up = [&](void *d, const void *h, size_t b) {
         return cudaMemcpy(d, h, b, cudaMemcpyHostToDevice);

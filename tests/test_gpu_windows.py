@@ -87,7 +87,7 @@ def test_kinbar_given_back_for_the_autotuner(clv, monkeypatch):
 
 
 def test_a_chain_of_more_than_half_needs_its_kinbar(clv, monkeypatch):
-    """Refused as before, with the allocation's error, and the next engine works."""
+    """Refused with the allocation's error, and the next engine works."""
     c = batch(clv, "spin1")[:1]
     monkeypatch.setenv("CLV_TEST_NO_KINBAR", "1")
     with pytest.raises(Exception, match="kinbar"):
@@ -96,3 +96,14 @@ def test_a_chain_of_more_than_half_needs_its_kinbar(clv, monkeypatch):
     with clv.Engine(c, model=clv.MODEL_SPIN1) as e:
         e.init_spin1()
         e.step(2)
+
+
+# (the second: large enough for the normals to be drawn in the reduce pass, on up to 152 SMs)
+@pytest.mark.parametrize("shape", [dict(nx=60, nt=25), dict(nx=128, ny=128, nt=39)], ids=["small", "drawn"])
+def test_a_chain_of_more_than_half_gives_its_stored_drift(clv, monkeypatch, shape):
+    c = [clv.ChainParams(**shape, eps=0.02, G=0.1, Q=0.02, P=0.05, mu=-0.5, DT=0.002, seed=3)]
+    a = run(clv, c, "ref4", "f64")
+    monkeypatch.setenv("CLV_TEST_NO_KINBAR", "1")
+    b = run(clv, c, "ref4", "f64")
+    same(a, b)
+    assert a["bytes"] - b["bytes"] > 1.9 * a["elems"]    # (16 bytes stay in the arrays' place or none)
