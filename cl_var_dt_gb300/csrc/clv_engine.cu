@@ -870,30 +870,23 @@ bool tiled_off() {
     return env && env[0] == '0';
 }
 
-// 1D batches of ln-site lines that the tiled path steps faster than the fused one (us a step,
-// fused / tiled; chains x sites x imaginary times).  The fused step saves the kinetic term's way
-// through HBM, but filters with a warp per line; the tile filter fills its warps whatever
-// the lines, and the tiled step overlaps noise and drift over more of them.
-//   * FP32 under the reference's rule, whose second pass filters once more (the step loop's
-//     small problems aside): 3 x 64 x 32 27 / 23, 8 x 256 x 64 47 / 38, 120 x 128 x 100 275 / 177.
-//   * FP64 from three blocks of sites an SM on, lines of 64 and, under the reference's rule,
-//     of 256: reference model 40 x 64 x 64 212 / 158, 120 x 256 x 100 2669 / 2172; spin-1 40 x 64
-//     x 64 159 / 122.  Others stay: reference model 120 x 128 x 100 1056 / 1113; 8 x 64 x 64
-//     64 / 64; spin-1 40 x 128 x 64 201 / 219, 40 x 256 x 64 328 / 384.
-//   * FP32, K/max rule: lines of 64 from 16 blocks an SM on (120 x 64 x 100 84 / 69; 40 x 64 x 64
-//     28 / 28; 120 x 128 x 100 104 / 113).
 bool tiled_is_faster(const clv_engine *e, int ln) {
-    const bool ref_rule = e->dt_rule == CLV_DT_REF_MEANMAX;
-    // its two more field-sized arrays (and the stored drift's) have to fit
-    size_t room = 0, all = 0;
+    LineBatch b{};
+    b.fp64 = e->precision == CLV_PREC_F64;
+    b.ref_rule = e->dt_rule == CLV_DT_REF_MEANMAX;
+    b.ln = ln;
+    b.sites = e->all_sites;
+    for (auto &d : e->chains_h) {
+        b.largest = std::max(b.largest, (long long)d.V * d.nt);
+        b.slices += d.nt;
+    }
+    b.field_bytes = e->all_sites * e->ncomp * e->elem_bytes;
+    b.num_sms = e->num_sms;
+    b.loop_ctas = e->loop_per_sm * e->num_sms;
+    size_t room = 0, all = 0;  // (the device's memory; what is free of it decides nothing)
     if (cudaMemGetInfo(&room, &all) != cudaSuccess) return false;
-    if ((double)e->all_sites * e->ncomp * e->elem_bytes * 8 > 0.95 * (double)room) return false;
-    const long long per_sm = e->all_sites / (256LL * e->num_sms);
-    if (e->precision == CLV_PREC_F64) return per_sm >= 3 && (ln == 64 || (ln == 256 && ref_rule));
-    if (!ref_rule) return ln == 64 && per_sm >= 16;
-    long long slices = 0;
-    for (auto &d : e->chains_h) slices += d.nt;
-    return 2 * slices > (long long)e->loop_per_sm * e->num_sms;
+    b.device_bytes = (long long)all;
+    return lines_on_the_tiled_path(b);
 }
 
 int plan_fused(clv_engine *e) {

@@ -110,4 +110,39 @@ inline int tile_pitch(int elem_bytes, int n, int lines) {
 // (128 sites: 0.2), from 270 to 2048 up to 2.2 times it, and 0.5 relative to the first site.
 constexpr int kBasedSites = 256;
 
+// A batch of 1D lines that both the fused and the tiled path can step.
+struct LineBatch {
+    bool fp64, ref_rule;
+    int ln;                        // sites of a line: 64, 128, 256
+    long long sites, largest;      // of all chains and imaginary times, of the largest chain
+    long long slices;              // imaginary times of all chains
+    long long field_bytes, device_bytes;
+    int num_sms, loop_ctas;        // the step loop's resident CTAs
+};
+
+// 1D batches of ln-site lines that the tiled path steps faster than the fused one (us a step,
+// fused / tiled; chains x sites x imaginary times).  The fused step saves the kinetic term's way
+// through HBM, but filters with a warp per line; the tile filter fills its warps whatever
+// the lines, and the tiled step overlaps noise and drift over more of them.
+//   * FP32 under the reference's rule, whose second pass filters once more (the step loop's
+//     small problems aside): 3 x 64 x 32 27 / 23, 8 x 256 x 64 47 / 38, 120 x 128 x 100 275 / 177.
+//   * FP64 from three blocks of sites an SM on, lines of 64 and, under the reference's rule,
+//     of 256: reference model 40 x 64 x 64 212 / 158, 120 x 256 x 100 2669 / 2172; spin-1 40 x 64
+//     x 64 159 / 122.  Others stay: reference model 120 x 128 x 100 1056 / 1113; 8 x 64 x 64
+//     64 / 64; spin-1 40 x 128 x 64 201 / 219, 40 x 256 x 64 328 / 384.
+//   * FP32, K/max rule: lines of 64 from 16 blocks an SM on (120 x 64 x 100 84 / 69; 40 x 64 x 64
+//     28 / 28; 120 x 128 x 100 104 / 113).
+// The two paths round differently, so sizes alone decide, not the memory that other engines leave:
+// that would change a chain's trajectory.  The tiled path steps in windows where kinbar does not
+// fit, which takes chains of at most half of the sites; batches of one large chain, a field of
+// over a 64th of the device's memory, stay fused, except for the reference model at FP64, which
+// can do without its stored drift.
+inline bool lines_on_the_tiled_path(const LineBatch &b) {
+    if (2 * b.largest > b.sites && !(b.ref_rule && b.fp64) && b.field_bytes > b.device_bytes / 64) return false;
+    const long long per_sm = b.sites / (256LL * b.num_sms);
+    if (b.fp64) return per_sm >= 3 && (b.ln == 64 || (b.ln == 256 && b.ref_rule));
+    if (!b.ref_rule) return b.ln == 64 && per_sm >= 16;
+    return 2 * b.slices > b.loop_ctas;
+}
+
 }  // namespace clv

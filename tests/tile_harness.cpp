@@ -95,6 +95,19 @@ extern "C" int tile_filter(const int *dims, int axes, int ns, int energy, double
     return 1;
 }
 
+extern "C" int line_path(int fp64, int ref_rule, int ln, int ncomp, int chains, int nt, long long device_bytes) {
+    LineBatch b{};
+    b.fp64 = fp64; b.ref_rule = ref_rule; b.ln = ln;
+    b.largest = (long long)ln * nt;
+    b.sites = chains * b.largest;
+    b.slices = (long long)chains * nt;
+    b.field_bytes = b.sites * ncomp * (fp64 ? 16 : 8);
+    b.device_bytes = device_bytes;
+    b.num_sms = 152;
+    b.loop_ctas = 152;
+    return lines_on_the_tiled_path(b);
+}
+
 // One line of n sites by FP64 butterflies of 8, 4, 2, 3 and 5 (Stockham passes), filter f
 // in the order of frequencies.
 template <int R, int S>
