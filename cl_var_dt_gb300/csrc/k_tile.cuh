@@ -455,16 +455,21 @@ __global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5
     }
 }
 
+// Allows the kernel the device's whole opt-in shared memory: it serves every shape, and a limit
+// raised by one engine could be lowered again by another that is created beside it.
 template <class R>
 cudaError_t setup_tile_filter(size_t smem_bytes, int threads, int *ctas_per_sm) {
     const void *fn = threads == 128 ? (const void *)tile_filter_kernel<R, 128> : (const void *)tile_filter_kernel<R, 256>;
-    cudaFuncAttributes fa;
-    cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaFuncAttributes fa{};
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, fn);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
     if (e != cudaSuccess) return e;
-    if ((int)smem_bytes > fa.maxDynamicSharedSizeBytes) {  // serves every shape: keep the largest request
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-        if (e != cudaSuccess) return e;
-    }
+    *ctas_per_sm = 0;
+    if (smem_bytes + fa.sharedSizeBytes > (size_t)optin) return cudaSuccess;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(ctas_per_sm, fn, threads, smem_bytes);
 }
 

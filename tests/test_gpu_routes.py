@@ -220,3 +220,27 @@ def test_spin1_sample_does_not_depend_on_the_batch(clv):
             got.append(e.spin1_samples(0)[0])
     for g in got[1:]:
         assert np.max(np.abs(g - got[0])) < 1e-12 * np.max(np.abs(got[0])), (got[0], g)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_engines_of_several_threads(clv, prec):
+    """Engines whose tiles differ in size, created, stepped and closed by four threads at once."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    shapes = [dict(nx=60, nt=6), dict(nx=48, ny=20, nt=3), dict(nx=600, nt=3), dict(nx=100, ny=81, nt=2)]
+
+    def work(k):
+        out = []
+        for r in range(12):
+            c = spin1(clv, seed=7 + k, **shapes[(k + r * (k % 2)) % 4])
+            with clv.Engine(c, model=clv.MODEL_SPIN1, precision=prec_of(clv, prec)) as e:
+                e.init_spin1()
+                e.step(2)
+                out.append(e.get_fields(0)[0])
+        return out
+
+    want = [work(k) for k in range(4)]
+    with ThreadPoolExecutor(4) as pool:
+        got = list(pool.map(work, range(4)))
+    for a, b in zip(want, got):
+        assert all(np.array_equal(x, y) for x, y in zip(a, b))
