@@ -1033,7 +1033,7 @@ int slices_per_tile(const clv_engine *e, const ChainDev &d, int nsum, int rows1,
     const int most = f64 ? tile_slice_max<double>() : tile_slice_max<float>();
     const int wide = f64 ? tile_wide<double>() : tile_wide<float>();
     auto resident = [&](int elems, size_t smem) {
-        const int by_regs = f64 ? (elems >= wide ? 2 : 5) : (elems >= wide ? 3 : 6);
+        const int th = elems >= wide ? 256 : 128, by_regs = f64 ? tile_min_ctas<double>(th) : tile_min_ctas<float>(th);
         return std::min(by_regs, std::max(1, (int)((size_t)(228 << 10) / (smem + 1024))));
     };
     const double total = (double)e->all_sites * d.ncomp * (energy ? 1 : 2);  // elements
@@ -1228,7 +1228,7 @@ int build_axis_groups(clv_engine *e, bool energy, std::vector<clv_engine::AxisGr
                 if (int rc = add_tile_axis(e, c, a, energy, groups)) return rc;
                 continue;
             }
-            const int W = axis_tile_lines<float>(n);
+            const int W = axis_tile_lines(n);
             int gi = -1;
             for (int g = 0; g < (int)groups.size(); ++g)
                 if (!groups[g].plane && !groups[g].tile && groups[g].axis == a && groups[g].n == n) gi = g;

@@ -276,6 +276,10 @@ template <class R> __host__ __device__ constexpr int tile_radix_max() { return s
 template <class R> __host__ __device__ constexpr int tile_target() { return sizeof(R) == 4 ? 4096 : 2048; }
 template <class R> __host__ __device__ constexpr int tile_slice_max() { return sizeof(R) == 4 ? 12288 : 6144; }
 template <class R> __host__ __device__ constexpr int tile_wide() { return sizeof(R) == 4 ? 6144 : 3072; }
+// CTAs an SM that its registers are budgeted for, by threads.
+template <class R> __host__ __device__ constexpr int tile_min_ctas(int threads) {
+    return sizeof(R) == 4 ? 768 / threads : (threads == 128 ? 5 : 2);
+}
 template <class R> cudaError_t launch_tile_filter(const LaunchTileFilter &L, cudaStream_t s);
 template <class R> cudaError_t setup_tile_filter(size_t smem_bytes, int threads, int *ctas_per_sm);
 
@@ -335,16 +339,15 @@ template <class R> cudaError_t launch_plane_filter(const LaunchAxis &L, cudaStre
 template <class R> cudaError_t setup_plane_filter(int n, int energy, size_t smem_bytes, int *ctas_per_sm);
 template <class R> cudaError_t launch_tiled(const LaunchTiled &L, cudaStream_t s);
 template <class R> cudaError_t setup_tiled(int model, int lean, int draw, int *ctas_per_sm);
-// Axis filter geometry, lines of 32, 64, 96, 128, 256 and 512 sites.  Lines per tile
-// (FP32; half at FP64): 64 for 32, 32 for 64, 16 for 96 and 128, 8 for 256 and 512, so that a
+// Axis filter geometry, FP32 lines of 32, 64, 96, 128, 256 and 512 sites.  Lines per tile:
+// 64 for 32, 32 for 64, 16 for 96 and 128, 8 for 256 and 512, so that a
 // radix-8 pass has about a butterfly for each of the 256 threads and a tile with
 // its scratch fits in a quarter of an SM's shared memory.
 __host__ __device__ constexpr bool axis_compile_time_plan(int n) {
     return n == 32 || n == 64 || n == 96 || n == 128 || n == 256 || n == 512;
 }
-template <class R>
 __host__ __device__ constexpr int axis_tile_lines(int n) {
-    return (n == 32 ? 64 : (n == 64 ? 32 : ((n == 96 || n == 128) ? 16 : 8))) / (sizeof(R) == 4 ? 1 : 2);
+    return n == 32 ? 64 : (n == 64 ? 32 : ((n == 96 || n == 128) ? 16 : 8));
 }
 // shared-memory bytes of the twiddle and filter tables for lines of n
 __host__ __device__ constexpr size_t axis_tab_bytes(int n, size_t esz) { return ((size_t)n * (esz + esz / 2) + 15) / 16 * 16; }

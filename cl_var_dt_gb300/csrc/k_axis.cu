@@ -151,7 +151,7 @@ struct AxisPlan {
 template <class R, int N>
 __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
     using C2 = typename Cx<R>::T;
-    constexpr int W = axis_tile_lines<R>(N);
+    constexpr int W = axis_tile_lines(N);
     constexpr int PER = W * N / 256;  // elements per thread of a full tile
     extern __shared__ __align__(128) unsigned char smem[];
     const AxisTask task = A.tasks[A.nfields == 2 ? blockIdx.x >> 1 : blockIdx.x];
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(256) axis_filter_kernel(const LaunchAxis A) {
 // memory, so a warp's loads and stores of one index are 32 consecutive elements), runs the
 // 64-point transform, the filter and the inverse, and writes the line back: no shared
 // memory and no barriers, 64 loads in flight per thread.
-static_assert(axis_tile_lines<float>(64) == 32, "one lane per line of a tile");
+static_assert(axis_tile_lines(64) == 32, "one lane per line of a tile");
 template <int N>
 __global__ void __launch_bounds__(64, 6) axis_line_kernel(const LaunchAxis A) {
     using C2 = float2;

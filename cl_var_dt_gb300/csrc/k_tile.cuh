@@ -249,7 +249,7 @@ inline void copy_async_wait() {}
 
 // TH threads: 128, or 256 for the large slices.
 template <class R, int TH>
-__global__ void __launch_bounds__(TH, sizeof(R) == 4 ? 768 / TH : (TH == 128 ? 5 : 2)) tile_filter_kernel(const LaunchTileFilter A) {
+__global__ void __launch_bounds__(TH, tile_min_ctas<R>(TH)) tile_filter_kernel(const LaunchTileFilter A) {
     using C2 = typename Cx<R>::T;
     using W = typename TileMath<R>::W;
     using F = typename TileMath<R>::F;

@@ -244,3 +244,16 @@ def test_engines_of_several_threads(clv, prec):
         got = list(pool.map(work, range(4)))
     for a, b in zip(want, got):
         assert all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+def test_the_sizes_above_take_the_forms_they_are_for():
+    """plan() names the path, not the form: the sizes of this file against the thresholds of
+    clv_engine.cu in blocks of 256 sites an SM (16: normals in the reduce pass, 8: two CTAs an SM,
+    3: FP64 lines on the tiled path; more chunks of 33 times than SMs for the fused form)."""
+    sms = pytest.importorskip("torch").cuda.get_device_properties(0).multi_processor_count
+    per_sm = lambda sites: sites // 256 / sms
+    assert per_sm(128 * 128 * 39) >= 16 and per_sm(50 * 30 * 200 + 27 * 25 * 300 + 128 * 64 * 20) >= 16
+    assert per_sm(20 * 27 * 127) < 8 and per_sm(20 * 27 * 127 + 128 * 128 * 48) >= 16
+    assert 8 <= per_sm(27 * 20 * sum(64 + i for i in range(10)))
+    assert 5 * 33 > sms > 3 * 33
+    assert per_sm(30 * 64 * 65) >= 3 and per_sm(8 * 256 * 64) >= 3 and per_sm(100 * 64 * 101) >= 16

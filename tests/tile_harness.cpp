@@ -13,6 +13,7 @@ extern "C" int tile_plan(int n, int most, int *fac) {
     int nf = 0;
     return tile_factors(n, most, fac, nf) ? nf : 0;
 }
+extern "C" int tile_pitch_of(int elem_bytes, int n, int lines) { return tile_pitch(elem_bytes, n, lines); }
 extern "C" void tile_frequencies(int n, int most, int *out) {
     int fac[kMaxTileFactors], nf;
     if (!tile_factors(n, most, fac, nf)) return;
