@@ -73,23 +73,27 @@ inline std::vector<WCplx> fixed_twiddles(int n) {
         return (a < 0) != (b < 0) ? -(i128)p : (i128)p;
     };
     const i128 one = (i128)1 << 96, twopi = ((i128)0x6487ED511ull << 64) | 0x0B4611A62633145Cull;
+    const i128 h = ((i128)0xB504F333ull << 64) | 0xF9DE6484597D89B3ull;  // sqrt(1/2)
+    constexpr int kTerms = 22;                                     // (pi / 8)^22 / 22! < 2^-99
+    i128 inv[kTerms + 1] = {one};                                  // 1 / j!
+    for (int j = 1; j <= kTerms; ++j) inv[j] = inv[j - 1] / j;
     std::vector<WCplx> tw(n);
-    for (int k = 0; k < n; ++k) {
+    for (int k = 0; 2 * k <= n; ++k) {
         const int o = (8 * k + n / 2) / n;                         // nearest multiple of pi / 4
-        const i128 t = twopi * (8 * k - o * n) / (8 * n);
-        i128 c = 0, s = 0, term = one;
-        for (int j = 1; term != 0; j += 2) {                       // cos, sin of t, |t| <= pi / 8
-            c += term;
-            term = mul(term, t) / j;
-            s += term;
-            term = -mul(term, t) / (j + 1);
+        const i128 t = twopi * (8 * k - o * n) / (8 * n), t2 = mul(t, t);
+        i128 c = inv[kTerms], s = inv[kTerms - 1];                 // cos, sin of t, |t| <= pi / 8
+        for (int j = kTerms - 2; j >= 0; j -= 2) {
+            c = inv[j] - mul(c, t2);
+            if (j > 0) s = inv[j - 1] - mul(s, t2);
         }
-        const i128 h = ((i128)0xB504F333ull << 64) | 0xF9DE6484597D89B3ull;  // sqrt(1/2)
+        s = mul(s, t);
         const i128 d = mul(h, c - s), e = mul(h, c + s);
         // angle o pi / 4 + t
         const i128 x[8] = {c, d, -s, -e, -c, -d, s, e}, y[8] = {s, e, c, d, -s, -e, -c, -d};
         auto round = [](i128 v) { return (long long)((v + ((i128)1 << 33)) >> 34); };
-        tw[k] = WCplx{wsplit(round(x[o & 7])), wsplit(round(-y[o & 7]))};
+        const long long wx = round(x[o & 7]), wy = round(y[o & 7]);
+        tw[k] = WCplx{wsplit(wx), wsplit(-wy)};
+        tw[(n - k) % n] = WCplx{wsplit(wx), wsplit(k ? wy : 0)};
     }
     return tw;
 }
