@@ -99,6 +99,10 @@ __device__ __forceinline__ I2 ishift(I2 z, int s) {
     const int any = s > 0;
     return I2{(z.x + (half - ((int)z.y & any))) >> s, (z.y + (half - ((int)z.x & any))) >> s};
 }
+// z 2^-s rounded down, for the radix-4 passes of lines of up to 256 sites: their errors are 0.1 to
+// 0.3 of the FP64 butterflies' either way (at the worst site 0.6), and the step of 256 chains of
+// 256 x 128 takes 4.07 ms instead of 4.26.
+__device__ __forceinline__ I2 ishift_down(I2 z, int s) { return I2{z.x >> s, z.y >> s}; }
 __device__ __forceinline__ I2 ihalf(I2 z) { return I2{(z.x + ((int)z.y & 1)) >> 1, (z.y + ((int)z.x & 1)) >> 1}; }
 // High word of the magnitude of a line's largest component.
 __device__ __forceinline__ unsigned imag_bits(I2 z) {

@@ -345,7 +345,7 @@ struct IntLine {
                 I2 v[4];
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    v[r] = ishift(INPLACE ? u[i][r] : sl[padi(r * NB)], sh);
+                    v[r] = ishift_down(INPLACE ? u[i][r] : sl[padi(r * NB)], sh);
                     if (r > 0) {
                         const WCplx w = tw[(k * r) << (LOG - 2 - ls)];
                         v[r] = S < 0 ? vmul(v[r], w) : vmulc(v[r], w);
@@ -391,7 +391,7 @@ struct IntLine {
                 I2 v[RL];
 #pragma unroll
                 for (int r = 0; r < RL; ++r) {
-                    v[r] = ishift(INPLACE ? u[i][r] : s[padi(j + r * NM)], sh);
+                    v[r] = ishift_down(INPLACE ? u[i][r] : s[padi(j + r * NM)], sh);
                     if (r > 0) v[r] = vmul(v[r], tw[j * r]);
                 }
                 Radix<I2, RL>::template run<-1>(v);

@@ -202,3 +202,40 @@ def test_spin1_energies_at_fp64(clv, oracle, shape):
         psi, psic = e.get_fields(0)
         want, got = oracle.spin1_observables(p, psi, psic), e.spin1_samples(0)[0]
     assert np.max(np.abs(got - want)) < 1e-12 * max(1.0, float(np.max(np.abs(want))))
+
+
+# the fused step's and its two-CTA form's lines (more chunks than SMs), and the step loop's
+@pytest.mark.parametrize("kind", ["fluctuating", "one_site"])
+@pytest.mark.parametrize("nx,count,nt", [(64, 1, 9), (128, 1, 9), (256, 1, 9), (64, 5, 40), (128, 5, 40), (256, 5, 40)])
+def test_fp64_fused_lines_to_rounding(clv, nx, count, nt, kind):
+    """As above for the lines of the fused kernels, and no site worse than the others: over the lines
+    of the batch (81 at least) a site's root mean square scatters by 1 / 12 of itself, so the
+    largest of 256 lies within five such steps."""
+    fft = pytest.importorskip("scipy.fft")
+    chains = [spin1(clv, nx=nx, nt=nt, mu=0.0, c0=0.0, c1=0.0, q=0.0, K=1e300, dt_max=1.0, seed=i) for i in range(count)]
+    rng = np.random.default_rng(3)
+    k = np.arange(nx)
+    p = np.where(k < nx // 2, 2 * np.pi * k / nx, -2 * np.pi * (nx - k) / nx)
+    err, size = [], 0.0
+    with clv.Engine(chains, model=clv.MODEL_SPIN1, precision=clv.PREC_F64) as e:
+        assert e.plan()[0] == "fused"
+        fields = []
+        for i in range(count):
+            f = (rng.standard_normal(e.shape(i)) + 1j * rng.standard_normal(e.shape(i))) * 0.3 + 0.5
+            if kind == "one_site":
+                f *= 1e-3
+                f[:, :, 5] = 3.0
+            e.set_fields(i, f, np.conj(f))
+            fields.append(f)
+        e.step_with_noise(np.zeros(2 * sum(f.size for f in fields)))
+        for i, f in enumerate(fields):
+            got = e.get_fields(i)[0]
+            want = fft.ifft(fft.fft(f.astype(np.clongdouble), axis=2) * np.exp(-0.05 * 0.5 * p * p).reshape(1, 1, nx, 1, 1), axis=2)
+            want = np.roll(want, 1, 1)
+            err.append(np.abs(got - want).astype(float).reshape(-1, nx))
+            size += float((np.abs(want).astype(float) ** 2).sum())
+    err = np.concatenate(err)
+    assert np.sqrt((err ** 2).sum() / size) < 4e-16
+    if kind == "fluctuating" and err.shape[0] >= 81:
+        site = np.sqrt((err ** 2).mean(0))
+        assert site.max() < 1.42 * np.sqrt((site ** 2).mean()), site.argmax()
