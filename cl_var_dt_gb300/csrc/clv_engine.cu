@@ -1308,7 +1308,7 @@ int plan_tiled(clv_engine *e) {
         e->store_drift = e->dt_rule == CLV_DT_REF_MEANMAX && sd[0] == '1';
     // Where that pass fills the GPU for a while it is bound by the FP64 pipe, so it also draws
     // the normals (integer pipes) into the buffer that the update overwrites: 128 x 128 x 128,
-    // reduce 672 -> 745 us and update 397 -> 190 us.  A short one is bound by latencies, and the
+    // reduce 754 -> 783 us and update 397 -> 190 us.  A short one is bound by latencies, and the
     // update draws them beside it (160 000 sites, 4 blocks an SM: 186 us a step, 200 drawn here).
     // A step kernel that draws beside its drift takes the same two CTAs an SM from 8 blocks on
     // (0.57 M sites, 14: 301 -> 229 us; 0.096 M, 2: 57 us, 70 in that form).

@@ -269,7 +269,7 @@ struct LaunchTileFilter {
     size_t smem_bytes;
 };
 // Largest radix of its passes: FP64 stops at 10, whose 10 elements of four words leave room
-// for five CTAs per SM (16: 168 registers, three CTAs; 128-site lines 568 against 530 us).
+// for five CTAs per SM (16: 168 registers, three CTAs; 128-site lines 7 % slower).
 template <class R> __host__ __device__ constexpr int tile_radix_max() { return sizeof(R) == 4 ? 16 : 10; }
 // Elements of a tile of lines, of a whole slice kept on chip (several CTAs per SM), and
 // where a CTA takes 256 threads instead of 128.

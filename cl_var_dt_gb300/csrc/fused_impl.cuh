@@ -518,7 +518,7 @@ template <> __device__ __forceinline__ const float *filt_of<float>(const AxisDev
 
 // TWO: the production variant of the FP64 spin-1 model where there is more than one CTA for an
 // SM: lines filtered in place and registers for two CTAs an SM.  One CTA's 8 warps issue on 21 %
-// of the clocks, waiting on their own arithmetic; two overlap (32 chains of 256 x 128: 771 -> 477
+// of the clocks, waiting on their own arithmetic; two overlap (32 chains of 256 x 128: 771 -> 480
 // us a step).  With an SM to itself a CTA is 3 % faster with all the registers.
 template <class R, int MODEL, int LN, bool FAST = false, bool TWO = false>
 // FP64 1D lines off the production variant (the reference's step rule on few CTAs):

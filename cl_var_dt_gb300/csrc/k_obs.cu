@@ -10,9 +10,9 @@
 //   imaginary times (29 FP64 operations each; the products of two times are summed among
 //   themselves and added to the running sum once: added one by one, each would be rounded at
 //   that sum's size, 2 to 3 times the error), a second kernel adds the chunks in order.
-//   Bound by the FP64 pipe on large lattices (4 components, 128^2 x 128: 405 -> 144 us), by
+//   Bound by the FP64 pipe on large lattices (4 components, 128^2 x 128: 405 -> 171 us), by
 //   latency on small ones, where a thread per site left one CTA to walk through imaginary
-//   time (256 x 32: 105 -> 33 us).
+//   time (256 x 32: 105 -> 17 us).
 // Spin-1 observables: density, F_z, F^2 = Fz^2 + F+F- and energy
 //   psibar (k^2/2 - q m^2) psi + c0/2 n^2 + c1/2 F^2, all with the point split
 //   (psibar(tau+1), psi(tau)); one FP64 sample per evaluate call and chain,

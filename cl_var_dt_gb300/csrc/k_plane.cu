@@ -117,7 +117,7 @@ __device__ __forceinline__ void plane_lines_in_registers(const LaunchAxis &A) {
 //   C  columns inverse, radix 8 and rows forward, radix RA: rows k + CB m, columns l + RB n  tile
 //   D  rows middle, radix RB:     columns RB q + i of row r                  tile
 //   E  rows inverse, radix RA:    columns l + RB n of 8 rows                 -> global
-// 768 planes of 128 (one chain, 3 components x 128 slices x 2 fields): 96.5 us in place -> 76
+// 768 planes of 128 (one chain, 3 components x 128 slices x 2 fields): 97 us in place -> 79
 // us (floor 30); 3840 planes of 96: 463 -> 422 us (floor 250).  Blocks of 128 (512 threads, one
 // CTA) prefetch the plane that follows on the SM into L2 (940 -> 902 us for 3840 planes); of 96
 // (192 threads, two CTAs that overlap) do not (422 -> 447 us).

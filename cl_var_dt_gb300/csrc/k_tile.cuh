@@ -22,9 +22,9 @@
 // writes.  A filter that vanishes at zero frequency (k^2: the reference's kinetic term and all
 // kinetic energies) does not see a constant, so its lines are taken relative to their first
 // site: a condensate would fill the top bits at a frequency that is then thrown away (lines of 1250
-// sites: 1.6 times the FP64 butterflies' error, now 0.5).  128-site lines, 4 components x 128 x 128 x 128 imaginary times, both fields: 1.37
-// (butterflies on the FP64 pipe, at its rate) -> 0.53 ms; 48-site lines of 48 x 40 x 36 x 24:
-// 0.93 -> 0.37 ms.  Bound by integer issue (46 % of the ALU) and instruction fetch.
+// sites: 2.2 times the FP64 butterflies' error, now 0.4 to 0.8; kBasedSites).  128-site lines, 4 components x 128 x 128 x 128 imaginary times, both fields: 1.37
+// (butterflies on the FP64 pipe, at its rate) -> 0.58 ms; 48-site lines of 48 x 40 x 36 x 24:
+// 0.93 -> 0.39 ms.  Bound by integer issue (48 % of the ALU) and instruction fetch.
 //
 // FP32 is bound by instruction issue (61 %, 170 instructions an element, a third of them
 // addresses) and the latency between its barriers.  64 ragged chains, 1.6 M sites: 78 us.

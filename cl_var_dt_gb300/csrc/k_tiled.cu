@@ -1,5 +1,5 @@
-// k_tiled.cu -- the Langevin step of chains whose slices are too large for the
-// fused kernel, after the kinetic terms have been filtered along every axis
+// k_tiled.cu -- the Langevin step of every lattice that the fused kernel does not
+// take, after the kinetic terms have been filtered along every axis
 // (k_axis.cu writes kin = e^{-eps H_kin} psi and kinbar for all imaginary times).
 //
 // A thread owns one spatial site of one chain over a chunk of imaginary times
@@ -243,7 +243,8 @@ __global__ void __launch_bounds__(256, LEAN || sizeof(R) == 4 ? 2 : 1) tiled_ste
 
 // The reference rule's reduce pass at FP64 that also draws the step's unit normals: the drift
 // keeps the FP64 pipe busy and the normals the integer pipes
-// (128 x 128 x 128: 672 us for the drift alone, 745 with the normals; the FP64 operations 510).
+// (128 x 128 x 128: 754 us for the drift alone, at one CTA an SM, 783 with the normals; the FP64
+// operations 560).
 template <int MODEL>
 __global__ void __launch_bounds__(256, 2) tiled_reduce_kernel(const LaunchTiled A) {
     tiled_task<double, MODEL, true, true>(A, A.tasks[blockIdx.x]);

@@ -111,7 +111,7 @@ inline int tile_pitch(int elem_bytes, int n, int lines) {
 // Lines (slices of a sum) of more sites than this are taken relative to their first site under a
 // filter that vanishes at zero frequency, the reference's k^2 and kinetic energies, where a
 // condensate costs precision: up to 256 sites at most 0.8 of the FP64 butterflies' error is left
-// (128 sites: 0.2), from 270 to 2048 up to 2.2 times it, and 0.5 relative to the first site.
+// (128 sites: 0.2), from 270 to 2048 up to 2.2 times it, and relative to the first site 0.8.
 constexpr int kBasedSites = 256;
 
 // A batch of 1D lines that both the fused and the tiled path can step.
