@@ -102,11 +102,11 @@ __device__ __forceinline__ I2 ishift(I2 z, int s) {
     const int any = s > 0;
     return I2{(z.x + (half - ((int)z.y & any))) >> s, (z.y + (half - ((int)z.x & any))) >> s};
 }
+__device__ __forceinline__ I2 ihalf(I2 z) { return I2{(z.x + ((int)z.y & 1)) >> 1, (z.y + ((int)z.x & 1)) >> 1}; }
 // z 2^-s rounded down, for the radix-4 passes of lines of up to 256 sites: their errors are 0.1 to
 // 0.3 of the FP64 butterflies' either way (at the worst site 0.6), and the step of 256 chains of
 // 256 x 128 takes 4.07 ms instead of 4.26.
 __device__ __forceinline__ I2 ishift_down(I2 z, int s) { return I2{z.x >> s, z.y >> s}; }
-__device__ __forceinline__ I2 ihalf(I2 z) { return I2{(z.x + ((int)z.y & 1)) >> 1, (z.y + ((int)z.x & 1)) >> 1}; }
 // High word of the magnitude of a line's largest component.
 __device__ __forceinline__ unsigned imag_bits(I2 z) {
     const int a = (int)(z.x >> 32), b = (int)(z.y >> 32);
@@ -116,9 +116,9 @@ __device__ __forceinline__ unsigned imag_bits(I2 z) {
 // Shifts before a butterfly of R inputs: the least that keeps R times a component below
 // 2^62.25, so that the outputs, of up to sqrt(2) times that, keep within 63 bits and their
 // products with twiddles too (imul's cross products: 2^30.75 2^31.5 + 2^31.5 2^30 < 2^63).
-// Counting R as the next power of two, and the component too, would leave up to two bits of the 62 unused
-// in every pass: a condensate fills them all at one frequency, and what it leaves to the others
-// is their precision (lines of 729 and 900 sites: 1.3 times the FP64 butterflies' error, now 0.7).
+// Counting R as the next power of two, and the component too, would leave up to two bits of the
+// 62 unused in every pass: a condensate fills them all at one frequency, and what it leaves to the
+// others is their precision (lines of 729 and 900 sites: 1.3 times the FP64 butterflies' error, now 0.7).
 // ishift_for: of a component with the high word mag; ifirst_for: of a double with the high
 // word raw, which to_fixed puts in [2^61, 2^62).
 __device__ __forceinline__ int ishift_for(unsigned mag, int r) {
